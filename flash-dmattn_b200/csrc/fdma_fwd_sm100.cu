@@ -92,7 +92,7 @@ struct Smem {
   static constexpr int kPosOff = kBmOff + kBmSlots * kBN * 4;
   static constexpr int kFlagsOff = kPosOff + kBmSlots * kBN * 4;   // two tables: this work item's and the next one's
   static constexpr int kBarOff = kFlagsOff + 2 * kMaxTiles;
-  static constexpr int kNumBars = 2 + 2 * kStages + 2 + 2 + 1 + 2 + 2 * kBmSlots + 1 + 4;
+  static constexpr int kNumBars = 2 + 2 * kStages + 2 + 2 + 2 + 2 + 2 * kBmSlots + 1 + 4;
   static constexpr int kMiscOff = kBarOff + kNumBars * 8;
   static constexpr int kTotal = kMiscOff + 16;
   static constexpr int kAlloc = kTotal + 1024;  // slack to align the base to 1024 B
@@ -180,8 +180,11 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
   uint64_t* bar_kv_empty = bar_kv_full + kStages;
   uint64_t* bar_s_full = bar_kv_empty + kStages;    // [2]
   uint64_t* bar_p_full = bar_s_full + 2;            // [2]
-  uint64_t* bar_o_done = bar_p_full + 2;            // every product of the item has completed
-  uint64_t* bar_o_free = bar_o_done + 1;            // [2] the softmax warps have read O_t out of tensor memory
+  // o_done / o_free only advance on items with at least one tile for query tile t, counted on both sides. A phase per
+  // item would let the MMA warp pass two phases of an item list with empty items (rows before the first kept key)
+  // while the softmax warps still look for the first of them; with the tile's own P hand-over in between it cannot.
+  uint64_t* bar_o_done = bar_p_full + 2;            // [2] every product of O_t of the item has completed
+  uint64_t* bar_o_free = bar_o_done + 2;            // [2] the softmax warps have read O_t out of tensor memory
   uint64_t* bar_bm_full = bar_o_free + 2;
   uint64_t* bar_bm_empty = bar_bm_full + kBmSlots;
   uint64_t* bar_stagger = bar_bm_empty + kBmSlots;  // warpgroup 0 -> warpgroup 1, once
@@ -229,11 +232,11 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
     for (int t = 0; t < 2; ++t) {
       mbar_init(bar_s_full + t, 1);
       mbar_init(bar_p_full + t, kBM);
+      mbar_init(bar_o_done + t, 1);
       mbar_init(bar_o_free + t, 4);  // one arrival per softmax warp of the query tile
       mbar_init(bar_flags_full + t, 1);
       mbar_init(bar_flags_empty + t, kFlagReaders);
     }
-    mbar_init(bar_o_done, 1);
     mbar_init(bar_stagger, kBM);
     for (int i = 0; i < kBmSlots; ++i) {
       mbar_init(bar_bm_full + i, 1);
@@ -311,6 +314,7 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
     const uint32_t q_addr = smem_u32(s_q), kv_addr = smem_u32(s_kv);
     FDMA_PROF_BEGIN();
     int a = 0;                    // ring position: K of the a-th kept tile (over all items) is ring item 2a, V 2a+1
+    uint32_t ocnt[2] = {0, 0};    // finished items with at least one tile, per query tile (barrier parity)
     uint32_t pcnt[2] = {0, 0};    // P hand-overs received per query tile, over all items (barrier parity)
     bool ok = true;
     for (int ic = 0; ok; ++ic) {
@@ -354,8 +358,8 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
           if (pfl & (1 << t)) {
             ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(3 + t, mbar_wait(bar_p_full + t, pcnt[t] & 1, ctl, kWaitP)));
             if (!ok) break;
-            if (pv_done[t] == 0 && ic > 0) {  // the previous item's O_t must have left tensor memory
-              ok = __all_sync(0xffffffffu, mbar_wait(bar_o_free + t, (ic - 1) & 1, ctl, kWaitOFree));
+            if (pv_done[t] == 0 && ocnt[t] > 0) {  // the previous item's O_t must have left tensor memory
+              ok = __all_sync(0xffffffffu, mbar_wait(bar_o_free + t, (ocnt[t] - 1) & 1, ctl, kWaitOFree));
               if (!ok) break;
             }
             tc_fence_after_sync();
@@ -391,7 +395,12 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
       }
       if (!ok) break;
       if (prev_j < 0) umma_commit(bar_q_empty);  // (an item without kept tiles never read its Q)
-      umma_commit(bar_o_done);
+#pragma unroll
+      for (int t = 0; t < kNQ; ++t)
+        if (pv_done[t] > 0) {
+          umma_commit(bar_o_done + t);
+          ++ocnt[t];
+        }
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_flags_empty + (ic & 1));
     }
@@ -539,6 +548,7 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
     const uint32_t o_taddr = tmem_base + lane_addr + kNQ * kBN + t * 128;
     FDMA_PROF_BEGIN();
     uint32_t scnt = 0;   // S tiles received over all items (barrier parity)
+    uint32_t ocnt = 0;   // items with at least one tile (barrier parity)
     int bi = 0;          // addend-ring position over all items
     bool ok = true;
     bool stagger_sent = false;
@@ -800,9 +810,12 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
     __syncwarp();
     if (lane == 0) mbar_arrive(bar_flags_empty + (ic & 1));
     // ---------------- epilogue of the item ----------------
-    ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(2, mbar_wait(bar_o_done, ic & 1, ctl, kWaitO)));
-    if (!ok) break;
-    tc_fence_after_sync();
+    if (sitem > 0) {
+      ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(2, mbar_wait(bar_o_done + t, ocnt & 1, ctl, kWaitO)));
+      if (!ok) break;
+      ++ocnt;
+      tc_fence_after_sync();
+    }
     {
       const bool in_range = qrow < Sq;  // TMEM loads below are warp-collective: every lane runs them
       const bool wide_o = (reinterpret_cast<uintptr_t>(p.out) & 31) == 0 &&
@@ -844,8 +857,6 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
           }
         }
       } else {
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar_o_free + t);
         if (in_range) {
 #pragma unroll
           for (int c = 0; c < D / 8; ++c) *reinterpret_cast<uint4*>(orow + c * 16) = make_uint4(0, 0, 0, 0);

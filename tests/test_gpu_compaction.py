@@ -197,3 +197,23 @@ def test_default_route_selection(dev):
         iface.set_compaction("auto")
     torch.cuda.synchronize()
     _kernel_status_ok()
+
+
+def test_left_padded_batch_with_empty_query_blocks(dev):
+    """Left-padded prompts: the leading query blocks of the shorter ones see no kept key at all, and there are more
+    work items than SMs, so a persistent CTA meets several empty items in a row between others."""
+    from flash_sparse_attn import flash_sparse_attn_func
+    from flash_sparse_attn.utils.mask import create_mask
+
+    B, S, H, Hk, d, W = 3, 2048, 32, 8, 128, 256
+    dtype = torch.bfloat16
+    q, k, v, bias, _ = (None if t is None else t.to(dev)
+                        for t in oracle.make_inputs(B, S, S, H, Hk, d, (B, Hk, 1, S), seed=6, dtype=dtype))
+    padding = torch.arange(S, device=dev)[None] >= torch.tensor([0, 700, 1500], device=dev)[:, None]
+    mask = create_mask(bias, padding, B, S, S, W, torch.finfo(dtype).min)
+    out = flash_sparse_attn_func(q, k, v, mask, bias, is_causal=True)
+    torch.cuda.synchronize()
+    _kernel_status_ok()
+    for b in range(B):
+        ref = oracle.attention_forward(q[b:b + 1], k[b:b + 1], v[b:b + 1], mask[b:b + 1], bias[b:b + 1], None, True)[0]
+        check(f"out[{b}]", out[b:b + 1], ref, dtype)
