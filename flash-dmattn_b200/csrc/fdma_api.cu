@@ -69,6 +69,13 @@ int validate_bwd(const fdma_bwd_params& p) {
     if (!(p.dbias_h == 1 || p.dbias_h == p.f.h_k || p.dbias_h == p.f.h)) return FDMA_ERR_BAD_ARG;
     if (!(p.dbias_rows == 1 || p.dbias_rows == p.f.seqlen_q)) return FDMA_ERR_BAD_ARG;
   }
+  if (p.scatter_pos) {
+    if (!(p.scatter_h == 1 || p.scatter_h == p.f.h_k) || p.scatter_rows <= 0) return FDMA_ERR_BAD_ARG;
+    if (p.dbias) {
+      if (p.dbias_rows != 1 || p.dbias_keys < p.scatter_rows || p.dbias_h % p.scatter_h) return FDMA_ERR_BAD_ARG;
+      if (p.scatter_batch_stride != 0 && p.dbias_b != p.f.b) return FDMA_ERR_BAD_ARG;
+    }
+  }
   return 0;
 }
 
@@ -234,7 +241,7 @@ size_t fdma_bwd_workspace_bytes(const fdma_bwd_params* pp) {
   fdma_bwd_params p = *pp;
   p.f = normalise(pp->f);
   if (p.f.path != FDMA_PATH_SIMT && tc_bwd_supported(p)) return tc_bwd_workspace_bytes(p);
-  return simt_bwd_workspace_bytes(p);
+  return simt_bwd_workspace_bytes(p);  // (with scatter_pos: refused by fdma_bwd)
 }
 
 int fdma_bwd(const fdma_bwd_params* pp, void* stream_) {
@@ -249,7 +256,8 @@ int fdma_bwd(const fdma_bwd_params* pp, void* stream_) {
   const bool tc_ok = tc_bwd_supported(p);
   if (p.f.path == FDMA_PATH_TCGEN05 && !tc_ok) return FDMA_ERR_UNSUPPORTED;
   if (p.f.path != FDMA_PATH_SIMT && tc_ok) return tc_bwd(p, stream);
-  if (p.f.mask && p.f.mask_bits) return FDMA_ERR_UNSUPPORTED;  // only the tcgen05 kernels read a bit-packed mask
+  // only the tcgen05 kernels read a bit-packed mask, and only they write gradients to the keys' positions
+  if ((p.f.mask && p.f.mask_bits) || p.scatter_pos) return FDMA_ERR_UNSUPPORTED;
   return simt_bwd(p, stream);
 }
 

@@ -1,4 +1,4 @@
-// Dynamic-mask attention backward for head dim 256 on Blackwell tensor cores (tcgen05 + TMEM + TMA), for
+// Dynamic-mask attention backward for head dims 136 to 256 on Blackwell tensor cores (tcgen05 + TMEM + TMA), for
 // row-broadcast masks and biases (the shape create_mask produces from a (B, Hk, 1, Sk) bias).
 //
 // Same mathematics and the same transposed products as the head-dim-128 kernel next door (fdma_bwd_sm100.cu; the
@@ -49,14 +49,14 @@ struct Bwd256Params {
   void* dk;
   void* dv;
   void* dbias;
-  float* dkv_part;     // nsplit > 1: fp32 partials [2: dV, dK][nsplit][B][h_k][NT*128][256]
-  float* dbias_part;   // nsplit > 1: fp32 partials [nsplit][B][h_k][NT*128]
+  float* dkv_part;     // null, or fp32 partials [2: dV, dK][nsplit][B][h_k][NT*128][256] instead of dk / dv
+  float* dbias_part;   // with dkv_part: fp32 partials [nsplit][B][h_k][NT*128]
   int* status;
   int64_t mask_batch_stride, mask_head_stride, bias_batch_stride, bias_head_stride;
   int64_t dk_batch_stride, dk_row_stride, dk_head_stride;
   int64_t dv_batch_stride, dv_row_stride, dv_head_stride;
   int64_t dbias_batch_stride, dbias_head_stride;
-  int b, seqlen_q, seqlen_k, sq_r, h, h_k, h_mask, h_bias;
+  int b, seqlen_q, seqlen_k, sq_r, h, h_k, h_mask, h_bias, d;
   int dbias_keys, want_dbias, nsplit, is_causal;
   const int32_t* key_pos;
   int64_t pos_batch_stride, pos_head_stride;
@@ -93,159 +93,6 @@ __device__ __forceinline__ float raw16_to_f(uint16_t u) {
 template <bool kBf16>
 __device__ __forceinline__ uint16_t f_to_raw16(float x) {
   return static_cast<uint16_t>(pack_16x2<kBf16>(x, 0.f) & 0xFFFFu);
-}
-
-// D = rowsum(dO o O), LSE in log2 units; rows [Sq, Sq_r) are padding (+inf / 0). One warp per (b, h, row): 32 lanes
-// x 8 elements = 256.
-template <bool kBf16>
-__global__ void __launch_bounds__(256) bwd256_prep_kernel(const void* __restrict__ out, const void* __restrict__ dout,
-                                                           const float* __restrict__ lse, float* __restrict__ lse2,
-                                                           float* __restrict__ dsum, int B, int H, int Sq, int Sq_r,
-                                                           int64_t ob, int64_t orow, int64_t oh, int64_t gb,
-                                                           int64_t grow, int64_t gh) {
-  const int lane = threadIdx.x & 31;
-  const int64_t w = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
-  const int64_t total = static_cast<int64_t>(B) * H * Sq_r;
-  if (w >= total) return;
-  const int q = static_cast<int>(w % Sq_r);
-  const int h = static_cast<int>((w / Sq_r) % H);
-  const int b = static_cast<int>(w / (static_cast<int64_t>(Sq_r) * H));
-  if (q >= Sq) {
-    if (lane == 0) {
-      lse2[w] = CUDART_INF_F;
-      dsum[w] = 0.f;
-    }
-    return;
-  }
-  const uint4 a = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(out) + b * ob +
-                                                  static_cast<int64_t>(q) * orow + h * oh + lane * 8);
-  const uint4 c = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(dout) + b * gb +
-                                                  static_cast<int64_t>(q) * grow + h * gh + lane * 8);
-  const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, cw[4] = {c.x, c.y, c.z, c.w};
-  float acc = 0.f;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    acc = fmaf(raw16_to_f<kBf16>(static_cast<uint16_t>(aw[j] & 0xFFFFu)),
-               raw16_to_f<kBf16>(static_cast<uint16_t>(cw[j] & 0xFFFFu)), acc);
-    acc = fmaf(raw16_to_f<kBf16>(static_cast<uint16_t>(aw[j] >> 16)), raw16_to_f<kBf16>(static_cast<uint16_t>(cw[j] >> 16)),
-               acc);
-  }
-#pragma unroll
-  for (int s = 16; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-  if (lane == 0) {
-    lse2[w] = lse[(static_cast<int64_t>(b) * H + h) * Sq + q] * kLog2e;
-    dsum[w] = acc;
-  }
-}
-
-// fp32 dQ accumulator (B,H,2,Sq,128) * scale -> dq (B,Sq,H,256 strided, 16-bit)
-template <bool kBf16>
-__global__ void bwd256_convert_dq_kernel(const float* __restrict__ acc, void* __restrict__ dq, int64_t n_vec, int Sq,
-                                         int H, int64_t sb, int64_t sr, int64_t sh, float scale) {
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n_vec;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t e = i * 8;
-    const int dd = static_cast<int>(e % 128);
-    const int q = static_cast<int>((e / 128) % Sq);
-    const int dh = static_cast<int>((e / (static_cast<int64_t>(128) * Sq)) % 2);
-    const int h = static_cast<int>((e / (static_cast<int64_t>(256) * Sq)) % H);
-    const int b = static_cast<int>(e / (static_cast<int64_t>(256) * Sq * H));
-    const float4 x = *reinterpret_cast<const float4*>(acc + e);
-    const float4 y = *reinterpret_cast<const float4*>(acc + e + 4);
-    uint4 o;
-    o.x = pack_16x2<kBf16>(x.x * scale, x.y * scale);
-    o.y = pack_16x2<kBf16>(x.z * scale, x.w * scale);
-    o.z = pack_16x2<kBf16>(y.x * scale, y.y * scale);
-    o.w = pack_16x2<kBf16>(y.z * scale, y.w * scale);
-    *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(dq) + b * sb + static_cast<int64_t>(q) * sr + h * sh +
-                              dh * 128 + dd) = o;
-  }
-}
-
-// Deterministic mode: the accumulator holds 64-bit fixed point (kDetFracBits256 fractional bits) instead of fp32.
-constexpr int kDetFracBits256 = 40;
-template <bool kBf16>
-__global__ void bwd256_convert_dq_fixed_kernel(const long long* __restrict__ acc, void* __restrict__ dq, int64_t n_vec,
-                                               int Sq, int H, int64_t sb, int64_t sr, int64_t sh, float scale,
-                                               const float* __restrict__ dsum, int sq_r) {
-  const float unit = scale * (1.0f / static_cast<float>(1ll << kDetFracBits256));
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n_vec;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t e = i * 8;
-    const int dd = static_cast<int>(e % 128);
-    const int q = static_cast<int>((e / 128) % Sq);
-    const int dh = static_cast<int>((e / (static_cast<int64_t>(128) * Sq)) % 2);
-    const int h = static_cast<int>((e / (static_cast<int64_t>(256) * Sq)) % H);
-    const int b = static_cast<int>(e / (static_cast<int64_t>(256) * Sq * H));
-    float x[8];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const longlong2 v = *reinterpret_cast<const longlong2*>(acc + e + 2 * j);
-      x[2 * j] = __ll2float_rn(v.x) * unit;
-      x[2 * j + 1] = __ll2float_rn(v.y) * unit;
-    }
-    // Fixed point cannot carry NaN / Inf. A non-finite dO or O element makes D = rowsum(dO o O) of its row
-    // non-finite, and with it every dS of the row: such rows come out as NaN, as the fp32 path would give.
-    if (!isfinite(dsum[(static_cast<int64_t>(b) * H + h) * sq_r + q])) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) x[j] = __int_as_float(0x7FC00000);
-    }
-    uint4 o;
-    o.x = pack_16x2<kBf16>(x[0], x[1]);
-    o.y = pack_16x2<kBf16>(x[2], x[3]);
-    o.z = pack_16x2<kBf16>(x[4], x[5]);
-    o.w = pack_16x2<kBf16>(x[6], x[7]);
-    *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(dq) + b * sb + static_cast<int64_t>(q) * sr + h * sh +
-                              dh * 128 + dd) = o;
-  }
-}
-
-// Sum of the query-range partials of dK or dV: part [nsplit][B][h_k][keys_r][256] fp32 -> 16-bit (B, Sk, h_k, 256).
-template <bool kBf16>
-__global__ void __launch_bounds__(256) bwd256_reduce_dkv_kernel(const float* __restrict__ part, void* __restrict__ dst,
-                                                                 int nsplit, int B, int Hk, int Sk, int keys_r,
-                                                                 int64_t sb, int64_t sr, int64_t sh) {
-  const int64_t n_vec = static_cast<int64_t>(B) * Hk * Sk * (kD / 8);
-  const int64_t split_stride = static_cast<int64_t>(B) * Hk * keys_r * kD;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n_vec;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int c = static_cast<int>(i % (kD / 8));
-    const int key = static_cast<int>((i / (kD / 8)) % Sk);
-    const int hk = static_cast<int>((i / (static_cast<int64_t>(kD / 8) * Sk)) % Hk);
-    const int b = static_cast<int>(i / (static_cast<int64_t>(kD / 8) * Sk * Hk));
-    const float* src = part + ((static_cast<int64_t>(b) * Hk + hk) * keys_r + key) * kD + c * 8;
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int s = 0; s < nsplit; ++s) {
-      const float4 a = *reinterpret_cast<const float4*>(src + s * split_stride);
-      const float4 d = *reinterpret_cast<const float4*>(src + s * split_stride + 4);
-      acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
-      acc[4] += d.x; acc[5] += d.y; acc[6] += d.z; acc[7] += d.w;
-    }
-    uint4 o;
-    o.x = pack_16x2<kBf16>(acc[0], acc[1]);
-    o.y = pack_16x2<kBf16>(acc[2], acc[3]);
-    o.z = pack_16x2<kBf16>(acc[4], acc[5]);
-    o.w = pack_16x2<kBf16>(acc[6], acc[7]);
-    *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(dst) + b * sb + static_cast<int64_t>(key) * sr + hk * sh +
-                              c * 8) = o;
-  }
-}
-
-// Sum of the query-range partials of the column-sum dBias: part [nsplit][B][h_k][keys_r] fp32 -> 16-bit
-// (B, h_k, 1, dbias_keys); keys beyond Sk are zero.
-template <bool kBf16>
-__global__ void __launch_bounds__(256) bwd256_reduce_dbias_kernel(const float* __restrict__ part, void* __restrict__ dst,
-                                                                   int nsplit, int B, int Hk, int dbias_keys, int Sk,
-                                                                   int keys_r, int64_t sb, int64_t sh) {
-  const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (i >= static_cast<int64_t>(B) * Hk * dbias_keys) return;
-  const int key = static_cast<int>(i % dbias_keys);
-  const int hk = static_cast<int>((i / dbias_keys) % Hk);
-  const int b = static_cast<int>(i / (static_cast<int64_t>(dbias_keys) * Hk));
-  float acc = 0.f;
-  if (key < Sk)
-    for (int s = 0; s < nsplit; ++s) acc += part[((static_cast<int64_t>(s) * B + b) * Hk + hk) * keys_r + key];
-  reinterpret_cast<uint16_t*>(dst)[b * sb + hk * sh + key] = f_to_raw16<kBf16>(acc);
 }
 
 template <bool kBf16, bool kDet>
@@ -568,7 +415,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd256_kernel(const __grid_consta
         named_bar_sync(1, 256);
         if (half == 0 && key < p.dbias_keys) {
           const float tot = key_ok ? colsum + s_red[krow] : 0.f;
-          if (p.nsplit > 1)
+          if (p.dkv_part)
             p.dbias_part[((static_cast<int64_t>(split) * p.b + b) * p.h_k + hk) * (NT * kBN) + key] = tot;
           else
             reinterpret_cast<uint16_t*>(p.dbias)[b * p.dbias_batch_stride + hk * p.dbias_head_stride + key] =
@@ -598,7 +445,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd256_kernel(const __grid_consta
 #pragma unroll
             for (int j = 0; j < 32; ++j) r[j] = 0u;
           }
-          if (p.nsplit > 1) {
+          if (p.dkv_part) {
 #pragma unroll
             for (int v4 = 0; v4 < 8; ++v4)
               *reinterpret_cast<float4*>(part + col + v4 * 4) =
@@ -607,6 +454,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd256_kernel(const __grid_consta
           } else if (key_ok) {
 #pragma unroll
             for (int v4 = 0; v4 < 4; ++v4) {
+              if (col + v4 * 8 >= p.d) break;
               uint4 o;
               o.x = pack_16x2<kBf16>(__uint_as_float(r[v4 * 8 + 0]) * mul, __uint_as_float(r[v4 * 8 + 1]) * mul);
               o.y = pack_16x2<kBf16>(__uint_as_float(r[v4 * 8 + 2]) * mul, __uint_as_float(r[v4 * 8 + 3]) * mul);
@@ -655,7 +503,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd256_kernel(const __grid_consta
             long long* s_dq64 = reinterpret_cast<long long*>(s_dq);
             long long* gdst64 = reinterpret_cast<long long*>(p.dq_acc) +
                                 (((static_cast<int64_t>(b) * p.h + h) * 2 + dh) * Sq + m * kBM) * 128;
-            constexpr float kFix = static_cast<float>(1ll << kDetFracBits256);
+            constexpr float kFix = static_cast<float>(1ll << kDetFracBits);
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
               if (tid == 384) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -669,13 +517,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd256_kernel(const __grid_consta
               named_bar_sync(3, 128);
               if (tid == 384) {
                 const int rows = min(8, Sq - (m * kBM + c * 8));
-                if (rows > 0) {
-                  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.u64 [%0], [%1], %2;"
-                               :
-                               : "l"(reinterpret_cast<uint64_t>(gdst64 + c * 8 * 128)), "r"(smem_u32(s_dq)),
-                                 "r"(static_cast<uint32_t>(rows * 128 * 8))
-                               : "memory");
-                }
+                if (rows > 0) bulk_reduce_add_u64(gdst64 + c * 8 * 128, s_dq, rows * 128 * 8);
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
               }
             }
@@ -692,13 +534,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd256_kernel(const __grid_consta
             named_bar_sync(3, 128);
             if (tid == 384) {
               const int rows = min(16, Sq - (m * kBM + c * 16));
-              if (rows > 0) {
-                asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;"
-                             :
-                             : "l"(reinterpret_cast<uint64_t>(gdst + c * 16 * 128)), "r"(smem_u32(s_dq)),
-                               "r"(static_cast<uint32_t>(rows * 128 * 4))
-                             : "memory");
-              }
+              if (rows > 0) bulk_reduce_add_f32(gdst + c * 16 * 128, s_dq, rows * 128 * 4);
               asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             }
           }
@@ -720,6 +556,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd256_kernel(const __grid_consta
 struct Plan256 {
   int sq_r, nsplit;
   bool want_dbias;
+  bool part;  // dK, dV and column sums leave the main kernel as fp32 partials
   size_t lse2_off, dsum_off, dq_off, part_off, dbpart_off, total;
 };
 
@@ -746,7 +583,8 @@ Plan256 plan256(const fdma_bwd_params& bp) {
   pl.dsum_off = o; o += align256(rows * 4);
   pl.dq_off = o;   o += align256(static_cast<size_t>(p.b) * p.seqlen_q * p.h * kD * (bp.deterministic ? 8 : 4));
   pl.part_off = pl.dbpart_off = o;
-  if (pl.nsplit > 1) {
+  pl.part = pl.nsplit > 1 || bp.scatter_pos != nullptr;
+  if (pl.part) {
     const size_t keys_r = round_up(p.seqlen_k, kBN);
     o += align256(static_cast<size_t>(2) * pl.nsplit * p.b * p.h_k * keys_r * kD * 4);
     pl.dbpart_off = o;
@@ -788,17 +626,14 @@ int launch256(const fdma_bwd_params& bp, const Plan256& pl, cudaStream_t stream)
   float* lse2 = reinterpret_cast<float*>(ws + pl.lse2_off);
   float* dsum = reinterpret_cast<float*>(ws + pl.dsum_off);
   float* dq_acc = reinterpret_cast<float*>(ws + pl.dq_off);
-  cudaError_t e = cudaMemsetAsync(dq_acc, 0, static_cast<size_t>(p.b) * p.seqlen_q * p.h * kD * (bp.deterministic ? 8 : 4),
-                                  stream);
-  if (e != cudaSuccess) return static_cast<int>(e);
   {
-    const int64_t warps = static_cast<int64_t>(p.b) * p.h * pl.sq_r;
-    const int64_t blocks = (warps * 32 + 255) / 256;
-    bwd256_prep_kernel<kBf16><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
-        p.out, bp.dout, p.lse, lse2, dsum, p.b, p.h, p.seqlen_q, pl.sq_r, p.o_batch_stride, p.o_row_stride,
-        p.o_head_stride, bp.do_batch_stride, bp.do_row_stride, bp.do_head_stride);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return static_cast<int>(e);
+    BwdPrepArgs a;
+    a.out = p.out; a.dout = bp.dout; a.lse = p.lse; a.lse2 = lse2; a.dsum = dsum; a.dq_acc = dq_acc;
+    a.b = p.b; a.h = p.h; a.sq = p.seqlen_q; a.sq_r = pl.sq_r; a.d = p.d; a.acc_bytes = bp.deterministic ? 8 : 4;
+    a.o_sb = p.o_batch_stride; a.o_sr = p.o_row_stride; a.o_sh = p.o_head_stride;
+    a.do_sb = bp.do_batch_stride; a.do_sr = bp.do_row_stride; a.do_sh = bp.do_head_stride;
+    st = launch_bwd_prep(a, kD, kBf16, stream);
+    if (st) return st;
     st = export_softmax_d(bp, dsum, pl.sq_r, stream);
     if (st) return st;
   }
@@ -810,7 +645,7 @@ int launch256(const fdma_bwd_params& bp, const Plan256& pl, cudaStream_t stream)
   kp.dk = bp.dk;
   kp.dv = bp.dv;
   kp.dbias = bp.dbias;
-  kp.dkv_part = reinterpret_cast<float*>(ws + pl.part_off);
+  kp.dkv_part = pl.part ? reinterpret_cast<float*>(ws + pl.part_off) : nullptr;
   kp.dbias_part = reinterpret_cast<float*>(ws + pl.dbpart_off);
   kp.status = kernel_status_ptr();
   if (!kp.status) return FDMA_ERR_DRIVER;
@@ -819,11 +654,11 @@ int launch256(const fdma_bwd_params& bp, const Plan256& pl, cudaStream_t stream)
   kp.dk_batch_stride = bp.dk_batch_stride; kp.dk_row_stride = bp.dk_row_stride; kp.dk_head_stride = bp.dk_head_stride;
   kp.dv_batch_stride = bp.dv_batch_stride; kp.dv_row_stride = bp.dv_row_stride; kp.dv_head_stride = bp.dv_head_stride;
   kp.dbias_batch_stride = bp.dbias_batch_stride; kp.dbias_head_stride = bp.dbias_head_stride;
-  kp.b = p.b; kp.seqlen_q = p.seqlen_q; kp.seqlen_k = p.seqlen_k; kp.sq_r = pl.sq_r; kp.h = p.h; kp.h_k = p.h_k;
+  kp.b = p.b; kp.seqlen_q = p.seqlen_q; kp.seqlen_k = p.seqlen_k; kp.sq_r = pl.sq_r; kp.h = p.h; kp.h_k = p.h_k; kp.d = p.d;
   // head extents equal to h only occur here with h == h_k (see tc_bwd256_supported): fold them onto h_k
   kp.h_mask = p.h_mask == p.h ? p.h_k : p.h_mask;
   kp.h_bias = p.h_bias == p.h ? p.h_k : p.h_bias;
-  kp.dbias_keys = bp.dbias ? bp.dbias_keys : 0;
+  kp.dbias_keys = !bp.dbias ? 0 : bp.scatter_pos ? p.seqlen_k : bp.dbias_keys;
   kp.want_dbias = pl.want_dbias ? 1 : 0;
   kp.nsplit = pl.nsplit;
   kp.is_causal = p.is_causal;
@@ -835,7 +670,7 @@ int launch256(const fdma_bwd_params& bp, const Plan256& pl, cudaStream_t stream)
   kp.scale = p.softmax_scale;
 
   auto kern = bp.deterministic ? bwd256_kernel<kBf16, true> : bwd256_kernel<kBf16, false>;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem256::kAlloc);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem256::kAlloc);
   if (e != cudaSuccess) return static_cast<int>(e);
   dim3 grid(((p.seqlen_k + kBN - 1) / kBN) * pl.nsplit, p.h_k, p.b);
   cudaEvent_t ev0, ev1;
@@ -846,45 +681,37 @@ int launch256(const fdma_bwd_params& bp, const Plan256& pl, cudaStream_t stream)
   e = cudaGetLastError();
   if (e != cudaSuccess) return static_cast<int>(e);
 
-  if (pl.nsplit > 1) {
-    const int keys_r = static_cast<int>(round_up(p.seqlen_k, kBN));
-    const int64_t n_vec = static_cast<int64_t>(p.b) * p.h_k * p.seqlen_k * (kD / 8);
-    const unsigned g = static_cast<unsigned>(std::min<int64_t>((n_vec + 255) / 256, sm_count() * 32));
-    for (int which = 0; which < 2; ++which) {  // 0: dV, 1: dK
-      const float* part = kp.dkv_part + static_cast<size_t>(which) * pl.nsplit * p.b * p.h_k * keys_r * kD;
-      bwd256_reduce_dkv_kernel<kBf16><<<g, 256, 0, stream>>>(
-          part, which == 0 ? bp.dv : bp.dk, pl.nsplit, p.b, p.h_k, p.seqlen_k, keys_r,
-          which == 0 ? bp.dv_batch_stride : bp.dk_batch_stride, which == 0 ? bp.dv_row_stride : bp.dk_row_stride,
-          which == 0 ? bp.dv_head_stride : bp.dk_head_stride);
-    }
+  BwdFinishArgs f = {};
+  f.dq_acc = dq_acc; f.dq = bp.dq; f.dsum = dsum;
+  f.dq_sb = bp.dq_batch_stride; f.dq_sr = bp.dq_row_stride; f.dq_sh = bp.dq_head_stride;
+  f.scale = p.softmax_scale;
+  f.b = p.b; f.h = p.h; f.sq = p.seqlen_q; f.sq_r = pl.sq_r; f.d = p.d; f.D = kD;
+  f.h_k = p.h_k; f.keys_r = static_cast<int>(round_up(p.seqlen_k, kBN));
+  f.rows_out = bp.scatter_pos ? bp.scatter_rows : p.seqlen_k;
+  f.pos = bp.scatter_pos; f.pos_sb = bp.scatter_batch_stride; f.pos_sh = bp.scatter_head_stride;
+  f.h_pos = bp.scatter_h; f.cap = p.seqlen_k;
+  if (pl.part) {
+    f.part = kp.dkv_part; f.nsplit = pl.nsplit;
+    f.split_stride = static_cast<int64_t>(p.b) * p.h_k * f.keys_r * kD;
+    f.dk = bp.dk; f.dk_sb = bp.dk_batch_stride; f.dk_sr = bp.dk_row_stride; f.dk_sh = bp.dk_head_stride;
+    f.dv = bp.dv; f.dv_sb = bp.dv_batch_stride; f.dv_sr = bp.dv_row_stride; f.dv_sh = bp.dv_head_stride;
     if (pl.want_dbias) {
-      const int64_t nk = static_cast<int64_t>(p.b) * p.h_k * bp.dbias_keys;
-      bwd256_reduce_dbias_kernel<kBf16><<<static_cast<unsigned>((nk + 255) / 256), 256, 0, stream>>>(
-          kp.dbias_part, bp.dbias, pl.nsplit, p.b, p.h_k, bp.dbias_keys, p.seqlen_k, keys_r, bp.dbias_batch_stride,
-          bp.dbias_head_stride);
+      f.db_part = kp.dbias_part; f.db_nsplit = pl.nsplit; f.db_pitch = f.keys_r;
+      f.db_split_stride = static_cast<int64_t>(p.b) * p.h_k * f.keys_r;
+      f.db_b = bp.dbias_b; f.db_h = bp.dbias_h; f.db_keys = bp.dbias_keys;
+      f.dbias = bp.dbias; f.db_sb = bp.dbias_batch_stride; f.db_sh = bp.dbias_head_stride;
     }
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return static_cast<int>(e);
   }
-  const int64_t n_vec = static_cast<int64_t>(p.b) * p.seqlen_q * p.h * kD / 8;
-  const unsigned g = static_cast<unsigned>(std::min<int64_t>((n_vec + 255) / 256, sm_count() * 32));
-  if (bp.deterministic)
-    bwd256_convert_dq_fixed_kernel<kBf16><<<g, 256, 0, stream>>>(reinterpret_cast<const long long*>(dq_acc), bp.dq, n_vec,
-                                                               p.seqlen_q, p.h, bp.dq_batch_stride, bp.dq_row_stride,
-                                                               bp.dq_head_stride, p.softmax_scale, dsum, pl.sq_r);
-  else
-    bwd256_convert_dq_kernel<kBf16><<<g, 256, 0, stream>>>(dq_acc, bp.dq, n_vec, p.seqlen_q, p.h, bp.dq_batch_stride,
-                                                           bp.dq_row_stride, bp.dq_head_stride, p.softmax_scale);
-  return static_cast<int>(cudaGetLastError());
+  return launch_bwd_finish(f, kBf16, bp.deterministic != 0, stream);
 }
 
 }  // namespace
 
-// Head dim 256 on the tensor-core backward: row-broadcast mask and bias with one row per kv head at most, dBias (if
+// Head dims above 128 on the tensor-core backward: row-broadcast mask and bias with one row per kv head at most, dBias (if
 // asked for) of shape (B, h_k, 1, keys); everything else at this head dim stays on the CUDA-core kernels.
 bool tc_bwd256_supported(const fdma_bwd_params& bp) {
   const fdma_fwd_params& p = bp.f;
-  if (p.d != kD || !tc_fwd_supported(p)) return false;
+  if (tile_head_dim(p.d) != kD || !tc_fwd_supported(p)) return false;
   if (p.h_k > 65535 || p.b > 65535) return false;
   const int G = p.h / p.h_k;
   const bool mask_b = !p.mask || p.mask_row_stride == 0 || p.seqlen_q == 1;

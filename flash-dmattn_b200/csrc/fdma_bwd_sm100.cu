@@ -1,4 +1,4 @@
-// Backward dynamic-mask attention for sm_100a (head dim 128): dQ, dK, dV and dBias from dO, O, LSE.
+// Backward dynamic-mask attention for sm_100a (head dims up to 128): dQ, dK, dV and dBias from dO, O, LSE.
 //
 // Math of the reference's compute_dq_dk_dv_1colblock (csrc/flash_sparse_attn/src/flash_bwd_kernel.h:79-1142):
 //   P = exp(S - LSE), dP = dO V^T, dS = P o (dP - D), D = rowsum(dO o O),
@@ -16,7 +16,10 @@
 // Query-broadcast bias gives dBias = column sums of dS: one fp32 register per softmax thread for the whole CTA.
 //
 // Warps: 0 TMA producer | 1 MMA issuer | 4-7, 8-11 softmax (query columns 0-31 / 32-63) | 12-15 dQ writer.
-// TMEM: St[2] 2x64 | dPt 64 | dQ^T 64 | dV 128 | dK 128 = 512 columns.
+// TMEM: St[2] 2x64 | dPt 64 | dQ^T 64 | dV D | dK D = 512 columns (D = 128) or 384 (D = 64).
+// Two instantiations: tiles of D = 64 for head dims up to 64, of D = 128 for 72 to 128. Columns beyond the head dim are
+// zeros that the TMA loads fill in, so nothing is padded in memory. (Head dim 64 ran on the D = 128 tiles before, with
+// padded copies of every tensor around it: 2 x the tensor work and 0.12 ms of copies at 4 x 2048 x 16 heads.)
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <math_constants.h>
@@ -29,13 +32,11 @@
 namespace fdma {
 namespace {
 
-constexpr int kD = 128;
 constexpr int kBN = 128;  // keys per CTA
 constexpr int kBM = 64;   // query rows per step
 constexpr int kQStages = 3;
 constexpr int kThreads = 512;
 constexpr int kMaxAct = 4096;  // bytes of the per-CTA tile-activity table
-constexpr int kDetFracBits = 40;  // deterministic dQ: |dQ / scale| < 2^23, resolution 2^-40
 constexpr float kLog2e = 1.4426950408889634f;
 
 enum DbiasMode { kDbNone = 0, kDbColsum = 1, kDbDirect = 2, kDbAtomic = 3 };
@@ -52,14 +53,14 @@ struct BwdKernelParams {
   const void* bias;
   const float* lse2;   // (B,H,Sq_r) LSE * log2(e); +inf for empty and padded rows
   const float* dsum;   // (B,H,Sq_r) D = rowsum(dO o O)
-  float* dq_acc;       // (B,H,Sq,128) fp32, zeroed by the launcher; deterministic kernels: the same shape in 64-bit
+  float* dq_acc;       // (B,H,Sq,D) fp32, zeroed by the launcher; deterministic kernels: the same shape in 64-bit
                        // fixed point (kDetFracBits fractional bits), whose sums do not depend on the order of addition
   void* dk;
   void* dv;
   void* dbias;         // direct / column-sum modes: the output tensor
   float* dbias_acc;    // atomic mode: fp32 buffer (dbias_b, dbias_h, dbias_rows, dbias_keys), zeroed
-  float* dkv_part;     // nsplit > 1: fp32 partials [2: dV, dK][nsplit][B][h_k][NT*128][128]
-  float* dbias_part;   // nsplit > 1, column-sum mode: fp32 partials [nsplit][B][h_k][NT*128]
+  float* dkv_part;     // null, or fp32 partials [2: dV, dK][nsplit][B][h_k][NT*128][D] instead of dk / dv
+  float* dbias_part;   // with dkv_part, column-sum mode: fp32 partials [nsplit][B][h_k][NT*128]
   int nsplit;          // query-range splits per key tile
   const uint8_t* act;  // per-query mask: activity bytes [B][h_mask][ceil(Sq/128)][ceil(Sk/128)], else null
   int mask_bits;       // per-query mask given as one bit per key (uint32 words, strides in words)
@@ -69,7 +70,7 @@ struct BwdKernelParams {
   int64_t dk_batch_stride, dk_row_stride, dk_head_stride;
   int64_t dv_batch_stride, dv_row_stride, dv_head_stride;
   int64_t dbias_batch_stride, dbias_head_stride, dbias_row_stride;
-  int b, seqlen_q, seqlen_k, sq_r, h, h_k, h_mask, h_bias;
+  int b, seqlen_q, seqlen_k, sq_r, h, h_k, h_mask, h_bias, d;
   int dbias_b, dbias_h, dbias_rows, dbias_keys, dbias_mode;
   int is_causal;
   const int32_t* key_pos;  // ascending positions of compacted keys, or null
@@ -78,7 +79,9 @@ struct BwdKernelParams {
   float scale_log2, scale;
 };
 
+template <int D>
 struct SmemB {
+  static constexpr int kD = D;
   static constexpr int kKOff = 0;
   static constexpr int kVOff = kBN * kD * 2;                       // 32 KB
   static constexpr int kQdoOff = 2 * kBN * kD * 2;                 // 64 KB
@@ -89,8 +92,8 @@ struct SmemB {
   static constexpr int kActOff = kDsOff + 2 * kDsBytes;            // 192 KB
   static constexpr int kLdOff = kActOff + kMaxAct;                 // per stage: 64 x LSE*log2e, 64 x D (fp32)
   static constexpr int kLdBytes = 2 * kBM * 4;
-  static constexpr int kDqOff = kLdOff + kQStages * kLdBytes;      // [32 q][128 d] fp32 staging tile of the dQ writer
-  static constexpr int kTrOff = kDqOff + 32 * kD * 4;              // per softmax warp: 1 KB transposition scratch
+  static constexpr int kDqOff = kLdOff + kQStages * kLdBytes;      // dQ writer's staging tile: [32 q][128 d] or [64 q][64 d] fp32
+  static constexpr int kTrOff = kDqOff + 16 * 1024;               // per softmax warp: 1 KB transposition scratch
   static constexpr int kTrBytes = 8 * 1024;
   static constexpr int kRedOff = kTrOff + kTrBytes;
   static constexpr int kBarOff = kRedOff + kBN * 4;
@@ -99,125 +102,6 @@ struct SmemB {
   static constexpr int kTotal = kMiscOff + 32;
   static constexpr int kAlloc = kTotal + 1024;
 };
-
-// D = rowsum(dO o O), LSE in log2 units; rows [Sq, Sq_r) are padding (+inf / 0). Head dim 128: sixteen lanes hold
-// one row (16 B each), a warp covers eight consecutive query rows of one (b, h) with all loads issued up front.
-template <bool kBf16>
-__global__ void __launch_bounds__(256) bwd_prep_kernel(const void* __restrict__ out, const void* __restrict__ dout,
-                                                        const float* __restrict__ lse, float* __restrict__ lse2,
-                                                        float* __restrict__ dsum, int B, int H, int Sq, int Sq_r,
-                                                        int64_t ob, int64_t orow, int64_t oh, int64_t gb, int64_t grow,
-                                                        int64_t gh) {
-  const int lane = threadIdx.x & 31, sub = lane >> 4, l16 = lane & 15;
-  const int64_t w = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
-  const int groups = Sq_r / 8;
-  const int64_t total = static_cast<int64_t>(B) * H * groups;
-  if (w >= total) return;
-  const int q0 = static_cast<int>(w % groups) * 8;
-  const int h = static_cast<int>((w / groups) % H);
-  const int b = static_cast<int>(w / (static_cast<int64_t>(groups) * H));
-  const uint16_t* o = reinterpret_cast<const uint16_t*>(out) + b * ob + h * oh + l16 * 8;
-  const uint16_t* g = reinterpret_cast<const uint16_t*>(dout) + b * gb + h * gh + l16 * 8;
-  uint4 a[4], c[4];
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int q = q0 + u * 2 + sub;
-    a[u] = c[u] = make_uint4(0, 0, 0, 0);
-    if (q < Sq) {
-      a[u] = *reinterpret_cast<const uint4*>(o + static_cast<int64_t>(q) * orow);
-      c[u] = *reinterpret_cast<const uint4*>(g + static_cast<int64_t>(q) * grow);
-    }
-  }
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const uint32_t aw[4] = {a[u].x, a[u].y, a[u].z, a[u].w}, cw[4] = {c[u].x, c[u].y, c[u].z, c[u].w};
-    float acc = 0.f;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float a0, a1, c0, c1;
-      if (kBf16) {
-        a0 = __uint_as_float(aw[j] << 16); a1 = __uint_as_float(aw[j] & 0xFFFF0000u);
-        c0 = __uint_as_float(cw[j] << 16); c1 = __uint_as_float(cw[j] & 0xFFFF0000u);
-      } else {
-        const __half2 ah = *reinterpret_cast<const __half2*>(&aw[j]);
-        const __half2 ch = *reinterpret_cast<const __half2*>(&cw[j]);
-        a0 = __low2float(ah); a1 = __high2float(ah); c0 = __low2float(ch); c1 = __high2float(ch);
-      }
-      acc = fmaf(a0, c0, acc);
-      acc = fmaf(a1, c1, acc);
-    }
-#pragma unroll
-    for (int sft = 8; sft > 0; sft >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, sft);
-    const int q = q0 + u * 2 + sub;
-    if (l16 == 0) {
-      const int64_t idx = (static_cast<int64_t>(b) * H + h) * Sq_r + q;
-      if (q < Sq) {
-        lse2[idx] = lse[(static_cast<int64_t>(b) * H + h) * Sq + q] * kLog2e;
-        dsum[idx] = acc;
-      } else {
-        lse2[idx] = CUDART_INF_F;
-        dsum[idx] = 0.f;
-      }
-    }
-  }
-}
-
-// fp32 dQ accumulator (B,H,Sq,128) * scale -> dq (B,Sq,H,128 strided, 16-bit)
-template <bool kBf16>
-__global__ void bwd_convert_dq_kernel(const float* __restrict__ acc, void* __restrict__ dq, int64_t n_vec, int Sq,
-                                      int H, int64_t sb, int64_t sr, int64_t sh, float scale) {
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n_vec;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t e = i * 8;
-    const int dd = static_cast<int>(e % kD);
-    const int q = static_cast<int>((e / kD) % Sq);
-    const int h = static_cast<int>((e / (static_cast<int64_t>(kD) * Sq)) % H);
-    const int b = static_cast<int>(e / (static_cast<int64_t>(kD) * Sq * H));
-    const float4 x = *reinterpret_cast<const float4*>(acc + e);
-    const float4 y = *reinterpret_cast<const float4*>(acc + e + 4);
-    uint4 o;
-    o.x = pack_16x2<kBf16>(x.x * scale, x.y * scale);
-    o.y = pack_16x2<kBf16>(x.z * scale, x.w * scale);
-    o.z = pack_16x2<kBf16>(y.x * scale, y.y * scale);
-    o.w = pack_16x2<kBf16>(y.z * scale, y.w * scale);
-    *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(dq) + b * sb + q * sr + h * sh + dd) = o;
-  }
-}
-
-// Deterministic mode: 64-bit fixed-point accumulator -> 16-bit dQ.
-template <bool kBf16>
-__global__ void bwd_convert_dq_fixed_kernel(const long long* __restrict__ acc, void* __restrict__ dq, int64_t n_vec,
-                                            int Sq, int H, int64_t sb, int64_t sr, int64_t sh, float scale,
-                                            const float* __restrict__ dsum, int sq_r) {
-  const float unit = scale * (1.0f / static_cast<float>(1ll << kDetFracBits));
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n_vec;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t e = i * 8;
-    const int dd = static_cast<int>(e % kD);
-    const int q = static_cast<int>((e / kD) % Sq);
-    const int h = static_cast<int>((e / (static_cast<int64_t>(kD) * Sq)) % H);
-    const int b = static_cast<int>(e / (static_cast<int64_t>(kD) * Sq * H));
-    float x[8];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const longlong2 v = *reinterpret_cast<const longlong2*>(acc + e + 2 * j);
-      x[2 * j] = __ll2float_rn(v.x) * unit;
-      x[2 * j + 1] = __ll2float_rn(v.y) * unit;
-    }
-    // Fixed point cannot carry NaN / Inf. A non-finite dO or O element makes D = rowsum(dO o O) of its row
-    // non-finite, and with it every dS of the row: such rows come out as NaN, as the fp32 path would give.
-    if (!isfinite(dsum[(static_cast<int64_t>(b) * H + h) * sq_r + q])) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) x[j] = __int_as_float(0x7FC00000);
-    }
-    uint4 o;
-    o.x = pack_16x2<kBf16>(x[0], x[1]);
-    o.y = pack_16x2<kBf16>(x[2], x[3]);
-    o.z = pack_16x2<kBf16>(x[4], x[5]);
-    o.w = pack_16x2<kBf16>(x[6], x[7]);
-    *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(dq) + b * sb + q * sr + h * sh + dd) = o;
-  }
-}
 
 // fp32 (nb,nh,nr,nk) contiguous -> strided 16-bit dbias
 template <bool kBf16>
@@ -245,9 +129,10 @@ __device__ __forceinline__ uint16_t float_to_raw16(float x) {
   return static_cast<uint16_t>(pack_16x2<kBf16>(x, 0.f) & 0xFFFFu);
 }
 
-template <bool kBf16, bool kBcast, bool kDet>
+template <int D, bool kBf16, bool kBcast, bool kDet>
 __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant__ BwdKernelParams p) {
-  using L = SmemB;
+  using L = SmemB<D>;
+  constexpr int kD = D;
   // Row-broadcast kernel: the two softmax warpgroups are two teams that take alternate steps (all 64 queries of
   // a step, in two passes of 32), so the fixed latencies of one team's step -- barrier round trips, TMEM loads and
   // stores, the hand-over to the MMA warp -- overlap the other team's arithmetic. Per-query kernel: both warpgroups
@@ -380,7 +265,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   __syncthreads();
   const uint32_t tmem_base = *s_tmem;
   const int n_steps = *s_nsteps;
-  constexpr uint32_t kColSt = 0, kColDp = 128, kColDq = 192, kColDv = 256, kColDk = 384;
+  constexpr uint32_t kColSt = 0, kColDp = 128, kColDq = 192, kColDv = 256, kColDk = 256 + kD;
 
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
@@ -390,7 +275,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         FDMA_PROF_BEGIN();
         mbar_arrive_expect_tx(bar_kv, 2 * kBN * kD * 2);
 #pragma unroll
-        for (int kb = 0; kb < 2; ++kb) {
+        for (int kb = 0; kb < kD / 64; ++kb) {
           tma_load_4d(s_k + kb * (kBN * 128), &p.tm_k, bar_kv, kb * 64, hk, n * kBN, b);
           tma_load_4d(s_v + kb * (kBN * 128), &p.tm_v, bar_kv, kb * 64, hk, n * kBN, b);
         }
@@ -409,7 +294,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
             bulk_load_1d(s_ld + stage * (2 * kBM), p.lse2 + row0, kBM * 4, bar_qdo_full + stage);
             bulk_load_1d(s_ld + stage * (2 * kBM) + kBM, p.dsum + row0, kBM * 4, bar_qdo_full + stage);
 #pragma unroll
-            for (int kb = 0; kb < 2; ++kb) {
+            for (int kb = 0; kb < kD / 64; ++kb) {
               tma_load_4d(dst + kb * (kBM * 128), &p.tm_q, bar_qdo_full + stage, kb * 64, h, m * kBM, b);
               tma_load_4d(dst + L::kQBytes + kb * (kBM * 128), &p.tm_do, bar_qdo_full + stage, kb * 64, h, m * kBM, b);
             }
@@ -423,7 +308,10 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
       if (n_steps > 0) {
         constexpr uint32_t idesc_s = umma_idesc(kBN, kBM, kBf16, false, false);  // St/dPt: 128 x 64, K-major
         constexpr uint32_t idesc_g = umma_idesc(kBN, kD, kBf16, false, true);    // dV/dK: A from TMEM, B MN-major
-        constexpr uint32_t idesc_q = umma_idesc(kD, kBM, kBf16, true, true);     // dQ^T: both MN-major
+        // dQ^T: both MN-major, M = 128. With D = 64 the second 64-row block of A is the first one again (block stride
+        // 0), so TMEM lanes 64-127 hold a second copy of dQ^T and all four writer warps have rows to move.
+        constexpr uint32_t idesc_q = umma_idesc(128, kBM, kBf16, true, true);
+        constexpr uint32_t k_blk = kD == 128 ? kBN * 128 : 0;
         const uint32_t k_addr = smem_u32(s_k), v_addr = smem_u32(s_v), qdo_addr = smem_u32(s_qdo),
                        ds_addr = smem_u32(s_ds);
         auto issue_st = [&](int step) {  // St[step & 1] = K Q^T
@@ -497,7 +385,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           // dQ^T = K^T dS^T : 8 k-steps of 16 keys
 #pragma unroll
           for (int s = 0; s < kBN / 16; ++s) {
-            umma_ss(tmem_base + kColDq, umma_desc_sw128(k_addr + s * 2048, kBN * 128, 1024),
+            umma_ss(tmem_base + kColDq, umma_desc_sw128(k_addr + s * 2048, k_blk, 1024),
                     umma_desc_sw128(ds_addr + (i & 1) * L::kDsBytes + s * 2048, 16, 1024), idesc_q, s > 0 ? 1u : 0u);
           }
           umma_commit(bar_dq_full);
@@ -872,7 +760,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
       if (half == 0 && key < p.dbias_keys) {
         // dbias_h == h_k: this CTA saw every query head of the group. dbias_h == h with a group of one: same.
         const float tot = colsum + s_red[krow];
-        if (p.nsplit > 1)
+        if (p.dkv_part)
           p.dbias_part[((static_cast<int64_t>(split) * p.b + b) * p.h_k + hk) * (NT * kBN) + key] = key_ok ? tot : 0.f;
         else
           dbias16[b * p.dbias_batch_stride + hk * p.dbias_head_stride + key] = float_to_raw16<kBf16>(key_ok ? tot : 0.f);
@@ -898,7 +786,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
 #pragma unroll
           for (int j = 0; j < 32; ++j) r[j] = 0u;
         }
-        if (p.nsplit > 1) {
+        if (p.dkv_part) {
           // fp32 partial: part[dv|dk][split][b][hk][key][d]
           float* part = p.dkv_part + ((((static_cast<int64_t>(half) * p.nsplit + split) * p.b + b) * p.h_k + hk) *
                                           (NT * kBN) + key) * kD + c * 32;
@@ -910,6 +798,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         } else if (key_ok) {
 #pragma unroll
           for (int v4 = 0; v4 < 4; ++v4) {
+            if (c * 32 + v4 * 8 >= p.d) break;
             uint4 o;
             o.x = pack_16x2<kBf16>(__uint_as_float(r[v4 * 8 + 0]) * mul, __uint_as_float(r[v4 * 8 + 1]) * mul);
             o.y = pack_16x2<kBf16>(__uint_as_float(r[v4 * 8 + 2]) * mul, __uint_as_float(r[v4 * 8 + 3]) * mul);
@@ -940,6 +829,55 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(0, mbar_wait(bar_dq_full, i & 1, ctl, kWaitDqFull)));
         if (!ok) break;
         tc_fence_after_sync();
+        float* gdst = p.dq_acc + ((static_cast<int64_t>(b) * p.h + h) * Sq + m * kBM) * kD;
+        if constexpr (kD == 64) {
+          // Lanes 64-127 hold the same 64 rows again: warps 0-1 move queries 0-31 (deterministic: 0-15 of each 32),
+          // warps 2-3 the others, and the staging tile takes all 64 queries at once (deterministic: 32).
+          const int d64 = dl & 63, hi = dl >> 6;
+          constexpr int kParts = kDet ? 2 : 1;
+          constexpr int kPer = kDet ? 16 : 32;  // queries per thread and part
+          uint32_t r[kParts][kPer];
+#pragma unroll
+          for (int c = 0; c < kParts; ++c) {
+            const uint32_t col = tmem_base + lane_addr + kColDq + (kDet ? c * 32 + hi * 16 : hi * 32);
+            if constexpr (kDet) tmem_ld_x16(col, r[c]);
+            else tmem_ld_x32(col, r[c]);
+          }
+          tmem_wait_ld();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_dq_empty);
+#pragma unroll
+          for (int c = 0; c < kParts; ++c) {
+            if (tid == 384) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            named_bar_sync(2, 128);
+#pragma unroll
+            for (int j = 0; j < kPer; ++j) {
+              const int row = hi * kPer + j;
+              if constexpr (kDet)
+                reinterpret_cast<long long*>(s_dq)[row * kD + d64] =
+                    __float2ll_rn(__uint_as_float(r[c][j]) * static_cast<float>(1ll << kDetFracBits));
+              else
+                s_dq[row * kD + d64] = __uint_as_float(r[c][j]);
+            }
+            fence_proxy_async_smem();
+            named_bar_sync(3, 128);
+            if (tid == 384) {
+              const int rows = min(2 * kPer, Sq - (m * kBM + c * 32));
+              if (rows > 0) {
+                if constexpr (kDet)
+                  bulk_reduce_add_u64(reinterpret_cast<long long*>(p.dq_acc) +
+                                          ((static_cast<int64_t>(b) * p.h + h) * Sq + m * kBM + c * 32) * kD,
+                                      s_dq, rows * kD * 8);
+                else
+                  bulk_reduce_add_f32(gdst, s_dq, rows * kD * 4);
+              }
+              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            }
+          }
+          ++i;
+          continue;
+        }
         uint32_t r0[32], r1[32];
         tmem_ld_x32(tmem_base + lane_addr + kColDq, r0);
         tmem_ld_x32(tmem_base + lane_addr + kColDq + 32, r1);
@@ -947,7 +885,6 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_dq_empty);  // dQ^T columns may be overwritten by the next step from here on
-        float* gdst = p.dq_acc + ((static_cast<int64_t>(b) * p.h + h) * Sq + m * kBM) * kD;
         if constexpr (kDet) {
           // 64-bit fixed point: integer sums are the same in any order. 16 queries fill the staging tile.
           long long* s_dq64 = reinterpret_cast<long long*>(s_dq);
@@ -967,13 +904,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
             named_bar_sync(3, 128);
             if (tid == 384) {
               const int rows = min(16, Sq - (m * kBM + c * 16));
-              if (rows > 0) {
-                asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.u64 [%0], [%1], %2;"
-                             :
-                             : "l"(reinterpret_cast<uint64_t>(gdst64 + c * 16 * kD)), "r"(smem_u32(s_dq)),
-                               "r"(static_cast<uint32_t>(rows * kD * 8))
-                             : "memory");
-              }
+              if (rows > 0) bulk_reduce_add_u64(gdst64 + c * 16 * kD, s_dq, rows * kD * 8);
               asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             }
           }
@@ -990,13 +921,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           named_bar_sync(3, 128);
           if (tid == 384) {
             const int rows = min(32, Sq - (m * kBM + c * 32));
-            if (rows > 0) {
-              asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;"
-                           :
-                           : "l"(reinterpret_cast<uint64_t>(gdst + c * 32 * kD)), "r"(smem_u32(s_dq)),
-                             "r"(static_cast<uint32_t>(rows * kD * 4))
-                           : "memory");
-            }
+            if (rows > 0) bulk_reduce_add_f32(gdst + c * 32 * kD, s_dq, rows * kD * 4);
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
         }
@@ -1016,56 +941,10 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   }
 }
 
-// Sum of the query-range partials of dK or dV: part [nsplit][B][h_k][keys_r][128] fp32 -> 16-bit (B, Sk, h_k, 128).
-template <bool kBf16>
-__global__ void __launch_bounds__(256) bwd_reduce_dkv_kernel(const float* __restrict__ part, void* __restrict__ dst,
-                                                              int nsplit, int B, int Hk, int Sk, int keys_r,
-                                                              int64_t sb, int64_t sr, int64_t sh) {
-  const int64_t n_vec = static_cast<int64_t>(B) * Hk * Sk * (kD / 8);
-  const int64_t split_stride = static_cast<int64_t>(B) * Hk * keys_r * kD;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n_vec;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int c = static_cast<int>(i % (kD / 8));
-    const int key = static_cast<int>((i / (kD / 8)) % Sk);
-    const int hk = static_cast<int>((i / (static_cast<int64_t>(kD / 8) * Sk)) % Hk);
-    const int b = static_cast<int>(i / (static_cast<int64_t>(kD / 8) * Sk * Hk));
-    const float* src = part + ((static_cast<int64_t>(b) * Hk + hk) * keys_r + key) * kD + c * 8;
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int s = 0; s < nsplit; ++s) {
-      const float4 a = *reinterpret_cast<const float4*>(src + s * split_stride);
-      const float4 d = *reinterpret_cast<const float4*>(src + s * split_stride + 4);
-      acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
-      acc[4] += d.x; acc[5] += d.y; acc[6] += d.z; acc[7] += d.w;
-    }
-    uint4 o;
-    o.x = pack_16x2<kBf16>(acc[0], acc[1]);
-    o.y = pack_16x2<kBf16>(acc[2], acc[3]);
-    o.z = pack_16x2<kBf16>(acc[4], acc[5]);
-    o.w = pack_16x2<kBf16>(acc[6], acc[7]);
-    *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(dst) + b * sb + static_cast<int64_t>(key) * sr + hk * sh +
-                              c * 8) = o;
-  }
-}
-
-// Sum of the query-range partials of the column-sum dBias: part [nsplit][B][h_k][keys_r] fp32 -> 16-bit
-// (B, h_k, 1, dbias_keys); keys beyond Sk are zero.
-template <bool kBf16>
-__global__ void __launch_bounds__(256) bwd_reduce_dbias_kernel(const float* __restrict__ part, void* __restrict__ dst,
-                                                                int nsplit, int B, int Hk, int dbias_keys, int Sk,
-                                                                int keys_r, int64_t sb, int64_t sh) {
-  const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (i >= static_cast<int64_t>(B) * Hk * dbias_keys) return;
-  const int key = static_cast<int>(i % dbias_keys);
-  const int hk = static_cast<int>((i / dbias_keys) % Hk);
-  const int b = static_cast<int>(i / (static_cast<int64_t>(dbias_keys) * Hk));
-  float acc = 0.f;
-  if (key < Sk)
-    for (int s = 0; s < nsplit; ++s) acc += part[((static_cast<int64_t>(s) * B + b) * Hk + hk) * keys_r + key];
-  reinterpret_cast<uint16_t*>(dst)[b * sb + hk * sh + key] = float_to_raw16<kBf16>(acc);
-}
-
 struct BwdPlan {
+  int D;
   bool bcast;
+  bool part;  // dK, dV (and column sums) leave the main kernel as fp32 partials
   bool needs_act;
   int dbias_mode;
   int sq_r;
@@ -1086,9 +965,13 @@ int pick_nsplit(const fdma_fwd_params& p) {
   return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(std::min(want, cap), 64)));
 }
 
+// Keys of the fp32 buffer of the atomic dBias mode: those of the tensor, or with gathered keys the gathered ones.
+int atomic_keys(const fdma_bwd_params& bp) { return bp.scatter_pos ? bp.f.seqlen_k : bp.dbias_keys; }
+
 BwdPlan plan(const fdma_bwd_params& bp) {
   const fdma_fwd_params& p = bp.f;
   BwdPlan pl;
+  pl.D = tile_head_dim(p.d);
   const bool mask_b = !p.mask || p.mask_row_stride == 0 || p.seqlen_q == 1;
   const bool bias_b = !p.bias || p.bias_row_stride == 0 || p.seqlen_q == 1;
   pl.bcast = mask_b && bias_b;
@@ -1111,18 +994,19 @@ BwdPlan plan(const fdma_bwd_params& bp) {
   const size_t rows = static_cast<size_t>(p.b) * p.h * pl.sq_r;
   pl.lse2_off = o; o += align256(rows * 4);
   pl.dsum_off = o; o += align256(rows * 4);
-  pl.dq_off = o;   o += align256(static_cast<size_t>(p.b) * p.seqlen_q * p.h * kD * (bp.deterministic ? 8 : 4));
+  pl.dq_off = o;   o += align256(static_cast<size_t>(p.b) * p.seqlen_q * p.h * pl.D * (bp.deterministic ? 8 : 4));
   pl.act_off = o;
   if (pl.needs_act)
     o += align256(static_cast<size_t>(p.b) * p.h_mask * ((p.seqlen_q + 127) / 128) * ((p.seqlen_k + 127) / 128));
   pl.dbias_off = o;
   if (pl.dbias_mode == kDbAtomic)
-    o += align256(static_cast<size_t>(bp.dbias_b) * bp.dbias_h * bp.dbias_rows * bp.dbias_keys * 4);
+    o += align256(static_cast<size_t>(bp.dbias_b) * bp.dbias_h * bp.dbias_rows * atomic_keys(bp) * 4);
   pl.nsplit = pick_nsplit(p);
+  pl.part = pl.nsplit > 1 || bp.scatter_pos != nullptr;
   pl.part_off = pl.dbpart_off = o;
-  if (pl.nsplit > 1) {
+  if (pl.part) {
     const size_t keys_r = round_up(p.seqlen_k, kBN);
-    o += align256(static_cast<size_t>(2) * pl.nsplit * p.b * p.h_k * keys_r * kD * 4);
+    o += align256(static_cast<size_t>(2) * pl.nsplit * p.b * p.h_k * keys_r * pl.D * 4);
     pl.dbpart_off = o;
     if (pl.dbias_mode == kDbColsum) o += align256(static_cast<size_t>(pl.nsplit) * p.b * p.h_k * keys_r * 4);
   }
@@ -1132,8 +1016,9 @@ BwdPlan plan(const fdma_bwd_params& bp) {
 
 bool aligned16(const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; }
 
-template <bool kBf16>
+template <int D, bool kBf16>
 int launch(const fdma_bwd_params& bp, const BwdPlan& pl, cudaStream_t stream) {
+  using L = SmemB<D>;
   const fdma_fwd_params& p = bp.f;
   if (!p.workspace || p.workspace_bytes < pl.total) return FDMA_ERR_WORKSPACE;
   char* ws = static_cast<char*>(p.workspace);
@@ -1162,20 +1047,18 @@ int launch(const fdma_bwd_params& bp, const BwdPlan& pl, cudaStream_t stream) {
   float* lse2 = reinterpret_cast<float*>(ws + pl.lse2_off);
   float* dsum = reinterpret_cast<float*>(ws + pl.dsum_off);
   float* dq_acc = reinterpret_cast<float*>(ws + pl.dq_off);
-  const size_t dq_bytes = static_cast<size_t>(p.b) * p.seqlen_q * p.h * kD * (bp.deterministic ? 8 : 4);
-  cudaError_t e = cudaMemsetAsync(dq_acc, 0, dq_bytes, stream);
-  if (e != cudaSuccess) return static_cast<int>(e);
   {
-    const int64_t warps = static_cast<int64_t>(p.b) * p.h * (pl.sq_r / 8);
-    const int64_t blocks = (warps * 32 + 255) / 256;
-    bwd_prep_kernel<kBf16><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
-        p.out, bp.dout, p.lse, lse2, dsum, p.b, p.h, p.seqlen_q, pl.sq_r, p.o_batch_stride, p.o_row_stride,
-        p.o_head_stride, bp.do_batch_stride, bp.do_row_stride, bp.do_head_stride);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return static_cast<int>(e);
+    BwdPrepArgs a;
+    a.out = p.out; a.dout = bp.dout; a.lse = p.lse; a.lse2 = lse2; a.dsum = dsum; a.dq_acc = dq_acc;
+    a.b = p.b; a.h = p.h; a.sq = p.seqlen_q; a.sq_r = pl.sq_r; a.d = p.d; a.acc_bytes = bp.deterministic ? 8 : 4;
+    a.o_sb = p.o_batch_stride; a.o_sr = p.o_row_stride; a.o_sh = p.o_head_stride;
+    a.do_sb = bp.do_batch_stride; a.do_sr = bp.do_row_stride; a.do_sh = bp.do_head_stride;
+    st = launch_bwd_prep(a, D, kBf16, stream);
+    if (st) return st;
     st = export_softmax_d(bp, dsum, pl.sq_r, stream);
     if (st) return st;
   }
+  cudaError_t e = cudaSuccess;
   kp.act = nullptr;
   kp.mask_bits = p.mask ? p.mask_bits : 0;
   if (pl.needs_act && p.tile_activity) {
@@ -1190,11 +1073,11 @@ int launch(const fdma_bwd_params& bp, const BwdPlan& pl, cudaStream_t stream) {
   if (pl.dbias_mode == kDbAtomic) {
     kp.dbias_acc = reinterpret_cast<float*>(ws + pl.dbias_off);
     e = cudaMemsetAsync(kp.dbias_acc, 0,
-                        static_cast<size_t>(bp.dbias_b) * bp.dbias_h * bp.dbias_rows * bp.dbias_keys * 4, stream);
+                        static_cast<size_t>(bp.dbias_b) * bp.dbias_h * bp.dbias_rows * atomic_keys(bp) * 4, stream);
     if (e != cudaSuccess) return static_cast<int>(e);
   }
   kp.nsplit = pl.nsplit;
-  kp.dkv_part = reinterpret_cast<float*>(ws + pl.part_off);
+  kp.dkv_part = pl.part ? reinterpret_cast<float*>(ws + pl.part_off) : nullptr;
   kp.dbias_part = reinterpret_cast<float*>(ws + pl.dbpart_off);
   kp.mask = static_cast<const uint8_t*>(p.mask);
   kp.bias = p.bias;
@@ -1214,9 +1097,10 @@ int launch(const fdma_bwd_params& bp, const BwdPlan& pl, cudaStream_t stream) {
   kp.dv_batch_stride = bp.dv_batch_stride; kp.dv_row_stride = bp.dv_row_stride; kp.dv_head_stride = bp.dv_head_stride;
   kp.dbias_batch_stride = bp.dbias_batch_stride; kp.dbias_head_stride = bp.dbias_head_stride;
   kp.dbias_row_stride = bp.dbias_row_stride;
-  kp.b = p.b; kp.seqlen_q = p.seqlen_q; kp.seqlen_k = p.seqlen_k; kp.sq_r = pl.sq_r; kp.h = p.h; kp.h_k = p.h_k;
+  kp.b = p.b; kp.seqlen_q = p.seqlen_q; kp.seqlen_k = p.seqlen_k; kp.sq_r = pl.sq_r; kp.h = p.h; kp.h_k = p.h_k; kp.d = p.d;
   kp.h_mask = p.h_mask; kp.h_bias = p.h_bias;
-  kp.dbias_b = bp.dbias_b; kp.dbias_h = bp.dbias_h; kp.dbias_rows = bp.dbias_rows; kp.dbias_keys = bp.dbias_keys;
+  kp.dbias_b = bp.dbias_b; kp.dbias_h = bp.dbias_h; kp.dbias_rows = bp.dbias_rows;
+  kp.dbias_keys = bp.scatter_pos ? p.seqlen_k : bp.dbias_keys;
   kp.dbias_mode = pl.dbias_mode;
   kp.is_causal = p.is_causal;
   kp.key_pos = p.key_pos;
@@ -1225,9 +1109,9 @@ int launch(const fdma_bwd_params& bp, const BwdPlan& pl, cudaStream_t stream) {
   kp.scale_log2 = p.softmax_scale * kLog2e;
   kp.scale = p.softmax_scale;
 
-  auto kern = bp.deterministic ? (pl.bcast ? bwd_kernel<kBf16, true, true> : bwd_kernel<kBf16, false, true>)
-                               : (pl.bcast ? bwd_kernel<kBf16, true, false> : bwd_kernel<kBf16, false, false>);
-  const int smem_bytes = SmemB::kAlloc;
+  auto kern = bp.deterministic ? (pl.bcast ? bwd_kernel<D, kBf16, true, true> : bwd_kernel<D, kBf16, false, true>)
+                               : (pl.bcast ? bwd_kernel<D, kBf16, true, false> : bwd_kernel<D, kBf16, false, false>);
+  const int smem_bytes = L::kAlloc;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
   if (e != cudaSuccess) return static_cast<int>(e);
   dim3 grid(((p.seqlen_k + kBN - 1) / kBN) * pl.nsplit, p.h_k, p.b);
@@ -1239,41 +1123,33 @@ int launch(const fdma_bwd_params& bp, const BwdPlan& pl, cudaStream_t stream) {
   e = cudaGetLastError();
   if (e != cudaSuccess) return static_cast<int>(e);
 
-  if (pl.nsplit > 1) {
-    const int keys_r = static_cast<int>(round_up(p.seqlen_k, kBN));
-    const int64_t n_vec = static_cast<int64_t>(p.b) * p.h_k * p.seqlen_k * (kD / 8);
-    const unsigned g = static_cast<unsigned>(std::min<int64_t>((n_vec + 255) / 256, sm_count() * 32));
-    for (int which = 0; which < 2; ++which) {  // 0: dV, 1: dK
-      const float* part = kp.dkv_part + static_cast<size_t>(which) * pl.nsplit * p.b * p.h_k * keys_r * kD;
-      bwd_reduce_dkv_kernel<kBf16><<<g, 256, 0, stream>>>(
-          part, which == 0 ? bp.dv : bp.dk, pl.nsplit, p.b, p.h_k, p.seqlen_k, keys_r,
-          which == 0 ? bp.dv_batch_stride : bp.dk_batch_stride, which == 0 ? bp.dv_row_stride : bp.dk_row_stride,
-          which == 0 ? bp.dv_head_stride : bp.dk_head_stride);
-    }
-    if (pl.dbias_mode == kDbColsum) {
-      const int64_t nk = static_cast<int64_t>(p.b) * p.h_k * bp.dbias_keys;
-      bwd_reduce_dbias_kernel<kBf16><<<static_cast<unsigned>((nk + 255) / 256), 256, 0, stream>>>(
-          kp.dbias_part, bp.dbias, pl.nsplit, p.b, p.h_k, bp.dbias_keys, p.seqlen_k, keys_r, bp.dbias_batch_stride,
-          bp.dbias_head_stride);
-    }
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return static_cast<int>(e);
+  BwdFinishArgs f = {};
+  f.dq_acc = dq_acc; f.dq = bp.dq; f.dsum = dsum;
+  f.dq_sb = bp.dq_batch_stride; f.dq_sr = bp.dq_row_stride; f.dq_sh = bp.dq_head_stride;
+  f.scale = p.softmax_scale;
+  f.b = p.b; f.h = p.h; f.sq = p.seqlen_q; f.sq_r = pl.sq_r; f.d = p.d; f.D = D;
+  f.h_k = p.h_k; f.keys_r = static_cast<int>(round_up(p.seqlen_k, kBN));
+  f.rows_out = bp.scatter_pos ? bp.scatter_rows : p.seqlen_k;
+  f.pos = bp.scatter_pos; f.pos_sb = bp.scatter_batch_stride; f.pos_sh = bp.scatter_head_stride;
+  f.h_pos = bp.scatter_h; f.cap = p.seqlen_k;
+  if (pl.part) {
+    f.part = kp.dkv_part; f.nsplit = pl.nsplit;
+    f.split_stride = static_cast<int64_t>(p.b) * p.h_k * f.keys_r * D;
+    f.dk = bp.dk; f.dk_sb = bp.dk_batch_stride; f.dk_sr = bp.dk_row_stride; f.dk_sh = bp.dk_head_stride;
+    f.dv = bp.dv; f.dv_sb = bp.dv_batch_stride; f.dv_sr = bp.dv_row_stride; f.dv_sh = bp.dv_head_stride;
   }
-  {
-    const int64_t n_vec = static_cast<int64_t>(p.b) * p.seqlen_q * p.h * kD / 8;
-    const unsigned g = static_cast<unsigned>(std::min<int64_t>((n_vec + 255) / 256, sm_count() * 32));
-    if (bp.deterministic)
-      bwd_convert_dq_fixed_kernel<kBf16><<<g, 256, 0, stream>>>(reinterpret_cast<const long long*>(dq_acc), bp.dq,
-                                                              n_vec, p.seqlen_q, p.h, bp.dq_batch_stride,
-                                                              bp.dq_row_stride, bp.dq_head_stride, p.softmax_scale,
-                                                              dsum, pl.sq_r);
-    else
-      bwd_convert_dq_kernel<kBf16><<<g, 256, 0, stream>>>(dq_acc, bp.dq, n_vec, p.seqlen_q, p.h, bp.dq_batch_stride,
-                                                          bp.dq_row_stride, bp.dq_head_stride, p.softmax_scale);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return static_cast<int>(e);
+  if (bp.dbias && bp.dbias_rows == 1 && (pl.dbias_mode == kDbAtomic || (pl.dbias_mode == kDbColsum && pl.part))) {
+    const bool atomic = pl.dbias_mode == kDbAtomic;
+    f.db_part = atomic ? kp.dbias_acc : kp.dbias_part;
+    f.db_nsplit = atomic ? 1 : pl.nsplit;
+    f.db_pitch = atomic ? atomic_keys(bp) : f.keys_r;
+    f.db_split_stride = static_cast<int64_t>(p.b) * p.h_k * f.keys_r;
+    f.db_b = bp.dbias_b; f.db_h = bp.dbias_h; f.db_keys = bp.dbias_keys;
+    f.dbias = bp.dbias; f.db_sb = bp.dbias_batch_stride; f.db_sh = bp.dbias_head_stride;
   }
-  if (pl.dbias_mode == kDbAtomic) {
+  st = launch_bwd_finish(f, kBf16, bp.deterministic != 0, stream);
+  if (st) return st;
+  if (pl.dbias_mode == kDbAtomic && bp.dbias_rows != 1) {
     const int64_t ndb = static_cast<int64_t>(bp.dbias_b) * bp.dbias_h * bp.dbias_rows * bp.dbias_keys;
     const unsigned g = static_cast<unsigned>(std::min<int64_t>((ndb + 255) / 256, sm_count() * 32));
     bwd_convert_dbias_kernel<kBf16><<<g, 256, 0, stream>>>(kp.dbias_acc, bp.dbias, bp.dbias_b, bp.dbias_h,
@@ -1288,9 +1164,8 @@ int launch(const fdma_bwd_params& bp, const BwdPlan& pl, cudaStream_t stream) {
 
 bool tc_bwd_supported(const fdma_bwd_params& bp) {
   const fdma_fwd_params& p = bp.f;
-  if (p.d == 256) return tc_bwd256_supported(bp);
   if (!tc_fwd_supported(p)) return false;
-  if (p.d != kD) return false;
+  if (tile_head_dim(p.d) == 256) return tc_bwd256_supported(bp);
   if (p.h_k > 65535) return false;
   if (p.key_pos && p.is_causal && p.h_pos == p.h && p.h != p.h_k) return false;  // positions per kv head at most
   const int G = p.h / p.h_k;
@@ -1305,18 +1180,20 @@ bool tc_bwd_supported(const fdma_bwd_params& bp) {
   for (int64_t s : strides)
     if (s % 8 != 0 || s < 0) return false;
   if (p.seqlen_q > 1 && bp.do_row_stride == 0) return false;
-  if (bp.dbias && bp.dbias_keys > round_up(p.seqlen_k, kBN)) return false;
+  if (bp.dbias && !bp.scatter_pos && bp.dbias_keys > round_up(p.seqlen_k, kBN)) return false;
   return true;
 }
 
 size_t tc_bwd_workspace_bytes(const fdma_bwd_params& p) {
-  return p.f.d == 256 ? tc_bwd256_workspace_bytes(p) : plan(p).total;
+  return tile_head_dim(p.f.d) == 256 ? tc_bwd256_workspace_bytes(p) : plan(p).total;
 }
 
 int tc_bwd(const fdma_bwd_params& p, cudaStream_t stream) {
-  if (p.f.d == 256) return tc_bwd256(p, stream);
+  const bool bf16 = p.f.dtype == FDMA_BF16;
+  if (tile_head_dim(p.f.d) == 256) return tc_bwd256(p, stream);
   const BwdPlan pl = plan(p);
-  return p.f.dtype == FDMA_BF16 ? launch<true>(p, pl, stream) : launch<false>(p, pl, stream);
+  if (pl.D == 64) return bf16 ? launch<64, true>(p, pl, stream) : launch<64, false>(p, pl, stream);
+  return bf16 ? launch<128, true>(p, pl, stream) : launch<128, false>(p, pl, stream);
 }
 
 }  // namespace fdma

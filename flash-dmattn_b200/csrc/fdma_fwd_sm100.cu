@@ -69,10 +69,11 @@ struct FwdKernelParams {
   int64_t mask_batch_stride, mask_head_stride, mask_row_stride;
   int64_t bias_batch_stride, bias_head_stride, bias_row_stride;
   int b, seqlen_q, seqlen_k, h, h_k, h_mask, h_bias;
+  int d;             // head dim, at most D: columns beyond it are zeros filled in by TMA and are not stored
   int is_causal;
   int n_mblk;        // query blocks (of kNQ tiles) per (batch, head)
   int n_items;       // work items = n_mblk * h * b
-  unsigned* sched;   // zeroed by the launcher: index of the next item nobody has taken yet
+  unsigned* sched;   // [0] next item nobody has taken yet, [1] CTAs that are done; both zero between launches
   float scale_log2;  // softmax_scale * log2(e)
 };
 
@@ -138,7 +139,7 @@ __global__ void tile_activity_kernel(const uint8_t* __restrict__ mask, int64_t s
 
 // Work item = one query block (kNQ query tiles of 128 rows) of one (batch, head). CTAs are persistent: the list is
 // ordered by decreasing causal extent (last query blocks first) and a CTA takes the next item nobody has taken yet
-// (one atomicAdd per item on a counter the launcher zeroes), which balances the SMs to within one short item. Barrier phases, ring positions and tensor memory carry over
+// (one atomicAdd per item), which balances the SMs to within one short item. Barrier phases, ring positions and tensor memory carry over
 // from one item to the next; nothing is re-initialised, and the pieces of an item that no role of the PREVIOUS
 // item needs any more start early: the tile flags of the next item are built by warp 3 during the current item,
 // its Q and first K / V tiles are loaded as soon as the tensor core has finished with the current Q, its first
@@ -842,24 +843,25 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
           if (in_range) {
 #pragma unroll
             for (int v8 = 0; v8 < 2; ++v8) {   // 16 outputs = 32 bytes per store where the alignment allows
+              if (c * 32 + v8 * 16 >= p.d) break;
               uint32_t o[8];
 #pragma unroll
               for (int e = 0; e < 8; ++e)
                 o[e] = pack_16x2<kBf16>(__uint_as_float(r[v8 * 16 + 2 * e]) * inv,
                                         __uint_as_float(r[v8 * 16 + 2 * e + 1]) * inv);
-              if (wide_o) {
+              if (wide_o && c * 32 + v8 * 16 + 16 <= p.d) {
                 st_v8(orow + c * 64 + v8 * 32, o);
               } else {
                 *reinterpret_cast<uint4*>(orow + c * 64 + v8 * 32) = make_uint4(o[0], o[1], o[2], o[3]);
-                *reinterpret_cast<uint4*>(orow + c * 64 + v8 * 32 + 16) = make_uint4(o[4], o[5], o[6], o[7]);
+                if (c * 32 + v8 * 16 + 8 < p.d)
+                  *reinterpret_cast<uint4*>(orow + c * 64 + v8 * 32 + 16) = make_uint4(o[4], o[5], o[6], o[7]);
               }
             }
           }
         }
       } else {
         if (in_range) {
-#pragma unroll
-          for (int c = 0; c < D / 8; ++c) *reinterpret_cast<uint4*>(orow + c * 16) = make_uint4(0, 0, 0, 0);
+          for (int c = 0; c < p.d / 8; ++c) *reinterpret_cast<uint4*>(orow + c * 16) = make_uint4(0, 0, 0, 0);
         }
       }
     }
@@ -875,13 +877,21 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 512);
   }
+  if (tid == 0) {  // the last CTA leaves the launch's counters as it found them (no memset node between launches)
+    __threadfence();
+    if (atomicAdd(p.sched + 1, 1u) == gridDim.x - 1) {
+      p.sched[0] = 0u;
+      p.sched[1] = 0u;
+      __threadfence();
+    }
+  }
 }
 
-// Item counters of the persistent forward: a ring of words in device memory that is part of the library image, one
-// word per launch (zeroed on the launch's stream just before it). Launches only share a word when more than
-// kSchedSlots of them are in flight on one device at the same time.
+// Item counters of the persistent forward: a ring of word pairs in device memory that is part of the library image, one
+// pair per launch, zero at load time and left at zero by the last CTA of every launch. Launches only share a pair when
+// more than kSchedSlots of them are in flight on one device at the same time.
 constexpr int kSchedSlots = 256;
-__device__ unsigned g_fwd_sched[kSchedSlots];
+__device__ unsigned g_fwd_sched[2 * kSchedSlots];
 
 unsigned* next_sched_slot() {
   static std::mutex mu;
@@ -895,7 +905,7 @@ unsigned* next_sched_slot() {
     if (cudaGetSymbolAddress(&ptr, g_fwd_sched) != cudaSuccess) return nullptr;
     base[dev] = static_cast<unsigned*>(ptr);
   }
-  return base[dev] + (next[dev]++ % kSchedSlots);
+  return base[dev] + 2 * (next[dev]++ % kSchedSlots);
 }
 
 struct FwdPlan {
@@ -953,7 +963,7 @@ int launch(const fdma_fwd_params& p, const FwdPlan& pl, cudaStream_t stream) {
   kp.mask_row_stride = p.mask_row_stride;
   kp.bias_batch_stride = p.bias_batch_stride; kp.bias_head_stride = p.bias_head_stride;
   kp.bias_row_stride = p.bias_row_stride;
-  kp.b = p.b; kp.seqlen_q = p.seqlen_q; kp.seqlen_k = p.seqlen_k; kp.h = p.h; kp.h_k = p.h_k;
+  kp.b = p.b; kp.seqlen_q = p.seqlen_q; kp.seqlen_k = p.seqlen_k; kp.h = p.h; kp.h_k = p.h_k; kp.d = p.d;
   kp.h_mask = p.h_mask; kp.h_bias = p.h_bias;
   kp.is_causal = p.is_causal;
   kp.key_pos = p.key_pos;
@@ -982,8 +992,6 @@ int launch(const fdma_fwd_params& p, const FwdPlan& pl, cudaStream_t stream) {
   dim3 grid(static_cast<unsigned>(std::min<int64_t>(n_items, sm_count())));  // persistent CTAs, one per SM
   kp.sched = next_sched_slot();
   if (!kp.sched) return FDMA_ERR_DRIVER;
-  e = cudaMemsetAsync(kp.sched, 0, sizeof(unsigned), stream);
-  if (e != cudaSuccess) return static_cast<int>(e);
   cudaEvent_t ev0, ev1;
   take_timing_events(&ev0, &ev1);
   if (ev0) cudaEventRecord(ev0, stream);
@@ -1015,7 +1023,7 @@ int launch_tile_activity(const fdma_fwd_params& p, uint8_t* act, cudaStream_t st
 }
 
 bool tc_fwd_supported(const fdma_fwd_params& p) {
-  if (p.d != 64 && p.d != 128 && p.d != 256) return false;
+  if (p.d <= 0 || p.d > 256 || p.d % 8) return false;  // rows are 16-byte multiples for TMA
   if (p.seqlen_k <= 0 || p.seqlen_k > kMaxTiles * kBN) return false;
   if (p.h > 65535 || p.b > 65535) return false;
   // TMA: 16-byte aligned bases and strides
@@ -1056,9 +1064,11 @@ size_t tc_fwd_workspace_bytes(const fdma_fwd_params& p) { return plan(p).act_byt
 
 int tc_fwd(const fdma_fwd_params& p, cudaStream_t stream) {
   const FwdPlan pl = plan(p);
-  if (p.d == 64) return launch_d<64>(p, pl, stream);
-  if (p.d == 256) return launch_d<256>(p, pl, stream);
-  return launch_d<128>(p, pl, stream);
+  switch (tile_head_dim(p.d)) {
+    case 64: return launch_d<64>(p, pl, stream);
+    case 128: return launch_d<128>(p, pl, stream);
+    default: return launch_d<256>(p, pl, stream);
+  }
 }
 
 }  // namespace fdma

@@ -34,6 +34,52 @@ bool tc_bwd_supported(const fdma_bwd_params& p);
 size_t tc_bwd_workspace_bytes(const fdma_bwd_params& p);
 int tc_bwd(const fdma_bwd_params& p, cudaStream_t stream);
 
+// ---- the kernels before and after every tensor-core backward (fdma_bwd_common.cu) ---------------
+constexpr int kDetFracBits = 40;  // deterministic dQ accumulator: fixed point, |dQ / scale| < 2^23, resolution 2^-40
+
+// Head dim the tensor-core kernels run a call at: tiles are 64, 128 or 256 wide; the columns beyond d are zeros that
+// the TMA loads fill in, so no tensor is ever padded in memory.
+inline int tile_head_dim(int d) { return d <= 64 ? 64 : d <= 128 ? 128 : 256; }
+
+struct BwdPrepArgs {
+  const void *out, *dout;
+  const float* lse;
+  float *lse2, *dsum;  // (B,H,sq_r)
+  void* dq_acc;        // zeroed: (B,H,D/min(D,128),Sq,min(D,128)) elements of acc_bytes
+  int b, h, sq, sq_r, d, acc_bytes;
+  int64_t o_sb, o_sr, o_sh, do_sb, do_sr, do_sh;
+};
+int launch_bwd_prep(const BwdPrepArgs& a, int D, bool bf16, cudaStream_t stream);
+
+struct BwdFinishArgs {
+  // dQ
+  const void* dq_acc;
+  void* dq;
+  const float* dsum;  // deterministic mode: rows with a non-finite D become NaN
+  int64_t dq_sb, dq_sr, dq_sh;
+  float scale;
+  int b, h, sq, sq_r, d, D;
+  // dK, dV: fp32 partials [2: dV, dK][nsplit][B][h_k][keys_r][D], or part = null (already written by the main kernel)
+  const float* part;
+  int64_t split_stride;
+  int nsplit, h_k, keys_r;
+  void *dk, *dv;
+  int64_t dk_sb, dk_sr, dk_sh, dv_sb, dv_sr, dv_sh;
+  int rows_out;  // key rows of dk / dv
+  // gathered keys: ascending positions ({B|1}, {h_k|1}, cap) of the partials' rows; null: row = key
+  const int32_t* pos;
+  int64_t pos_sb, pos_sh;
+  int h_pos, cap;
+  // row-broadcast dBias: fp32 sums [db_nsplit][db_b * db_h][db_pitch], or db_part = null
+  const float* db_part;
+  int64_t db_split_stride;
+  int db_nsplit, db_pitch, db_b, db_h, db_keys;
+  void* dbias;
+  int64_t db_sb, db_sh;
+  int kv_blocks, db_blocks;  // set by the launcher
+};
+int launch_bwd_finish(BwdFinishArgs a, bool bf16, bool deterministic, cudaStream_t stream);
+
 // ---- single-query (decode) forward: row-granular skipping, split over keys + merge -------------
 bool decode_supported(const fdma_fwd_params& p);
 size_t decode_workspace_bytes(const fdma_fwd_params& p);

@@ -183,6 +183,20 @@ __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gmem_sr
                : "memory");
 }
 
+// Bulk reduce-add shared -> global (16-byte aligned addresses, size a multiple of 16 bytes); the caller commits the group.
+__device__ __forceinline__ void bulk_reduce_add_f32(float* gmem_dst, const void* smem_src, uint32_t bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;"
+               :
+               : "l"(reinterpret_cast<uint64_t>(gmem_dst)), "r"(smem_u32(smem_src)), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_reduce_add_u64(long long* gmem_dst, const void* smem_src, uint32_t bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.u64 [%0], [%1], %2;"
+               :
+               : "l"(reinterpret_cast<uint64_t>(gmem_dst)), "r"(smem_u32(smem_src)), "r"(bytes)
+               : "memory");
+}
+
 // ---------------------------------------------------------------------------------------------
 // TMEM allocation (one warp executes these, all 32 lanes converged)
 // ---------------------------------------------------------------------------------------------

@@ -39,6 +39,8 @@ class BwdParams(Structure):
         + [(f"dbias_{s}_stride", c_int64) for s in ("batch", "head", "row")]
         + [(n, c_int32) for n in ("dbias_b", "dbias_h", "dbias_rows", "dbias_keys", "deterministic", "reserved")]
         + [("softmax_d", c_void_p)]
+        + [("scatter_pos", c_void_p), ("scatter_batch_stride", c_int64), ("scatter_head_stride", c_int64)]
+        + [("scatter_h", c_int32), ("scatter_rows", c_int32)]
     )
 
 
@@ -71,6 +73,7 @@ EXPORTED_SYMBOLS = (
     "fdma_static_scratch_limit",
     "fdma_compact_index",
     "fdma_gather_rows",
+    "fdma_gather_kept",
     "fdma_scatter_rows",
     "fdma_merge_partials",
 )
@@ -98,6 +101,18 @@ class RowsParams(ctypes.Structure):
         ("b", c_int32), ("heads", c_int32), ("h_pos", c_int32), ("rows_full", c_int32),
         ("capacity", c_int32), ("row_elems", c_int32), ("dtype", c_int32), ("reserved_", c_int32),
     ]
+
+
+class KeptParams(ctypes.Structure):
+    """fdma_kept_params of include/fdma.h."""
+
+    _fields_ = (
+        [(n, c_void_p) for n in ("k", "v", "bias", "k_c", "v_c", "bias_c", "key_pos")]
+        + [("key_pos_batch_stride", c_int64), ("key_pos_head_stride", c_int64)]
+        + [(f"{t}_{s}_stride", c_int64) for t in ("k", "v") for s in ("batch", "row", "head")]
+        + [(f"bias_{s}_stride", c_int64) for s in ("batch", "head", "key")]
+        + [(n, c_int32) for n in ("b", "h_k", "h_pos", "seqlen_k", "capacity", "d", "bias_b", "bias_h", "dtype", "reserved")]
+    )
 
 
 class MergeParams(ctypes.Structure):
@@ -150,6 +165,8 @@ def load():
     lib.fdma_compact_index.argtypes = [POINTER(CompactParams), c_void_p]
     lib.fdma_gather_rows.restype = c_int
     lib.fdma_gather_rows.argtypes = [POINTER(RowsParams), c_void_p]
+    lib.fdma_gather_kept.restype = c_int
+    lib.fdma_gather_kept.argtypes = [POINTER(KeptParams), c_void_p]
     lib.fdma_scatter_rows.restype = c_int
     lib.fdma_scatter_rows.argtypes = [POINTER(RowsParams), c_void_p]
     lib.fdma_merge_partials.restype = c_int

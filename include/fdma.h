@@ -43,7 +43,7 @@ enum fdma_status {
 };
 
 /* Which kernel family the launcher picks. AUTO: the row-gather decode kernel for single-query calls
- * (seqlen_q == 1, head dim 64/128/256), tcgen05/TMA kernels where shape and alignment allow, the
+ * (seqlen_q == 1, head dim 64/128/256), tcgen05/TMA kernels (any head dim that is a multiple of 8) where shape and alignment allow, the
  * CUDA-core kernels otherwise. The other values force one family (tests use them); forcing a family
  * on a shape it does not handle returns FDMA_ERR_UNSUPPORTED. */
 enum fdma_path { FDMA_PATH_AUTO = 0, FDMA_PATH_SIMT = 1, FDMA_PATH_TCGEN05 = 2, FDMA_PATH_DECODE = 3 };
@@ -143,6 +143,15 @@ typedef struct fdma_bwd_params {
   float* softmax_d; /* optional out, may be NULL: D = rowsum(dOut o Out) as fp32 (B, H, round_up(Sq,128)) contiguous,
                        zeros in the padding columns -- the `softmax_d` tensor mha_bwd returns (flash_api.cpp:952,
                        :1049) */
+  /* Optional, for K / V that were gathered to the kept keys (fdma_gather_kept): the ascending positions
+   * ({B|1}, scatter_h in {1, h_k}, seqlen_k) int32 of the gathered rows among scatter_rows key rows. dk, dv are then
+   * (B, scatter_rows, h_k, d) and dbias (dbias_b, dbias_h, 1, dbias_keys >= scatter_rows): every gathered row's
+   * gradient is written to its position and every other row is zero. Row-broadcast bias only; a per-head position list
+   * needs dbias_h to be a multiple of scatter_h, a per-batch one dbias_b == B. NULL: gradients of k, v, bias as given. */
+  const int32_t* scatter_pos;
+  int64_t scatter_batch_stride, scatter_head_stride;
+  int32_t scatter_h;
+  int32_t scatter_rows;
 } fdma_bwd_params;
 
 size_t fdma_bwd_workspace_bytes(const fdma_bwd_params* p);
@@ -294,6 +303,26 @@ typedef struct fdma_rows_params {
   int32_t reserved_;
 } fdma_rows_params;
 int fdma_gather_rows(const fdma_rows_params* p, void* stream);
+/*
+ * fdma_gather_kept: the kept rows of K, V and (optionally) a row-broadcast bias in one launch: k_c, v_c
+ * (b, capacity, h_k, d) and bias_c (bias_b, bias_h, 1, capacity), all dense, zeros in slots whose position is outside
+ * [0, seqlen_k). Positions ({b|1}, h_pos in {1, h_k}, capacity), batch stride 0 for a shared list; bias strides in
+ * elements, 0 where it is broadcast; bias_h a multiple of h_pos, bias_b == b when the list has a batch stride. The
+ * gradients go back with fdma_bwd_params::scatter_pos.
+ */
+typedef struct fdma_kept_params {
+  const void *k, *v, *bias; /* bias may be NULL */
+  void *k_c, *v_c, *bias_c;
+  const int32_t* key_pos;
+  int64_t key_pos_batch_stride, key_pos_head_stride;
+  int64_t k_batch_stride, k_row_stride, k_head_stride;
+  int64_t v_batch_stride, v_row_stride, v_head_stride;
+  int64_t bias_batch_stride, bias_head_stride, bias_key_stride;
+  int32_t b, h_k, h_pos, seqlen_k, capacity, d, bias_b, bias_h;
+  int32_t dtype;            /* FDMA_BF16 or FDMA_FP16 */
+  int32_t reserved;
+} fdma_kept_params;
+int fdma_gather_kept(const fdma_kept_params* p, void* stream);
 int fdma_scatter_rows(const fdma_rows_params* p, void* stream);
 
 /*
