@@ -1,0 +1,588 @@
+// Native host path of the operator layer: what flash_sparse_attn_func and create_mask do between the Python call and the
+// kernel launches -- checks, route choice, allocation, the autograd node -- in C++ on top of the C ABI of
+// libfdma_sm100.so (include/fdma.h), which is opened at run time.
+//
+// Why: a training call at S = 256 spends 0.05 ms on the GPU and spent 0.6 ms in Python (custom-op dispatch, ctypes
+// structures field by field, one allocation call per tensor). Every function here returns an empty result for inputs it
+// does not handle (wrong types, odd layouts, tracing); the Python layer then runs its own path, which also raises the
+// argument errors.
+#include <ATen/ATen.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <dlfcn.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <algorithm>
+#include <optional>
+#include <stdexcept>
+#include <string>
+#include <vector>
+
+#include "../../include/fdma.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+namespace {
+
+struct Api {
+  decltype(&fdma_fwd_workspace_bytes) fwd_workspace_bytes;
+  decltype(&fdma_fwd) fwd;
+  decltype(&fdma_bwd_workspace_bytes) bwd_workspace_bytes;
+  decltype(&fdma_bwd) bwd;
+  decltype(&fdma_create_mask) create_mask;
+  decltype(&fdma_gather_kept) gather_kept;
+  decltype(&fdma_strerror) strerror;
+  decltype(&fdma_poll_kernel_status) poll_kernel_status;
+  decltype(&fdma_last_kernel_status) last_kernel_status;
+} api;
+
+void init(const std::string& path) {
+  void* h = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
+  if (!h) throw std::runtime_error(std::string("cannot open ") + path + ": " + dlerror());
+  auto get = [&](auto& fn, const char* name) {
+    fn = reinterpret_cast<std::remove_reference_t<decltype(fn)>>(dlsym(h, name));
+    if (!fn) throw std::runtime_error(path + " does not export " + name);
+  };
+  get(api.fwd_workspace_bytes, "fdma_fwd_workspace_bytes");
+  get(api.fwd, "fdma_fwd");
+  get(api.bwd_workspace_bytes, "fdma_bwd_workspace_bytes");
+  get(api.bwd, "fdma_bwd");
+  get(api.create_mask, "fdma_create_mask");
+  get(api.gather_kept, "fdma_gather_kept");
+  get(api.strerror, "fdma_strerror");
+  get(api.poll_kernel_status, "fdma_poll_kernel_status");
+  get(api.last_kernel_status, "fdma_last_kernel_status");
+}
+
+constexpr int64_t kTile = 128;
+int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
+
+void check(int status, const char* what) {
+  if (status != 0)
+    throw std::runtime_error(std::string(what) + " failed: " + api.strerror(status) + " (status " + std::to_string(status) + ")");
+}
+
+cudaStream_t stream_of(const Tensor& t) { return at::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+
+// A kernel whose bounded wait gave up surfaces at the next operator call (one host load, no GPU work).
+void raise_if_timed_out(cudaStream_t stream) {
+  if (api.poll_kernel_status(nullptr) == 0) return;
+  int32_t detail = 0;
+  api.last_kernel_status(stream, &detail);
+  throw std::runtime_error("an earlier attention kernel on this device gave up a bounded wait (code " + std::to_string(detail) +
+                           "): " + api.strerror(FDMA_ERR_TIMEOUT) + "; results of calls since then are not valid");
+}
+
+Tensor empty(at::IntArrayRef sizes, at::ScalarType type, const Tensor& like) {
+  return at::detail::empty_cuda(sizes, type, like.device(), std::nullopt);
+}
+Tensor empty_as(const Tensor& t) {
+  return t.is_contiguous() ? empty(t.sizes(), t.scalar_type(), t) : at::empty_like(t);
+}
+Tensor inner_contiguous(const Tensor& t) { return t.stride(-1) == 1 ? t : t.contiguous(); }
+const Tensor& get(const OptTensor& t) {
+  static const Tensor none;
+  return t.has_value() ? *t : none;
+}
+
+int dtype_code(const Tensor& t) {
+  switch (t.scalar_type()) {
+    case at::kBFloat16: return FDMA_BF16;
+    case at::kHalf: return FDMA_FP16;
+    case at::kFloat: return FDMA_FP32;
+    default: return -1;
+  }
+}
+
+struct Bsh {
+  int64_t b, r, h;
+};
+// (batch, row, head) element strides of a (B, S, H, d) tensor; dimensions of extent 1 get a dense stride
+Bsh bsh(const Tensor& t) {
+  Bsh s{t.stride(0), t.stride(1), t.stride(2)};
+  if (t.size(2) == 1) s.h = t.size(3);
+  if (t.size(1) == 1 && s.h == t.size(3)) s.r = t.size(2) * t.size(3);
+  if (t.size(0) == 1) s.b = std::max<int64_t>(s.b, 1);
+  return s;
+}
+int64_t bcast_stride(const Tensor& t, int dim) { return t.size(dim) == 1 ? 0 : t.stride(dim); }
+
+// Everything one attention call needs besides q, k, v: the same struct serves the forward call and the autograd node.
+struct Call {
+  float scale = 0.f;
+  bool causal = false, deterministic = false, bits = false, gathered = false;
+  int path = FDMA_PATH_AUTO;
+  int64_t seqlen_k = 0;      // keys of the caller's K
+  int64_t bias_keys = 0;     // key extent of the caller's bias
+  std::vector<int64_t> bias_c;  // gathered: shape of the gathered bias (empty: no bias)
+};
+
+// Gathered K, V and bias live in one buffer: [K_c | V_c | bias_c], each 256-byte aligned.
+struct KvB {
+  void *k, *v, *bias;
+};
+KvB split_kvb(const Tensor& buf, int64_t kv_elems, bool has_bias) {
+  char* p = static_cast<char*>(buf.data_ptr());
+  const int64_t step = round_up(kv_elems * 2, 256);
+  return {p, p + step, has_bias ? p + 2 * step : nullptr};
+}
+
+void fill_geometry(fdma_fwd_params& p, const Tensor& q, int64_t seqlen_k, int64_t h_k, const Call& c) {
+  p.q = q.data_ptr();
+  const Bsh sq = bsh(q);
+  p.q_batch_stride = sq.b; p.q_row_stride = sq.r; p.q_head_stride = sq.h;
+  p.b = static_cast<int32_t>(q.size(0));
+  p.seqlen_q = static_cast<int32_t>(q.size(1));
+  p.seqlen_k = static_cast<int32_t>(seqlen_k);
+  p.h = static_cast<int32_t>(q.size(2));
+  p.h_k = static_cast<int32_t>(h_k);
+  p.h_mask = p.h_bias = 1;
+  p.d = static_cast<int32_t>(q.size(3));
+  p.dtype = dtype_code(q);
+  p.is_causal = c.causal ? 1 : 0;
+  p.softmax_scale = c.scale;
+  p.path = c.path;
+}
+void fill_kv(fdma_fwd_params& p, const Tensor& k, const Tensor& v) {
+  const Bsh sk = bsh(k), sv = bsh(v);
+  p.k = k.data_ptr(); p.v = v.data_ptr();
+  p.k_batch_stride = sk.b; p.k_row_stride = sk.r; p.k_head_stride = sk.h;
+  p.v_batch_stride = sv.b; p.v_row_stride = sv.r; p.v_head_stride = sv.h;
+}
+void fill_out(fdma_fwd_params& p, const Tensor& out, const Tensor& lse) {
+  const Bsh so = bsh(out);
+  p.out = out.data_ptr(); p.lse = lse.data_ptr<float>();
+  p.o_batch_stride = so.b; p.o_row_stride = so.r; p.o_head_stride = so.h;
+}
+void fill_mask_bias(fdma_fwd_params& p, const Tensor& mask, const Tensor& bias, const Tensor& activity, const Call& c) {
+  if (mask.defined()) {
+    p.mask = mask.data_ptr();
+    p.h_mask = static_cast<int32_t>(mask.size(1));
+    if (c.bits) {
+      p.mask_bits = 1;
+      p.mask_batch_stride = mask.stride(0);
+      p.mask_head_stride = bcast_stride(mask, 1);
+      p.mask_row_stride = mask.stride(2);
+      p.tile_activity = static_cast<const uint8_t*>(activity.data_ptr());
+    } else {
+      p.mask_batch_stride = bcast_stride(mask, 0);
+      p.mask_head_stride = bcast_stride(mask, 1);
+      p.mask_row_stride = bcast_stride(mask, 2);
+    }
+  }
+  if (bias.defined()) {
+    p.bias = bias.data_ptr();
+    p.h_bias = static_cast<int32_t>(bias.size(1));
+    p.bias_batch_stride = bcast_stride(bias, 0);
+    p.bias_head_stride = bcast_stride(bias, 1);
+    p.bias_row_stride = bcast_stride(bias, 2);
+  }
+}
+// gathered keys: dense (B, cap, Hk, d) rows and their positions
+void fill_gathered(fdma_fwd_params& p, const KvB& kv, const Tensor& key_pos, const Tensor& slot_mask, const Call& c) {
+  const int64_t cap = key_pos.size(2), hk = p.h_k, d = p.d;
+  p.k = kv.k; p.v = kv.v;
+  p.k_batch_stride = p.v_batch_stride = cap * hk * d;
+  p.k_row_stride = p.v_row_stride = hk * d;
+  p.k_head_stride = p.v_head_stride = d;
+  p.mask = slot_mask.data_ptr();
+  p.h_mask = static_cast<int32_t>(slot_mask.size(1));
+  p.mask_batch_stride = bcast_stride(slot_mask, 0);
+  p.mask_head_stride = bcast_stride(slot_mask, 1);
+  p.mask_row_stride = 0;
+  if (!c.bias_c.empty()) {
+    p.bias = kv.bias;
+    p.h_bias = static_cast<int32_t>(c.bias_c[1]);
+    p.bias_batch_stride = c.bias_c[0] == 1 ? 0 : c.bias_c[1] * cap;
+    p.bias_head_stride = c.bias_c[1] == 1 ? 0 : cap;
+    p.bias_row_stride = 0;
+  }
+  p.key_pos = key_pos.data_ptr<int32_t>();
+  p.key_pos_batch_stride = bcast_stride(key_pos, 0);
+  p.key_pos_head_stride = key_pos.stride(1);
+  p.h_pos = static_cast<int32_t>(key_pos.size(1));
+  p.causal_shift = static_cast<int32_t>(c.seqlen_k - p.seqlen_q);
+}
+
+// ---- backward --------------------------------------------------------------------------------------------------
+// One node for the three routes. Saved: dense   q, k, v, mask, bias, out, lse
+//                                       bits    q, k, v, bits, bias, out, lse, activity
+//                                       gathered q, kvb, -, slot_mask, -, out, lse, key_pos
+struct AttnBackward : public torch::autograd::Node {
+  Call c;
+  SavedVariable q, k, v, mask, bias, out, lse, extra;
+  at::SmallVector<int64_t, 4> k_sizes, v_like;
+  bool want_bias = false;
+  std::vector<int64_t> bias_sizes;
+
+  std::string name() const override { return "FlashSparseAttnBackward"; }
+  void release_variables() override {
+    for (SavedVariable* s : {&q, &k, &v, &mask, &bias, &out, &lse, &extra}) s->reset_data();
+  }
+  variable_list apply(variable_list&& grads) override;
+};
+
+variable_list AttnBackward::apply(variable_list&& grads) {
+  variable_list res(4);
+  if (!grads[0].defined()) return res;
+  at::AutoDispatchBelowADInplaceOrView guard;
+  const Tensor tq = q.unpack(), tk = k.unpack(), tmask = mask.unpack(), tlse = lse.unpack(), textra = extra.unpack();
+  const Tensor tout = out.unpack(getptr());
+  const c10::cuda::CUDAGuard device(tq.device());
+  const cudaStream_t stream = stream_of(tq);
+  raise_if_timed_out(stream);
+  const Tensor dout = inner_contiguous(grads[0]);
+
+  fdma_bwd_params bp = {};
+  Tensor dq = empty_as(tq), dk, dv, dbias;
+  if (c.gathered) {
+    dk = empty(k_sizes, tq.scalar_type(), tq);
+    dv = empty(k_sizes, tq.scalar_type(), tq);
+    const int64_t cap = textra.size(2), hk = k_sizes[2], d = tq.size(3);
+    fill_geometry(bp.f, tq, cap, hk, c);
+    fill_gathered(bp.f, split_kvb(tk, tq.size(0) * cap * hk * d, !c.bias_c.empty()), textra, tmask, c);
+    bp.scatter_pos = textra.data_ptr<int32_t>();
+    bp.scatter_batch_stride = bp.f.key_pos_batch_stride;
+    bp.scatter_head_stride = bp.f.key_pos_head_stride;
+    bp.scatter_h = bp.f.h_pos;
+    bp.scatter_rows = static_cast<int32_t>(c.seqlen_k);
+    if (want_bias) dbias = empty(bias_sizes, tq.scalar_type(), tq);
+  } else {
+    const Tensor tv = v.unpack(), tbias = bias.unpack();
+    dk = empty_as(tk);
+    dv = empty_as(tv);
+    fill_geometry(bp.f, tq, tk.size(1), tk.size(2), c);
+    fill_kv(bp.f, tk, tv);
+    fill_mask_bias(bp.f, tmask, tbias, textra, c);
+    if (want_bias) dbias = empty(tbias.sizes(), tbias.scalar_type(), tbias);
+  }
+  fill_out(bp.f, tout, tlse);
+  const Bsh so = bsh(dout), sq = bsh(dq), sk = bsh(dk), sv = bsh(dv);
+  bp.dout = dout.data_ptr();
+  bp.do_batch_stride = so.b; bp.do_row_stride = so.r; bp.do_head_stride = so.h;
+  bp.dq = dq.data_ptr(); bp.dk = dk.data_ptr(); bp.dv = dv.data_ptr();
+  bp.dq_batch_stride = sq.b; bp.dq_row_stride = sq.r; bp.dq_head_stride = sq.h;
+  bp.dk_batch_stride = sk.b; bp.dk_row_stride = sk.r; bp.dk_head_stride = sk.h;
+  bp.dv_batch_stride = sv.b; bp.dv_row_stride = sv.r; bp.dv_head_stride = sv.h;
+  if (dbias.defined()) {
+    bp.dbias = dbias.data_ptr();
+    bp.dbias_batch_stride = dbias.stride(0); bp.dbias_head_stride = dbias.stride(1); bp.dbias_row_stride = dbias.stride(2);
+    bp.dbias_b = static_cast<int32_t>(dbias.size(0));
+    bp.dbias_h = static_cast<int32_t>(dbias.size(1));
+    bp.dbias_rows = static_cast<int32_t>(dbias.size(2));
+    bp.dbias_keys = static_cast<int32_t>(dbias.size(3));
+  }
+  bp.deterministic = c.deterministic ? 1 : 0;
+  const size_t bytes = api.bwd_workspace_bytes(&bp);
+  Tensor ws;
+  if (bytes) {
+    ws = empty({static_cast<int64_t>(bytes)}, at::kByte, tq);
+    bp.f.workspace = ws.data_ptr();
+    bp.f.workspace_bytes = bytes;
+  }
+  check(api.bwd(&bp, stream), "fdma_bwd");
+  if (dbias.defined() && !c.gathered && c.bias_keys != dbias.size(3)) {
+    dbias = dbias.narrow(3, 0, c.seqlen_k);
+    if (c.bias_keys == 1) dbias = dbias.sum({3}, /*keepdim=*/true);
+  }
+  res[0] = dq; res[1] = dk; res[2] = dv; res[3] = dbias;
+  return res;
+}
+
+// ---- forward ---------------------------------------------------------------------------------------------------
+bool plain(const Tensor& t) { return t.defined() && t.is_cuda() && t.layout() == at::kStrided && t.dim() == 4; }
+
+bool needs_grad(const Tensor& t) { return t.defined() && t.requires_grad(); }
+
+Tensor fit_keys(const Tensor& t, int64_t keys_r) {
+  if (t.size(3) == keys_r) return t;
+  if (t.size(3) == 1) return t.expand({t.size(0), t.size(1), t.size(2), keys_r});
+  return at::constant_pad_nd(t, {0, keys_r - t.size(3)}, 0);
+}
+
+// mask / bias extents the kernels take; anything else goes to the Python path, which raises the right error
+bool broadcastable(const Tensor& t, int64_t B, int64_t H, int64_t Hk, int64_t Sq) {
+  return (t.size(0) == 1 || t.size(0) == B) && (t.size(1) == 1 || t.size(1) == Hk || t.size(1) == H) &&
+         (t.size(2) == 1 || t.size(2) == Sq);
+}
+
+// Runs one attention call; nullopt for inputs this path does not take. Exactly one form of mask is given: a bool tensor,
+// the position list of the kept keys (key_pos, slot_mask), bits with their tile activity, or none.
+std::optional<Tensor> attention(const Tensor& q0, const Tensor& k0, const Tensor& v0, const OptTensor& mask_, const OptTensor& bias_,
+                                const OptTensor& key_pos_, const OptTensor& slot_mask_, const OptTensor& bits_,
+                                const OptTensor& activity_, double scale, bool causal, bool deterministic, int path) {
+  const Tensor &mask0 = get(mask_), &bias0 = get(bias_), &key_pos = get(key_pos_), &slot_mask = get(slot_mask_),
+               &bits = get(bits_), &activity = get(activity_);
+  if (!plain(q0) || !plain(k0) || !plain(v0)) return std::nullopt;
+  const auto type = q0.scalar_type();
+  if ((type != at::kBFloat16 && type != at::kHalf) || k0.scalar_type() != type || v0.scalar_type() != type) return std::nullopt;
+  const int64_t B = q0.size(0), Sq = q0.size(1), H = q0.size(2), d = q0.size(3), Sk = k0.size(1), Hk = k0.size(2);
+  if (B <= 0 || Sq <= 0 || Sk <= 0 || H <= 0 || Hk <= 0 || H % Hk || d % 8 || d <= 0 || d > 256) return std::nullopt;
+  if (k0.size(0) != B || k0.size(3) != d || v0.sizes() != k0.sizes()) return std::nullopt;
+  if (k0.device() != q0.device() || v0.device() != q0.device()) return std::nullopt;
+  if (bias0.defined() && (!plain(bias0) || bias0.scalar_type() != type || bias0.device() != q0.device() ||
+                          !broadcastable(bias0, B, H, Hk, Sq)))
+    return std::nullopt;
+  const int64_t Sk_r = round_up(Sk, kTile);
+
+  Call c;
+  c.scale = static_cast<float>(scale);
+  c.causal = causal;
+  c.deterministic = deterministic;
+  c.path = path;
+  c.seqlen_k = Sk;
+  c.bias_keys = bias0.defined() ? bias0.size(3) : 0;
+  if (key_pos.defined()) {
+    c.gathered = true;
+    const int64_t Bm = key_pos.size(0), Hm = key_pos.size(1), cap = key_pos.size(2);
+    if (Sq <= 1 || (Bm != 1 && Bm != B) || (Hm != 1 && Hm != Hk) || cap % kTile || !key_pos.is_contiguous() ||
+        !slot_mask.is_contiguous() || slot_mask.numel() != key_pos.numel())
+      return std::nullopt;
+    if (k0.stride(3) != 1 || v0.stride(3) != 1) return std::nullopt;
+    for (int i = 0; i < 3; ++i)
+      if (k0.stride(i) % 8 || v0.stride(i) % 8) return std::nullopt;
+    if ((reinterpret_cast<uintptr_t>(k0.data_ptr()) | reinterpret_cast<uintptr_t>(v0.data_ptr())) & 15) return std::nullopt;
+    if (bias0.defined()) {
+      // the gathered bias has the bias' own extents: the list must not vary along a dimension the bias is shared over
+      if (bias0.size(2) != 1 || bias0.size(3) < Sk || bias0.size(3) == 1) return std::nullopt;
+      if ((Bm > 1 && bias0.size(0) != B) || bias0.size(1) % Hm) return std::nullopt;
+      if (d > 128 && H != Hk && bias0.size(1) == H) return std::nullopt;  // gradients of such a bias: CUDA-core kernels
+      if (d > 128 && (bias0.size(0) != B || bias0.size(1) != Hk)) return std::nullopt;
+      c.bias_c = {bias0.size(0), bias0.size(1), 1, cap};
+    }
+  } else if (bits.defined()) {
+    c.bits = true;
+    if (d > 128 || Sq == 1 || bits.size(0) != B || bits.size(2) != Sq || bits.size(3) != Sk_r / 32) return std::nullopt;
+    if (bits.size(1) != 1 && bits.size(1) != Hk && bits.size(1) != H) return std::nullopt;
+    if (!bits.is_contiguous() || !activity.is_contiguous()) return std::nullopt;
+  } else if (mask0.defined()) {
+    if (!plain(mask0) || mask0.scalar_type() != at::kBool || mask0.device() != q0.device() ||
+        !broadcastable(mask0, B, H, Hk, Sq) || (mask0.size(3) != 1 && mask0.size(3) != Sk && mask0.size(3) != Sk_r))
+      return std::nullopt;
+  }
+  if (!c.gathered && bias0.defined() && bias0.size(3) != 1 && bias0.size(3) != Sk && bias0.size(3) != Sk_r) return std::nullopt;
+
+  const bool grad = at::GradMode::is_enabled() && (needs_grad(q0) || needs_grad(k0) || needs_grad(v0) || needs_grad(bias0));
+  Tensor out, lse, q, k, v, mask, bias, kvb;
+  {
+    at::AutoDispatchBelowADInplaceOrView guard;
+    const c10::cuda::CUDAGuard device(q0.device());
+    const cudaStream_t stream = stream_of(q0);
+    raise_if_timed_out(stream);
+    q = inner_contiguous(q0);
+    out = empty_as(q);
+    lse = empty({B, H, Sq}, at::kFloat, q);
+    fdma_fwd_params p = {};
+    if (c.gathered) {
+      const int64_t cap = key_pos.size(2), kv_elems = B * cap * Hk * d;
+      const bool has_bias = bias0.defined();
+      const int64_t bytes = 2 * round_up(kv_elems * 2, 256) + (has_bias ? c.bias_c[0] * c.bias_c[1] * cap * 2 : 0);
+      kvb = empty({bytes}, at::kByte, q);
+      const KvB kv = split_kvb(kvb, kv_elems, has_bias);
+      fdma_kept_params g = {};
+      const Bsh sk = bsh(k0), sv = bsh(v0);
+      g.k = k0.data_ptr(); g.v = v0.data_ptr();
+      g.k_c = kv.k; g.v_c = kv.v;
+      g.k_batch_stride = sk.b; g.k_row_stride = sk.r; g.k_head_stride = sk.h;
+      g.v_batch_stride = sv.b; g.v_row_stride = sv.r; g.v_head_stride = sv.h;
+      if (B == 1) g.k_batch_stride = g.v_batch_stride = 0;
+      g.key_pos = key_pos.data_ptr<int32_t>();
+      g.key_pos_batch_stride = bcast_stride(key_pos, 0);
+      g.key_pos_head_stride = key_pos.stride(1);
+      g.b = static_cast<int32_t>(B); g.h_k = static_cast<int32_t>(Hk); g.h_pos = static_cast<int32_t>(key_pos.size(1));
+      g.seqlen_k = static_cast<int32_t>(Sk); g.capacity = static_cast<int32_t>(cap); g.d = static_cast<int32_t>(d);
+      g.dtype = dtype_code(q);
+      if (has_bias) {
+        g.bias = bias0.data_ptr(); g.bias_c = kv.bias;
+        g.bias_batch_stride = bcast_stride(bias0, 0); g.bias_head_stride = bcast_stride(bias0, 1);
+        g.bias_key_stride = bias0.stride(3);
+        g.bias_b = static_cast<int32_t>(c.bias_c[0]); g.bias_h = static_cast<int32_t>(c.bias_c[1]);
+      }
+      check(api.gather_kept(&g, stream), "fdma_gather_kept");
+      fill_geometry(p, q, cap, Hk, c);
+      fill_gathered(p, kv, key_pos, slot_mask, c);
+    } else {
+      k = inner_contiguous(k0);
+      v = inner_contiguous(v0);
+      if (c.bits) mask = bits;
+      else if (mask0.defined()) mask = inner_contiguous(fit_keys(mask0, Sk_r));
+      if (bias0.defined()) bias = inner_contiguous(fit_keys(bias0, Sk_r));
+      fill_geometry(p, q, Sk, Hk, c);
+      fill_kv(p, k, v);
+      fill_mask_bias(p, mask, bias, activity, c);
+    }
+    fill_out(p, out, lse);
+    const size_t bytes = api.fwd_workspace_bytes(&p);
+    Tensor ws;
+    if (bytes) {
+      ws = empty({static_cast<int64_t>(bytes)}, at::kByte, q);
+      p.workspace = ws.data_ptr();
+      p.workspace_bytes = bytes;
+    }
+    check(api.fwd(&p, stream), "fdma_fwd");
+  }
+  if (grad) {
+    auto node = std::shared_ptr<AttnBackward>(new AttnBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(q0, k0, v0, bias0));
+    torch::autograd::set_history(out, node);
+    node->want_bias = bias0.defined() && (needs_grad(bias0));
+    node->k_sizes.assign(k0.sizes().begin(), k0.sizes().end());
+    if (bias0.defined()) node->bias_sizes = bias0.sizes().vec();
+    // tensors made here are saved as they are; the caller's own go in with their version, so in-place edits are noticed
+    node->q = SavedVariable(q.is_same(q0) ? q0 : q, false);
+    if (c.gathered) {
+      node->k = SavedVariable(kvb, false);
+      node->mask = SavedVariable(slot_mask, false);
+      node->extra = SavedVariable(key_pos, false);
+    } else {
+      node->k = SavedVariable(k, false);
+      node->v = SavedVariable(v, false);
+      if (mask.defined()) node->mask = SavedVariable(mask, false);
+      if (bias.defined()) node->bias = SavedVariable(bias, false);
+      if (activity.defined()) node->extra = SavedVariable(activity, false);
+    }
+    node->out = SavedVariable(out, /*is_output=*/true);
+    node->lse = SavedVariable(lse, false);
+    node->c = std::move(c);
+  }
+  return out;
+}
+
+// ---- create_mask -------------------------------------------------------------------------------------------------
+// Top-k selection: (mask, key_pos, count, slot_mask) for a row-broadcast bias, (mask, bits, activity) for a per-query one
+// where the kernel writes bits, (mask) otherwise. Empty for inputs this path does not take.
+std::vector<Tensor> topk_mask(const Tensor& bias, const OptTensor& premask_, int64_t window, double min_value) {
+  const Tensor& pm = get(premask_);
+  std::vector<Tensor> res;
+  if (!plain(bias) || bias.stride(3) != 1 || dtype_code(bias) < 0) return res;
+  const int64_t keys = bias.size(3);
+  if (window <= 0 || window > keys) return res;
+  int64_t shape[3];
+  for (int i = 0; i < 3; ++i) shape[i] = bias.size(i);
+  if (pm.defined()) {
+    if (!plain(pm) || pm.scalar_type() != at::kBool || pm.device() != bias.device() || pm.stride(3) != 1 || pm.size(3) != keys)
+      return res;
+    for (int i = 0; i < 3; ++i) {
+      if (pm.size(i) != shape[i] && pm.size(i) != 1 && shape[i] != 1) return res;
+      if (pm.size(i) != 1) shape[i] = pm.size(i);
+    }
+  }
+  const int64_t B = shape[0], Hm = shape[1], rows = shape[2];
+  if (B * Hm * rows * keys == 0) return res;
+  at::AutoDispatchBelowADInplaceOrView guard;
+  const c10::cuda::CUDAGuard device(bias.device());
+  const cudaStream_t stream = stream_of(bias);
+  fdma_mask_params p = {};
+  p.bias = bias.data_ptr();
+  p.bias_batch_stride = bcast_stride(bias, 0); p.bias_head_stride = bcast_stride(bias, 1); p.bias_row_stride = bcast_stride(bias, 2);
+  if (pm.defined()) {
+    p.premask = pm.data_ptr();
+    p.pm_batch_stride = bcast_stride(pm, 0); p.pm_head_stride = bcast_stride(pm, 1); p.pm_row_stride = bcast_stride(pm, 2);
+  }
+  p.out_b = static_cast<int32_t>(B); p.out_h = static_cast<int32_t>(Hm); p.out_rows = static_cast<int32_t>(rows);
+  p.keys = static_cast<int32_t>(keys);
+  p.window = static_cast<int32_t>(window);
+  p.dtype = dtype_code(bias);
+  p.kind = FDMA_MASK_TOPK;
+  p.min_value = static_cast<float>(min_value);
+  Tensor mask = empty({B, Hm, rows, keys}, at::kBool, bias);
+  p.out = mask.data_ptr();
+  res.push_back(mask);
+  if (rows == 1) {
+    const int64_t cap = std::max(kTile, round_up(std::min(window, keys), kTile));
+    Tensor key_pos = empty({B, Hm, cap}, at::kInt, bias), count = empty({B, Hm}, at::kInt, bias),
+           slot_mask = empty({B, Hm, 1, cap}, at::kBool, bias);
+    p.key_pos = key_pos.data_ptr<int32_t>();
+    p.count = count.data_ptr<int32_t>();
+    p.slot_mask = slot_mask.data_ptr();
+    p.capacity = static_cast<int32_t>(cap);
+    res.insert(res.end(), {key_pos, count, slot_mask});
+    check(api.create_mask(&p, stream), "fdma_create_mask");
+    return res;
+  }
+  const int64_t keys_r = round_up(keys, kTile);
+  Tensor bits = empty({B, Hm, rows, keys_r / 32}, at::kInt, bias);
+  if (keys != keys_r) bits.zero_();  // the kernel writes the bits of keys [0, keys)
+  Tensor act = empty({B, Hm, (rows + 127) / 128, keys_r / kTile}, at::kByte, bias);
+  p.bits = reinterpret_cast<uint32_t*>(bits.data_ptr<int32_t>());
+  p.activity = static_cast<uint8_t*>(act.data_ptr());
+  int st = api.create_mask(&p, stream);
+  if (st == FDMA_ERR_UNSUPPORTED) {  // rows the bit-writing kernel does not serve: bool mask alone
+    p.bits = nullptr;
+    p.activity = nullptr;
+    st = api.create_mask(&p, stream);
+  } else {
+    res.push_back(bits);
+    res.push_back(act);
+  }
+  check(st, "fdma_create_mask");
+  return res;
+}
+
+// ---- Python -----------------------------------------------------------------------------------------------------
+// Only exact torch.Tensor / Parameter objects and no active dispatch mode (fake tensors, tracing): everything else is the
+// Python path's.
+bool exact(PyObject* o) { return THPVariable_CheckExact(o); }
+bool as_tensor(const py::handle& o, OptTensor& t) {
+  if (o.is_none()) return true;
+  if (!exact(o.ptr())) return false;
+  t = THPVariable_Unpack(o.ptr());
+  return true;
+}
+
+py::object py_attention(py::handle q, py::handle k, py::handle v, py::handle mask, py::handle bias, py::handle key_pos,
+                        py::handle slot_mask, py::handle bits, py::handle activity, py::handle scale, bool causal,
+                        bool deterministic, int path) {
+  OptTensor t[9];
+  const py::handle in[9] = {q, k, v, mask, bias, key_pos, slot_mask, bits, activity};
+  for (int i = 0; i < 9; ++i)
+    if (!as_tensor(in[i], t[i])) return py::none();
+  if (!t[0] || !t[1] || !t[2] || c10::impl::TorchDispatchModeTLS::any_modes_set()) return py::none();
+  double s;
+  if (scale.is_none()) {
+    if (t[0]->dim() != 4) return py::none();
+    s = 1.0 / std::sqrt(static_cast<double>(t[0]->size(3)));
+  } else {
+    s = py::cast<double>(scale);
+  }
+  std::optional<Tensor> out;
+  {
+    py::gil_scoped_release release;
+    out = attention(*t[0], *t[1], *t[2], t[3], t[4], t[5], t[6], t[7], t[8], s, causal, deterministic, path);
+  }
+  if (!out) return py::none();
+  return py::reinterpret_steal<py::object>(THPVariable_Wrap(*out));
+}
+
+py::object py_topk_mask(py::handle bias, py::handle premask, int64_t window, double min_value) {
+  OptTensor b, pm;
+  if (!as_tensor(bias, b) || !as_tensor(premask, pm) || !b || c10::impl::TorchDispatchModeTLS::any_modes_set()) return py::none();
+  std::vector<Tensor> res;
+  {
+    py::gil_scoped_release release;
+    res = topk_mask(*b, pm, window, min_value);
+  }
+  if (res.empty()) return py::none();
+  py::tuple out(res.size());
+  for (size_t i = 0; i < res.size(); ++i) out[i] = py::reinterpret_steal<py::object>(THPVariable_Wrap(res[i]));
+  return out;
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_fdma_torch, m) {
+  m.def("init", &init);
+  m.def("attention", &py_attention);
+  m.def("topk_mask", &py_topk_mask);
+}

@@ -17,7 +17,8 @@ from typing import NamedTuple, Optional, Tuple
 import ctypes
 import torch
 
-from . import _lib
+from . import _lib, _native
+from . import flash_sparse_attn_interface as iface
 from .flash_sparse_attn_interface import (_bsh, _check_inputs, _dtype_code, _fill_fwd, _raise_if_kernel_timed_out,
                                           _stream_ptr, round_multiple)
 
@@ -401,5 +402,10 @@ def flash_sparse_attn_compact_func(
         key_pos, count, slot_mask = torch.ops.flash_sparse_attn._index_kept_keys(m, int(capacity))
         if not trusted and int(count.max().item()) > key_pos.shape[-1]:
             raise RuntimeError(f"a mask row keeps more than capacity={key_pos.shape[-1]} keys")
+    if not torch.compiler.is_compiling() and iface._kernel_path in (_lib.PATH_AUTO, _lib.PATH_TCGEN05):
+        out = _native.load().attention(query, key, value, None, attn_bias, key_pos, slot_mask, None, None, softmax_scale,
+                                       is_causal, bool(deterministic), iface._kernel_path)
+        if out is not None:
+            return out
     return _CompactAttnFunc.apply(query, key, value, attn_bias, key_pos, slot_mask, softmax_scale, is_causal,
                                   bool(deterministic))

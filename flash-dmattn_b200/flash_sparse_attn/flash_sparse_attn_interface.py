@@ -11,7 +11,7 @@ from typing import Any, Optional, Tuple
 import ctypes
 import torch
 
-from . import _lib
+from . import _lib, _native
 
 __all__ = ["flash_sparse_attn_func", "flash_sparse_attn_varlen_func", "FlashDMAttnFunc", "set_kernel_path",
            "set_compaction"]
@@ -101,6 +101,44 @@ def _cached_packed_mask(attn_mask):
     if tag is not None and tag[1] == attn_mask._version and tuple(tag[0].shape) == tuple(attn_mask.shape):
         return tag[0]
     return None
+
+
+def _native_attention(query, key, value, attn_mask, attn_bias, softmax_scale, is_causal, deterministic):
+    """The call through the native host path, or None when that path does not take it: while tracing, with a forced
+    kernel family, for a row-broadcast bool mask whose kept keys are still to be counted, and for whatever
+    csrc/fdma_torch.cpp declines (it checks shapes, types and layouts itself)."""
+    if torch.compiler.is_compiling() or _kernel_path not in (_lib.PATH_AUTO, _lib.PATH_TCGEN05):
+        return None
+    key_pos = slot_mask = bits = activity = None
+    mask = attn_mask
+    if mask is not None:
+        tensor = isinstance(mask, torch.Tensor)
+        kept = packed = None
+        if tensor:
+            if mask.dim() != 4 or key.dim() != 4 or query.dim() != 4:
+                return None
+            tag = getattr(mask, "_fdma_kept", None)
+            if tag is not None and tag[1] == mask._version:
+                kept = tag[0]
+            else:
+                tag = getattr(mask, "_fdma_packed", None)
+                if tag is not None and tag[1] == mask._version and mask.shape[3] == tag[0].seqlen_k:
+                    packed = tag[0]
+        elif hasattr(mask, "key_pos"):
+            kept = mask
+        else:
+            packed = mask
+        if kept is not None and _compaction == "auto" and query.shape[1] > 1 and kept.seqlen_k == key.shape[1]:
+            if 4 * kept.key_pos.shape[-1] <= 3 * round_multiple(kept.seqlen_k, _KEY_PAD):
+                key_pos, slot_mask, mask = kept.key_pos, kept.slot_mask, None
+        elif packed is not None and packed.seqlen_k == key.shape[1] and query.shape[1] > 1 and query.shape[3] <= 128:
+            bits, activity, mask = packed.bits, packed.activity, None
+        elif tensor and kept is None and mask.shape[2] == 1 and query.shape[1] > 1 and _compaction == "auto":
+            return None  # its kept keys are counted first
+        if mask is not None and not tensor:
+            return None
+    return _native.load().attention(query, key, value, mask, attn_bias, key_pos, slot_mask, bits, activity, softmax_scale,
+                                    bool(is_causal), bool(deterministic), _kernel_path)
 
 
 def _raise_if_kernel_timed_out(lib) -> None:
@@ -442,6 +480,10 @@ def flash_sparse_attn_func(
     A row-broadcast mask (one keep-set per batch and kv head) is run over its gathered kept keys, which gives the
     same result in far fewer key tiles when the kept keys are scattered; `set_compaction("off")` disables that.
     """
+    if not softcap and not return_attn_probs:
+        out = _native_attention(query, key, value, attn_mask, attn_bias, softmax_scale, is_causal, deterministic)
+        if out is not None:
+            return out
     from .packed import PackedMask
     from .utils.mask import KeptKeys
 

@@ -9,7 +9,8 @@ from typing import NamedTuple, Optional
 
 import torch
 
-from .. import _lib
+from .. import _lib, _native
+from ..packed import PackedMask
 
 _TILE = 128
 
@@ -68,8 +69,6 @@ def _launch(attention_bias, attention_mask, window_size, min_dtype, block_size, 
     kept = None
     packed = None
     if want_bits:  # one bit per key (the kernel writes keys [0, keys); padding bits must be zero) + tile activity
-        from ..packed import PackedMask
-
         words = (keys + _TILE - 1) // _TILE * (_TILE // 32)
         alloc = torch.empty if keys % _TILE == 0 else torch.zeros
         bits = alloc(tuple(out_shape[:3]) + (words,), dtype=torch.int32, device=bias.device)
@@ -166,6 +165,20 @@ def _reshape_padding_mask(attention_mask, batch_size, query_len, key_len):
     return attention_mask
 
 
+def _native_topk(attention_bias, attention_mask, window_size, min_dtype):
+    """The plain top-k mask through the native host path (csrc/fdma_torch.cpp), with the caches `create_mask` attaches
+    to it; None for inputs that path does not take."""
+    res = _native.load().topk_mask(attention_bias, attention_mask, int(window_size), float(min_dtype))
+    if res is None:
+        return None
+    mask = res[0]
+    if len(res) == 4:
+        mask._fdma_kept = (KeptKeys(res[1], res[2], res[3], mask.shape[3]), mask._version)
+    elif len(res) == 3:
+        mask._fdma_packed = (PackedMask(res[1], res[2], mask.shape[3]), mask._version)
+    return mask
+
+
 def create_mask(
     attention_bias: torch.Tensor,
     attention_mask: Optional[torch.Tensor],
@@ -188,6 +201,10 @@ def create_mask(
     if type == "topk":
         if block_size is not None and block_size <= 0:
             raise ValueError(f"block_size must be a positive integer, got {block_size}.")
+        if (block_size is None or block_size <= 1) and not torch.compiler.is_compiling():
+            mask = _native_topk(attention_bias, attention_mask, window_size, min_dtype)
+            if mask is not None:
+                return mask
         rows = attention_bias.shape[2] if attention_bias.dim() == 4 else 0
         if attention_mask is not None and attention_mask.dim() == 4:
             rows = max(rows, attention_mask.shape[2])
