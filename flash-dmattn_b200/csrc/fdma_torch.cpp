@@ -42,6 +42,8 @@ struct Api {
   decltype(&fdma_bwd) bwd;
   decltype(&fdma_create_mask) create_mask;
   decltype(&fdma_gather_kept) gather_kept;
+  decltype(&fdma_decode_kept) decode_kept;
+  decltype(&fdma_decode_kept_workspace_bytes) decode_kept_workspace_bytes;
   decltype(&fdma_strerror) strerror;
   decltype(&fdma_poll_kernel_status) poll_kernel_status;
   decltype(&fdma_last_kernel_status) last_kernel_status;
@@ -60,6 +62,8 @@ void init(const std::string& path) {
   get(api.bwd, "fdma_bwd");
   get(api.create_mask, "fdma_create_mask");
   get(api.gather_kept, "fdma_gather_kept");
+  get(api.decode_kept, "fdma_decode_kept");
+  get(api.decode_kept_workspace_bytes, "fdma_decode_kept_workspace_bytes");
   get(api.strerror, "fdma_strerror");
   get(api.poll_kernel_status, "fdma_poll_kernel_status");
   get(api.last_kernel_status, "fdma_last_kernel_status");
@@ -317,6 +321,41 @@ bool broadcastable(const Tensor& t, int64_t B, int64_t H, int64_t Hk, int64_t Sq
          (t.size(2) == 1 || t.size(2) == Sq);
 }
 
+// A single query over the kept keys of the list; nullopt for layouts the decode kernel does not take.
+std::optional<Tensor> decode(const Tensor& q0, const Tensor& k, const Tensor& v, const Tensor& bias0, const Tensor& key_pos, const Call& c) {
+  const int64_t B = q0.size(0), H = q0.size(2), Hk = k.size(2), Sk = k.size(1);
+  if (k.stride(3) != 1 || v.stride(3) != 1 || q0.stride(3) != 1 || !key_pos.is_contiguous()) return std::nullopt;
+  if ((key_pos.size(0) != 1 && key_pos.size(0) != B) || (key_pos.size(1) != 1 && key_pos.size(1) != Hk && key_pos.size(1) != H))
+    return std::nullopt;
+  if (bias0.defined() && (bias0.size(2) != 1 || bias0.size(3) < Sk || bias0.stride(3) != 1)) return std::nullopt;
+  at::AutoDispatchBelowADInplaceOrView guard;
+  const c10::cuda::CUDAGuard device(q0.device());
+  const cudaStream_t stream = stream_of(q0);
+  raise_if_timed_out(stream);
+  Tensor out = empty_as(q0), lse = empty({B, H, 1}, at::kFloat, q0);
+  fdma_decode_params p = {};
+  fill_geometry(p.f, q0, Sk, Hk, c);
+  fill_kv(p.f, k, v);
+  fill_mask_bias(p.f, Tensor(), bias0, Tensor(), c);
+  fill_out(p.f, out, lse);
+  p.kept_pos = key_pos.data_ptr<int32_t>();
+  p.kept_batch_stride = bcast_stride(key_pos, 0);
+  p.kept_head_stride = bcast_stride(key_pos, 1);
+  p.kept_h = static_cast<int32_t>(key_pos.size(1));
+  p.kept_capacity = static_cast<int32_t>(key_pos.size(2));
+  const size_t bytes = api.decode_kept_workspace_bytes(&p);
+  Tensor ws;
+  if (bytes) {
+    ws = empty({static_cast<int64_t>(bytes)}, at::kByte, q0);
+    p.f.workspace = ws.data_ptr();
+    p.f.workspace_bytes = bytes;
+  }
+  const int st = api.decode_kept(&p, stream);
+  if (st == FDMA_ERR_UNSUPPORTED) return std::nullopt;
+  check(st, "fdma_decode_kept");
+  return out;
+}
+
 // Runs one attention call; nullopt for inputs this path does not take. Exactly one form of mask is given: a bool tensor,
 // the position list of the kept keys (key_pos, slot_mask), bits with their tile activity, or none.
 std::optional<Tensor> attention(const Tensor& q0, const Tensor& k0, const Tensor& v0, const OptTensor& mask_, const OptTensor& bias_,
@@ -335,6 +374,7 @@ std::optional<Tensor> attention(const Tensor& q0, const Tensor& k0, const Tensor
                           !broadcastable(bias0, B, H, Hk, Sq)))
     return std::nullopt;
   const int64_t Sk_r = round_up(Sk, kTile);
+  const bool grad = at::GradMode::is_enabled() && (needs_grad(q0) || needs_grad(k0) || needs_grad(v0) || needs_grad(bias0));
 
   Call c;
   c.scale = static_cast<float>(scale);
@@ -343,6 +383,10 @@ std::optional<Tensor> attention(const Tensor& q0, const Tensor& k0, const Tensor
   c.path = path;
   c.seqlen_k = Sk;
   c.bias_keys = bias0.defined() ? bias0.size(3) : 0;
+  if (key_pos.defined() && Sq == 1) {
+    if (grad) return std::nullopt;
+    return decode(q0, k0, v0, bias0, key_pos, c);
+  }
   if (key_pos.defined()) {
     c.gathered = true;
     const int64_t Bm = key_pos.size(0), Hm = key_pos.size(1), cap = key_pos.size(2);
@@ -373,7 +417,6 @@ std::optional<Tensor> attention(const Tensor& q0, const Tensor& k0, const Tensor
   }
   if (!c.gathered && bias0.defined() && bias0.size(3) != 1 && bias0.size(3) != Sk && bias0.size(3) != Sk_r) return std::nullopt;
 
-  const bool grad = at::GradMode::is_enabled() && (needs_grad(q0) || needs_grad(k0) || needs_grad(v0) || needs_grad(bias0));
   Tensor out, lse, q, k, v, mask, bias, kvb;
   {
     at::AutoDispatchBelowADInplaceOrView guard;

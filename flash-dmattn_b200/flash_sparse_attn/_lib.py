@@ -62,6 +62,8 @@ EXPORTED_SYMBOLS = (
     "fdma_strerror",
     "fdma_fwd_workspace_bytes",
     "fdma_fwd",
+    "fdma_decode_kept",
+    "fdma_decode_kept_workspace_bytes",
     "fdma_bwd_workspace_bytes",
     "fdma_bwd",
     "fdma_create_mask",
@@ -100,6 +102,16 @@ class RowsParams(ctypes.Structure):
         ("dst_batch_stride", c_int64), ("dst_row_stride", c_int64), ("dst_head_stride", c_int64),
         ("b", c_int32), ("heads", c_int32), ("h_pos", c_int32), ("rows_full", c_int32),
         ("capacity", c_int32), ("row_elems", c_int32), ("dtype", c_int32), ("reserved_", c_int32),
+    ]
+
+
+class DecodeParams(ctypes.Structure):
+    """fdma_decode_params of include/fdma.h."""
+
+    _fields_ = [
+        ("f", FwdParams), ("kept_pos", c_void_p), ("kept_batch_stride", c_int64), ("kept_head_stride", c_int64),
+        ("kept_count", c_void_p), ("count_batch_stride", c_int64), ("count_head_stride", c_int64),
+        ("kept_h", c_int32), ("kept_capacity", c_int32),
     ]
 
 
@@ -146,6 +158,10 @@ def load():
     lib.fdma_fwd_workspace_bytes.argtypes = [POINTER(FwdParams)]
     lib.fdma_fwd.restype = c_int
     lib.fdma_fwd.argtypes = [POINTER(FwdParams), c_void_p]
+    lib.fdma_decode_kept.restype = c_int
+    lib.fdma_decode_kept.argtypes = [POINTER(DecodeParams), c_void_p]
+    lib.fdma_decode_kept_workspace_bytes.restype = c_size_t
+    lib.fdma_decode_kept_workspace_bytes.argtypes = [POINTER(DecodeParams)]
     lib.fdma_bwd_workspace_bytes.restype = c_size_t
     lib.fdma_bwd_workspace_bytes.argtypes = [POINTER(BwdParams)]
     lib.fdma_bwd.restype = c_int

@@ -128,8 +128,12 @@ def _native_attention(query, key, value, attn_mask, attn_bias, softmax_scale, is
             kept = mask
         else:
             packed = mask
-        if kept is not None and _compaction == "auto" and query.shape[1] > 1 and kept.seqlen_k == key.shape[1]:
-            if 4 * kept.key_pos.shape[-1] <= 3 * round_multiple(kept.seqlen_k, _KEY_PAD):
+        if kept is not None and _compaction == "auto" and kept.seqlen_k == key.shape[1]:
+            if query.shape[1] == 1:  # a decode step reads the kept rows themselves, whatever their share
+                if not tensor or not (torch.is_grad_enabled() and (query.requires_grad or key.requires_grad or
+                                      value.requires_grad or (attn_bias is not None and attn_bias.requires_grad))):
+                    key_pos, slot_mask, mask = kept.key_pos, kept.slot_mask, None
+            elif 4 * kept.key_pos.shape[-1] <= 3 * round_multiple(kept.seqlen_k, _KEY_PAD):
                 key_pos, slot_mask, mask = kept.key_pos, kept.slot_mask, None
         elif packed is not None and packed.seqlen_k == key.shape[1] and query.shape[1] > 1 and query.shape[3] <= 128:
             bits, activity, mask = packed.bits, packed.activity, None

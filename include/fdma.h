@@ -43,7 +43,7 @@ enum fdma_status {
 };
 
 /* Which kernel family the launcher picks. AUTO: the row-gather decode kernel for single-query calls
- * (seqlen_q == 1, head dim 64/128/256), tcgen05/TMA kernels (any head dim that is a multiple of 8) where shape and alignment allow, the
+ * (seqlen_q == 1), tcgen05/TMA kernels (any head dim that is a multiple of 8) where shape and alignment allow, the
  * CUDA-core kernels otherwise. The other values force one family (tests use them); forcing a family
  * on a shape it does not handle returns FDMA_ERR_UNSUPPORTED. */
 enum fdma_path { FDMA_PATH_AUTO = 0, FDMA_PATH_SIMT = 1, FDMA_PATH_TCGEN05 = 2, FDMA_PATH_DECODE = 3 };
@@ -107,6 +107,25 @@ typedef struct fdma_fwd_params {
 
 size_t fdma_fwd_workspace_bytes(const fdma_fwd_params* p);
 int fdma_fwd(const fdma_fwd_params* p, void* stream);
+
+/*
+ * Single-query forward over a list of kept keys (what fdma_create_mask writes through fdma_mask_params::key_pos): f as
+ * for fdma_fwd with seqlen_q = 1 over the FULL K / V (f.mask and f.key_pos are ignored, the key positions come from the
+ * list); kept_pos ascending int32 positions ({B|1}, kept_h in {1, h_k, h}, kept_capacity), batch stride 0 for a shared
+ * list; kept_count, if given, the entries in use of each list (strides 0 where shared), otherwise entries outside
+ * [0, seqlen_k) are skipped. No bool mask is read. Scratch: f.workspace, of the size the second function returns (0 for
+ * most calls). Rows 16-byte aligned, d a multiple of 8; FDMA_ERR_UNSUPPORTED otherwise.
+ */
+typedef struct fdma_decode_params {
+  fdma_fwd_params f;
+  const int32_t* kept_pos;
+  int64_t kept_batch_stride, kept_head_stride;
+  const int32_t* kept_count;
+  int64_t count_batch_stride, count_head_stride;
+  int32_t kept_h, kept_capacity;
+} fdma_decode_params;
+int fdma_decode_kept(const fdma_decode_params* p, void* stream);
+size_t fdma_decode_kept_workspace_bytes(const fdma_decode_params* p);
 
 /*
  * Backward: dQ, dK, dV and dBias for the forward above, given dOut, Out and LSE.
@@ -252,9 +271,8 @@ int fdma_selftest_wait_timeout(uint32_t limit_us, int* result_dev, void* stream)
  * nothing. Two kinds of call need scratch, and the limit applies to each as fdma_fwd_workspace_bytes reports it
  * (query it first to know):
  *   - a per-query mask: one activity byte per 128x128 tile, B * h_mask * ceil(Sq/128) * ceil(Sk/128) bytes;
- *   - a single-query call (seqlen_q == 1, with or without a mask) on the row-gather decode kernel: per-split
- *     partials B * H * splits * 8 * (d + 2) * 4 bytes (splits >= 1, chosen from Sk and the SM count), e.g. 1.02 MiB --
- *     over the limit -- at B * H = 256, d = 128 with one split.
+ *   - a single-query call (seqlen_q == 1) on the row-gather decode kernel: with a bool mask the position lists derived
+ *     from it, B * h_mask * round_up(Sk,128) * 4 bytes, and for long key ranges with few heads fp32 partials.
  * A call needing more than the limit returns FDMA_ERR_TOO_LARGE and launches nothing. The first call on each
  * device resolves the array's address: issue it outside any stream capture. Calls share the array; calls whose
  * GPU work overlaps in time race and must be serialised by the caller.
