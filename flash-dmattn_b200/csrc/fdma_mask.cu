@@ -5,6 +5,7 @@
 //
 // One CTA per row. The row's keys are staged once in shared memory (when they fit), so HBM traffic is
 // the algorithmic minimum: bias row in, (pre-mask row in,) bool row out.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -309,8 +310,7 @@ __device__ __forceinline__ uint32_t key_pair16(uint32_t u) {
 
 constexpr int kTieSlots = 32;  // up to this many keys tied at the threshold are ranked by one warp
 
-// kPos: also (or, with a null `out`, only) writes the ascending positions of the selected keys.
-template <int DT, int CHUNKS, bool kPos>
+template <int DT, int CHUNKS>
 __global__ void __launch_bounds__(kThreads, CHUNKS <= 4 ? 4 : 1) topk16_reg_kernel(const fdma_mask_params p) {
   using KT = KeyTraits<DT>;
   __shared__ int s_hist[kWarps][256];
@@ -456,9 +456,6 @@ __global__ void __launch_bounds__(kThreads, CHUNKS <= 4 ? 4 : 1) topk16_reg_kern
   const bool check_min = thr <= min_key;  // only then can a selected key hold the value min_dtype
 
   // ---- write pass: two output bytes per packed word (bit 0 = low key, bit 8 = high key) ----
-  uint32_t selbits[(CHUNKS + 3) / 4];
-#pragma unroll
-  for (int i = 0; i < (CHUNKS + 3) / 4; ++i) selbits[i] = 0u;
   auto emit = [&](int c, uint32_t (&ob)[4]) {
     const int k = c * kChunk + tid * kPerThread;
     if (k >= n) return;
@@ -473,10 +470,9 @@ __global__ void __launch_bounds__(kThreads, CHUNKS <= 4 ? 4 : 1) topk16_reg_kern
     o.x = ob[0] | (ob[1] << 16);
     o.y = ob[2] | (ob[3] << 16);
     if (rp.out) *reinterpret_cast<uint2*>(rp.out + k) = o;
-    if (kPos || bits_row) {  // bit j of the chunk's byte = key k + j selected
+    if (bits_row) {  // bit j of the byte = key k + j selected; every byte of keys [0, n), the caller zeroed the rest
       const uint32_t b8 = (((o.x & 0x01010101u) * 0x01020408u) >> 24) | ((((o.y & 0x01010101u) * 0x01020408u) >> 24) << 4);
-      if (kPos) selbits[c >> 2] |= b8 << ((c & 3) * 8);
-      if (bits_row) bits_row[k >> 3] = static_cast<uint8_t>(b8);  // every byte of keys [0, n); the caller zeroed the rest
+      bits_row[k >> 3] = static_cast<uint8_t>(b8);
     }
   };
   if (all_eq) {  // every key equal to the threshold is kept
@@ -490,7 +486,7 @@ __global__ void __launch_bounds__(kThreads, CHUNKS <= 4 ? 4 : 1) topk16_reg_kern
       }
       emit(c, ob);
     }
-  } else if (!kPos && s_eq_total <= kTieSlots) {
+  } else if (s_eq_total <= kTieSlots) {
     // A handful of keys tied at the threshold (the usual case): the lowest key indices win. Every thread writes the
     // keys above the threshold and drops the index of each tied key of its own into a short list; after a barrier
     // warp 0 ranks the list (one entry per lane, 32 shuffles) and sets the bytes of the winners itself. The
@@ -587,47 +583,6 @@ __global__ void __launch_bounds__(kThreads, CHUNKS <= 4 ? 4 : 1) topk16_reg_kern
       emit(c, ob);
     }
   }
-  if (kPos) {
-    // ascending positions: selections are counted chunk by chunk, thread by thread, with one block-wide scan
-    __syncthreads();  // s_scan may still be read by the tie ranking above
-    int excl[CHUNKS];
-#pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) {
-      const int cnt = __popc((selbits[c >> 2] >> ((c & 3) * 8)) & 0xFFu);
-      int incl = cnt;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      excl[c] = incl - cnt;
-      if (lane == 31) s_scan[c * kWarps + warp] = incl;
-    }
-    __syncthreads();
-    int32_t* prow = p.key_pos + row * p.capacity;
-    int base = 0;
-#pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) {
-      int warp_base = 0, total = 0;
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w) {
-        const int v = s_scan[c * kWarps + w];
-        if (w < warp) warp_base += v;
-        total += v;
-      }
-      uint32_t bits = (selbits[c >> 2] >> ((c & 3) * 8)) & 0xFFu;
-      int slot = base + warp_base + excl[c];
-      const int k = c * kChunk + tid * kPerThread;
-      while (bits) {
-        const int j = __ffs(bits) - 1;
-        bits &= bits - 1;
-        if (slot < p.capacity) prow[slot] = k + j;
-        ++slot;
-      }
-      base += total;
-    }
-    finish_positions(p, row, base, tid, kThreads);
-  }
   __syncthreads();  // the shared selection state is rewritten at the top of the next row
   }  // row loop
 }
@@ -670,19 +625,347 @@ bool reg_path_ok(const fdma_mask_params& p) {
   return (reinterpret_cast<uintptr_t>(p.out) & 7u) == 0;  // a null `out` (positions only) passes
 }
 
-template <int DT, bool kPos>
-void launch_reg_p(const fdma_mask_params& p, unsigned rows, cudaStream_t stream) {
-  const int chunks = (p.keys + kChunk - 1) / kChunk;
-  if (chunks <= 1) topk16_reg_kernel<DT, 1, kPos><<<rows, kThreads, 0, stream>>>(p);
-  else if (chunks <= 2) topk16_reg_kernel<DT, 2, kPos><<<rows, kThreads, 0, stream>>>(p);
-  else if (chunks <= 4) topk16_reg_kernel<DT, 4, kPos><<<rows, kThreads, 0, stream>>>(p);
-  else if (chunks <= 8) topk16_reg_kernel<DT, 8, kPos><<<rows, kThreads, 0, stream>>>(p);
-  else topk16_reg_kernel<DT, 16, kPos><<<rows, kThreads, 0, stream>>>(p);
-}
 template <int DT>
 void launch_reg(const fdma_mask_params& p, unsigned rows, cudaStream_t stream) {
-  if (p.key_pos) launch_reg_p<DT, true>(p, rows, stream);
-  else launch_reg_p<DT, false>(p, rows, stream);
+  const int chunks = (p.keys + kChunk - 1) / kChunk;
+  if (chunks <= 1) topk16_reg_kernel<DT, 1><<<rows, kThreads, 0, stream>>>(p);
+  else if (chunks <= 2) topk16_reg_kernel<DT, 2><<<rows, kThreads, 0, stream>>>(p);
+  else if (chunks <= 4) topk16_reg_kernel<DT, 4><<<rows, kThreads, 0, stream>>>(p);
+  else if (chunks <= 8) topk16_reg_kernel<DT, 8><<<rows, kThreads, 0, stream>>>(p);
+  else topk16_reg_kernel<DT, 16><<<rows, kThreads, 0, stream>>>(p);
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// 16-bit rows whose positions are wanted (row-broadcast masks: few rows, up to very long ones), and rows the register
+// kernel above does not take (odd lengths, unaligned bases). A row is shared by a cluster of up to 8 CTAs, each
+// with an even segment in registers; histograms are summed and counts exchanged through distributed shared
+// memory. The first digit has 11 bits, the second 5: an 8-bit first digit is sign and exponent of a bfloat16, four to
+// six values in all for normally distributed biases, and its shared-memory atomics serialise.
+// Bound by latency: loads, four cluster barriers and the passes over a CTA's keys. One CTA per row before, now: 1 row of 65536 keys
+// 99 -> 17 us, 8 x 32768 51 -> 13.5 us, 8 x 3001 9.8 -> 7.2 us, 256 x 65536 170 -> 151 us.
+// ---------------------------------------------------------------------------------------------------------
+constexpr int kBins = 2048;
+constexpr int kMaxRowCtas = 8;
+
+template <int DT, int CHUNKS>
+__global__ void __launch_bounds__(kThreads, CHUNKS <= 4 ? 4 : 2) topk16_cluster_kernel(const fdma_mask_params p) {
+  namespace cg = cooperative_groups;
+  using KT = KeyTraits<DT>;
+  __shared__ __align__(16) int s_hist[kBins];
+  __shared__ int s_low[32];            // second digit, among the keys that share the first
+  __shared__ int s_warp[kWarps];
+  __shared__ int s_scan[CHUNKS * kWarps];
+  __shared__ int s_digit, s_need;
+  __shared__ int s_eq_total, s_eq_before;
+  __shared__ int s_selected;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int nrank = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
+  const int64_t row = blockIdx.x / nrank;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n = p.keys;
+  const int seg = (((n + nrank - 1) / nrank) + kPerThread - 1) / kPerThread * kPerThread;  // at most CHUNKS * kChunk
+  const int k_lo = min(n, rank * seg), k_hi = min(n, k_lo + seg);
+  const RowPtrs rp = locate(p, row, 2);
+  const uint16_t* bias = static_cast<const uint16_t*>(rp.bias);
+  const uint32_t min_key = KT::key(KT::from_float(p.min_value));
+  const uint32_t min2 = min_key | (min_key << 16);
+  auto sync_row = [&]() {
+    if (nrank > 1) cluster.sync();
+    else __syncthreads();
+  };
+
+  // ---- keys [k_lo + c*2048 + tid*8, +8) as integer pairs; 0, below every real key, where there is none ----
+  uint32_t kw[CHUNKS][4];
+  const bool vec = (reinterpret_cast<uintptr_t>(bias) & 15u) == 0;  // k_lo is a multiple of 8
+  const bool vec_pm = (reinterpret_cast<uintptr_t>(rp.pm) & 7u) == 0;
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c) {
+    const int k = k_lo + c * kChunk + tid * kPerThread;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    uint2 m = make_uint2(0x01010101u, 0x01010101u);
+    if (k < k_hi) {
+      if (vec && k + kPerThread <= n) {
+        v = *reinterpret_cast<const uint4*>(bias + k);
+      } else {
+        uint32_t w[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int j = 0; j < kPerThread; ++j)
+          if (k + j < n) w[j >> 1] |= static_cast<uint32_t>(bias[k + j]) << ((j & 1) * 16);
+        v = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+      if (rp.pm) {
+        if (vec_pm && k + kPerThread <= n) {
+          m = *reinterpret_cast<const uint2*>(rp.pm + k);
+        } else {
+          uint32_t w[2] = {0, 0};
+#pragma unroll
+          for (int j = 0; j < kPerThread; ++j)
+            if (k + j < n) w[j >> 2] |= (rp.pm[k + j] ? 1u : 0u) << ((j & 3) * 8);
+          m = make_uint2(w[0], w[1]);
+        }
+      }
+    }
+    const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
+    const uint32_t mb[2] = {m.x, m.y};
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const uint32_t two = mb[w >> 1] >> ((w & 1) * 16);  // bytes of keys 2w, 2w+1
+      const uint32_t keep = ((two & 0xFFu) ? 0x0000FFFFu : 0u) | ((two & 0xFF00u) ? 0xFFFF0000u : 0u);
+      const uint32_t key = (key_pair16<DT>(vw[w]) & keep) | (min2 & ~keep);
+      const uint32_t real = (k + 2 * w < k_hi ? 0x0000FFFFu : 0u) | (k + 2 * w + 1 < k_hi ? 0xFFFF0000u : 0u);
+      kw[c][w] = key & real;
+    }
+  }
+  for (int i = tid; i < kBins; i += kThreads) s_hist[i] = 0;
+  if (tid < 32) s_low[tid] = 0;
+  __syncthreads();
+  // ---- first digit ----
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c) {
+    if (k_lo + c * kChunk + tid * kPerThread < k_hi) {
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        // (a missing key adds to bin 0, which no real key falls into: those would be NaN patterns, mapped to 0xFFFF)
+        atomicAdd(&s_hist[(kw[c][w] >> 5) & 0x7FFu], 1);
+        atomicAdd(&s_hist[kw[c][w] >> 21], 1);
+      }
+    }
+  }
+  sync_row();
+  {  // thread t owns bins [8t, 8t + 8) of the whole row
+    int cnt[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 4
+    for (int r = 0; r < nrank; ++r) {
+      const int4* h = reinterpret_cast<const int4*>(nrank > 1 ? cluster.map_shared_rank(s_hist, r) : s_hist) + tid * 2;
+      const int4 a = h[0], b = h[1];
+      cnt[0] += a.x; cnt[1] += a.y; cnt[2] += a.z; cnt[3] += a.w;
+      cnt[4] += b.x; cnt[5] += b.y; cnt[6] += b.z; cnt[7] += b.w;
+    }
+    int sum = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sum += cnt[j];
+    int above = sum;  // suffix sum over the lanes, then over the warps
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_down_sync(0xffffffffu, above, o);
+      if (lane + o < 32) above += v;
+    }
+    if (lane == 0) s_warp[warp] = above;
+    above -= sum;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w)
+      if (w > warp) above += s_warp[w];
+    const int need = min(p.window, n);
+#pragma unroll
+    for (int j = 7; j >= 0; --j) {
+      if (above < need && above + cnt[j] >= need) {
+        s_digit = tid * 8 + j;
+        s_need = need - above;
+      }
+      above += cnt[j];
+    }
+  }
+  __syncthreads();
+  const uint32_t hi = static_cast<uint32_t>(s_digit);
+  // ---- second digit ----
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c) {
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const uint32_t x = kw[c][w];
+      if (((x >> 5) & 0x7FFu) == hi) atomicAdd(&s_low[x & 31u], 1);
+      if ((x >> 21) == hi) atomicAdd(&s_low[(x >> 16) & 31u], 1);
+    }
+  }
+  sync_row();
+  if (warp == 0) {
+    int cnt = 0, before = 0;  // keys with this digit in the row / in the CTAs before this one
+    for (int r = 0; r < nrank; ++r) {
+      const int v = nrank > 1 ? cluster.map_shared_rank(s_low, r)[lane] : s_low[lane];
+      cnt += v;
+      if (r < rank) before += v;
+    }
+    int above = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_down_sync(0xffffffffu, above, o);
+      if (lane + o < 32) above += v;
+    }
+    above -= cnt;
+    const int need = s_need;
+    __syncwarp();
+    if (above < need && above + cnt >= need) {
+      s_digit = lane;
+      s_need = need - above;
+      s_eq_total = cnt;
+      s_eq_before = before;
+    }
+  }
+  __syncthreads();
+  const uint32_t thr = (hi << 5) | static_cast<uint32_t>(s_digit);
+  const int need_eq = s_need;
+  const bool all_eq = need_eq >= s_eq_total;
+  // number of items before this thread's, per chunk, in key order: `excl` inside the warp, s_scan the warps' totals
+  auto scan_counts = [&](const int (&cnt)[CHUNKS], int (&excl)[CHUNKS]) {
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+      int incl = cnt[c];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      excl[c] = incl - cnt[c];
+      if (lane == 31) s_scan[c * kWarps + warp] = incl;
+    }
+    __syncthreads();
+    int base = 0;
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {
+        if (w == warp) excl[c] += base;
+        base += s_scan[c * kWarps + w];
+      }
+    }
+    __syncthreads();  // s_scan is used again
+    return base;
+  };
+
+  // ---- selection: bit j of sel[c] = key j of the chunk; ties at the threshold go to the lowest key indices ----
+  uint32_t sel[CHUNKS];
+  {
+    int rank_eq[CHUNKS];
+    if (!all_eq) {
+      int cnt[CHUNKS];
+#pragma unroll
+      for (int c = 0; c < CHUNKS; ++c) {
+        cnt[c] = 0;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) cnt[c] += ((kw[c][w] & 0xFFFFu) == thr ? 1 : 0) + ((kw[c][w] >> 16) == thr ? 1 : 0);
+      }
+      scan_counts(cnt, rank_eq);
+    }
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+      uint32_t bits = 0;
+      int r = all_eq ? 0 : rank_eq[c] + s_eq_before;
+#pragma unroll
+      for (int j = 0; j < kPerThread; ++j) {
+        const uint32_t key = (kw[c][j >> 1] >> ((j & 1) * 16)) & 0xFFFFu;
+        bool s = key > thr;
+        if (key == thr) {
+          s = all_eq || r < need_eq;
+          ++r;
+        }
+        if (s && key != min_key) bits |= 1u << j;  // a value equal to min_dtype is never marked
+      }
+      sel[c] = bits;
+    }
+  }
+  if (rp.out) {
+    const bool vec_out = (reinterpret_cast<uintptr_t>(rp.out) & 7u) == 0;
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+      const int k = k_lo + c * kChunk + tid * kPerThread;
+      if (k >= k_hi) continue;
+      if (vec_out && k + kPerThread <= n) {
+        // four bits to the low bits of four bytes: copies of the nibble at bit offsets 0, 7, 14, 21
+        const uint32_t lo = ((sel[c] & 15u) * 0x00204081u) & 0x01010101u;
+        const uint32_t up = ((sel[c] >> 4) * 0x00204081u) & 0x01010101u;
+        *reinterpret_cast<uint2*>(rp.out + k) = make_uint2(lo, up);
+      } else {
+#pragma unroll
+        for (int j = 0; j < kPerThread; ++j)
+          if (k + j < n) rp.out[k + j] = (sel[c] >> j) & 1u;
+      }
+    }
+  }
+  if (p.bits) {  // one byte per 8 keys (whole bytes: see reg_path_ok); the caller zeroed the bytes beyond the row's keys
+    uint8_t* bits_row = reinterpret_cast<uint8_t*>(p.bits + row * (((n + 127) / 128) * 4));
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+      const int k = k_lo + c * kChunk + tid * kPerThread;
+      if (k < k_hi) bits_row[k >> 3] = static_cast<uint8_t>(sel[c]);
+    }
+  }
+  if (p.key_pos) {  // ascending positions of the selected keys
+    int cnt[CHUNKS], slot0[CHUNKS];
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) cnt[c] = __popc(sel[c]);
+    const int mine = scan_counts(cnt, slot0);
+    int before = 0, total = mine;
+    if (nrank > 1) {
+      if (tid == 0) s_selected = mine;
+      cluster.sync();
+      for (int r = 0; r < nrank; ++r) {
+        const int v = *cluster.map_shared_rank(&s_selected, r);
+        if (r < rank) before += v;
+        if (r != rank) total += v;
+      }
+    }
+    int32_t* prow = p.key_pos + row * p.capacity;
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+      uint32_t bits = sel[c];
+      int slot = before + slot0[c];
+      while (bits) {
+        const int j = __ffs(bits) - 1;
+        bits &= bits - 1;
+        if (slot < p.capacity) prow[slot] = k_lo + c * kChunk + tid * kPerThread + j;
+        ++slot;
+      }
+    }
+    finish_positions(p, row, total, rank * kThreads + tid, nrank * kThreads);
+  }
+  if (nrank > 1) cluster.sync();  // nobody leaves while its shared memory may still be read
+}
+
+template <int DT, int CHUNKS>
+int launch_cluster_c(const fdma_mask_params& p, unsigned rows, int ctas, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(rows * ctas);
+  cfg.blockDim = dim3(kThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ctas;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, topk16_cluster_kernel<DT, CHUNKS>, p));
+}
+
+// Longest row a cluster holds: 8 CTAs x 16 chunks.
+bool cluster_path_ok(const fdma_mask_params& p, int64_t rows) {
+  return p.keys <= kMaxRowCtas * 16 * kChunk && rows <= 0x7FFFFFFF / kMaxRowCtas;
+}
+
+// Keys per CTA: as few as keep the CTAs of all rows resident at once (four per SM), because a row's time is the time of
+// one CTA; where there are too many rows for that, four chunks (four CTAs per SM still fit), and more only for rows that
+// 8 such CTAs cannot hold, or rows in such number that one CTA each is enough.
+template <int DT>
+int launch_cluster(const fdma_mask_params& p, unsigned rows, cudaStream_t stream) {
+  const int64_t resident = 4ll * sm_count();
+  auto ctas_for = [&](int chunks) {
+    int c = 1;
+    while (static_cast<int64_t>(c) * chunks * kChunk < p.keys) c *= 2;
+    return c;
+  };
+  int chunks = 0;
+  for (int c = 1; c <= 16 && !chunks; c *= 2)
+    if (ctas_for(c) == 1 || (ctas_for(c) <= kMaxRowCtas && rows * static_cast<int64_t>(ctas_for(c)) <= resident)) chunks = c;
+  if (!chunks || (chunks > 4 && ctas_for(4) <= kMaxRowCtas))
+    for (chunks = 4; ctas_for(chunks) > kMaxRowCtas;) chunks *= 2;
+  const int ctas = ctas_for(chunks);
+  switch (chunks) {
+    case 1: return launch_cluster_c<DT, 1>(p, rows, ctas, stream);
+    case 2: return launch_cluster_c<DT, 2>(p, rows, ctas, stream);
+    case 4: return launch_cluster_c<DT, 4>(p, rows, ctas, stream);
+    case 8: return launch_cluster_c<DT, 8>(p, rows, ctas, stream);
+    default: return launch_cluster_c<DT, 16>(p, rows, ctas, stream);
+  }
 }
 
 template <int DT>
@@ -729,8 +1012,13 @@ int launch_mask(const fdma_mask_params& p, cudaStream_t stream) {
   if (p.bits && (p.kind != FDMA_MASK_TOPK || !reg_path_ok<DT>(p))) return FDMA_ERR_UNSUPPORTED;  // register kernel only
   if (p.kind == FDMA_MASK_RELU) {
     relu_mask_kernel<DT><<<static_cast<unsigned>(rows), kThreads, 0, stream>>>(p);
-  } else if (reg_path_ok<DT>(p)) {
+  } else if (DT != FDMA_FP32 && reg_path_ok<DT>(p) && !p.key_pos) {
     if constexpr (DT != FDMA_FP32) launch_reg<DT>(p, static_cast<unsigned>(rows), stream);
+  } else if (DT != FDMA_FP32 && cluster_path_ok(p, rows)) {
+    if constexpr (DT != FDMA_FP32) {
+      const int st = launch_cluster<DT>(p, static_cast<unsigned>(rows), stream);
+      if (st) return st;
+    }
   } else {
     const size_t stage = static_cast<size_t>(p.keys) * sizeof(typename KT::key_t);
     if (stage <= kMaxStageBytes) {
