@@ -577,11 +577,19 @@ std::vector<Tensor> topk_mask(const Tensor& bias, const OptTensor& premask_, int
 // Only exact torch.Tensor / Parameter objects and no active dispatch mode (fake tensors, tracing): everything else is the
 // Python path's.
 bool exact(PyObject* o) { return THPVariable_CheckExact(o); }
+// Tensors that stand for something else (vmap and grad transforms, functionalisation, lazy conjugation) or carry a
+// forward-mode tangent are the Python path's as well: the node below has neither batching rules nor a jvp.
+bool ordinary(const Tensor& t) {
+  constexpr c10::DispatchKeySet kWrapped({c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
+                                          c10::DispatchKey::Functionalize, c10::DispatchKey::Python, c10::DispatchKey::Conjugate,
+                                          c10::DispatchKey::Negative, c10::DispatchKey::ZeroTensor});
+  return !t.key_set().has_any(kWrapped) && !t._fw_grad(0).defined();
+}
 bool as_tensor(const py::handle& o, OptTensor& t) {
   if (o.is_none()) return true;
   if (!exact(o.ptr())) return false;
   t = THPVariable_Unpack(o.ptr());
-  return true;
+  return ordinary(*t);
 }
 
 py::object py_attention(py::handle q, py::handle k, py::handle v, py::handle mask, py::handle bias, py::handle key_pos,

@@ -121,3 +121,14 @@ def test_threads_and_streams(dev):
     _kernel_status_ok()
     for r in results.values():
         assert all(torch.equal(a, b) for a, b in zip(r, want))
+
+
+def test_forward_mode_tangent_is_not_dropped(dev):
+    """The node has no jvp: a dual tensor must reach the Python path, which refuses it, and not lose its tangent."""
+    from flash_sparse_attn import flash_sparse_attn_func
+
+    q, k, v = (torch.randn(1, 128, 2, 64, device=dev, dtype=torch.bfloat16) for _ in range(3))
+    with torch.autograd.forward_ad.dual_level():
+        dual = torch.autograd.forward_ad.make_dual(q, torch.ones_like(q))
+        with pytest.raises((RuntimeError, NotImplementedError)):
+            flash_sparse_attn_func(dual, k, v, is_causal=True)
