@@ -76,6 +76,7 @@ struct BwdKernelParams {
   const int32_t* key_pos;  // ascending positions of compacted keys, or null
   int64_t pos_batch_stride, pos_head_stride;
   int h_pos, causal_shift;
+  const int2* key_rows;  // packed sequences: query rows [x, y) that see each key (both ascending), or null
   float scale_log2, scale;
 };
 
@@ -177,7 +178,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   const int M64_all = (Sq + kBM - 1) / kBM;
   const int m_chunk = (M64_all + p.nsplit - 1) / p.nsplit;
   const int m_lo = split * m_chunk;
-  const int M64 = min(M64_all, m_lo + m_chunk);  // end of this CTA's query range
+  int M64 = min(M64_all, m_lo + m_chunk);  // end of this CTA's query range
   const bool causal = p.is_causal != 0;
   const int act_g = (p.h_mask == p.h && G > 1) ? G : 1;  // activity differs per query head only for per-head masks
   // Compacted keys carry their original positions (ascending); the causal test then runs on positions.
@@ -191,6 +192,11 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     m_start = static_cast<int>(max(static_cast<int64_t>(0), min(first, static_cast<int64_t>(M64))));
   } else if (causal) {
     m_start = max(0, (n * kBN - off) / kBM);  // first query tile with a row that sees key n*128
+  }
+  const bool packed = kBcast && p.key_rows != nullptr;
+  if (packed) {
+    m_start = p.key_rows[n * kBN].x / kBM;
+    M64 = min(M64, (p.key_rows[min(n * kBN + kBN, Sk) - 1].y + kBM - 1) / kBM);
   }
   m_start = max(m_start, m_lo);
   const WaitCtl ctl{s_abort, p.status};
@@ -425,6 +431,16 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     // (clamped so that ckey - coff cannot overflow; padding slots hold INT_MAX and are masked out anyway)
     const int ckey = pos_row ? (key_ok ? min(pos_row[key], 0x3FFFFFFF) : 0x3FFFFFFF) : key;
     const int ckey_wmax = pos_row ? __shfl_sync(0xffffffffu, ckey, 31) : n * kBN + (warp & 3) * 32 + 31;
+    // Row-broadcast kernel: query rows [qlo, qhi) see this key, those of [qlo_max, qhi_min) all keys of the warp.
+    int qlo = causal ? ckey - coff : -0x7FFFFFFF, qhi = 0x7FFFFFFF;
+    int qlo_max = causal ? ckey_wmax - coff : -0x7FFFFFFF, qhi_min = 0x7FFFFFFF;
+    if (packed) {
+      const int2 r = p.key_rows[min(key, Sk - 1)];
+      qlo = r.x;
+      qhi = r.y;
+      qlo_max = __shfl_sync(0xffffffffu, qlo, 31);
+      qhi_min = __shfl_sync(0xffffffffu, qhi, 0);
+    }
     const int mode = p.dbias_mode;
     float colsum = 0.f;       // column-sum mode
     float dacc[32];           // direct mode with dbias_h == h_k: sum over the head group
@@ -644,13 +660,13 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           // LSE*log2e and D of the step's 64 queries arrive in shared memory with the Q/dO stage
           const float* lrow = s_ld + (i % kQStages) * (2 * kBM) + qh * 32;
           const float* drow = lrow + kBM;
-          const bool diag = causal && static_cast<int64_t>(ckey_wmax) > static_cast<int64_t>(q0s) + coff;  // warp-uniform
+          const bool diag = qlo_max > q0s || qhi_min < q0s + 32;  // warp-uniform
           const bool per_elem = !kBcast || diag;
           if (kBcast && diag) {
 #pragma unroll
             for (int j = 0; j < 16; ++j)
-              bias2[j] = make_float2(ckey - coff > q0s + 2 * j ? -CUDART_INF_F : bv,
-                                     ckey - coff > q0s + 2 * j + 1 ? -CUDART_INF_F : bv);
+              bias2[j] = make_float2(q0s + 2 * j < qlo || q0s + 2 * j >= qhi ? -CUDART_INF_F : bv,
+                                     q0s + 2 * j + 1 < qlo || q0s + 2 * j + 1 >= qhi ? -CUDART_INF_F : bv);
           }
           uint32_t dsk[16];
           uint32_t rs[32], rp[32];
@@ -1017,7 +1033,7 @@ BwdPlan plan(const fdma_bwd_params& bp) {
 bool aligned16(const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; }
 
 template <int D, bool kBf16>
-int launch(const fdma_bwd_params& bp, const BwdPlan& pl, cudaStream_t stream) {
+int launch(const fdma_bwd_params& bp, const BwdPlan& pl, const int32_t* key_rows, cudaStream_t stream) {
   using L = SmemB<D>;
   const fdma_fwd_params& p = bp.f;
   if (!p.workspace || p.workspace_bytes < pl.total) return FDMA_ERR_WORKSPACE;
@@ -1102,7 +1118,8 @@ int launch(const fdma_bwd_params& bp, const BwdPlan& pl, cudaStream_t stream) {
   kp.dbias_b = bp.dbias_b; kp.dbias_h = bp.dbias_h; kp.dbias_rows = bp.dbias_rows;
   kp.dbias_keys = bp.scatter_pos ? p.seqlen_k : bp.dbias_keys;
   kp.dbias_mode = pl.dbias_mode;
-  kp.is_causal = p.is_causal;
+  kp.is_causal = key_rows ? 0 : p.is_causal;  // (packed: the causal limit is part of the rows)
+  kp.key_rows = reinterpret_cast<const int2*>(key_rows);
   kp.key_pos = p.key_pos;
   kp.pos_batch_stride = p.key_pos_batch_stride; kp.pos_head_stride = p.key_pos_head_stride;
   kp.h_pos = p.h_pos; kp.causal_shift = p.causal_shift;
@@ -1188,12 +1205,12 @@ size_t tc_bwd_workspace_bytes(const fdma_bwd_params& p) {
   return tile_head_dim(p.f.d) == 256 ? tc_bwd256_workspace_bytes(p) : plan(p).total;
 }
 
-int tc_bwd(const fdma_bwd_params& p, cudaStream_t stream) {
+int tc_bwd(const fdma_bwd_params& p, cudaStream_t stream, const int32_t* key_rows) {
   const bool bf16 = p.f.dtype == FDMA_BF16;
   if (tile_head_dim(p.f.d) == 256) return tc_bwd256(p, stream);
   const BwdPlan pl = plan(p);
-  if (pl.D == 64) return bf16 ? launch<64, true>(p, pl, stream) : launch<64, false>(p, pl, stream);
-  return bf16 ? launch<128, true>(p, pl, stream) : launch<128, false>(p, pl, stream);
+  if (pl.D == 64) return bf16 ? launch<64, true>(p, pl, key_rows, stream) : launch<64, false>(p, pl, key_rows, stream);
+  return bf16 ? launch<128, true>(p, pl, key_rows, stream) : launch<128, false>(p, pl, key_rows, stream);
 }
 
 }  // namespace fdma

@@ -40,6 +40,9 @@ struct Api {
   decltype(&fdma_fwd) fwd;
   decltype(&fdma_bwd_workspace_bytes) bwd_workspace_bytes;
   decltype(&fdma_bwd) bwd;
+  decltype(&fdma_packed_limits) packed_limits;
+  decltype(&fdma_fwd_packed) fwd_packed;
+  decltype(&fdma_bwd_packed) bwd_packed;
   decltype(&fdma_create_mask) create_mask;
   decltype(&fdma_gather_kept) gather_kept;
   decltype(&fdma_decode_kept) decode_kept;
@@ -60,6 +63,9 @@ void init(const std::string& path) {
   get(api.fwd, "fdma_fwd");
   get(api.bwd_workspace_bytes, "fdma_bwd_workspace_bytes");
   get(api.bwd, "fdma_bwd");
+  get(api.packed_limits, "fdma_packed_limits");
+  get(api.fwd_packed, "fdma_fwd_packed");
+  get(api.bwd_packed, "fdma_bwd_packed");
   get(api.create_mask, "fdma_create_mask");
   get(api.gather_kept, "fdma_gather_kept");
   get(api.decode_kept, "fdma_decode_kept");
@@ -125,7 +131,7 @@ int64_t bcast_stride(const Tensor& t, int dim) { return t.size(dim) == 1 ? 0 : t
 // Everything one attention call needs besides q, k, v: the same struct serves the forward call and the autograd node.
 struct Call {
   float scale = 0.f;
-  bool causal = false, deterministic = false, bits = false, gathered = false;
+  bool causal = false, deterministic = false, bits = false, gathered = false, packed = false;
   int path = FDMA_PATH_AUTO;
   int64_t seqlen_k = 0;      // keys of the caller's K
   int64_t bias_keys = 0;     // key extent of the caller's bias
@@ -220,9 +226,10 @@ void fill_gathered(fdma_fwd_params& p, const KvB& kv, const Tensor& key_pos, con
 }
 
 // ---- backward --------------------------------------------------------------------------------------------------
-// One node for the three routes. Saved: dense   q, k, v, mask, bias, out, lse
+// One node for the four routes. Saved: dense   q, k, v, mask, bias, out, lse
 //                                       bits    q, k, v, bits, bias, out, lse, activity
 //                                       gathered q, kvb, -, slot_mask, -, out, lse, key_pos
+//                                       packed  q, k, v, -, -, out, lse, the query rows that see each key
 struct AttnBackward : public torch::autograd::Node {
   Call c;
   SavedVariable q, k, v, mask, bias, out, lse, extra;
@@ -235,7 +242,40 @@ struct AttnBackward : public torch::autograd::Node {
     for (SavedVariable* s : {&q, &k, &v, &mask, &bias, &out, &lse, &extra}) s->reset_data();
   }
   variable_list apply(variable_list&& grads) override;
+  variable_list apply_packed(const Tensor& tq, const Tensor& tk, const Tensor& tv, const Tensor& tout, const Tensor& tlse,
+                             const Tensor& key_rows, const Tensor& dout, cudaStream_t stream);
 };
+
+// Gradients of packed sequences: (tokens, heads, d) tensors, one row of tokens for the kernels.
+variable_list AttnBackward::apply_packed(const Tensor& tq, const Tensor& tk, const Tensor& tv, const Tensor& tout, const Tensor& tlse,
+                                         const Tensor& key_rows, const Tensor& dout, cudaStream_t stream) {
+  variable_list res(3);
+  Tensor dq = empty(tq.sizes(), tq.scalar_type(), tq), dk = empty(tk.sizes(), tk.scalar_type(), tk), dv = empty(tv.sizes(), tv.scalar_type(), tv);
+  fdma_bwd_params bp = {};
+  const Tensor q4 = tq.unsqueeze(0), k4 = tk.unsqueeze(0);
+  fill_geometry(bp.f, q4, tk.size(0), tk.size(1), c);
+  fill_kv(bp.f, k4, tv.unsqueeze(0));
+  fill_out(bp.f, tout.unsqueeze(0), tlse);
+  const Bsh so = bsh(dout.unsqueeze(0)), sq = bsh(dq.unsqueeze(0)), sk = bsh(dk.unsqueeze(0));
+  bp.dout = dout.data_ptr();
+  bp.do_batch_stride = so.b; bp.do_row_stride = so.r; bp.do_head_stride = so.h;
+  bp.dq = dq.data_ptr(); bp.dk = dk.data_ptr(); bp.dv = dv.data_ptr();
+  bp.dq_batch_stride = sq.b; bp.dq_row_stride = sq.r; bp.dq_head_stride = sq.h;
+  bp.dk_batch_stride = bp.dv_batch_stride = sk.b;
+  bp.dk_row_stride = bp.dv_row_stride = sk.r;
+  bp.dk_head_stride = bp.dv_head_stride = sk.h;
+  bp.deterministic = c.deterministic ? 1 : 0;
+  const size_t bytes = api.bwd_workspace_bytes(&bp);
+  Tensor ws;
+  if (bytes) {
+    ws = empty({static_cast<int64_t>(bytes)}, at::kByte, tq);
+    bp.f.workspace = ws.data_ptr();
+    bp.f.workspace_bytes = bytes;
+  }
+  check(api.bwd_packed(&bp, key_rows.data_ptr<int32_t>(), stream), "fdma_bwd_packed");
+  res[0] = dq; res[1] = dk; res[2] = dv;
+  return res;
+}
 
 variable_list AttnBackward::apply(variable_list&& grads) {
   variable_list res(4);
@@ -246,6 +286,7 @@ variable_list AttnBackward::apply(variable_list&& grads) {
   const c10::cuda::CUDAGuard device(tq.device());
   const cudaStream_t stream = stream_of(tq);
   raise_if_timed_out(stream);
+  if (c.packed) return apply_packed(tq, tk, v.unpack(), tout, tlse, textra, grads[0].contiguous(), stream);
   const Tensor dout = inner_contiguous(grads[0]);
 
   fdma_bwd_params bp = {};
@@ -502,6 +543,67 @@ std::optional<Tensor> attention(const Tensor& q0, const Tensor& k0, const Tensor
   return out;
 }
 
+// Packed sequences in one launch: q (Tq, H, d), k and v (Tk, Hk, d), cu_q / cu_k (n + 1) int32 on the device, ascending from 0
+// to Tq / Tk (the caller has looked). Returns (out, lse (1, H, Tq)); empty for inputs this path does not take.
+std::vector<Tensor> packed_attention(const Tensor& q0, const Tensor& k0, const Tensor& v0, const Tensor& cu_q, const Tensor& cu_k,
+                                     double scale, bool causal, bool deterministic) {
+  for (const Tensor* t : {&q0, &k0, &v0})
+    if (!t->defined() || !t->is_cuda() || t->layout() != at::kStrided || t->dim() != 3 || t->device() != q0.device()) return {};
+  const auto type = q0.scalar_type();
+  if ((type != at::kBFloat16 && type != at::kHalf) || k0.scalar_type() != type || v0.scalar_type() != type) return {};
+  const int64_t Tq = q0.size(0), H = q0.size(1), d = q0.size(2), Tk = k0.size(0), Hk = k0.size(1);
+  if (Tq <= 0 || Tk <= 0 || H <= 0 || Hk <= 0 || H % Hk || d <= 0 || d % 8 || d > 128 || k0.size(2) != d || v0.sizes() != k0.sizes()) return {};
+  if (Hk > 65535 || H > 65535 || Tq > (1 << 19) || Tk > (1 << 20)) return {};  // the kernels' tile tables
+  for (const Tensor* t : {&cu_q, &cu_k})
+    if (!t->is_cuda() || t->device() != q0.device() || t->scalar_type() != at::kInt || t->dim() != 1 || !t->is_contiguous() || t->size(0) < 2) return {};
+  // what the kernels' TMA loads ask of the tensors; anything else goes sequence by sequence
+  for (const Tensor* t : {&q0, &k0, &v0}) {
+    if (t->stride(2) != 1 || (reinterpret_cast<uintptr_t>(t->data_ptr()) & 15)) return {};
+    for (int i = 0; i < 2; ++i)
+      if (t->size(i) > 1 && (t->stride(i) <= 0 || t->stride(i) % 8)) return {};
+  }
+  const bool grad = at::GradMode::is_enabled() && (needs_grad(q0) || needs_grad(k0) || needs_grad(v0));
+  Call c;
+  c.scale = static_cast<float>(scale);
+  c.causal = causal;
+  c.deterministic = deterministic;
+  c.packed = true;
+  c.seqlen_k = Tk;
+  Tensor out, lse, key_rows;
+  {
+    at::AutoDispatchBelowADInplaceOrView guard;
+    const c10::cuda::CUDAGuard device(q0.device());
+    const cudaStream_t stream = stream_of(q0);
+    raise_if_timed_out(stream);
+    out = empty(q0.sizes(), type, q0);
+    lse = empty({1, H, Tq}, at::kFloat, q0);
+    const Tensor row_keys = empty({Tq, 2}, at::kInt, q0);
+    key_rows = empty({Tk, 2}, at::kInt, q0);
+    check(api.packed_limits(cu_q.data_ptr<int32_t>(), cu_k.data_ptr<int32_t>(), static_cast<int32_t>(cu_q.size(0) - 1),
+                            static_cast<int32_t>(Tq), static_cast<int32_t>(Tk), causal ? 1 : 0, row_keys.data_ptr<int32_t>(),
+                            key_rows.data_ptr<int32_t>(), stream), "fdma_packed_limits");
+    fdma_fwd_params p = {};
+    const Tensor q4 = q0.unsqueeze(0), k4 = k0.unsqueeze(0);
+    fill_geometry(p, q4, Tk, Hk, c);
+    fill_kv(p, k4, v0.unsqueeze(0));
+    fill_out(p, out.unsqueeze(0), lse);
+    check(api.fwd_packed(&p, row_keys.data_ptr<int32_t>(), stream), "fdma_fwd_packed");
+  }
+  if (grad) {
+    auto node = std::shared_ptr<AttnBackward>(new AttnBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(q0, k0, v0));
+    torch::autograd::set_history(out, node);
+    node->q = SavedVariable(q0, false);
+    node->k = SavedVariable(k0, false);
+    node->v = SavedVariable(v0, false);
+    node->out = SavedVariable(out, /*is_output=*/true);
+    node->lse = SavedVariable(lse, false);
+    node->extra = SavedVariable(key_rows, false);
+    node->c = std::move(c);
+  }
+  return {out, lse};
+}
+
 // ---- create_mask -------------------------------------------------------------------------------------------------
 // Top-k selection: (mask, key_pos, count, slot_mask) for a row-broadcast bias, (mask, bits, activity) for a per-query one
 // where the kernel writes bits, (mask) otherwise. Empty for inputs this path does not take.
@@ -616,6 +718,24 @@ py::object py_attention(py::handle q, py::handle k, py::handle v, py::handle mas
   return py::reinterpret_steal<py::object>(THPVariable_Wrap(*out));
 }
 
+py::object py_packed_attention(py::handle q, py::handle k, py::handle v, py::handle cu_q, py::handle cu_k, double scale, bool causal,
+                               bool deterministic) {
+  OptTensor t[5];
+  const py::handle in[5] = {q, k, v, cu_q, cu_k};
+  for (int i = 0; i < 5; ++i)
+    if (!as_tensor(in[i], t[i]) || !t[i]) return py::none();
+  if (c10::impl::TorchDispatchModeTLS::any_modes_set()) return py::none();
+  std::vector<Tensor> res;
+  {
+    py::gil_scoped_release release;
+    res = packed_attention(*t[0], *t[1], *t[2], *t[3], *t[4], scale, causal, deterministic);
+  }
+  if (res.empty()) return py::none();
+  py::tuple out(res.size());
+  for (size_t i = 0; i < res.size(); ++i) out[i] = py::reinterpret_steal<py::object>(THPVariable_Wrap(res[i]));
+  return out;
+}
+
 py::object py_topk_mask(py::handle bias, py::handle premask, int64_t window, double min_value) {
   OptTensor b, pm;
   if (!as_tensor(bias, b) || !as_tensor(premask, pm) || !b || c10::impl::TorchDispatchModeTLS::any_modes_set()) return py::none();
@@ -635,5 +755,6 @@ py::object py_topk_mask(py::handle bias, py::handle premask, int64_t window, dou
 PYBIND11_MODULE(_fdma_torch, m) {
   m.def("init", &init);
   m.def("attention", &py_attention);
+  m.def("packed_attention", &py_packed_attention);
   m.def("topk_mask", &py_topk_mask);
 }

@@ -533,6 +533,21 @@ def flash_sparse_attn_func(
     )
 
 
+def _one_launch(query, key, value, cu_q, cu_k, cq, ck, max_q, max_k, softmax_scale, is_causal, deterministic):
+    """Packed sequences in one launch: (out, lse (1, H, total_q)), or None for calls that go sequence by sequence -- lengths
+    that leave tokens out, decrease or exceed the given maxima (the loop raises the right error), tracing, forced kernel
+    families, and the layouts the native path declines."""
+    if _kernel_path != _lib.PATH_AUTO or torch.compiler.is_compiling() or not query.is_cuda:
+        return None
+    if cq[0] or ck[0] or cq[-1] != query.shape[0] or ck[-1] != key.shape[0]:
+        return None
+    for i in range(len(cq) - 1):
+        if not (0 <= cq[i + 1] - cq[i] <= max_q and 0 <= ck[i + 1] - ck[i] <= max_k):
+            return None
+    scale = query.shape[-1] ** (-0.5) if softmax_scale is None else float(softmax_scale)
+    return _native.load().packed_attention(query, key, value, cu_q, cu_k, scale, bool(is_causal), bool(deterministic))
+
+
 def flash_sparse_attn_varlen_func(
     query: torch.Tensor,
     key: torch.Tensor,
@@ -557,9 +572,10 @@ def flash_sparse_attn_varlen_func(
     of key / value; is_causal aligns each sequence's causal mask to ITS bottom-right corner. Returns out
     (total_q, H, d), or with return_attn_probs=True (out, softmax_lse (H, total_q) fp32, empty tensor).
 
-    Each sequence is a contiguous slice of the packed tensors, so it is handed to the dense kernels as a zero-copy
-    (1, L, H, d) view: one forward (and backward) launch sequence per packed sequence, no padding, no mask. The
-    boundaries are read on the host (one device synchronisation per call). A paged KV cache (`block_table`) is not
+    Sequences that cover the tokens without a gap run in one launch per direction, where every query row carries its
+    own first and last key (head dims up to 128). Anything else goes sequence by sequence: each is a contiguous slice of the packed
+    tensors, handed to the dense kernels as a zero-copy (1, L, H, d) view. No padding and no mask in either form. The
+    boundaries are read on the host (one device synchronisation per call) for the checks below. A paged KV cache (`block_table`) is not
     built and raises NotImplementedError."""
     if block_table is not None:
         raise NotImplementedError("paged KV (block_table) is not built into the B200 kernels")
@@ -567,10 +583,19 @@ def flash_sparse_attn_varlen_func(
         raise RuntimeError("query, key and value must be (total_tokens, nheads, headdim)")
     if cu_seqlens_q.numel() != cu_seqlens_k.numel() or cu_seqlens_q.numel() < 2:
         raise RuntimeError("cu_seqlens_q and cu_seqlens_k must both have batch_size + 1 entries")
-    cq, ck = cu_seqlens_q.tolist(), cu_seqlens_k.tolist()
+    cq = cu_seqlens_q.tolist()
+    ck = cq if cu_seqlens_k is cu_seqlens_q else cu_seqlens_k.tolist()
     if cq[-1] > query.shape[0] or ck[-1] > key.shape[0]:
         raise RuntimeError("cu_seqlens exceed the number of packed tokens")
     H, d = query.shape[1], query.shape[2]
+    res = None
+    if not softcap and len(cq) > 2:
+        res = _one_launch(query, key, value, cu_seqlens_q, cu_seqlens_k, cq, ck, max_seqlen_q, max_seqlen_k, softmax_scale,
+                          is_causal, deterministic)
+    if res is not None:
+        if not return_attn_probs:
+            return res[0]
+        return res[0], res[1][0], torch.empty((0,), dtype=query.dtype, device=query.device)
     outs, lses = [], []
     if cq[0] > 0:  # tokens before the first boundary belong to no sequence
         outs.append(query.new_zeros((cq[0], H, d)))
