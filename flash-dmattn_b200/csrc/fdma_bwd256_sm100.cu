@@ -1,21 +1,30 @@
 // Dynamic-mask attention backward for head dims 136 to 256 on Blackwell tensor cores (tcgen05 + TMEM + TMA), for
 // row-broadcast masks and biases (the shape create_mask produces from a (B, Hk, 1, Sk) bias).
 //
-// Same mathematics and the same transposed products as the head-dim-128 kernel next door (fdma_bwd_sm100.cu; the
-// reference kernel is csrc/flash_sparse_attn/src/flash_bwd_kernel.h:79-1142):
-//     St = K Q^T, dPt = V dO^T, P = exp2(St*scale*log2e + bias*log2e - LSE*log2e), dS = P o (dPt - D),
-//     dV += P^T dO, dK += dS^T Q (x scale at the end), dQ^T = K^T dS^T (x scale in the convert pass),
-//     dBias[key] = sum over queries and the head group of dS.
-// What differs is the budget. At d = 256 the dK and dV accumulators of a 128-key tile need 256 TMEM columns EACH, all
-// 512 there are, and K + V + one Q/dO step fill 192 KiB of shared memory. So a CTA walks its (query tile, head) steps
-// TWICE, recomputing St / dPt / dS:
-//     pass A: TMEM  St | dPt | dQ^T low | dQ^T high | dV (256)   -> dV, dQ, dBias
-//     pass B: TMEM  St | dPt |     (free)           | dK (256)   -> dK
-// and the Q/dO ring has ONE slot: a step is load -> St, dPt -> softmax -> dV (+ dQ) or dK -> next load. That is 14
-// GEMM units per step pair instead of the 10 a single pass would need, and no overlap between the steps of one CTA;
-// it still beats the CUDA-core kernel, the only other implementation at this head dim, by two orders of magnitude.
-// Query-range splits (fp32 partial dK / dV / column sums + a reduction kernel) spread small grids over the GPU as in
-// the d = 128 kernel. Every mbarrier wait is bounded.
+// Same mathematics as the head-dim-128 kernel next door (fdma_bwd_sm100.cu; the reference kernel is
+// csrc/flash_sparse_attn/src/flash_bwd_kernel.h:79-1142). What differs is the budget: at d = 256 the accumulator of ONE
+// gradient of a 128-row tile takes 256 of the 512 TMEM columns and a 128-row operand 64 KB of shared memory. So every
+// gradient has its own pass, and all three are the same pipeline over a stationary 128-row tile and 64-row tiles that
+// stream by:
+//              stationary        streamed, 64 rows    scores          gradient product
+//     kDk      K, V (128 keys)   Q, dO (each head)    St, dPt         dK += dS^T Q
+//     kDv      K    (128 keys)   Q, dO (each head)    St              dV += P^T dO
+//     kDq      Q, dO (128 rows)  K, V                 S, dP           dQ += dS K
+// with scores[row, column] = (stationary row) . (streamed row), the probabilities or dS written back in 16 bit over the
+// scores as the A operand (from TMEM), and the B operand read MN-major from the streamed tile. dK's pass also sums dS over its queries
+// for dBias. dQ is complete in TMEM: no accumulator in memory, nothing to zero, add to or convert, and the same bits every time.
+//
+// TMEM: scores[2] 2 x 64 | dP[2] 2 x 64 | accumulator 256. The products of step i+1 are issued before the gradient
+// product of step i, so the softmax of a step runs under 1536 cycles of tensor work of the next (d = 256, N = 64 products are bound by the
+// shared-memory reads of their operands: 48 cycles per 16 columns of d against 32 of arithmetic). Shared memory: the operand of the
+// gradient product must stay until that product is done and has two slots, the other streamed operand one (two for kDv).
+// 8 products of 128 x 64 x 256 per tile pair instead of the 7 of a two-pass form (dV and dQ in one pass, dK in the other) that had
+// one slot for everything, no overlap between steps and an fp32 dQ buffer in memory. 65536 queries, 16 heads over one kv head,
+// 2048 kept keys: kernel 8.3 -> 5.5 ms, with the kernels around it 8.95 -> 5.8 ms.
+// One launch: the CTAs of the three passes are mixed, dK first.
+//
+// Warps: 0 TMA producer | 1 MMA issuer | 2 row vectors (LSE and D of 64 queries, or addend and position of 64 keys) |
+// 4-7, 8-11 softmax and epilogue (thread = stationary row; score columns 0-31 / 32-63). Every mbarrier wait is bounded.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <math_constants.h>
@@ -29,23 +38,25 @@ namespace fdma {
 namespace {
 
 constexpr int kD = 256;
-constexpr int kBN = 128;  // keys per CTA
-constexpr int kBM = 64;   // query rows per step
-constexpr int kThreads = 512;
+constexpr int kBN = 128;  // stationary rows per CTA
+constexpr int kBM = 64;   // streamed rows per step
+constexpr int kThreads = 384;
+constexpr int kMaxBits = 4096;  // 64-key tiles the activity bits of a dQ pass can hold; beyond, every tile is worked on
 constexpr float kLog2e = 1.4426950408889634f;
 
+enum Pass { kDk = 0, kDv = 1, kDq = 2 };
 enum WaitCode256 {
-  kW256Kv = 301, kW256StageEmpty = 302, kW256StageFull = 303, kW256SFull = 304, kW256Pds = 305, kW256DqFull = 306,
-  kW256DqEmpty = 307, kW256DsEmpty = 308, kW256AccFree = 309, kW256Final = 310
+  kW256X = 301, kW256AEmpty = 302, kW256AFull = 303, kW256SFull = 304, kW256Pds = 305, kW256BEmpty = 306,
+  kW256BFull = 307, kW256VecEmpty = 308, kW256VecFull = 309, kW256Final = 310
 };
 
 struct Bwd256Params {
-  CUtensorMap tm_q, tm_do, tm_k, tm_v;  // q/do: 64-row boxes, k/v: 128-row boxes, 64 elements wide
+  CUtensorMap tm_q, tm_do, tm_k, tm_v;  // boxes of 64 rows x 64 elements
   const uint8_t* mask;
   const void* bias;
   const float* lse2;   // (B,H,Sq_r) LSE * log2(e); +inf for empty and padded rows
   const float* dsum;   // (B,H,Sq_r) D = rowsum(dO o O)
-  float* dq_acc;       // (B,H,2,Sq,128) fp32: the two halves of d kept apart so that 16 query rows are contiguous
+  void* dq;
   void* dk;
   void* dv;
   void* dbias;
@@ -53,11 +64,13 @@ struct Bwd256Params {
   float* dbias_part;   // with dkv_part: fp32 partials [nsplit][B][h_k][NT*128]
   int* status;
   int64_t mask_batch_stride, mask_head_stride, bias_batch_stride, bias_head_stride;
+  int64_t dq_batch_stride, dq_row_stride, dq_head_stride;
   int64_t dk_batch_stride, dk_row_stride, dk_head_stride;
   int64_t dv_batch_stride, dv_row_stride, dv_head_stride;
   int64_t dbias_batch_stride, dbias_head_stride;
   int b, seqlen_q, seqlen_k, sq_r, h, h_k, h_mask, h_bias, d;
   int dbias_keys, want_dbias, nsplit, is_causal;
+  int n_kv_ctas;       // CTAs of the dK pass, and of the dV pass
   const int32_t* key_pos;
   int64_t pos_batch_stride, pos_head_stride;
   int h_pos, causal_shift;
@@ -65,20 +78,16 @@ struct Bwd256Params {
 };
 
 struct Smem256 {
-  static constexpr int kKOff = 0;                                   // 4 blocks of [128 keys][64 d]
-  static constexpr int kVOff = kBN * kD * 2;                        // 64 KB
-  static constexpr int kQOff = 2 * kBN * kD * 2;                    // 128 KB: Q step, 4 blocks of [64 q][64 d]
-  static constexpr int kQBytes = kBM * kD * 2;                      // 32 KB
-  static constexpr int kDoOff = kQOff + kQBytes;                    // dO step
-  static constexpr int kDsOff = kDoOff + kQBytes;                   // 192 KB: dS^T tile [128 keys][64 q] 16-bit
-  static constexpr int kDsBytes = kBN * kBM * 2;                    // 16 KB
-  static constexpr int kDqOff = kDsOff + kDsBytes;                  // [16 q][128 d] fp32 staging tile of the dQ writer
-  static constexpr int kDqRows = 16;
-  static constexpr int kLdOff = kDqOff + kDqRows * 128 * 4;         // 64 x LSE*log2e, 64 x D (fp32)
-  static constexpr int kLdBytes = 2 * kBM * 4;
-  static constexpr int kRedOff = kLdOff + kLdBytes;
-  static constexpr int kBarOff = kRedOff + kBN * 4;
-  static constexpr int kNumBars = 12;
+  static constexpr int kTile = kBN * kD * 2;                // 64 KB: 4 blocks of [128 rows][64 d]
+  static constexpr int kStep = kBM * kD * 2;                // 32 KB: 4 blocks of [64 rows][64 d]
+  static constexpr int kXOff = 0;                           // stationary operand of the scores
+  static constexpr int kX2Off = kTile;                      // ... of dP; kDv: second slot of the other streamed operand
+  static constexpr int kAOff = 2 * kTile;                   // two slots: streamed operand of the gradient product
+  static constexpr int kBOff = kAOff + 2 * kStep;           // one slot: the other streamed operand
+  static constexpr int kVecOff = kBOff + kStep;             // [2][128] 32-bit values of the step's 64 columns
+  static constexpr int kBitsOff = kVecOff + 2 * 128 * 4;
+  static constexpr int kBarOff = kBitsOff + kMaxBits / 8;
+  static constexpr int kNumBars = 18;
   static constexpr int kMiscOff = kBarOff + kNumBars * 8;
   static constexpr int kTotal = kMiscOff + 32;
   static constexpr int kAlloc = kTotal + 1024;  // slack to align the base to 1024 B
@@ -95,80 +104,91 @@ __device__ __forceinline__ uint16_t f_to_raw16(float x) {
   return static_cast<uint16_t>(pack_16x2<kBf16>(x, 0.f) & 0xFFFFu);
 }
 
-template <bool kBf16, bool kDet>
-__global__ void __launch_bounds__(kThreads, 1) bwd256_kernel(const __grid_constant__ Bwd256Params p) {
+template <bool kBf16, int kPass>
+__device__ __forceinline__ void pass256(const Bwd256Params& p, unsigned char* smem, int item) {
   using L = Smem256;
-  extern __shared__ unsigned char smem_dyn[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) &
-                                                         ~static_cast<uintptr_t>(1023));
-  unsigned char* s_k = smem + L::kKOff;
-  unsigned char* s_v = smem + L::kVOff;
-  unsigned char* s_q = smem + L::kQOff;
-  unsigned char* s_do = smem + L::kDoOff;
-  unsigned char* s_ds = smem + L::kDsOff;
-  float* s_dq = reinterpret_cast<float*>(smem + L::kDqOff);
-  float* s_ld = reinterpret_cast<float*>(smem + L::kLdOff);
-  float* s_red = reinterpret_cast<float*>(smem + L::kRedOff);
+  constexpr bool kKeys = kPass != kDq;     // stationary rows are keys
+  constexpr bool kDp = kPass != kDv;       // the pass needs dP
+  constexpr int kBSlots = kDp ? 1 : 2;
+  float* s_vec = reinterpret_cast<float*>(smem + L::kVecOff);
+  uint32_t* s_bits = reinterpret_cast<uint32_t*>(smem + L::kBitsOff);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBarOff);
-  uint64_t* bar_kv = bars;
-  uint64_t* bar_stage_full = bars + 1;
-  uint64_t* bar_stage_empty = bars + 2;
-  uint64_t* bar_s_full = bars + 3;
-  uint64_t* bar_pds = bars + 4;
-  uint64_t* bar_dq_full = bars + 5;
-  uint64_t* bar_dq_empty = bars + 6;
-  uint64_t* bar_ds_empty = bars + 7;
-  uint64_t* bar_acc_free = bars + 8;
-  uint64_t* bar_final = bars + 9;  // [2]: end of pass A, end of pass B
+  uint64_t* bar_x = bars;
+  uint64_t* bar_a_full = bars + 1;       // [2]
+  uint64_t* bar_a_empty = bars + 3;      // [2]
+  uint64_t* bar_b_full = bars + 5;       // [2], kDk and kDq use the first
+  uint64_t* bar_b_empty = bars + 7;      // [2]
+  uint64_t* bar_s_full = bars + 9;       // [2]
+  uint64_t* bar_pds = bars + 11;         // [2]
+  uint64_t* bar_vec_full = bars + 13;    // [2]
+  uint64_t* bar_vec_empty = bars + 15;   // [2]
+  uint64_t* bar_final = bars + 17;
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + L::kMiscOff);
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem + L::kMiscOff + 4);
-  int* s_active = reinterpret_cast<int*>(smem + L::kMiscOff + 8);
+  int* s_count = reinterpret_cast<int*>(smem + L::kMiscOff + 8);   // [0] active 64-key tiles, [1] visible kept keys
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int hk = blockIdx.y, b = blockIdx.z;
   const int G = p.h / p.h_k;
   const int Sq = p.seqlen_q, Sk = p.seqlen_k;
-  const int off = Sk - Sq;
   const int NT = (Sk + kBN - 1) / kBN;
-  // blockIdx.x = (query-range split, key tile): the CTA covers the 64-row query tiles [m_start, M64) of its key tile;
-  // with more than one split it leaves fp32 partials. The last ranges, never emptied by causal masking, run first.
-  const int n = blockIdx.x % NT;
-  const int split = p.nsplit - 1 - blockIdx.x / NT;
-  const int M64_all = (Sq + kBM - 1) / kBM;
-  const int m_chunk = (M64_all + p.nsplit - 1) / p.nsplit;
-  const int m_lo = split * m_chunk;
-  const int M64 = min(M64_all, m_lo + m_chunk);
   const bool causal = p.is_causal != 0;
+  // the CTA's stationary tile n, its (kv) head and batch element; key passes: its range of 64-row query tiles
+  int n, hk, b, h = 0, split = 0;
+  if (kKeys) {
+    // (query-range split, key tile): with more than one split the CTA covers the query tiles [m_start, M64) of its key tile
+    // and leaves fp32 partials. The last ranges, never emptied by causal masking, run first.
+    const int per = NT * p.nsplit;
+    n = item % per % NT;
+    split = p.nsplit - 1 - item % per / NT;
+    hk = item / per % p.h_k;
+    b = item / per / p.h_k;
+  } else {
+    const int per = p.h * p.b;  // the last query tiles, which see most keys, run first; heads of a group meet in L2
+    n = (Sq + kBN - 1) / kBN - 1 - item / per;
+    h = item % per % p.h;
+    b = item % per / p.h;
+    hk = h / G;
+  }
   const int32_t* pos_row = nullptr;  // compacted keys: the causal test runs on their original positions
   if (causal && p.key_pos)
     pos_row = p.key_pos + b * p.pos_batch_stride + (p.h_pos == p.h_k ? hk : 0) * p.pos_head_stride;
-  const int coff = pos_row ? p.causal_shift : off;
-  int m_start = 0;
-  if (pos_row) {
-    const int64_t first = (static_cast<int64_t>(pos_row[n * kBN]) - coff) / kBM;
-    m_start = static_cast<int>(max(static_cast<int64_t>(0), min(first, static_cast<int64_t>(M64))));
-  } else if (causal) {
-    m_start = max(0, (n * kBN - off) / kBM);
-  }
-  m_start = max(m_start, m_lo);
-  const WaitCtl ctl{s_abort, p.status};
+  const int coff = pos_row ? p.causal_shift : Sk - Sq;
   const int hm = p.h_mask == p.h_k ? hk : 0;  // heads of mask / bias are 1 or h_k here (or h == h_k)
   const int hb = p.h_bias == p.h_k ? hk : 0;
+  const uint8_t* mrow = p.mask ? p.mask + b * p.mask_batch_stride + hm * p.mask_head_stride : nullptr;
+  const uint16_t* brow = p.bias ? reinterpret_cast<const uint16_t*>(p.bias) + b * p.bias_batch_stride + hb * p.bias_head_stride
+                                : nullptr;
+  int m_start = 0, M64 = 0;
+  if (kKeys) {
+    const int M64_all = (Sq + kBM - 1) / kBM;
+    const int m_chunk = (M64_all + p.nsplit - 1) / p.nsplit;
+    M64 = min(M64_all, (split + 1) * m_chunk);
+    if (pos_row) {
+      const int64_t first = (static_cast<int64_t>(pos_row[n * kBN]) - coff) / kBM;
+      m_start = static_cast<int>(max(static_cast<int64_t>(0), min(first, static_cast<int64_t>(M64))));
+    } else if (causal) {
+      m_start = max(0, (n * kBN - coff) / kBM);
+    }
+    m_start = max(m_start, split * m_chunk);
+  }
+  const WaitCtl ctl{s_abort, p.status};
 
   // ---------------- set-up ----------------
   if (tid == 0) {
     *s_abort = 0;
-    mbar_init(bar_kv, 1);
-    mbar_init(bar_stage_full, 1);
-    mbar_init(bar_stage_empty, 1);
-    mbar_init(bar_s_full, 1);
-    mbar_init(bar_pds, 256);
-    mbar_init(bar_dq_full, 1);
-    mbar_init(bar_dq_empty, 128);
-    mbar_init(bar_ds_empty, 1);
-    mbar_init(bar_acc_free, 256);
-    mbar_init(bar_final + 0, 1);
-    mbar_init(bar_final + 1, 1);
+    s_count[0] = s_count[1] = 0;
+    mbar_init(bar_x, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar_a_full + i, 1);
+      mbar_init(bar_a_empty + i, 1);
+      mbar_init(bar_b_full + i, 1);
+      mbar_init(bar_b_empty + i, 1);
+      mbar_init(bar_s_full + i, 1);
+      mbar_init(bar_pds + i, 8);  // one arrival per softmax warp
+      mbar_init(bar_vec_full + i, 1);
+      mbar_init(bar_vec_empty + i, 8);
+    }
+    mbar_init(bar_final, 1);
     fence_mbar_init();
   }
   if (warp == 1) {
@@ -181,367 +201,348 @@ __global__ void __launch_bounds__(kThreads, 1) bwd256_kernel(const __grid_consta
     prefetch_tmap(&p.tm_k);
     prefetch_tmap(&p.tm_v);
   }
-  if (warp == 2) {  // does this key tile hold a kept key at all?
-    bool any = true;
-    if (p.mask) {
-      const uint8_t* mrow = p.mask + b * p.mask_batch_stride + hm * p.mask_head_stride + n * kBN;
-      any = false;
-      for (int i = lane; i < kBN; i += 32) any = any || (n * kBN + i < Sk && mrow[i] != 0);
+  // dQ pass: one activity bit per 64-key tile, where there is a mask and the table is large enough
+  const bool use_bits = !kKeys && mrow && (Sk + kBM - 1) / kBM <= kMaxBits;
+  if (use_bits)
+    for (int i = tid; i < kMaxBits / 32; i += kThreads) s_bits[i] = 0;
+  __syncthreads();
+  const int q_last = min(n * kBN + kBN, Sq) - 1;  // dQ pass: last query row of the tile
+  if (kKeys) {
+    if (warp == 2) {  // does this key tile hold a kept key at all?
+      bool any = !mrow;
+      if (mrow)
+        for (int i = lane; i < kBN; i += 32) any = any || (n * kBN + i < Sk && mrow[n * kBN + i] != 0);
       any = __any_sync(0xffffffffu, any);
+      if (lane == 0) s_count[0] = any ? 1 : 0;
     }
-    if (lane == 0) *s_active = any ? 1 : 0;
+  } else {
+    if (use_bits) {
+      for (int c = tid; c < (Sk + 15) / 16; c += kThreads) {
+        const uint4 v = *reinterpret_cast<const uint4*>(mrow + c * 16);
+        uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        if (c * 16 + 16 > Sk) {
+#pragma unroll
+          for (int e = 0; e < 16; ++e)
+            if (c * 16 + e >= Sk) w[e >> 2] &= ~(0xFFu << ((e & 3) * 8));
+        }
+        if (w[0] | w[1] | w[2] | w[3]) atomicOr(&s_bits[c >> 7], 1u << ((c >> 2) & 31));
+      }
+    }
+    if (pos_row) {  // keys the last query row sees: a prefix of the ascending positions
+      int cnt = 0;
+      for (int k = tid; k < Sk; k += kThreads) cnt += static_cast<int64_t>(pos_row[k]) <= static_cast<int64_t>(q_last) + coff ? 1 : 0;
+#pragma unroll
+      for (int s = 16; s > 0; s >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, s);
+      if (lane == 0) atomicAdd(&s_count[1], cnt);
+    }
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *s_tmem;
-  const int n_steps = (*s_active && M64 > m_start) ? (M64 - m_start) * G : 0;  // per pass
-  constexpr uint32_t kColSt = 0, kColDp = 64, kColDq = 128, kColAcc = 256;
-
-  if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-    if (warp == 0) {
-      // ---------------- TMA producer ----------------
-      if (lane == 0 && n_steps > 0) {
-        mbar_arrive_expect_tx(bar_kv, 2 * kBN * kD * 2);
-#pragma unroll
-        for (int kb = 0; kb < kD / 64; ++kb) {
-          tma_load_4d(s_k + kb * (kBN * 128), &p.tm_k, bar_kv, kb * 64, hk, n * kBN, b);
-          tma_load_4d(s_v + kb * (kBN * 128), &p.tm_v, bar_kv, kb * 64, hk, n * kBN, b);
-        }
-        int it = 0;
-        bool ok = true;
-        for (int pass = 0; pass < 2 && ok; ++pass) {
-          for (int m = m_start; m < M64 && ok; ++m) {
-            for (int g = 0; g < G; ++g) {
-              ok = mbar_wait(bar_stage_empty, (it & 1) ^ 1, ctl, kW256StageEmpty);
-              if (!ok) break;
-              mbar_arrive_expect_tx(bar_stage_full, 2 * L::kQBytes + L::kLdBytes);
-              const int h = hk * G + g;
-              const int64_t row0 = (static_cast<int64_t>(b) * p.h + h) * p.sq_r + m * kBM;
-              bulk_load_1d(s_ld, p.lse2 + row0, kBM * 4, bar_stage_full);
-              bulk_load_1d(s_ld + kBM, p.dsum + row0, kBM * 4, bar_stage_full);
-#pragma unroll
-              for (int kb = 0; kb < kD / 64; ++kb) {
-                tma_load_4d(s_q + kb * (kBM * 128), &p.tm_q, bar_stage_full, kb * 64, h, m * kBM, b);
-                tma_load_4d(s_do + kb * (kBM * 128), &p.tm_do, bar_stage_full, kb * 64, h, m * kBM, b);
-              }
-              ++it;
-            }
-          }
-        }
-      }
-    } else if (warp == 1) {
-      // ---------------- MMA issuer (whole warp, uniform control flow; the issue wrappers elect one lane) -------
-      if (n_steps > 0) {
-        constexpr uint32_t idesc_s = umma_idesc(kBN, kBM, kBf16, false, false);  // St/dPt: 128 x 64, K-major
-        constexpr uint32_t idesc_g = umma_idesc(kBN, kD, kBf16, false, true);    // dV/dK: A from TMEM, B MN-major
-        constexpr uint32_t idesc_q = umma_idesc(128, kBM, kBf16, true, true);    // dQ^T half: both MN-major
-        const uint32_t k_addr = smem_u32(s_k), v_addr = smem_u32(s_v), q_addr = smem_u32(s_q),
-                       do_addr = smem_u32(s_do), ds_addr = smem_u32(s_ds);
-        bool ok = __all_sync(0xffffffffu, mbar_wait(bar_kv, 0, ctl, kW256Kv));
-        int it = 0;
-        for (int pass = 0; pass < 2 && ok; ++pass) {
-          for (int i = 0; i < n_steps && ok; ++i, ++it) {
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_stage_full, it & 1, ctl, kW256StageFull));
-            if (!ok) break;
-            tc_fence_after_sync();
-#pragma unroll
-            for (int kk = 0; kk < kD / 16; ++kk) {  // St = K Q^T
-              const uint32_t ko = (kk >> 2) * (kBN * 128) + (kk & 3) * 32;
-              const uint32_t qo = (kk >> 2) * (kBM * 128) + (kk & 3) * 32;
-              umma_ss(tmem_base + kColSt, umma_desc_sw128(k_addr + ko, 16, 1024), umma_desc_sw128(q_addr + qo, 16, 1024),
-                      idesc_s, kk > 0 ? 1u : 0u);
-            }
-#pragma unroll
-            for (int kk = 0; kk < kD / 16; ++kk) {  // dPt = V dO^T
-              const uint32_t ko = (kk >> 2) * (kBN * 128) + (kk & 3) * 32;
-              const uint32_t qo = (kk >> 2) * (kBM * 128) + (kk & 3) * 32;
-              umma_ss(tmem_base + kColDp, umma_desc_sw128(v_addr + ko, 16, 1024),
-                      umma_desc_sw128(do_addr + qo, 16, 1024), idesc_s, kk > 0 ? 1u : 0u);
-            }
-            umma_commit(bar_s_full);
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_pds, it & 1, ctl, kW256Pds));
-            if (!ok) break;
-            tc_fence_after_sync();
-            const uint32_t acc = i > 0 ? 1u : 0u;
-            // A operands from TMEM: queries 0-31 sit in columns [0,16) of the St / dPt block, queries 32-63 in
-            // columns [32,48) (each softmax warpgroup writes back into the columns it read).
-            if (pass == 0) {
-#pragma unroll
-              for (int s = 0; s < 4; ++s) {  // dV += P^T dO
-                const uint32_t a_col = (s < 2 ? s * 8 : 32 + (s - 2) * 8);
-                umma_ts(tmem_base + kColAcc, tmem_base + kColSt + a_col,
-                        umma_desc_sw128(do_addr + s * 2048, kBM * 128, 1024), idesc_g, (acc || s > 0) ? 1u : 0u);
-              }
-              if (i > 0) {
-                ok = __all_sync(0xffffffffu, mbar_wait(bar_dq_empty, (i - 1) & 1, ctl, kW256DqEmpty));
-                if (!ok) break;
-                tc_fence_after_sync();
-              }
-#pragma unroll
-              for (int dh = 0; dh < 2; ++dh) {  // dQ^T halves = K_half^T dS^T : 8 k-steps of 16 keys
-#pragma unroll
-                for (int s = 0; s < kBN / 16; ++s) {
-                  umma_ss(tmem_base + kColDq + dh * kBM,
-                          umma_desc_sw128(k_addr + dh * 2 * (kBN * 128) + s * 2048, kBN * 128, 1024),
-                          umma_desc_sw128(ds_addr + s * 2048, 16, 1024), idesc_q, s > 0 ? 1u : 0u);
-                }
-              }
-              umma_commit(bar_dq_full);
-              umma_commit(bar_ds_empty);
-            } else {
-              if (i == 0) {  // the dV accumulator has been read out: its columns now take dK
-                ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_free, 0, ctl, kW256AccFree));
-                if (!ok) break;
-                tc_fence_after_sync();
-              }
-#pragma unroll
-              for (int s = 0; s < 4; ++s) {  // dK += dS^T Q
-                const uint32_t a_col = (s < 2 ? s * 8 : 32 + (s - 2) * 8);
-                umma_ts(tmem_base + kColAcc, tmem_base + kColDp + a_col,
-                        umma_desc_sw128(q_addr + s * 2048, kBM * 128, 1024), idesc_g, (acc || s > 0) ? 1u : 0u);
-              }
-            }
-            umma_commit(bar_stage_empty);
-          }
-          if (ok) umma_commit(bar_final + pass);
-        }
-      }
-    }
-  } else if (warp < 12) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 176;");
-    // ---------------- softmax warpgroups: thread = key = TMEM lane; warpgroup `half` takes 32 of the 64 queries ----
-    const int half = (warp - 4) >> 2;
-    const int krow = (warp & 3) * 32 + lane;
-    const int key = n * kBN + krow;
-    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const bool key_ok = key < Sk;
-    // value compared with q + coff in the causal test: the key's position (clamped so that ckey - coff cannot
-    // overflow; padding slots of a gathered key list hold INT_MAX and are masked out anyway)
-    const int ckey = pos_row ? (key_ok ? min(pos_row[key], 0x3FFFFFFF) : 0x3FFFFFFF) : key;
-    const int ckey_wmax = pos_row ? __shfl_sync(0xffffffffu, ckey, 31) : n * kBN + (warp & 3) * 32 + 31;
-    float bv = -CUDART_INF_F;  // bias*log2e of this key, or -inf when the key is masked out
-    {
-      bool kp = key_ok;
-      if (p.mask && kp) kp = p.mask[b * p.mask_batch_stride + hm * p.mask_head_stride + key] != 0;
-      if (kp)
-        bv = p.bias ? raw16_to_f<kBf16>(reinterpret_cast<const uint16_t*>(
-                          p.bias)[b * p.bias_batch_stride + hb * p.bias_head_stride + key]) * kLog2e
-                    : 0.f;
-    }
-    const int m_begin = n_steps > 0 ? m_start : M64;
-    float colsum = 0.f;
-    int it = 0;
-    bool ok = true;
-    for (int pass = 0; pass < 2; ++pass) {
-      int i = 0;  // step inside the pass
-      for (int m = m_begin; m < M64 && ok; ++m) {
-        const int q0 = m * kBM + half * 32;
-        for (int g = 0; g < G && ok; ++g, ++i, ++it) {
-          const bool diag = causal && static_cast<int64_t>(ckey_wmax) > static_cast<int64_t>(q0) + coff;  // warp-uniform
-          float2 bias2[16];
-          if (diag) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-              bias2[j] = make_float2(ckey - coff > q0 + 2 * j ? -CUDART_INF_F : bv,
-                                     ckey - coff > q0 + 2 * j + 1 ? -CUDART_INF_F : bv);
-          }
-          const float* lrow = s_ld + half * 32;
-          const float* drow = lrow + kBM;
-          // the stage barrier makes the bulk-copied LSE / D values visible; s_full covers St and dPt
-          ok = __all_sync(0xffffffffu, mbar_wait(bar_stage_full, it & 1, ctl, kW256StageFull));
-          if (!ok) break;
-          ok = __all_sync(0xffffffffu, mbar_wait(bar_s_full, it & 1, ctl, kW256SFull));
-          if (!ok) break;
-          tc_fence_after_sync();
-          uint32_t dsk[16], pk[16];
-          {
-            uint32_t rs[32], rp[32];
-            tmem_ld_x32(tmem_base + lane_addr + kColSt + half * 32, rs);
-            tmem_ld_x32(tmem_base + lane_addr + kColDp + half * 32, rp);
-            tmem_wait_ld();
-            float2 part[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-            const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
-            const float2 bv2 = make_float2(bv, bv);
-            const float2 neg1 = make_float2(-1.f, -1.f);
-#pragma unroll
-            for (int j4 = 0; j4 < 8; ++j4) {
-              const float4 l4 = reinterpret_cast<const float4*>(lrow)[j4];
-              const float4 d4 = reinterpret_cast<const float4*>(drow)[j4];
-#pragma unroll
-              for (int e = 0; e < 2; ++e) {
-                const int j = j4 * 2 + e;  // pair of queries
-                const float2 lv = e == 0 ? make_float2(l4.x, l4.y) : make_float2(l4.z, l4.w);
-                const float2 dv = e == 0 ? make_float2(d4.x, d4.y) : make_float2(d4.z, d4.w);
-                const float2 addend = __ffma2_rn(lv, neg1, diag ? bias2[j] : bv2);  // bias - LSE
-                const float2 x = __ffma2_rn(
-                    make_float2(__uint_as_float(rs[2 * j]), __uint_as_float(rs[2 * j + 1])), sc2, addend);
-                const float2 pj = make_float2(fast_exp2(x.x), fast_exp2(x.y));
-                const float2 dpd =
-                    __ffma2_rn(dv, neg1, make_float2(__uint_as_float(rp[2 * j]), __uint_as_float(rp[2 * j + 1])));
-                const float2 ds = __fmul2_rn(pj, dpd);
-                part[e] = __fadd2_rn(part[e], ds);
-                pk[j] = pack_16x2<kBf16>(pj.x, pj.y);
-                dsk[j] = pack_16x2<kBf16>(ds.x, ds.y);
-              }
-            }
-            if (pass == 0) colsum += (part[0].x + part[0].y) + (part[1].x + part[1].y);
-          }
-          if (pass == 0) tmem_st_x16(tmem_base + lane_addr + kColSt + half * 32, pk);
-          tmem_st_x16(tmem_base + lane_addr + kColDp + half * 32, dsk);
-          if (pass == 0) {
-            // dS^T tile to shared memory for the dQ products: row = key, 64 queries x 2 B = 128 B, 128-byte swizzle.
-            // The previous step's dQ products must have finished reading the tile.
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_ds_empty, (i & 1) ^ 1, ctl, kW256DsEmpty));
-            if (!ok) break;
-            unsigned char* rowp = s_ds + krow * 128;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const int chunk = (half * 4 + c) ^ (krow & 7);
-              *reinterpret_cast<uint4*>(rowp + chunk * 16) =
-                  make_uint4(dsk[c * 4], dsk[c * 4 + 1], dsk[c * 4 + 2], dsk[c * 4 + 3]);
-            }
-          }
-          tmem_wait_st();
-          fence_proxy_async_smem();
-          tc_fence_before_sync();
-          mbar_arrive(bar_pds);
-        }
-      }
-      // ---------------- end of the pass: dV (pass A) or dK (pass B); column-sum dBias after pass A ----------------
-      if (pass == 0 && p.want_dbias) {
-        if (half == 1) s_red[krow] = colsum;
-        named_bar_sync(1, 256);
-        if (half == 0 && key < p.dbias_keys) {
-          const float tot = key_ok ? colsum + s_red[krow] : 0.f;
-          if (p.dkv_part)
-            p.dbias_part[((static_cast<int64_t>(split) * p.b + b) * p.h_k + hk) * (NT * kBN) + key] = tot;
-          else
-            reinterpret_cast<uint16_t*>(p.dbias)[b * p.dbias_batch_stride + hk * p.dbias_head_stride + key] =
-                f_to_raw16<kBf16>(tot);
-        }
-      }
-      if (ok && n_steps > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_final + pass, 0, ctl, kW256Final));
-      tc_fence_after_sync();
-      if (ok) {
-        const float mul = pass == 0 ? 1.f : p.scale;
-        const int64_t krow_g = static_cast<int64_t>(min(key, Sk - 1));
-        uint16_t* dst = pass == 0 ? reinterpret_cast<uint16_t*>(p.dv) + b * p.dv_batch_stride + hk * p.dv_head_stride +
-                                        krow_g * p.dv_row_stride
-                                  : reinterpret_cast<uint16_t*>(p.dk) + b * p.dk_batch_stride + hk * p.dk_head_stride +
-                                        krow_g * p.dk_row_stride;
-        // partial: part[dv|dk][split][b][hk][key][256]
-        float* part = p.dkv_part + ((((static_cast<int64_t>(pass) * p.nsplit + split) * p.b + b) * p.h_k + hk) *
-                                        (NT * kBN) + key) * kD;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {  // this warpgroup's 128 of the 256 columns
-          const int col = half * 128 + c * 32;
-          uint32_t r[32];
-          if (n_steps > 0) {
-            tmem_ld_x32(tmem_base + lane_addr + kColAcc + col, r);
-            tmem_wait_ld();
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) r[j] = 0u;
-          }
-          if (p.dkv_part) {
-#pragma unroll
-            for (int v4 = 0; v4 < 8; ++v4)
-              *reinterpret_cast<float4*>(part + col + v4 * 4) =
-                  make_float4(__uint_as_float(r[v4 * 4 + 0]) * mul, __uint_as_float(r[v4 * 4 + 1]) * mul,
-                              __uint_as_float(r[v4 * 4 + 2]) * mul, __uint_as_float(r[v4 * 4 + 3]) * mul);
-          } else if (key_ok) {
-#pragma unroll
-            for (int v4 = 0; v4 < 4; ++v4) {
-              if (col + v4 * 8 >= p.d) break;
-              uint4 o;
-              o.x = pack_16x2<kBf16>(__uint_as_float(r[v4 * 8 + 0]) * mul, __uint_as_float(r[v4 * 8 + 1]) * mul);
-              o.y = pack_16x2<kBf16>(__uint_as_float(r[v4 * 8 + 2]) * mul, __uint_as_float(r[v4 * 8 + 3]) * mul);
-              o.z = pack_16x2<kBf16>(__uint_as_float(r[v4 * 8 + 4]) * mul, __uint_as_float(r[v4 * 8 + 5]) * mul);
-              o.w = pack_16x2<kBf16>(__uint_as_float(r[v4 * 8 + 6]) * mul, __uint_as_float(r[v4 * 8 + 7]) * mul);
-              *reinterpret_cast<uint4*>(dst + col + v4 * 8) = o;
-            }
-          }
-        }
-        if (pass == 0 && n_steps > 0) {  // the accumulator columns may now take dK
-          tc_fence_before_sync();
-          mbar_arrive(bar_acc_free);
-        }
-      }
-    }
+  int n_steps, n_sub = 0;
+  if (kKeys) {
+    n_steps = (s_count[0] && M64 > m_start) ? (M64 - m_start) * G : 0;
   } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
-    // ---------------- dQ writer (pass A only): thread = head-dim index inside a half of d (row of dQ^T) ----------
-    // Each half of dQ^T (128 d x 64 q, fp32) leaves TMEM in four pieces of 16 queries: transposed into a
-    // [16 q][128 d] fp32 staging tile in shared memory, then ONE bulk reduce-add per piece into the fp32 dQ buffer,
-    // whose (B,H,2,Sq,128) layout makes the 16 rows contiguous.
-    const int dl = (warp & 3) * 32 + lane;
-    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const int m_begin = n_steps > 0 ? m_start : M64;
-    int i = 0;
-    bool ok = true;
-    for (int m = m_begin; m < M64 && ok; ++m) {
-      for (int g = 0; g < G && ok; ++g, ++i) {
-        const int h = hk * G + g;
-        ok = __all_sync(0xffffffffu, mbar_wait(bar_dq_full, i & 1, ctl, kW256DqFull));
-        if (!ok) break;
-        tc_fence_after_sync();
+    int vis = Sk;
+    if (pos_row) vis = s_count[1];
+    else if (causal) vis = static_cast<int>(max(static_cast<int64_t>(0), min(static_cast<int64_t>(Sk), static_cast<int64_t>(q_last) + coff + 1)));
+    n_sub = (vis + kBM - 1) / kBM;
+    n_steps = n_sub;
+    if (use_bits) {
+      n_steps = 0;
+      for (int w = 0; w * 32 < n_sub; ++w)
+        n_steps += __popc(s_bits[w] & (n_sub - w * 32 >= 32 ? 0xFFFFFFFFu : (1u << (n_sub - w * 32)) - 1u));
+    }
+  }
+  // Steps: (query tile m, head g of the group), or key tile m
+  int m = kKeys ? m_start : -1, g = 0;
+  auto next = [&]() {
+    if (kKeys) {
+      if (++g == G) {
+        g = 0;
+        ++m;
+      }
+    } else {
+      do ++m;
+      while (use_bits && m < n_sub && !((s_bits[m >> 5] >> (m & 31)) & 1u));
+    }
+  };
+  if (!kKeys) next();  // to the first active tile
+  constexpr uint32_t kColS = 0, kColDp = 128, kColAcc = 256;
+  auto b_slot = [&](int i) { return smem + ((kBSlots == 2 && (i & 1)) ? L::kX2Off : L::kBOff); };
+
+  if (warp == 0) {
+    // ---------------- TMA producer ----------------
+    if (lane == 0 && n_steps > 0) {
+      const int hx = kKeys ? hk : h;
+      mbar_arrive_expect_tx(bar_x, (kDp ? 2 : 1) * L::kTile);
 #pragma unroll
-        for (int dh = 0; dh < 2; ++dh) {
-          uint32_t r0[32], r1[32];
-          tmem_ld_x32(tmem_base + lane_addr + kColDq + dh * kBM, r0);
-          tmem_ld_x32(tmem_base + lane_addr + kColDq + dh * kBM + 32, r1);
-          tmem_wait_ld();
-          if (dh == 1) {  // both halves are in registers: the dQ^T columns may be overwritten by the next step
-            tc_fence_before_sync();
-            mbar_arrive(bar_dq_empty);
-          }
-          float* gdst = p.dq_acc + (((static_cast<int64_t>(b) * p.h + h) * 2 + dh) * Sq + m * kBM) * 128;
-          if constexpr (kDet) {
-            // 64-bit fixed point: integer sums are the same in any order. 8 queries fill the staging tile.
-            long long* s_dq64 = reinterpret_cast<long long*>(s_dq);
-            long long* gdst64 = reinterpret_cast<long long*>(p.dq_acc) +
-                                (((static_cast<int64_t>(b) * p.h + h) * 2 + dh) * Sq + m * kBM) * 128;
-            constexpr float kFix = static_cast<float>(1ll << kDetFracBits);
+      for (int kb = 0; kb < kD / 64; ++kb)
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-              if (tid == 384) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-              named_bar_sync(2, 128);
+        for (int r = 0; r < 2; ++r) {
+          const int dst = kb * (kBN * 128) + r * (kBM * 128), row = n * kBN + r * kBM;
+          tma_load_4d(smem + L::kXOff + dst, kKeys ? &p.tm_k : &p.tm_q, bar_x, kb * 64, hx, row, b);
+          if (kDp) tma_load_4d(smem + L::kX2Off + dst, kKeys ? &p.tm_v : &p.tm_do, bar_x, kb * 64, hx, row, b);
+        }
+      const CUtensorMap* tm_a = kPass == kDk ? &p.tm_q : kPass == kDv ? &p.tm_do : &p.tm_k;
+      const CUtensorMap* tm_b = kPass == kDk ? &p.tm_do : kPass == kDv ? &p.tm_q : &p.tm_v;
+      bool ok = true;
+      for (int i = 0; i < n_steps && ok; ++i, next()) {
+        const int head = kKeys ? hk * G + g : hk, row = m * kBM;
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                const uint32_t raw = c < 4 ? r0[(c & 3) * 8 + j] : r1[(c & 3) * 8 + j];
-                s_dq64[j * 128 + dl] = __float2ll_rn(__uint_as_float(raw) * kFix);
-              }
-              fence_proxy_async_smem();
-              named_bar_sync(3, 128);
-              if (tid == 384) {
-                const int rows = min(8, Sq - (m * kBM + c * 8));
-                if (rows > 0) bulk_reduce_add_u64(gdst64 + c * 8 * 128, s_dq, rows * 128 * 8);
-                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-              }
-            }
-            continue;
-          }
+        for (int k = 0; k < 2; ++k) {
+          // in the order the products want them: kDv computes its scores from the other operand
+          if ((k == 0) == kDp) {
+            ok = mbar_wait(bar_a_empty + (i & 1), ((i >> 1) & 1) ^ 1, ctl, kW256AEmpty);
+            if (!ok) break;
+            mbar_arrive_expect_tx(bar_a_full + (i & 1), L::kStep);
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            if (tid == 384) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // staging tile free again
-            named_bar_sync(2, 128);
+            for (int kb = 0; kb < kD / 64; ++kb)
+              tma_load_4d(smem + L::kAOff + (i & 1) * L::kStep + kb * (kBM * 128), tm_a, bar_a_full + (i & 1), kb * 64, head, row, b);
+          } else {
+            const int slot = i % kBSlots;
+            ok = mbar_wait(bar_b_empty + slot, ((i / kBSlots) & 1) ^ 1, ctl, kW256BEmpty);
+            if (!ok) break;
+            mbar_arrive_expect_tx(bar_b_full + slot, L::kStep);
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-              s_dq[j * 128 + dl] = __uint_as_float(c < 2 ? r0[(c & 1) * 16 + j] : r1[(c & 1) * 16 + j]);
-            fence_proxy_async_smem();
-            named_bar_sync(3, 128);
-            if (tid == 384) {
-              const int rows = min(16, Sq - (m * kBM + c * 16));
-              if (rows > 0) bulk_reduce_add_f32(gdst + c * 16 * 128, s_dq, rows * 128 * 4);
-              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-            }
+            for (int kb = 0; kb < kD / 64; ++kb)
+              tma_load_4d(b_slot(i) + kb * (kBM * 128), tm_b, bar_b_full + slot, kb * 64, head, row, b);
           }
         }
       }
     }
-    if (tid == 384) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  } else if (warp == 1) {
+    // ---------------- MMA issuer (whole warp, uniform control flow; the issue wrappers elect one lane) -------
+    if (n_steps > 0) {
+      constexpr uint32_t idesc_s = umma_idesc(kBN, kBM, kBf16, false, false);  // scores, dP: 128 x 64, K-major
+      constexpr uint32_t idesc_g = umma_idesc(kBN, kD, kBf16, false, true);    // gradient: A from TMEM, B MN-major
+      const uint32_t x_addr = smem_u32(smem + L::kXOff), x2_addr = smem_u32(smem + L::kX2Off);
+      auto product = [&](uint32_t col, uint32_t x, uint32_t y) {  // [128 x 64] = x y^T
+#pragma unroll
+        for (int kk = 0; kk < kD / 16; ++kk)
+          umma_ss(tmem_base + col, umma_desc_sw128(x + (kk >> 2) * (kBN * 128) + (kk & 3) * 32, 16, 1024),
+                  umma_desc_sw128(y + (kk >> 2) * (kBM * 128) + (kk & 3) * 32, 16, 1024), idesc_s, kk > 0 ? 1u : 0u);
+      };
+      auto wait = [&](uint64_t* bar, int phase, int code) {
+        const bool r = __all_sync(0xffffffffu, mbar_wait(bar, phase & 1, ctl, code));
+        tc_fence_after_sync();
+        return r;
+      };
+      auto scores = [&](int i) {
+        const uint32_t a_addr = smem_u32(smem + L::kAOff + (i & 1) * L::kStep), b_addr = smem_u32(b_slot(i));
+        if (kDp) {
+          if (!wait(bar_a_full + (i & 1), i >> 1, kW256AFull)) return false;
+          product(kColS + (i & 1) * kBM, x_addr, a_addr);
+          if (!wait(bar_b_full, i, kW256BFull)) return false;
+          product(kColDp + (i & 1) * kBM, x2_addr, b_addr);
+        } else {
+          if (!wait(bar_b_full + (i & 1), i >> 1, kW256BFull)) return false;
+          product(kColS + (i & 1) * kBM, x_addr, b_addr);
+        }
+        umma_commit(bar_s_full + (i & 1));
+        umma_commit(bar_b_empty + i % kBSlots);
+        return true;
+      };
+      bool ok = wait(bar_x, 0, kW256X) && scores(0);
+      for (int i = 0; i < n_steps && ok; ++i) {
+        // The buffers of step i+1 were last used by step i-1: its scores by the gradient product issued before, its dP by
+        // softmax warps that have handed step i-1 over.
+        if (i + 1 < n_steps) ok = scores(i + 1);
+        if (ok) ok = wait(bar_pds + (i & 1), i >> 1, kW256Pds);
+        if (ok && !kDp) ok = wait(bar_a_full + (i & 1), i >> 1, kW256AFull);
+        if (!ok) break;
+        const uint32_t a_addr = smem_u32(smem + L::kAOff + (i & 1) * L::kStep);
+#pragma unroll
+        for (int s = 0; s < 4; ++s)  // columns 0-31 of the step sit in [0,16) of the score block, 32-63 in [32,48)
+          umma_ts(tmem_base + kColAcc, tmem_base + kColS + (i & 1) * kBM + (s < 2 ? s * 8 : 32 + (s - 2) * 8),
+                  umma_desc_sw128(a_addr + s * 2048, kBM * 128, 1024), idesc_g, (i > 0 || s > 0) ? 1u : 0u);
+        umma_commit(bar_a_empty + (i & 1));
+      }
+      if (ok) umma_commit(bar_final);
+    }
+  } else if (warp == 2) {
+    // ---------------- vectors of the step's 64 columns ----------------
+    bool ok = true;
+    for (int i = 0; i < n_steps && ok; ++i, next()) {
+      uint4 v;
+      int2 pos = make_int2(0, 0);
+      if (kKeys) {  // LSE (lanes 0-15) and D (16-31) of 64 queries
+        const int64_t row0 = (static_cast<int64_t>(b) * p.h + hk * G + g) * p.sq_r + m * kBM;
+        v = *reinterpret_cast<const uint4*>((lane < 16 ? p.lse2 : p.dsum) + row0 + (lane & 15) * 4);
+      } else {  // addend (bias in log2 units, or -inf where masked out) and position of two keys per lane
+        const int k = m * kBM + lane * 2;
+        const uint32_t mb = mrow ? *reinterpret_cast<const uint16_t*>(mrow + k) : 0x0101u;
+        const uint32_t bb = brow ? *reinterpret_cast<const uint32_t*>(brow + k) : 0u;
+        v.x = __float_as_uint(k < Sk && (mb & 0xFFu) ? raw16_to_f<kBf16>(static_cast<uint16_t>(bb & 0xFFFFu)) * kLog2e : -CUDART_INF_F);
+        v.y = __float_as_uint(k + 1 < Sk && (mb >> 8) ? raw16_to_f<kBf16>(static_cast<uint16_t>(bb >> 16)) * kLog2e : -CUDART_INF_F);
+        pos = make_int2(k, k + 1);
+        if (pos_row) pos = make_int2(k < Sk ? pos_row[k] : 0x7FFFFFFF, k + 1 < Sk ? pos_row[k + 1] : 0x7FFFFFFF);
+      }
+      ok = __all_sync(0xffffffffu, mbar_wait(bar_vec_empty + (i & 1), ((i >> 1) & 1) ^ 1, ctl, kW256VecEmpty));
+      if (!ok) break;
+      float* dst = s_vec + (i & 1) * 128;
+      if (kKeys) {
+        reinterpret_cast<uint4*>(dst)[lane] = v;
+      } else {
+        reinterpret_cast<uint2*>(dst)[lane] = make_uint2(v.x, v.y);
+        reinterpret_cast<int2*>(dst + 64)[lane] = pos;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_vec_full + (i & 1));
+    }
+  } else if (warp >= 4) {
+    // ---------------- softmax warpgroups: thread = stationary row = TMEM lane; `half` takes 32 of the 64 columns ----
+    const int half = (warp - 4) >> 2;
+    const int row = n * kBN + (warp & 3) * 32 + lane;
+    const int warp_row = n * kBN + (warp & 3) * 32;
+    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const bool row_ok = row < (kKeys ? Sk : Sq);
+    // key passes: addend of this key, and the value compared with q + coff in the causal test, its position
+    // (clamped so that ckey - coff cannot overflow; padding slots hold INT_MAX and are masked out anyway)
+    float bv = -CUDART_INF_F;
+    int ckey = 0, ckey_wmax = 0;
+    // dQ pass: LSE and D of this query, and the last position it (and the warp's first query) sees
+    float lse = CUDART_INF_F, dsum = 0.f;
+    int qlim = 0x7FFFFFFE, qlim_wmin = 0x7FFFFFFE;
+    if (kKeys) {
+      ckey = pos_row ? (row_ok ? min(pos_row[row], 0x3FFFFFFF) : 0x3FFFFFFF) : row;
+      ckey_wmax = pos_row ? __shfl_sync(0xffffffffu, ckey, 31) : warp_row + 31;
+      if (row_ok && (!mrow || mrow[row])) bv = brow ? raw16_to_f<kBf16>(brow[row]) * kLog2e : 0.f;
+    } else {
+      if (row_ok) {
+        const int64_t idx = (static_cast<int64_t>(b) * p.h + h) * p.sq_r + row;
+        lse = p.lse2[idx];
+        dsum = p.dsum[idx];
+      }
+      if (causal) {
+        auto clamp = [](int64_t x) { return static_cast<int>(max(static_cast<int64_t>(-1), min(x, static_cast<int64_t>(0x7FFFFFFE)))); };
+        qlim = clamp(static_cast<int64_t>(row) + coff);
+        qlim_wmin = clamp(static_cast<int64_t>(warp_row) + coff);
+      }
+    }
+    float colsum = 0.f;
+    bool ok = true;
+    const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
+    const float2 neg1 = make_float2(-1.f, -1.f);
+    for (int i = 0; i < n_steps && ok; ++i, next()) {
+      const float* vec = s_vec + (i & 1) * 128 + half * 32;
+      ok = __all_sync(0xffffffffu, mbar_wait(bar_vec_full + (i & 1), (i >> 1) & 1, ctl, kW256VecFull));
+      if (!ok) break;
+      ok = __all_sync(0xffffffffu, mbar_wait(bar_s_full + (i & 1), (i >> 1) & 1, ctl, kW256SFull));
+      if (!ok) break;
+      tc_fence_after_sync();
+      uint32_t rs[32], rp[32], pk[16];
+      tmem_ld_x32(tmem_base + lane_addr + kColS + (i & 1) * kBM + half * 32, rs);
+      if (kDp) tmem_ld_x32(tmem_base + lane_addr + kColDp + (i & 1) * kBM + half * 32, rp);
+      tmem_wait_ld();
+      const int* pos = reinterpret_cast<const int*>(vec + 64);
+      const int q0 = m * kBM + half * 32;
+      const bool diag = causal && (kKeys ? static_cast<int64_t>(ckey_wmax) > static_cast<int64_t>(q0) + coff
+                                         : pos[31] > qlim_wmin);  // warp-uniform
+      float2 part[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+      for (int j4 = 0; j4 < 8; ++j4) {
+        const float4 v4 = reinterpret_cast<const float4*>(vec)[j4];
+        float4 d4 = make_float4(dsum, dsum, dsum, dsum);
+        if (kKeys && kDp) d4 = reinterpret_cast<const float4*>(vec + 64)[j4];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int j = j4 * 2 + e;  // pair of columns
+          const float2 vv = e == 0 ? make_float2(v4.x, v4.y) : make_float2(v4.z, v4.w);
+          const float2 dv = e == 0 ? make_float2(d4.x, d4.y) : make_float2(d4.z, d4.w);
+          float2 add;  // bias - LSE, or -inf
+          if (kKeys) {
+            float2 b2 = make_float2(bv, bv);
+            if (diag) {
+              if (ckey - coff > q0 + 2 * j) b2.x = -CUDART_INF_F;
+              if (ckey - coff > q0 + 2 * j + 1) b2.y = -CUDART_INF_F;
+            }
+            add = __ffma2_rn(vv, neg1, b2);
+          } else {
+            add = __fadd2_rn(vv, make_float2(-lse, -lse));
+            if (diag) {
+              if (pos[2 * j] > qlim) add.x = -CUDART_INF_F;
+              if (pos[2 * j + 1] > qlim) add.y = -CUDART_INF_F;
+            }
+          }
+          const float2 x = __ffma2_rn(make_float2(__uint_as_float(rs[2 * j]), __uint_as_float(rs[2 * j + 1])), sc2, add);
+          const float2 pj = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+          if (kDp) {
+            const float2 dpd = __ffma2_rn(dv, neg1, make_float2(__uint_as_float(rp[2 * j]), __uint_as_float(rp[2 * j + 1])));
+            const float2 ds = __fmul2_rn(pj, dpd);
+            if (kPass == kDk) part[e] = __fadd2_rn(part[e], ds);
+            pk[j] = pack_16x2<kBf16>(ds.x, ds.y);
+          } else {
+            pk[j] = pack_16x2<kBf16>(pj.x, pj.y);
+          }
+        }
+      }
+      if (kPass == kDk) colsum += (part[0].x + part[0].y) + (part[1].x + part[1].y);
+      tmem_st_x16(tmem_base + lane_addr + kColS + (i & 1) * kBM + half * 32, pk);
+      tmem_wait_st();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(bar_vec_empty + (i & 1));
+        mbar_arrive(bar_pds + (i & 1));
+      }
+    }
+    // ---------------- the gradient tile; dBias sums of the dK pass ----------------
+    if (kPass == kDk && p.want_dbias) {
+      named_bar_sync(1, 256);  // the step vectors have been read: their place takes the sums of the second half
+      if (half == 1) s_vec[row - n * kBN] = colsum;
+      named_bar_sync(1, 256);
+      if (half == 0 && row < p.dbias_keys) {
+        const float tot = row_ok ? colsum + s_vec[row - n * kBN] : 0.f;
+        if (p.dkv_part)
+          p.dbias_part[((static_cast<int64_t>(split) * p.b + b) * p.h_k + hk) * (NT * kBN) + row] = tot;
+        else
+          reinterpret_cast<uint16_t*>(p.dbias)[b * p.dbias_batch_stride + hk * p.dbias_head_stride + row] = f_to_raw16<kBf16>(tot);
+      }
+    }
+    if (ok && n_steps > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_final, 0, ctl, kW256Final));
+    tc_fence_after_sync();
+    if (ok) {
+      const float mul = kPass == kDv ? 1.f : p.scale;
+      const int64_t row_g = min(row, (kKeys ? Sk : Sq) - 1);
+      uint16_t* dst = kPass == kDv   ? reinterpret_cast<uint16_t*>(p.dv) + b * p.dv_batch_stride + hk * p.dv_head_stride + row_g * p.dv_row_stride
+                      : kPass == kDk ? reinterpret_cast<uint16_t*>(p.dk) + b * p.dk_batch_stride + hk * p.dk_head_stride + row_g * p.dk_row_stride
+                                     : reinterpret_cast<uint16_t*>(p.dq) + b * p.dq_batch_stride + h * p.dq_head_stride + row_g * p.dq_row_stride;
+      // partial: part[dv|dk][split][b][hk][key][256]
+      float* part = p.dkv_part + ((((static_cast<int64_t>(kPass == kDk ? 1 : 0) * p.nsplit + split) * p.b + b) * p.h_k + hk) *
+                                      (NT * kBN) + row) * kD;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {  // this warpgroup's 128 of the 256 columns
+        const int col = half * 128 + c * 32;
+        uint32_t r[32];
+        if (n_steps > 0) {
+          tmem_ld_x32(tmem_base + lane_addr + kColAcc + col, r);
+          tmem_wait_ld();
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) r[j] = 0u;
+        }
+        if (kKeys && p.dkv_part) {
+#pragma unroll
+          for (int v4 = 0; v4 < 8; ++v4)
+            *reinterpret_cast<float4*>(part + col + v4 * 4) =
+                make_float4(__uint_as_float(r[v4 * 4 + 0]) * mul, __uint_as_float(r[v4 * 4 + 1]) * mul,
+                            __uint_as_float(r[v4 * 4 + 2]) * mul, __uint_as_float(r[v4 * 4 + 3]) * mul);
+        } else if (row_ok) {
+#pragma unroll
+          for (int v4 = 0; v4 < 4; ++v4) {
+            if (col + v4 * 8 >= p.d) break;
+            uint4 o;
+            o.x = pack_16x2<kBf16>(__uint_as_float(r[v4 * 8 + 0]) * mul, __uint_as_float(r[v4 * 8 + 1]) * mul);
+            o.y = pack_16x2<kBf16>(__uint_as_float(r[v4 * 8 + 2]) * mul, __uint_as_float(r[v4 * 8 + 3]) * mul);
+            o.z = pack_16x2<kBf16>(__uint_as_float(r[v4 * 8 + 4]) * mul, __uint_as_float(r[v4 * 8 + 5]) * mul);
+            o.w = pack_16x2<kBf16>(__uint_as_float(r[v4 * 8 + 6]) * mul, __uint_as_float(r[v4 * 8 + 7]) * mul);
+            *reinterpret_cast<uint4*>(dst + col + v4 * 8) = o;
+          }
+        }
+      }
+    }
   }
 
   // ---------------- tear-down ----------------
@@ -553,20 +554,32 @@ __global__ void __launch_bounds__(kThreads, 1) bwd256_kernel(const __grid_consta
   }
 }
 
+template <bool kBf16>
+__global__ void __launch_bounds__(kThreads, 1) bwd256_kernel(const __grid_constant__ Bwd256Params p) {
+  extern __shared__ unsigned char smem_dyn[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) &
+                                                         ~static_cast<uintptr_t>(1023));
+  const int item = blockIdx.x;
+  if (item < p.n_kv_ctas) pass256<kBf16, kDk>(p, smem, item);
+  else if (item < 2 * p.n_kv_ctas) pass256<kBf16, kDv>(p, smem, item - p.n_kv_ctas);
+  else pass256<kBf16, kDq>(p, smem, item - 2 * p.n_kv_ctas);
+}
+
 struct Plan256 {
   int sq_r, nsplit;
   bool want_dbias;
   bool part;  // dK, dV and column sums leave the main kernel as fp32 partials
-  size_t lse2_off, dsum_off, dq_off, part_off, dbpart_off, total;
+  size_t lse2_off, dsum_off, part_off, dbpart_off, total;
 };
 
-// Query-range splits per key tile: as in the d = 128 kernel, a grid that cannot fill the GPU twice is cut along the
-// query dimension until about eight CTAs per SM exist; every split keeps at least 32 steps.
+// Query-range splits per key tile: a grid that cannot fill the GPU twice is cut along the query dimension until each of the
+// two key passes has about two CTAs per SM (the many short CTAs of the dQ pass, last in the launch, even out what is left);
+// every split keeps at least 32 steps. More splits only add partials: 37 instead of 19 at 2048 kept keys write and read 80 MB more.
 int pick_nsplit256(const fdma_fwd_params& p) {
   const int64_t ctas = static_cast<int64_t>((p.seqlen_k + kBN - 1) / kBN) * p.h_k * p.b;
   if (ctas >= 2 * sm_count()) return 1;
   const int64_t steps = static_cast<int64_t>((p.seqlen_q + kBM - 1) / kBM) * (p.h / p.h_k);
-  const int64_t want = (8 * sm_count() + ctas - 1) / ctas;
+  const int64_t want = (2 * sm_count() + ctas - 1) / ctas;
   const int64_t cap = std::max<int64_t>(1, steps / 32);
   return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(std::min(want, cap), 64)));
 }
@@ -581,7 +594,6 @@ Plan256 plan256(const fdma_bwd_params& bp) {
   const size_t rows = static_cast<size_t>(p.b) * p.h * pl.sq_r;
   pl.lse2_off = o; o += align256(rows * 4);
   pl.dsum_off = o; o += align256(rows * 4);
-  pl.dq_off = o;   o += align256(static_cast<size_t>(p.b) * p.seqlen_q * p.h * kD * (bp.deterministic ? 8 : 4));
   pl.part_off = pl.dbpart_off = o;
   pl.part = pl.nsplit > 1 || bp.scatter_pos != nullptr;
   if (pl.part) {
@@ -602,8 +614,7 @@ int launch256(const fdma_bwd_params& bp, const Plan256& pl, cudaStream_t stream)
   if (!p.workspace || p.workspace_bytes < pl.total) return FDMA_ERR_WORKSPACE;
   char* ws = static_cast<char*>(p.workspace);
   Bwd256Params kp;
-  auto encode = [&](CUtensorMap* tm, const void* base, int heads, int rows, int box_rows, int64_t sb, int64_t sr,
-                    int64_t sh) {
+  auto encode = [&](CUtensorMap* tm, const void* base, int heads, int rows, int64_t sb, int64_t sr, int64_t sh) {
     if (heads == 1) sh = p.d;
     if (rows == 1) sr = static_cast<int64_t>(heads) * p.d;
     if (p.b == 1) sb = static_cast<int64_t>(rows) * heads * p.d;
@@ -611,25 +622,24 @@ int launch256(const fdma_bwd_params& bp, const Plan256& pl, cudaStream_t stream)
                               static_cast<uint64_t>(p.b)};
     const uint64_t str[3] = {static_cast<uint64_t>(sh) * 2, static_cast<uint64_t>(sr) * 2,
                              static_cast<uint64_t>(sb) * 2};
-    const uint32_t box[4] = {64, 1, static_cast<uint32_t>(box_rows), 1};
+    const uint32_t box[4] = {64, 1, static_cast<uint32_t>(kBM), 1};
     return encode_tmap_4d(tm, base, 2, dims, str, box);
   };
-  int st = encode(&kp.tm_q, p.q, p.h, p.seqlen_q, kBM, p.q_batch_stride, p.q_row_stride, p.q_head_stride);
+  int st = encode(&kp.tm_q, p.q, p.h, p.seqlen_q, p.q_batch_stride, p.q_row_stride, p.q_head_stride);
   if (st) return st;
-  st = encode(&kp.tm_do, bp.dout, p.h, p.seqlen_q, kBM, bp.do_batch_stride, bp.do_row_stride, bp.do_head_stride);
+  st = encode(&kp.tm_do, bp.dout, p.h, p.seqlen_q, bp.do_batch_stride, bp.do_row_stride, bp.do_head_stride);
   if (st) return st;
-  st = encode(&kp.tm_k, p.k, p.h_k, p.seqlen_k, kBN, p.k_batch_stride, p.k_row_stride, p.k_head_stride);
+  st = encode(&kp.tm_k, p.k, p.h_k, p.seqlen_k, p.k_batch_stride, p.k_row_stride, p.k_head_stride);
   if (st) return st;
-  st = encode(&kp.tm_v, p.v, p.h_k, p.seqlen_k, kBN, p.v_batch_stride, p.v_row_stride, p.v_head_stride);
+  st = encode(&kp.tm_v, p.v, p.h_k, p.seqlen_k, p.v_batch_stride, p.v_row_stride, p.v_head_stride);
   if (st) return st;
 
   float* lse2 = reinterpret_cast<float*>(ws + pl.lse2_off);
   float* dsum = reinterpret_cast<float*>(ws + pl.dsum_off);
-  float* dq_acc = reinterpret_cast<float*>(ws + pl.dq_off);
   {
     BwdPrepArgs a;
-    a.out = p.out; a.dout = bp.dout; a.lse = p.lse; a.lse2 = lse2; a.dsum = dsum; a.dq_acc = dq_acc;
-    a.b = p.b; a.h = p.h; a.sq = p.seqlen_q; a.sq_r = pl.sq_r; a.d = p.d; a.acc_bytes = bp.deterministic ? 8 : 4;
+    a.out = p.out; a.dout = bp.dout; a.lse = p.lse; a.lse2 = lse2; a.dsum = dsum; a.dq_acc = nullptr;
+    a.b = p.b; a.h = p.h; a.sq = p.seqlen_q; a.sq_r = pl.sq_r; a.d = p.d; a.acc_bytes = 0;
     a.o_sb = p.o_batch_stride; a.o_sr = p.o_row_stride; a.o_sh = p.o_head_stride;
     a.do_sb = bp.do_batch_stride; a.do_sr = bp.do_row_stride; a.do_sh = bp.do_head_stride;
     st = launch_bwd_prep(a, kD, kBf16, stream);
@@ -641,7 +651,7 @@ int launch256(const fdma_bwd_params& bp, const Plan256& pl, cudaStream_t stream)
   kp.bias = p.bias;
   kp.lse2 = lse2;
   kp.dsum = dsum;
-  kp.dq_acc = dq_acc;
+  kp.dq = bp.dq;
   kp.dk = bp.dk;
   kp.dv = bp.dv;
   kp.dbias = bp.dbias;
@@ -651,6 +661,7 @@ int launch256(const fdma_bwd_params& bp, const Plan256& pl, cudaStream_t stream)
   if (!kp.status) return FDMA_ERR_DRIVER;
   kp.mask_batch_stride = p.mask_batch_stride; kp.mask_head_stride = p.mask_head_stride;
   kp.bias_batch_stride = p.bias_batch_stride; kp.bias_head_stride = p.bias_head_stride;
+  kp.dq_batch_stride = bp.dq_batch_stride; kp.dq_row_stride = bp.dq_row_stride; kp.dq_head_stride = bp.dq_head_stride;
   kp.dk_batch_stride = bp.dk_batch_stride; kp.dk_row_stride = bp.dk_row_stride; kp.dk_head_stride = bp.dk_head_stride;
   kp.dv_batch_stride = bp.dv_batch_stride; kp.dv_row_stride = bp.dv_row_stride; kp.dv_head_stride = bp.dv_head_stride;
   kp.dbias_batch_stride = bp.dbias_batch_stride; kp.dbias_head_stride = bp.dbias_head_stride;
@@ -669,10 +680,14 @@ int launch256(const fdma_bwd_params& bp, const Plan256& pl, cudaStream_t stream)
   kp.scale_log2 = p.softmax_scale * kLog2e;
   kp.scale = p.softmax_scale;
 
-  auto kern = bp.deterministic ? bwd256_kernel<kBf16, true> : bwd256_kernel<kBf16, false>;
+  auto kern = bwd256_kernel<kBf16>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem256::kAlloc);
   if (e != cudaSuccess) return static_cast<int>(e);
-  dim3 grid(((p.seqlen_k + kBN - 1) / kBN) * pl.nsplit, p.h_k, p.b);
+  const int64_t kv = static_cast<int64_t>((p.seqlen_k + kBN - 1) / kBN) * pl.nsplit * p.h_k * p.b;
+  const int64_t ctas = 2 * kv + static_cast<int64_t>((p.seqlen_q + kBN - 1) / kBN) * p.h * p.b;
+  if (ctas > 0x7FFFFFFF) return FDMA_ERR_TOO_LARGE;
+  kp.n_kv_ctas = static_cast<int>(kv);
+  const dim3 grid(static_cast<unsigned>(ctas));
   cudaEvent_t ev0, ev1;
   take_timing_events(&ev0, &ev1);
   if (ev0) cudaEventRecord(ev0, stream);
@@ -682,9 +697,6 @@ int launch256(const fdma_bwd_params& bp, const Plan256& pl, cudaStream_t stream)
   if (e != cudaSuccess) return static_cast<int>(e);
 
   BwdFinishArgs f = {};
-  f.dq_acc = dq_acc; f.dq = bp.dq; f.dsum = dsum;
-  f.dq_sb = bp.dq_batch_stride; f.dq_sr = bp.dq_row_stride; f.dq_sh = bp.dq_head_stride;
-  f.scale = p.softmax_scale;
   f.b = p.b; f.h = p.h; f.sq = p.seqlen_q; f.sq_r = pl.sq_r; f.d = p.d; f.D = kD;
   f.h_k = p.h_k; f.keys_r = static_cast<int>(round_up(p.seqlen_k, kBN));
   f.rows_out = bp.scatter_pos ? bp.scatter_rows : p.seqlen_k;
@@ -702,7 +714,7 @@ int launch256(const fdma_bwd_params& bp, const Plan256& pl, cudaStream_t stream)
       f.dbias = bp.dbias; f.db_sb = bp.dbias_batch_stride; f.db_sh = bp.dbias_head_stride;
     }
   }
-  return launch_bwd_finish(f, kBf16, bp.deterministic != 0, stream);
+  return launch_bwd_finish(f, kBf16, false, stream);
 }
 
 }  // namespace

@@ -1,5 +1,5 @@
 // The two small kernels on either side of every tensor-core backward kernel (head dims 64, 128, 256):
-//   bwd_prep_kernel    D = rowsum(dO o O), LSE in log2 units, and the zero fill of the fp32 dQ accumulator
+//   bwd_prep_kernel    D = rowsum(dO o O), LSE in log2 units, and the zero fill of the fp32 dQ accumulator (head dims up to 128)
 //   bwd_finish_kernel  dQ accumulator -> 16-bit dQ; sum of the query-range partials -> 16-bit dK, dV; fp32 column sums
 //                      -> 16-bit dBias; for gathered keys every gradient row goes straight to its key's position and all
 //                      other rows are written as zeros
@@ -58,16 +58,10 @@ __global__ void __launch_bounds__(kThreads) bwd_prep_kernel(const BwdPrepArgs a)
       y[u] = *reinterpret_cast<const uint4*>(g + static_cast<int64_t>(q) * a.do_sr);
     }
   }
-  {  // accumulator rows of this warp: (B,H,D/kPitch,Sq,kPitch) elements of acc_bytes each
-    constexpr int kPitch = D < 128 ? D : 128;
-    const int rows = min(8, a.sq - q0);
-#pragma unroll
-    for (int half = 0; half < D / kPitch; ++half) {
-      char* base = static_cast<char*>(a.dq_acc) +
-                   ((static_cast<int64_t>(bh) * (D / kPitch) + half) * a.sq + q0) * kPitch * a.acc_bytes;
-      const int n16 = rows * kPitch * a.acc_bytes / 16;
-      for (int i = lane; i < n16; i += 32) reinterpret_cast<uint4*>(base)[i] = make_uint4(0, 0, 0, 0);
-    }
+  if (D <= 128) {  // accumulator rows of this warp: (B,H,Sq,D) elements of acc_bytes each
+    char* base = static_cast<char*>(a.dq_acc) + (static_cast<int64_t>(bh) * a.sq + q0) * D * a.acc_bytes;
+    const int n16 = min(8, a.sq - q0) * D * a.acc_bytes / 16;
+    for (int i = lane; i < n16; i += 32) reinterpret_cast<uint4*>(base)[i] = make_uint4(0, 0, 0, 0);
   }
 #pragma unroll
   for (int u = 0; u < kPasses; ++u) {
@@ -197,17 +191,14 @@ __global__ void __launch_bounds__(kThreads) bwd_finish_kernel(const BwdFinishArg
     return;
   }
   blk -= a.db_blocks;
-  // ---- dQ: accumulator (B,H,D/pitch,Sq,pitch) * scale -> (B,Sq,H,d) 16-bit ----
+  // ---- dQ: accumulator (B,H,Sq,D), D = 64 or 128, * scale -> (B,Sq,H,d) 16-bit ----
   const uint32_t dq_blocks = gridDim.x - a.kv_blocks - a.db_blocks;
-  const int pitch_log2 = a.D >= 128 ? 7 : 6;
-  const int halves = a.D >> pitch_log2;
-  const uint32_t vec_log2 = pitch_log2 - 3;
-  const int64_t n_vec = (static_cast<int64_t>(a.b) * a.h * halves * a.sq) << vec_log2;
+  const uint32_t vec_log2 = a.D == 128 ? 4 : 3;
+  const int64_t n_vec = (static_cast<int64_t>(a.b) * a.h * a.sq) << vec_log2;
   for (int64_t i = blk * static_cast<int64_t>(kThreads) + tid; i < n_vec; i += static_cast<int64_t>(dq_blocks) * kThreads) {
     const uint32_t row = static_cast<uint32_t>(i >> vec_log2);
-    const uint32_t hh = row / a.sq, q = row - hh * a.sq;
-    const uint32_t bh = halves == 1 ? hh : hh >> 1;
-    const int dd = (static_cast<int>(i) & ((1 << vec_log2) - 1)) * 8 + (halves == 1 ? 0 : (hh & 1) << pitch_log2);
+    const uint32_t bh = row / a.sq, q = row - bh * a.sq;
+    const int dd = (static_cast<int>(i) & ((1 << vec_log2) - 1)) * 8;
     if (dd >= a.d) continue;
     const uint32_t b = bh / a.h, h = bh - b * a.h;
     float x[8];
@@ -271,7 +262,8 @@ int launch_bwd_finish(BwdFinishArgs a, bool bf16, bool deterministic, cudaStream
   }
   // dQ rows: a grid-stride loop of at least four 32-byte pieces per thread on large tensors
   const int64_t n_vec = static_cast<int64_t>(a.b) * a.h * a.sq * (a.D / 8);
-  const int64_t dq = std::max<int64_t>(1, std::min<int64_t>((n_vec + kThreads - 1) / kThreads, sm_count() * 32));
+  const int64_t dq = a.dq_acc ? std::max<int64_t>(1, std::min<int64_t>((n_vec + kThreads - 1) / kThreads, sm_count() * 32)) : 0;
+  if (kv + db + dq == 0) return 0;
   if (kv + db + dq > 0x7FFFFFFF) return FDMA_ERR_TOO_LARGE;
   a.kv_blocks = static_cast<int>(kv);
   a.db_blocks = static_cast<int>(db);

@@ -46,14 +46,14 @@ struct BwdPrepArgs {
   const void *out, *dout;
   const float* lse;
   float *lse2, *dsum;  // (B,H,sq_r)
-  void* dq_acc;        // zeroed: (B,H,D/min(D,128),Sq,min(D,128)) elements of acc_bytes
+  void* dq_acc;        // D <= 128: zeroed, (B,H,Sq,D) elements of acc_bytes
   int b, h, sq, sq_r, d, acc_bytes;
   int64_t o_sb, o_sr, o_sh, do_sb, do_sr, do_sh;
 };
 int launch_bwd_prep(const BwdPrepArgs& a, int D, bool bf16, cudaStream_t stream);
 
 struct BwdFinishArgs {
-  // dQ
+  // dQ, or dq_acc = null (already written by the main kernel)
   const void* dq_acc;
   void* dq;
   const float* dsum;  // deterministic mode: rows with a non-finite D become NaN
