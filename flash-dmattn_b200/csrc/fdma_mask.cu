@@ -642,7 +642,7 @@ void launch_reg(const fdma_mask_params& p, unsigned rows, cudaStream_t stream) {
 // memory. The first digit has 11 bits, the second 5: an 8-bit first digit is sign and exponent of a bfloat16, four to
 // six values in all for normally distributed biases, and its shared-memory atomics serialise.
 // Bound by latency: loads, four cluster barriers and the passes over a CTA's keys. One CTA per row before, now: 1 row of 65536 keys
-// 99 -> 17 us, 8 x 32768 51 -> 13.5 us, 8 x 3001 9.8 -> 7.2 us, 256 x 65536 170 -> 151 us.
+// 99 -> 16 us, 8 x 32768 51 -> 13 us, 8 x 3001 9.8 -> 7.2 us, 256 x 65536 170 -> 139 us (148 with the row's stores ahead of the last exchange).
 // ---------------------------------------------------------------------------------------------------------
 constexpr int kBins = 2048;
 constexpr int kMaxRowCtas = 8;
@@ -706,17 +706,24 @@ __global__ void __launch_bounds__(kThreads, CHUNKS <= 4 ? 4 : 2) topk16_cluster_
       }
     }
     const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
-    const uint32_t mb[2] = {m.x, m.y};
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const uint32_t two = mb[w >> 1] >> ((w & 1) * 16);  // bytes of keys 2w, 2w+1
-      const uint32_t keep = ((two & 0xFFu) ? 0x0000FFFFu : 0u) | ((two & 0xFF00u) ? 0xFFFF0000u : 0u);
-      const uint32_t key = (key_pair16<DT>(vw[w]) & keep) | (min2 & ~keep);
-      const uint32_t real = (k + 2 * w < k_hi ? 0x0000FFFFu : 0u) | (k + 2 * w + 1 < k_hi ? 0xFFFF0000u : 0u);
-      kw[c][w] = key & real;
+    for (int w = 0; w < 4; ++w) kw[c][w] = key_pair16<DT>(vw[w]);
+    if (rp.pm) {
+      const uint32_t mb[2] = {m.x, m.y};
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const uint32_t two = mb[w >> 1] >> ((w & 1) * 16);  // bytes of keys 2w, 2w+1
+        const uint32_t keep = ((two & 0xFFu) ? 0x0000FFFFu : 0u) | ((two & 0xFF00u) ? 0xFFFF0000u : 0u);
+        kw[c][w] = (kw[c][w] & keep) | (min2 & ~keep);
+      }
+    }
+    if (k + kPerThread > k_hi) {  // past the end of the segment
+#pragma unroll
+      for (int w = 0; w < 4; ++w)
+        kw[c][w] &= (k + 2 * w < k_hi ? 0x0000FFFFu : 0u) | (k + 2 * w + 1 < k_hi ? 0xFFFF0000u : 0u);
     }
   }
-  for (int i = tid; i < kBins; i += kThreads) s_hist[i] = 0;
+  for (int i = tid; i < kBins / 4; i += kThreads) reinterpret_cast<int4*>(s_hist)[i] = make_int4(0, 0, 0, 0);
   if (tid < 32) s_low[tid] = 0;
   __syncthreads();
   // ---- first digit ----
@@ -864,6 +871,27 @@ __global__ void __launch_bounds__(kThreads, CHUNKS <= 4 ? 4 : 2) topk16_cluster_
       sel[c] = bits;
     }
   }
+  // ---- selected keys in the CTAs before this one; then the last reads of other CTAs' shared memory are done. The row's global
+  // stores come after, so that no cluster barrier waits for them ----
+  int slot0[CHUNKS], before = 0, total = 0;
+  if (p.key_pos) {
+    int cnt[CHUNKS];
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) cnt[c] = __popc(sel[c]);
+    total = scan_counts(cnt, slot0);
+    if (nrank > 1) {
+      if (tid == 0) s_selected = total;
+      cluster.sync();
+      total = 0;
+      for (int r = 0; r < nrank; ++r) {
+        const int v = *cluster.map_shared_rank(&s_selected, r);
+        if (r < rank) before += v;
+        total += v;
+      }
+    }
+  }
+  __syncwarp();
+  if (nrank > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   if (rp.out) {
     const bool vec_out = (reinterpret_cast<uintptr_t>(rp.out) & 7u) == 0;
 #pragma unroll
@@ -891,20 +919,6 @@ __global__ void __launch_bounds__(kThreads, CHUNKS <= 4 ? 4 : 2) topk16_cluster_
     }
   }
   if (p.key_pos) {  // ascending positions of the selected keys
-    int cnt[CHUNKS], slot0[CHUNKS];
-#pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) cnt[c] = __popc(sel[c]);
-    const int mine = scan_counts(cnt, slot0);
-    int before = 0, total = mine;
-    if (nrank > 1) {
-      if (tid == 0) s_selected = mine;
-      cluster.sync();
-      for (int r = 0; r < nrank; ++r) {
-        const int v = *cluster.map_shared_rank(&s_selected, r);
-        if (r < rank) before += v;
-        if (r != rank) total += v;
-      }
-    }
     int32_t* prow = p.key_pos + row * p.capacity;
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {
@@ -919,7 +933,8 @@ __global__ void __launch_bounds__(kThreads, CHUNKS <= 4 ? 4 : 2) topk16_cluster_
     }
     finish_positions(p, row, total, rank * kThreads + tid, nrank * kThreads);
   }
-  if (nrank > 1) cluster.sync();  // nobody leaves while its shared memory may still be read
+  __syncwarp();
+  if (nrank > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // nobody leaves while its shared memory may still be read
 }
 
 template <int DT, int CHUNKS>
