@@ -280,13 +280,15 @@ variable_list AttnBackward::apply_packed(const Tensor& tq, const Tensor& tk, con
 variable_list AttnBackward::apply(variable_list&& grads) {
   variable_list res(4);
   if (!grads[0].defined()) return res;
+  // Unpacked before anything is switched off: a hook may recompute the region the call belongs to (checkpointing), which
+  // has to record a graph of its own while it does.
+  const Tensor tq = q.unpack(), tk = k.unpack(), tv = v.unpack(), tmask = mask.unpack(), tbias = bias.unpack(),
+               tlse = lse.unpack(), textra = extra.unpack(), tout = out.unpack(getptr());
   at::AutoDispatchBelowADInplaceOrView guard;
-  const Tensor tq = q.unpack(), tk = k.unpack(), tmask = mask.unpack(), tlse = lse.unpack(), textra = extra.unpack();
-  const Tensor tout = out.unpack(getptr());
   const c10::cuda::CUDAGuard device(tq.device());
   const cudaStream_t stream = stream_of(tq);
   raise_if_timed_out(stream);
-  if (c.packed) return apply_packed(tq, tk, v.unpack(), tout, tlse, textra, grads[0].contiguous(), stream);
+  if (c.packed) return apply_packed(tq, tk, tv, tout, tlse, textra, grads[0].contiguous(), stream);
   const Tensor dout = inner_contiguous(grads[0]);
 
   fdma_bwd_params bp = {};
@@ -304,7 +306,6 @@ variable_list AttnBackward::apply(variable_list&& grads) {
     bp.scatter_rows = static_cast<int32_t>(c.seqlen_k);
     if (want_bias) dbias = empty(bias_sizes, tq.scalar_type(), tq);
   } else {
-    const Tensor tv = v.unpack(), tbias = bias.unpack();
     dk = empty_as(tk);
     dv = empty_as(tv);
     fill_geometry(bp.f, tq, tk.size(1), tk.size(2), c);

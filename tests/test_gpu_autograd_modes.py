@@ -1,0 +1,76 @@
+"""The autograd node of the native host path under the autograd features a training program combines it with: saved-tensor
+hooks and checkpointing, compiled autograd, second derivatives, threads that share a graph, tracing. The results are compared
+with those of a plain call, bit for bit (deterministic gradients)."""
+import threading
+
+import pytest
+import torch
+
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+DTYPE = torch.bfloat16
+ROUTES = ["gathered", "bits", "dense", "packed"]
+
+
+@pytest.fixture(scope="module")
+def dev():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    return torch.device("cuda:0")
+
+
+def make(dev, route, d=64, seed=3):
+    """(leaves, dout, call): one attention call on the given route of the native path as a function of its leaves."""
+    from flash_sparse_attn import flash_sparse_attn_func, flash_sparse_attn_varlen_func
+    from flash_sparse_attn.utils.mask import create_mask
+
+    B, S, H, Hk = 2, 256, 4, 2
+    rows = S if route == "bits" else 1
+    q, k, v, bias, dout = (t.to(dev) for t in oracle.make_inputs(B, S, S, H, Hk, d, (B, Hk, rows, S), seed=seed, dtype=DTYPE))
+    if route == "packed":
+        leaves = [t.reshape(B * S, -1, d).requires_grad_(True) for t in (q, k, v)]
+        cu = torch.tensor([0, 200, B * S], device=dev, dtype=torch.int32)
+
+        def call(q, k, v):
+            return flash_sparse_attn_varlen_func(q, k, v, cu, cu, 312, 312, is_causal=True, deterministic=True)
+
+        return leaves, dout.reshape(B * S, H, d), call
+    leaves = [t.requires_grad_(True) for t in (q, k, v, bias)]
+    mask = create_mask(bias.detach(), None, B, S, S, 100, torch.finfo(DTYPE).min) if route != "dense" else None
+
+    def call(q, k, v, bias):
+        return flash_sparse_attn_func(q, k, v, mask, bias, is_causal=True, deterministic=True)
+
+    return leaves, dout, call
+
+
+def plain(leaves, dout, call):
+    out = call(*leaves)
+    assert out.grad_fn.name() == "FlashSparseAttnBackward"
+    return (out.detach(), *torch.autograd.grad(out, leaves, dout))
+
+
+def same(got, want):
+    torch.cuda.synchronize()
+    assert len(got) == len(want)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("route", ROUTES)
+@pytest.mark.parametrize("tail", [False, True])
+def test_non_reentrant_checkpoint(dev, route, tail):
+    """A checkpointed region that ends with the attention (the first node to unpack), or goes on after it."""
+    from torch.utils.checkpoint import checkpoint
+
+    leaves, dout, call = make(dev, route)
+
+    def region(*t):
+        out = call(*(x * 1.0 for x in t))
+        return out * 1.0 if tail else out
+
+    want = torch.autograd.grad(region(*leaves), leaves, dout)
+    got = torch.autograd.grad(checkpoint(region, *leaves, use_reentrant=False), leaves, dout)
+    same(got, want)
