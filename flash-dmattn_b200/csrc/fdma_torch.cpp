@@ -17,9 +17,12 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/dynamo/compiled_autograd.h>
 #include <torch/csrc/utils/pybind.h>
 
 #include <algorithm>
+#include <array>
+#include <mutex>
 #include <optional>
 #include <stdexcept>
 #include <string>
@@ -230,25 +233,98 @@ void fill_gathered(fdma_fwd_params& p, const KvB& kv, const Tensor& key_pos, con
 //                                       bits    q, k, v, bits, bias, out, lse, activity
 //                                       gathered q, kvb, -, slot_mask, -, out, lse, key_pos
 //                                       packed  q, k, v, -, -, out, lse, the query rows that see each key
-struct AttnBackward : public torch::autograd::Node {
+enum { kQ, kK, kV, kMask, kBias, kOut, kLse, kExtra, kNumSaved };
+using SavedTensors = std::array<Tensor, kNumSaved>;
+
+// What the node knows besides tensors, and the same as plain values for compiled autograd.
+struct Meta {
   Call c;
-  SavedVariable q, k, v, mask, bias, out, lse, extra;
-  at::SmallVector<int64_t, 4> k_sizes, v_like;
+  std::vector<int64_t> k_sizes, bias_sizes;  // of the caller's tensors
   bool want_bias = false;
-  std::vector<int64_t> bias_sizes;
+
+  std::vector<int64_t> pack() const {
+    std::vector<int64_t> x = {c.causal, c.deterministic, c.bits, c.gathered, c.packed, c.path, c.seqlen_k, c.bias_keys, want_bias};
+    for (const auto* v : {&c.bias_c, &k_sizes, &bias_sizes}) {
+      x.push_back(static_cast<int64_t>(v->size()));
+      x.insert(x.end(), v->begin(), v->end());
+    }
+    return x;
+  }
+  static Meta unpack(const std::vector<int64_t>& x, double scale) {
+    Meta m;
+    size_t i = 0;
+    auto next = [&] { return x.at(i++); };
+    m.c.scale = static_cast<float>(scale);
+    m.c.causal = next(); m.c.deterministic = next(); m.c.bits = next(); m.c.gathered = next(); m.c.packed = next();
+    m.c.path = static_cast<int>(next());
+    m.c.seqlen_k = next(); m.c.bias_keys = next(); m.want_bias = next();
+    for (auto* v : {&m.c.bias_c, &m.k_sizes, &m.bias_sizes}) {
+      v->resize(next());
+      for (int64_t& e : *v) e = next();
+    }
+    return m;
+  }
+};
+
+variable_list backward(const Tensor& grad, const SavedTensors& t, const Meta& meta);
+
+struct AttnBackward : public torch::autograd::Node {
+  Meta meta;
+  std::array<SavedVariable, kNumSaved> saved;
 
   std::string name() const override { return "FlashSparseAttnBackward"; }
   void release_variables() override {
-    for (SavedVariable* s : {&q, &k, &v, &mask, &bias, &out, &lse, &extra}) s->reset_data();
+    std::lock_guard<std::mutex> lock(mutex_);  // another thread may run this node
+    for (SavedVariable& s : saved) s.reset_data();
   }
-  variable_list apply(variable_list&& grads) override;
-  variable_list apply_packed(const Tensor& tq, const Tensor& tk, const Tensor& tv, const Tensor& tout, const Tensor& tlse,
-                             const Tensor& key_rows, const Tensor& dout, cudaStream_t stream);
+  SavedTensors unpack() {
+    SavedTensors t;
+    for (int i = 0; i < kNumSaved; ++i) t[i] = saved[i].unpack(i == kOut ? getptr() : nullptr);
+    return t;
+  }
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    // Unpacked before anything is switched off: a hook may recompute the region the call belongs to (checkpointing),
+    // which has to record a graph of its own while it does.
+    return backward(grads[0], unpack(), meta);
+  }
+
+  // Compiled autograd: the node is one opaque call in the graph it captures.
+  void compiled_args(torch::dynamo::autograd::CompiledNodeArgs& args) const override {
+    for (int i = 0; i < kNumSaved; ++i) args.collect(saved[i], /*is_output=*/i == kOut);
+    args.collect(static_cast<double>(meta.c.scale));
+    args.collect(meta.pack());
+  }
+  variable_list apply_with_saved(const variable_list& grads, torch::dynamo::autograd::SwapSavedVariables& swap) override {
+    namespace ca = torch::dynamo::autograd;
+    for (SavedVariable& s : saved) swap.before(s);
+    ca::PackedArgs packed;
+    for (const Tensor& t : unpack()) packed.pack(t);
+    packed.pack(static_cast<double>(meta.c.scale));
+    packed.pack(meta.pack());
+    const std::vector<at::IValue> args = packed.vec();
+    std::vector<at::TypePtr> schema;
+    for (const at::IValue& x : args) schema.push_back(x.isTensor() ? at::TypePtr(at::TensorType::get()) : x.type());
+    const auto outputs = ca::IValuePacker<std::vector<std::optional<torch::autograd::InputMetadata>>>::pack(ca::get_input_metadata(next_edges()));
+    const auto& compiler = ca::getPyCompilerInterface();
+    const std::string fn = compiler->bind_function(swap.get_py_compiler(), name(), &functional, schema, /*is_custom_function=*/true,
+                                                   /*is_traceable=*/false);
+    variable_list res = compiler->call_function(swap.get_py_compiler(), "apply_functional", fn, grads, args, outputs);
+    for (SavedVariable& s : saved) swap.after(s);
+    return res;
+  }
+  static variable_list functional(const variable_list& grads, const std::vector<at::IValue>& args) {
+    torch::dynamo::autograd::PackedArgs packed(args);
+    SavedTensors t;
+    for (Tensor& x : t) x = packed.unpack<Tensor>();
+    const double scale = packed.unpack<double>();
+    return backward(grads[0], t, Meta::unpack(packed.unpack<std::vector<int64_t>>(), scale));
+  }
 };
 
 // Gradients of packed sequences: (tokens, heads, d) tensors, one row of tokens for the kernels.
-variable_list AttnBackward::apply_packed(const Tensor& tq, const Tensor& tk, const Tensor& tv, const Tensor& tout, const Tensor& tlse,
-                                         const Tensor& key_rows, const Tensor& dout, cudaStream_t stream) {
+variable_list packed_backward(const SavedTensors& t, const Call& c, const Tensor& dout, cudaStream_t stream) {
+  const Tensor &tq = t[kQ], &tk = t[kK], &tv = t[kV], &tout = t[kOut], &tlse = t[kLse], &key_rows = t[kExtra];
   variable_list res(3);
   Tensor dq = empty(tq.sizes(), tq.scalar_type(), tq), dk = empty(tk.sizes(), tk.scalar_type(), tk), dv = empty(tv.sizes(), tv.scalar_type(), tv);
   fdma_bwd_params bp = {};
@@ -277,26 +353,24 @@ variable_list AttnBackward::apply_packed(const Tensor& tq, const Tensor& tk, con
   return res;
 }
 
-variable_list AttnBackward::apply(variable_list&& grads) {
+variable_list backward(const Tensor& grad, const SavedTensors& t, const Meta& meta) {
+  const Call& c = meta.c;
   variable_list res(4);
-  if (!grads[0].defined()) return res;
-  // Unpacked before anything is switched off: a hook may recompute the region the call belongs to (checkpointing), which
-  // has to record a graph of its own while it does.
-  const Tensor tq = q.unpack(), tk = k.unpack(), tv = v.unpack(), tmask = mask.unpack(), tbias = bias.unpack(),
-               tlse = lse.unpack(), textra = extra.unpack(), tout = out.unpack(getptr());
+  if (!grad.defined()) return res;
+  const Tensor &tq = t[kQ], &tk = t[kK], &tv = t[kV], &tmask = t[kMask], &tbias = t[kBias], &tlse = t[kLse], &textra = t[kExtra], &tout = t[kOut];
   at::AutoDispatchBelowADInplaceOrView guard;
   const c10::cuda::CUDAGuard device(tq.device());
   const cudaStream_t stream = stream_of(tq);
   raise_if_timed_out(stream);
-  if (c.packed) return apply_packed(tq, tk, tv, tout, tlse, textra, grads[0].contiguous(), stream);
-  const Tensor dout = inner_contiguous(grads[0]);
+  if (c.packed) return packed_backward(t, c, grad.contiguous(), stream);
+  const Tensor dout = inner_contiguous(grad);
 
   fdma_bwd_params bp = {};
   Tensor dq = empty_as(tq), dk, dv, dbias;
   if (c.gathered) {
-    dk = empty(k_sizes, tq.scalar_type(), tq);
-    dv = empty(k_sizes, tq.scalar_type(), tq);
-    const int64_t cap = textra.size(2), hk = k_sizes[2], d = tq.size(3);
+    dk = empty(meta.k_sizes, tq.scalar_type(), tq);
+    dv = empty(meta.k_sizes, tq.scalar_type(), tq);
+    const int64_t cap = textra.size(2), hk = meta.k_sizes[2], d = tq.size(3);
     fill_geometry(bp.f, tq, cap, hk, c);
     fill_gathered(bp.f, split_kvb(tk, tq.size(0) * cap * hk * d, !c.bias_c.empty()), textra, tmask, c);
     bp.scatter_pos = textra.data_ptr<int32_t>();
@@ -304,14 +378,14 @@ variable_list AttnBackward::apply(variable_list&& grads) {
     bp.scatter_head_stride = bp.f.key_pos_head_stride;
     bp.scatter_h = bp.f.h_pos;
     bp.scatter_rows = static_cast<int32_t>(c.seqlen_k);
-    if (want_bias) dbias = empty(bias_sizes, tq.scalar_type(), tq);
+    if (meta.want_bias) dbias = empty(meta.bias_sizes, tq.scalar_type(), tq);
   } else {
     dk = empty_as(tk);
     dv = empty_as(tv);
     fill_geometry(bp.f, tq, tk.size(1), tk.size(2), c);
     fill_kv(bp.f, tk, tv);
     fill_mask_bias(bp.f, tmask, tbias, textra, c);
-    if (want_bias) dbias = empty(tbias.sizes(), tbias.scalar_type(), tbias);
+    if (meta.want_bias) dbias = empty(tbias.sizes(), tbias.scalar_type(), tbias);
   }
   fill_out(bp.f, tout, tlse);
   const Bsh so = bsh(dout), sq = bsh(dq), sk = bsh(dk), sv = bsh(dv);
@@ -521,25 +595,25 @@ std::optional<Tensor> attention(const Tensor& q0, const Tensor& k0, const Tensor
     auto node = std::shared_ptr<AttnBackward>(new AttnBackward(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(q0, k0, v0, bias0));
     torch::autograd::set_history(out, node);
-    node->want_bias = bias0.defined() && (needs_grad(bias0));
-    node->k_sizes.assign(k0.sizes().begin(), k0.sizes().end());
-    if (bias0.defined()) node->bias_sizes = bias0.sizes().vec();
+    node->meta.want_bias = bias0.defined() && (needs_grad(bias0));
+    node->meta.k_sizes = k0.sizes().vec();
+    if (bias0.defined()) node->meta.bias_sizes = bias0.sizes().vec();
     // tensors made here are saved as they are; the caller's own go in with their version, so in-place edits are noticed
-    node->q = SavedVariable(q.is_same(q0) ? q0 : q, false);
+    node->saved[kQ] = SavedVariable(q.is_same(q0) ? q0 : q, false);
     if (c.gathered) {
-      node->k = SavedVariable(kvb, false);
-      node->mask = SavedVariable(slot_mask, false);
-      node->extra = SavedVariable(key_pos, false);
+      node->saved[kK] = SavedVariable(kvb, false);
+      node->saved[kMask] = SavedVariable(slot_mask, false);
+      node->saved[kExtra] = SavedVariable(key_pos, false);
     } else {
-      node->k = SavedVariable(k, false);
-      node->v = SavedVariable(v, false);
-      if (mask.defined()) node->mask = SavedVariable(mask, false);
-      if (bias.defined()) node->bias = SavedVariable(bias, false);
-      if (activity.defined()) node->extra = SavedVariable(activity, false);
+      node->saved[kK] = SavedVariable(k, false);
+      node->saved[kV] = SavedVariable(v, false);
+      if (mask.defined()) node->saved[kMask] = SavedVariable(mask, false);
+      if (bias.defined()) node->saved[kBias] = SavedVariable(bias, false);
+      if (activity.defined()) node->saved[kExtra] = SavedVariable(activity, false);
     }
-    node->out = SavedVariable(out, /*is_output=*/true);
-    node->lse = SavedVariable(lse, false);
-    node->c = std::move(c);
+    node->saved[kOut] = SavedVariable(out, /*is_output=*/true);
+    node->saved[kLse] = SavedVariable(lse, false);
+    node->meta.c = std::move(c);
   }
   return out;
 }
@@ -594,13 +668,13 @@ std::vector<Tensor> packed_attention(const Tensor& q0, const Tensor& k0, const T
     auto node = std::shared_ptr<AttnBackward>(new AttnBackward(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(q0, k0, v0));
     torch::autograd::set_history(out, node);
-    node->q = SavedVariable(q0, false);
-    node->k = SavedVariable(k0, false);
-    node->v = SavedVariable(v0, false);
-    node->out = SavedVariable(out, /*is_output=*/true);
-    node->lse = SavedVariable(lse, false);
-    node->extra = SavedVariable(key_rows, false);
-    node->c = std::move(c);
+    node->saved[kQ] = SavedVariable(q0, false);
+    node->saved[kK] = SavedVariable(k0, false);
+    node->saved[kV] = SavedVariable(v0, false);
+    node->saved[kOut] = SavedVariable(out, /*is_output=*/true);
+    node->saved[kLse] = SavedVariable(lse, false);
+    node->saved[kExtra] = SavedVariable(key_rows, false);
+    node->meta.c = std::move(c);
   }
   return {out, lse};
 }

@@ -74,3 +74,51 @@ def test_non_reentrant_checkpoint(dev, route, tail):
     want = torch.autograd.grad(region(*leaves), leaves, dout)
     got = torch.autograd.grad(checkpoint(region, *leaves, use_reentrant=False), leaves, dout)
     same(got, want)
+
+
+@pytest.mark.parametrize("route", ROUTES)
+def test_compiled_autograd(dev, route):
+    from torch._dynamo import compiled_autograd
+
+    leaves, dout, call = make(dev, route)
+    want = plain(leaves, dout, call)
+    for _ in range(2):  # the second time from the cache of compiled graphs
+        for t in leaves:
+            t.grad = None
+        out = call(*leaves)
+        with compiled_autograd._enable(torch.compile(backend="eager", dynamic=False)):
+            out.backward(dout)
+        same([t.grad for t in leaves], want[1:])
+
+
+@pytest.mark.parametrize("route", ROUTES)
+def test_backward_twice(dev, route):
+    leaves, dout, call = make(dev, route)
+    want = plain(leaves, dout, call)
+    out = call(*leaves)
+    same(torch.autograd.grad(out, leaves, dout, retain_graph=True), want[1:])
+    same(torch.autograd.grad(out, leaves, dout), want[1:])
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(out, leaves, dout)
+
+
+def test_threads_share_a_graph(dev):
+    """Two threads run the same graph backward, which is kept: neither sees the other's release of it."""
+    leaves, dout, call = make(dev, "gathered")
+    want = plain(leaves, dout, call)
+    out = call(*leaves)
+    torch.cuda.synchronize()
+    results = []
+
+    def work():
+        for _ in range(10):
+            results.append(torch.autograd.grad(out, leaves, dout, retain_graph=True))
+
+    threads = [threading.Thread(target=work) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(results) == 20
+    for r in results:
+        same(r, want[1:])
