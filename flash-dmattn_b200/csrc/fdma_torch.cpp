@@ -355,7 +355,7 @@ variable_list packed_backward(const SavedTensors& t, const Call& c, const Tensor
 
 variable_list backward(const Tensor& grad, const SavedTensors& t, const Meta& meta) {
   const Call& c = meta.c;
-  variable_list res(4);
+  variable_list res(c.packed ? 3 : 4);
   if (!grad.defined()) return res;
   const Tensor &tq = t[kQ], &tk = t[kK], &tv = t[kV], &tmask = t[kMask], &tbias = t[kBias], &tlse = t[kLse], &textra = t[kExtra], &tout = t[kOut];
   at::AutoDispatchBelowADInplaceOrView guard;

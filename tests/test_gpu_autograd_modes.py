@@ -122,3 +122,21 @@ def test_threads_share_a_graph(dev):
     assert len(results) == 20
     for r in results:
         same(r, want[1:])
+
+
+@pytest.mark.parametrize("route", ROUTES)
+def test_undefined_gradient(dev, route):
+    """A consumer that returns no gradient for its input: the node is run without one."""
+    leaves, dout, call = make(dev, route)
+
+    class Drop(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x):
+            return x.clone()
+
+        @staticmethod
+        def backward(ctx, g):
+            return None
+
+    grads = torch.autograd.grad(Drop.apply(call(*leaves)), leaves, dout, allow_unused=True)
+    assert all(g is None or not g.any() for g in grads)
