@@ -13,6 +13,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <dlfcn.h>
 #include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
@@ -286,7 +287,15 @@ struct AttnBackward : public torch::autograd::Node {
     std::lock_guard<std::mutex> lock(mutex_);
     // Unpacked before anything is switched off: a hook may recompute the region the call belongs to (checkpointing),
     // which has to record a graph of its own while it does.
-    return backward(grads[0], unpack(), meta);
+    variable_list res = backward(grads[0], unpack(), meta);
+    if (!at::GradMode::is_enabled()) return res;
+    // create_graph: the gradients come from kernels without a derivative. They carry a node that says so when it is
+    // reached; without one a gradient penalty would silently leave the attention out.
+    for (Tensor& t : res)
+      if (t.defined()) t.set_requires_grad(true);
+    auto error = std::make_shared<torch::autograd::DelayedError>(
+        "trying to differentiate twice through flash_sparse_attn, whose backward has no derivative", static_cast<int64_t>(res.size()));
+    return error->apply(std::move(res));
   }
 
   // Compiled autograd: the node is one opaque call in the graph it captures.

@@ -140,3 +140,16 @@ def test_undefined_gradient(dev, route):
 
     grads = torch.autograd.grad(Drop.apply(call(*leaves)), leaves, dout, allow_unused=True)
     assert all(g is None or not g.any() for g in grads)
+
+
+@pytest.mark.parametrize("route", ROUTES)
+def test_second_derivative_is_refused(dev, route):
+    """The gradients have no derivative of their own: a gradient penalty must fail, not train without the attention."""
+    leaves, dout, call = make(dev, route)
+    want = plain(leaves, dout, call)
+    out = call(*leaves)
+    grads = torch.autograd.grad(out, leaves, dout, create_graph=True)
+    same([g.detach() for g in grads], want[1:])
+    assert all(g.requires_grad for g in grads)
+    with pytest.raises(RuntimeError, match="twice|second|not implemented|once_differentiable"):
+        sum(g.float().pow(2).sum() for g in grads).backward()
