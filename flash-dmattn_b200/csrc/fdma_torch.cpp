@@ -105,6 +105,14 @@ Tensor empty_as(const Tensor& t) {
   return t.is_contiguous() ? empty(t.sizes(), t.scalar_type(), t) : at::empty_like(t);
 }
 Tensor inner_contiguous(const Tensor& t) { return t.stride(-1) == 1 ? t : t.contiguous(); }
+// A (.., rows, heads, d) tensor as the tensor-core kernels load it: 16-byte aligned base and strides, nothing expanded. Calls
+// that only those kernels serve (gathered keys, bit masks, packed sequences) get a dense copy of anything else: an output
+// gradient that `sum` expanded or that was cut out of wider rows, a query slice with an odd stride.
+Tensor kernel_layout(const Tensor& t) {
+  bool ok = t.stride(-1) == 1 && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+  for (int64_t i = 0; i + 1 < t.dim(); ++i) ok = ok && t.stride(i) > 0 && t.stride(i) % 8 == 0;
+  return ok ? t : t.clone(at::MemoryFormat::Contiguous);
+}
 const Tensor& get(const OptTensor& t) {
   static const Tensor none;
   return t.has_value() ? *t : none;
@@ -371,8 +379,8 @@ variable_list backward(const Tensor& grad, const SavedTensors& t, const Meta& me
   const c10::cuda::CUDAGuard device(tq.device());
   const cudaStream_t stream = stream_of(tq);
   raise_if_timed_out(stream);
-  if (c.packed) return packed_backward(t, c, grad.contiguous(), stream);
-  const Tensor dout = inner_contiguous(grad);
+  if (c.packed) return packed_backward(t, c, kernel_layout(grad), stream);
+  const Tensor dout = c.gathered || c.bits ? kernel_layout(grad) : inner_contiguous(grad);
 
   fdma_bwd_params bp = {};
   Tensor dq = empty_as(tq), dk, dv, dbias;
