@@ -80,6 +80,8 @@ void init(const std::string& path) {
 }
 
 constexpr int64_t kTile = 128;
+// What the tile tables of the tensor-core kernels hold. The gradients of gathered keys and bit masks have no other kernels.
+constexpr int64_t kMaxKeys = 1 << 20, kMaxQueries = 1 << 19;
 int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
 
 void check(int status, const char* what) {
@@ -530,6 +532,7 @@ std::optional<Tensor> attention(const Tensor& q0, const Tensor& k0, const Tensor
     for (int i = 0; i < 3; ++i)
       if (k0.stride(i) % 8 || v0.stride(i) % 8) return std::nullopt;
     if ((reinterpret_cast<uintptr_t>(k0.data_ptr()) | reinterpret_cast<uintptr_t>(v0.data_ptr())) & 15) return std::nullopt;
+    if (cap > kMaxKeys || (d <= 128 && Sq > kMaxQueries) || H > 65535 || B > 65535) return std::nullopt;
     if (bias0.defined()) {
       // the gathered bias has the bias' own extents: the list must not vary along a dimension the bias is shared over
       if (bias0.size(2) != 1 || bias0.size(3) < Sk || bias0.size(3) == 1) return std::nullopt;
@@ -556,7 +559,7 @@ std::optional<Tensor> attention(const Tensor& q0, const Tensor& k0, const Tensor
     const c10::cuda::CUDAGuard device(q0.device());
     const cudaStream_t stream = stream_of(q0);
     raise_if_timed_out(stream);
-    q = inner_contiguous(q0);
+    q = c.gathered ? kernel_layout(q0) : inner_contiguous(q0);
     out = empty_as(q);
     lse = empty({B, H, Sq}, at::kFloat, q);
     fdma_fwd_params p = {};

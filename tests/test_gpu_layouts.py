@@ -104,3 +104,49 @@ def test_output_gradient(dev, route, use, d, dtype):
     _kernel_status_ok()
     for n, a, b in zip(("dq", "dk", "dv", "dbias"), got, want):
         close(n, a, b, dtype)
+
+
+@pytest.mark.parametrize("d", [64, 96, 128, 256])
+@pytest.mark.parametrize("layout", list(LAYOUTS))
+@pytest.mark.parametrize("which", ["q", "kv", "bias", "all"])
+@pytest.mark.parametrize("route", ["gathered", "packed", "dense"])
+def test_inputs(dev, route, which, layout, d):
+    from flash_sparse_attn.utils.mask import create_mask
+
+    if d == 256 and route not in ("gathered", "dense"):
+        pytest.skip("no other kernel at this head dim")
+    if route == "packed" and (which == "bias" or layout == "expanded"):
+        pytest.skip("packed calls have no bias and no batch")
+    dtype = torch.bfloat16
+    q, k, v, bias, dout = inputs(dev, route, d, dtype)
+    B, S = q.shape[:2]
+    f = LAYOUTS[layout]
+    if route == "packed":
+        q, k, v = (t.flatten(0, 1) for t in (q, k, v))
+        dout = dout.flatten(0, 1)
+    if which in ("q", "all"):
+        q = f(q)
+    if which in ("kv", "all"):
+        k, v = f(k), f(v)
+    if which in ("bias", "all"):
+        bias = f(bias)
+
+    def step(q, k, v, bias):
+        t = [x.detach().requires_grad_(True) for x in (q, k, v, bias)]
+        mask = create_mask(bias.contiguous(), None, B, S, S, 100, torch.finfo(dtype).min) if route in ("gathered", "bits") else None
+        if route == "packed":
+            from flash_sparse_attn import flash_sparse_attn_varlen_func
+
+            cu = torch.tensor([0, 100, B * S], device=dev, dtype=torch.int32)
+            out = flash_sparse_attn_varlen_func(t[0], t[1], t[2], cu, cu, B * S, B * S, is_causal=True, deterministic=True)
+            t = t[:3]
+        else:
+            out = attend(route, *t, mask)
+        return (out.detach(), *torch.autograd.grad(out, t, dout))
+
+    got = step(q, k, v, bias)
+    want = step(*(x.contiguous().clone(memory_format=torch.contiguous_format) for x in (q, k, v, bias)))
+    torch.cuda.synchronize()
+    _kernel_status_ok()
+    for n, a, b in zip(("out", "dq", "dk", "dv", "dbias"), got, want):
+        close(n, a, b, dtype)
