@@ -545,7 +545,9 @@ std::optional<Tensor> attention(const Tensor& q0, const Tensor& k0, const Tensor
     c.bits = true;
     if (d > 128 || Sq == 1 || bits.size(0) != B || bits.size(2) != Sq || bits.size(3) != Sk_r / 32) return std::nullopt;
     if (bits.size(1) != 1 && bits.size(1) != Hk && bits.size(1) != H) return std::nullopt;
-    if (!bits.is_contiguous() || !activity.is_contiguous()) return std::nullopt;
+    if (!bits.is_contiguous() || !activity.is_contiguous() || (reinterpret_cast<uintptr_t>(bits.data_ptr()) & 15)) return std::nullopt;
+    // (the tile table of the backward holds one row of tiles per query head whose mask differs)
+    if (Sk > kMaxKeys || round_up(Sq, kTile) * (bits.size(1) == H ? H / Hk : 1) > kMaxQueries || H > 65535 || B > 65535) return std::nullopt;
   } else if (mask0.defined()) {
     if (!plain(mask0) || mask0.scalar_type() != at::kBool || mask0.device() != q0.device() ||
         !broadcastable(mask0, B, H, Hk, Sq) || (mask0.size(3) != 1 && mask0.size(3) != Sk && mask0.size(3) != Sk_r))
@@ -559,7 +561,8 @@ std::optional<Tensor> attention(const Tensor& q0, const Tensor& k0, const Tensor
     const c10::cuda::CUDAGuard device(q0.device());
     const cudaStream_t stream = stream_of(q0);
     raise_if_timed_out(stream);
-    q = c.gathered ? kernel_layout(q0) : inner_contiguous(q0);
+    const auto layout = c.gathered || c.bits ? kernel_layout : inner_contiguous;
+    q = layout(q0);
     out = empty_as(q);
     lse = empty({B, H, Sq}, at::kFloat, q);
     fdma_fwd_params p = {};
@@ -592,11 +595,16 @@ std::optional<Tensor> attention(const Tensor& q0, const Tensor& k0, const Tensor
       fill_geometry(p, q, cap, Hk, c);
       fill_gathered(p, kv, key_pos, slot_mask, c);
     } else {
-      k = inner_contiguous(k0);
-      v = inner_contiguous(v0);
+      k = layout(k0);
+      v = layout(v0);
       if (c.bits) mask = bits;
       else if (mask0.defined()) mask = inner_contiguous(fit_keys(mask0, Sk_r));
       if (bias0.defined()) bias = inner_contiguous(fit_keys(bias0, Sk_r));
+      if (c.bits && bias0.defined()) {  // 16-byte loads; expanded dimensions are fine
+        bool ok = (reinterpret_cast<uintptr_t>(bias.data_ptr()) & 15) == 0;
+        for (int i = 0; i < 3; ++i) ok = ok && bcast_stride(bias, i) % 8 == 0;
+        if (!ok) bias = bias.clone(at::MemoryFormat::Contiguous);
+      }
       fill_geometry(p, q, Sk, Hk, c);
       fill_kv(p, k, v);
       fill_mask_bias(p, mask, bias, activity, c);

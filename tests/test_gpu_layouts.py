@@ -109,7 +109,7 @@ def test_output_gradient(dev, route, use, d, dtype):
 @pytest.mark.parametrize("d", [64, 96, 128, 256])
 @pytest.mark.parametrize("layout", list(LAYOUTS))
 @pytest.mark.parametrize("which", ["q", "kv", "bias", "all"])
-@pytest.mark.parametrize("route", ["gathered", "packed", "dense"])
+@pytest.mark.parametrize("route", ["gathered", "bits", "packed", "dense"])
 def test_inputs(dev, route, which, layout, d):
     from flash_sparse_attn.utils.mask import create_mask
 
