@@ -7,6 +7,7 @@
 // does not handle (wrong types, odd layouts, tracing); the Python layer then runs its own path, which also raises the
 // argument errors.
 #include <ATen/ATen.h>
+#include <ATen/TracerMode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
@@ -779,8 +780,9 @@ std::vector<Tensor> topk_mask(const Tensor& bias, const OptTensor& premask_, int
 }
 
 // ---- Python -----------------------------------------------------------------------------------------------------
-// Only exact torch.Tensor / Parameter objects and no active dispatch mode (fake tensors, tracing): everything else is the
-// Python path's.
+// Only exact torch.Tensor / Parameter objects, no active dispatch mode (fake tensors, make_fx) and no torch.jit.trace, which
+// records dispatched operators only: everything else is the Python path's.
+bool eager() { return !c10::impl::TorchDispatchModeTLS::any_modes_set() && !at::tracer::impl::is_dispatch_enabled(); }
 bool exact(PyObject* o) { return THPVariable_CheckExact(o); }
 // Tensors that stand for something else (vmap and grad transforms, functionalisation, lazy conjugation) or carry a
 // forward-mode tangent are the Python path's as well: the node below has neither batching rules nor a jvp.
@@ -804,7 +806,7 @@ py::object py_attention(py::handle q, py::handle k, py::handle v, py::handle mas
   const py::handle in[9] = {q, k, v, mask, bias, key_pos, slot_mask, bits, activity};
   for (int i = 0; i < 9; ++i)
     if (!as_tensor(in[i], t[i])) return py::none();
-  if (!t[0] || !t[1] || !t[2] || c10::impl::TorchDispatchModeTLS::any_modes_set()) return py::none();
+  if (!t[0] || !t[1] || !t[2] || !eager()) return py::none();
   double s;
   if (scale.is_none()) {
     if (t[0]->dim() != 4) return py::none();
@@ -827,7 +829,7 @@ py::object py_packed_attention(py::handle q, py::handle k, py::handle v, py::han
   const py::handle in[5] = {q, k, v, cu_q, cu_k};
   for (int i = 0; i < 5; ++i)
     if (!as_tensor(in[i], t[i]) || !t[i]) return py::none();
-  if (c10::impl::TorchDispatchModeTLS::any_modes_set()) return py::none();
+  if (!eager()) return py::none();
   std::vector<Tensor> res;
   {
     py::gil_scoped_release release;
@@ -841,7 +843,7 @@ py::object py_packed_attention(py::handle q, py::handle k, py::handle v, py::han
 
 py::object py_topk_mask(py::handle bias, py::handle premask, int64_t window, double min_value) {
   OptTensor b, pm;
-  if (!as_tensor(bias, b) || !as_tensor(premask, pm) || !b || c10::impl::TorchDispatchModeTLS::any_modes_set()) return py::none();
+  if (!as_tensor(bias, b) || !as_tensor(premask, pm) || !b || !eager()) return py::none();
   std::vector<Tensor> res;
   {
     py::gil_scoped_release release;

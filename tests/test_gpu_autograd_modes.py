@@ -153,3 +153,18 @@ def test_second_derivative_is_refused(dev, route):
     assert all(g.requires_grad for g in grads)
     with pytest.raises(RuntimeError, match="twice|second|not implemented|once_differentiable"):
         sum(g.float().pow(2).sum() for g in grads).backward()
+
+
+def test_jit_trace_records_the_call(dev):
+    """A traced function computes on its inputs; the call must not be baked in as a constant."""
+    from flash_sparse_attn import flash_sparse_attn_func
+
+    q, k, v, bias, _ = (t.to(dev) for t in oracle.make_inputs(1, 128, 128, 2, 1, 64, (1, 1, 128, 128), seed=1, dtype=DTYPE))
+
+    def f(q, k, v, bias):
+        return flash_sparse_attn_func(q, k, v, None, bias, is_causal=True)
+
+    with torch.no_grad():
+        traced = torch.jit.trace(f, (q, k, v, bias), check_trace=False)
+        q2 = q.flip(1)
+        assert torch.equal(traced(q2, k, v, bias), f(q2, k, v, bias))
