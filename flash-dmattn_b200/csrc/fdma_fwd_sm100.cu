@@ -25,7 +25,6 @@
 #include <math_constants.h>
 
 #include <algorithm>
-#include <mutex>
 
 #include <type_traits>
 
@@ -51,7 +50,7 @@ constexpr unsigned kPolyPairs = FDMA_POLY_PAIRS;  // bit i: pair i of every 16 p
 enum WaitCode {
   kWaitQ = 101, kWaitKvEmpty = 102, kWaitKvFullK = 103, kWaitKvFullV = 104, kWaitP = 105, kWaitS = 106,
   kWaitO = 107, kWaitBmEmpty = 108, kWaitBmFull = 109, kWaitQEmpty = 110, kWaitOFree = 111, kWaitFlagsFull = 112,
-  kWaitFlagsEmpty = 113
+  kWaitFlagsEmpty = 113, kWaitItem = 114
 };
 
 struct FwdKernelParams {
@@ -74,7 +73,6 @@ struct FwdKernelParams {
   const int2* row_keys;  // packed sequences: keys [x, y) each query row sees (both ascending), or null
   int n_mblk;        // query blocks (of kNQ tiles) per (batch, head)
   int n_items;       // work items = n_mblk * h * b
-  unsigned* sched;   // [0] next item nobody has taken yet, [1] CTAs that are done; both zero between launches
   float scale_log2;  // softmax_scale * log2(e)
 };
 
@@ -98,8 +96,9 @@ struct Smem {
   static constexpr int kPosOff = kBmOff + kBmSlots * kBN * 4;
   static constexpr int kFlagsOff = kPosOff + kBmSlots * kBN * 4;   // two tables: this work item's and the next one's
   static constexpr int kBarOff = kFlagsOff + 2 * kMaxTiles;
-  static constexpr int kNumBars = 2 + 2 * kStages + 2 + 2 + 2 + 2 + 2 * kBmSlots + 1 + 4 + 1;
-  static constexpr int kMiscOff = kBarOff + kNumBars * 8;
+  static constexpr int kNumBars = 2 + 2 * kStages + 2 + 2 + 2 + 2 + 2 * kBmSlots + 1 + 4 + 1 + 1;
+  static constexpr int kClcOff = (kBarOff + kNumBars * 8 + 15) / 16 * 16;  // answer of the launch control
+  static constexpr int kMiscOff = kClcOff + 16;
   static constexpr int kTotal = kMiscOff + 48;
   static constexpr int kAlloc = kTotal + 1024;  // slack to align the base to 1024 B
 };
@@ -142,9 +141,10 @@ __global__ void tile_activity_kernel(const uint8_t* __restrict__ mask, int64_t s
   if (lane == 0) act[w] = any ? 1 : 0;
 }
 
-// Work item = one query block (kNQ query tiles of 128 rows) of one (batch, head). CTAs are persistent: the list is
-// ordered by decreasing causal extent (last query blocks first) and a CTA takes the next item nobody has taken yet
-// (one atomicAdd per item), which balances the SMs to within one short item. Barrier phases, ring positions and tensor memory carry over
+// Work item = one query block (kNQ query tiles of 128 rows) of one (batch, head). The grid has one CTA per item, ordered by
+// decreasing causal extent (last query blocks first), and the CTAs that run are persistent: each takes over the next item
+// whose CTA has not started yet (cluster launch control), which balances the SMs to within one short item. There is no
+// counter in memory that launches could share or leave behind. Barrier phases, ring positions and tensor memory carry over
 // from one item to the next; nothing is re-initialised, and the pieces of an item that no role of the PREVIOUS
 // item needs any more start early: the tile flags of the next item are built by warp 3 during the current item,
 // its Q and first K / V tiles are loaded as soon as the tensor core has finished with the current Q, its first
@@ -202,6 +202,7 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
   uint64_t* bar_flags_full = bar_stagger + 1;       // [2]
   uint64_t* bar_flags_empty = bar_flags_full + 2;   // [2]
   uint64_t* bar_pv = bar_flags_empty + 2;           // one query tile: a P V product has completed (phase per product)
+  uint64_t* bar_clc = bar_pv + 1;                   // the launch control has answered (phase per question)
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + L::kMiscOff);
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem + L::kMiscOff + 4);
   volatile int* s_item = reinterpret_cast<volatile int*>(smem + L::kMiscOff + 8);  // [2]: item of the flag table
@@ -266,6 +267,7 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
     }
     mbar_init(bar_stagger, kBM);
     mbar_init(bar_pv, 1);
+    mbar_init(bar_clc, 1);
     for (int i = 0; i < kBmSlots; ++i) {
       mbar_init(bar_bm_full + i, 1);
       mbar_init(bar_bm_empty + i, 4 * kNQ);  // one arrival per softmax warp
@@ -552,12 +554,28 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
     // warp 3: tile flags of every item, one item ahead of the other roles. Bit t of flags[j] = key tile j is
     // processed for query tile t.
     bool ok = true;
+    int asked = 0, answered = 0;  // questions to the launch control
+    auto ask = [&]() {
+      if (lane == 0) {
+        fence_proxy_async_smem();  // (the previous answer has been read)
+        mbar_arrive_expect_tx(bar_clc, 16);
+        clc_try_cancel(smem + L::kClcOff, bar_clc);
+      }
+      ++asked;
+    };
     for (int ic = 0; ok; ++ic) {
       ok = __all_sync(0xffffffffu, mbar_wait(bar_flags_empty + (ic & 1), ((ic >> 1) & 1) ^ 1, ctl, kWaitFlagsEmpty));
       if (!ok) break;
-      int item = 0;
-      if (lane == 0) item = static_cast<int>(min(atomicAdd(p.sched, 1u), static_cast<unsigned>(p.n_items)));
-      item = __shfl_sync(0xffffffffu, item, 0);
+      int item = blockIdx.x;
+      if (ic > 0) {  // the first item is the CTA's own
+        ask();
+        ok = __all_sync(0xffffffffu, mbar_wait(bar_clc, (asked - 1) & 1, ctl, kWaitItem));
+        if (!ok) break;
+        answered = asked;
+        item = clc_answer(smem + L::kClcOff);
+        if (item < 0) item = p.n_items;
+        __syncwarp();  // every lane has read the answer
+      }
       if (lane == 0) s_item[ic & 1] = item;  // n_items = no item left: the other roles leave their loops on it
       if (item >= p.n_items) {
         __syncwarp();
@@ -633,6 +651,14 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_flags_full + (ic & 1));
+    }
+    // A wait gave up: the items nobody has started are taken off the launch, so that it does not wait for each of them.
+    while (!ok && asked == answered) {
+      ask();
+      for (int i = 0; i < (1 << 20) && answered != asked; ++i)
+        if (__all_sync(0xffffffffu, mbar_try_wait(smem_u32(bar_clc), (asked - 1) & 1))) answered = asked;
+      if (answered != asked || clc_answer(smem + L::kClcOff) < 0) break;
+      __syncwarp();
     }
   }
   } else {
@@ -1001,35 +1027,6 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 512);
   }
-  if (tid == 0) {  // the last CTA leaves the launch's counters as it found them (no memset node between launches)
-    __threadfence();
-    if (atomicAdd(p.sched + 1, 1u) == gridDim.x - 1) {
-      p.sched[0] = 0u;
-      p.sched[1] = 0u;
-      __threadfence();
-    }
-  }
-}
-
-// Item counters of the persistent forward: a ring of word pairs in device memory that is part of the library image, one
-// pair per launch, zero at load time and left at zero by the last CTA of every launch. Launches only share a pair when
-// more than kSchedSlots of them are in flight on one device at the same time.
-constexpr int kSchedSlots = 256;
-__device__ unsigned g_fwd_sched[2 * kSchedSlots];
-
-unsigned* next_sched_slot() {
-  static std::mutex mu;
-  static unsigned* base[64] = {nullptr};
-  static unsigned next[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  std::lock_guard<std::mutex> lock(mu);
-  if (!base[dev]) {
-    void* ptr = nullptr;
-    if (cudaGetSymbolAddress(&ptr, g_fwd_sched) != cudaSuccess) return nullptr;
-    base[dev] = static_cast<unsigned*>(ptr);
-  }
-  return base[dev] + 2 * (next[dev]++ % kSchedSlots);
 }
 
 struct FwdPlan {
@@ -1114,9 +1111,7 @@ int launch(const fdma_fwd_params& p, const FwdPlan& pl, const int32_t* row_keys,
   const int64_t n_items = static_cast<int64_t>(kp.n_mblk) * p.h * p.b;
   if (n_items > 0x7FFFFFFF) return FDMA_ERR_TOO_LARGE;
   kp.n_items = static_cast<int>(n_items);
-  dim3 grid(static_cast<unsigned>(std::min<int64_t>(n_items, sm_count())));  // persistent CTAs, one per SM
-  kp.sched = next_sched_slot();
-  if (!kp.sched) return FDMA_ERR_DRIVER;
+  const dim3 grid(static_cast<unsigned>(n_items));
   cudaEvent_t ev0, ev1;
   take_timing_events(&ev0, &ev1);
   if (ev0) cudaEventRecord(ev0, stream);

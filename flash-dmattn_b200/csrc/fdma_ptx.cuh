@@ -198,6 +198,37 @@ __device__ __forceinline__ void bulk_reduce_add_u64(long long* gmem_dst, const v
 }
 
 // ---------------------------------------------------------------------------------------------
+// Cluster launch control: a running CTA takes over the work of a CTA of its own grid that has not started yet
+// ---------------------------------------------------------------------------------------------
+// Asks for one such CTA. The 16-byte answer arrives at smem_answer (16-byte aligned) and completes 16 bytes on the barrier.
+// Not to be asked again once the answer was that none is left.
+__device__ __forceinline__ void clc_try_cancel(void* smem_answer, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+               :
+               : "r"(smem_u32(smem_answer)), "r"(smem_u32(bar))
+               : "memory");
+}
+// The answer: blockIdx.x of the CTA taken over, or -1 when none was left.
+__device__ __forceinline__ int clc_answer(const void* smem_answer) {
+  uint32_t taken, x;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .b128 r;\n\t"
+      ".reg .b32 y, z, w;\n\t"
+      "ld.shared.b128 r, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "mov.u32 %1, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, y, z, w}, r;\n\t"
+      "}"
+      : "=r"(taken), "=r"(x)
+      : "r"(smem_u32(smem_answer))
+      : "memory");
+  return taken ? static_cast<int>(x) : -1;
+}
+
+// ---------------------------------------------------------------------------------------------
 // TMEM allocation (one warp executes these, all 32 lanes converged)
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_result, uint32_t ncols) {

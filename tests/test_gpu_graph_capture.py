@@ -80,3 +80,33 @@ def test_forward_backward_in_a_cuda_graph():
         check("dk", got[2].cpu(), ref[3], dtype, reduced=True)
         check("dv", got[3].cpu(), ref[4], dtype, reduced=True)
         check("dbias", got[4].cpu(), ref[5], dtype, reduced=True)
+
+
+def test_replay_beside_eager_launches():
+    """A captured forward replayed on one stream while eager calls of another size run on a second one, several hundred of
+    each: every launch hands out its own work items, whatever runs beside it."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from flash_sparse_attn import flash_sparse_attn_func
+
+    dev, dtype = torch.device("cuda:0"), torch.bfloat16
+    g = torch.Generator(device=dev).manual_seed(2)
+    small = [torch.randn(1, 1024, h, 64, generator=g, device=dev, dtype=dtype) for h in (4, 2, 2)]
+    large = [torch.randn(2, 2048, h, 64, generator=g, device=dev, dtype=dtype) for h in (16, 2, 2)]
+    with torch.no_grad():
+        want_small, want_large = (flash_sparse_attn_func(*t, is_causal=True) for t in (small, large))
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = flash_sparse_attn_func(*small, is_causal=True)
+        streams = torch.cuda.Stream(), torch.cuda.Stream()
+        replays, eager = [], []
+        for i in range(600):
+            with torch.cuda.stream(streams[0]):
+                out.fill_(float("nan"))
+                graph.replay()
+                replays.append((out == want_small).all())
+            with torch.cuda.stream(streams[1]):
+                eager.append((flash_sparse_attn_func(*large, is_causal=True) == want_large).all())
+        torch.cuda.synchronize()
+    assert torch.stack(replays).all() and torch.stack(eager).all()
