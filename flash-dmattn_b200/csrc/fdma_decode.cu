@@ -113,6 +113,15 @@ __device__ __forceinline__ uint16_t f_to_raw(float x) {
   if (kBf16) return __bfloat16_as_ushort(__float2bfloat16_rn(x));
   return __half_as_ushort(__float2half_rn(x));
 }
+// (lo, hi) as 16-bit values, and what that leaves of them: three in a row add up to all 24 significant bits of a number (bf16:
+// 3 x 8; fp16: 3 x 11, cut at 2^-24).
+template <bool kBf16>
+__device__ __forceinline__ uint32_t split_off2(float& lo, float& hi) {
+  const uint32_t u = pack2<kBf16>(lo, hi);
+  lo -= raw_to_f<kBf16>(static_cast<uint16_t>(u & 0xFFFFu));
+  hi -= raw_to_f<kBf16>(static_cast<uint16_t>(u >> 16));
+  return u;
+}
 __device__ __forceinline__ float exp2_or_zero(float x) { return x == -CUDART_INF_F ? 0.f : exp2f(x); }
 
 // kM16: 9 to 16 query heads (both halves of the M rows of the products), else up to 8. Fragments of mma.m16n8k16
@@ -123,6 +132,11 @@ __global__ void __launch_bounds__(kThreads, NJ <= 4 ? 3 : 1) decode_rows_kernel(
   constexpr int D = NJ * 32;
   constexpr int kHalves = kM16 ? 2 : 1;
   constexpr int kHeads = 8 * kHalves;
+  // Head dims above 128: the probabilities keep their 32 bits, as sums of three 16-bit values with a product each. fp16 holds
+  // them times 2^14, away from its smallest numbers. (8 x 65536 keys, 4096 kept, 32 heads over 8, d = 256: 104 us with 16-bit
+  // probabilities, which are 15 % further from the exact result, 113 us so.)
+  constexpr int kTerms = D > 128 ? 3 : 1;
+  constexpr float kPScale = kTerms > 1 && !kBf16 ? 16384.f : 1.f;
   extern __shared__ __align__(16) unsigned char s_dyn[];  // the warps' rings; afterwards [kWarps][kHeads][D] fp32 partials
   __shared__ uint32_t s_q[kHalves][2 * NJ][2][32];        // A fragments of Q, one word per lane
   __shared__ float s_m[kWarps][kHeads], s_l[kWarps][kHeads];
@@ -243,7 +257,7 @@ __global__ void __launch_bounds__(kThreads, NJ <= 4 ? 3 : 1) decode_rows_kernel(
         mma_16816<kBf16>(s0[u], kM16 ? s8[u] : zero, q0, q1, q2, q3, f[2 * u], f[2 * u + 1]);
     }
     const float kbf = raw_to_f<kBf16>(kb) * kLog2e;
-    uint32_t pa[kHalves][2];
+    uint32_t pa[kTerms][kHalves][2];
 #pragma unroll
     for (int t = 0; t < kHalves; ++t) {
       float x[2][2];
@@ -276,9 +290,12 @@ __global__ void __launch_bounds__(kThreads, NJ <= 4 ? 3 : 1) decode_rows_kernel(
       const float base = m[t] == -CUDART_INF_F ? 0.f : m[t];
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        const float p0 = exp2f(x[u][0] - base), p1 = exp2f(x[u][1] - base);
+        float p0 = exp2f(x[u][0] - base), p1 = exp2f(x[u][1] - base);
         l[t] += p0 + p1;
-        pa[t][u] = pack2<kBf16>(p0, p1);
+        p0 *= kPScale;
+        p1 *= kPScale;
+#pragma unroll
+        for (int term = 0; term < kTerms; ++term) pa[term][t][u] = split_off2<kBf16>(p0, p1);
       }
     }
 #pragma unroll
@@ -287,8 +304,11 @@ __global__ void __launch_bounds__(kThreads, NJ <= 4 ? 3 : 1) decode_rows_kernel(
       ldmatrix_x4_trans(f, vaddr + j * 32);
 #pragma unroll
       for (int r = 0; r < 2; ++r)
-        mma_16816<kBf16>(o[0][2 * j + r], kM16 ? o[kHalves - 1][2 * j + r] : zero, pa[0][0], kM16 ? pa[kHalves - 1][0] : 0u,
-                         pa[0][1], kM16 ? pa[kHalves - 1][1] : 0u, f[2 * r], f[2 * r + 1]);
+#pragma unroll
+        for (int term = kTerms - 1; term >= 0; --term)
+          mma_16816<kBf16>(o[0][2 * j + r], kM16 ? o[kHalves - 1][2 * j + r] : zero, pa[term][0][0],
+                           kM16 ? pa[term][kHalves - 1][0] : 0u, pa[term][0][1], kM16 ? pa[term][kHalves - 1][1] : 0u, f[2 * r],
+                           f[2 * r + 1]);
     }
     __syncwarp();  // every lane has read the stage before it is overwritten
   };
@@ -329,7 +349,7 @@ __global__ void __launch_bounds__(kThreads, NJ <= 4 ? 3 : 1) decode_rows_kernel(
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) cm = fmaxf(cm, s_m[w][head]);
     const float base = cm == -CUDART_INF_F ? 0.f : cm;
-    const float f = exp2_or_zero(m[t] - base);
+    const float f = exp2_or_zero(m[t] - base) * (1.f / kPScale);
     if (warp == 0 && c == 0) {
       float cl = 0.f;
 #pragma unroll
