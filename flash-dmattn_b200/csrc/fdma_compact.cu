@@ -7,9 +7,11 @@
 //
 // The reference's CUDA backend has no such path; its Triton prototype gathers keys by top-k index
 // (flash_sparse_attn/flash_dmattn_triton.py:49-211). All three kernels are plain HBM-bound copies.
+#include <cooperative_groups.h>
+#include <cuda_runtime.h>
+
 #include <cstdint>
 #include <utility>
-#include <cuda_runtime.h>
 
 #include "fdma_internal.h"
 
@@ -19,27 +21,30 @@ namespace {
 constexpr int kIdxThreads = 256;
 constexpr int kIdxPerThread = 16;  // mask bytes scanned per thread and round
 
-// One CTA per mask row: running exclusive scan of the keep flags; kept key k lands in slot (number of kept keys
-// before it). Slots beyond the count are filled with INT32_MAX, mask_out marks the filled slots.
+// One cluster per mask row, an even segment of the keys per CTA: running exclusive scan of the keep flags; kept key k lands in
+// slot (number of kept keys before it). Slots beyond the count are filled with INT32_MAX, mask_out marks the filled slots.
+// A CTA of a cluster first counts its segment, which gives the others their first slot; the second pass finds it in L2.
 __global__ void __launch_bounds__(kIdxThreads) compact_index_kernel(const uint8_t* __restrict__ mask, int64_t sb,
                                                                      int64_t sh, int Hm, int Sk, int cap,
                                                                      int32_t* __restrict__ key_pos,
                                                                      int32_t* __restrict__ count,
                                                                      uint8_t* __restrict__ mask_out) {
+  namespace cg = cooperative_groups;
   __shared__ int s_warp[kIdxThreads / 32];
-  __shared__ int s_base;
-  const int row = blockIdx.x;
+  __shared__ int s_base, s_count;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int nrank = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
+  const int row = blockIdx.x / nrank;
   const int b = row / Hm, hm = row % Hm;
   const uint8_t* mrow = mask + b * sb + hm * sh;
   int32_t* prow = key_pos + static_cast<int64_t>(row) * cap;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) s_base = 0;
-  __syncthreads();
+  const int seg = ((Sk + nrank - 1) / nrank + kIdxPerThread - 1) / kIdxPerThread * kIdxPerThread;
+  const int k_lo = min(Sk, rank * seg), k_hi = min(Sk, k_lo + seg);
   const bool vec_ok = (reinterpret_cast<uintptr_t>(mrow) & 15u) == 0;
-  for (int k0 = 0; k0 < Sk; k0 += kIdxThreads * kIdxPerThread) {
-    const int k = k0 + tid * kIdxPerThread;
-    uint32_t bits = 0;  // bit i = key k + i kept
-    if (vec_ok && k + kIdxPerThread <= Sk) {
+  auto keep_bits = [&](int k) {  // bit i = key k + i kept
+    uint32_t bits = 0;
+    if (vec_ok && k + kIdxPerThread <= k_hi) {
       const uint4 v = *reinterpret_cast<const uint4*>(mrow + k);
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -47,8 +52,25 @@ __global__ void __launch_bounds__(kIdxThreads) compact_index_kernel(const uint8_
         if ((w[i >> 2] >> ((i & 3) * 8)) & 0xFFu) bits |= 1u << i;
     } else {
       for (int i = 0; i < kIdxPerThread; ++i)
-        if (k + i < Sk && mrow[k + i]) bits |= 1u << i;
+        if (k + i < k_hi && mrow[k + i]) bits |= 1u << i;
     }
+    return bits;
+  };
+  if (tid == 0) s_base = s_count = 0;
+  __syncthreads();
+  if (nrank > 1) {
+    int mine = 0;
+#pragma unroll 4
+    for (int k = k_lo + tid * kIdxPerThread; k < k_hi; k += kIdxThreads * kIdxPerThread) mine += __popc(keep_bits(k));
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane == 0) atomicAdd(&s_count, mine);
+    cluster.sync();
+    if (tid < rank) atomicAdd(&s_base, *cluster.map_shared_rank(&s_count, tid));
+    __syncthreads();
+  }
+  for (int k0 = k_lo; k0 < k_hi; k0 += kIdxThreads * kIdxPerThread) {
+    const int k = k0 + tid * kIdxPerThread;
+    uint32_t bits = keep_bits(k);
     const int mine = __popc(bits);
     int incl = mine;
 #pragma unroll
@@ -67,12 +89,17 @@ __global__ void __launch_bounds__(kIdxThreads) compact_index_kernel(const uint8_
       ++before;
     }
     __syncthreads();
-    if (tid == kIdxThreads - 1) s_base = before;  // the last thread's running total is the row's
+    if (tid == kIdxThreads - 1) s_base = before;  // the last thread's running total
     __syncthreads();
   }
-  const int total = s_base;
-  if (tid == 0) count[row] = total;
-  for (int s = tid; s < cap; s += kIdxThreads) {
+  int total = s_base;
+  if (nrank > 1) {
+    total = 0;
+    for (int r = 0; r < nrank; ++r) total += *cluster.map_shared_rank(&s_count, r);
+    cluster.sync();  // nobody leaves while its shared memory may still be read
+  }
+  if (rank == 0 && tid == 0) count[row] = total;
+  for (int s = rank * kIdxThreads + tid; s < cap; s += nrank * kIdxThreads) {
     if (s >= total) prow[s] = 0x7FFFFFFF;
     if (mask_out) mask_out[static_cast<int64_t>(row) * cap + s] = s < total ? 1 : 0;
   }
@@ -253,10 +280,22 @@ extern "C" int fdma_compact_index(const fdma_compact_params* p, void* stream) {
   if (p->b_mask <= 0 || p->h_mask <= 0 || p->seqlen_k <= 0 || p->capacity <= 0) return FDMA_ERR_BAD_ARG;
   const int64_t rows = static_cast<int64_t>(p->b_mask) * p->h_mask;
   if (rows > 0x7FFFFFFF) return FDMA_ERR_TOO_LARGE;
-  compact_index_kernel<<<static_cast<unsigned>(rows), kIdxThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint8_t*>(p->mask), p->mask_batch_stride, p->mask_head_stride, p->h_mask, p->seqlen_k,
-      p->capacity, p->key_pos, p->count, static_cast<uint8_t*>(p->mask_out));
-  return static_cast<int>(cudaGetLastError());
+  // CTAs per row: one round of the kernel (4096 keys) each, as long as the CTAs of all rows fit the GPU at once
+  int ctas = 1;
+  while (ctas < 8 && p->seqlen_k > ctas * kIdxThreads * kIdxPerThread && rows * ctas * 2 <= 4ll * sm_count()) ctas *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(rows) * ctas);
+  cfg.blockDim = dim3(kIdxThreads);
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ctas;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, compact_index_kernel, static_cast<const uint8_t*>(p->mask),
+                                             p->mask_batch_stride, p->mask_head_stride, p->h_mask, p->seqlen_k, p->capacity,
+                                             p->key_pos, p->count, static_cast<uint8_t*>(p->mask_out)));
 }
 
 extern "C" int fdma_gather_rows(const fdma_rows_params* p, void* stream) {

@@ -217,3 +217,28 @@ def test_left_padded_batch_with_empty_query_blocks(dev):
     for b in range(B):
         ref = oracle.attention_forward(q[b:b + 1], k[b:b + 1], v[b:b + 1], mask[b:b + 1], bias[b:b + 1], None, True)[0]
         check(f"out[{b}]", out[b:b + 1], ref, dtype)
+
+
+@pytest.mark.parametrize("rows,keys", [((1, 1), 1), ((1, 1), 4096), ((1, 1), 4097), ((1, 3), 8193), ((2, 1), 20001), ((1, 2), 32768),
+                                       ((1, 1), 300007), ((20, 8), 16400), ((80, 8), 9000)])
+@pytest.mark.parametrize("share", [0.0, 0.02, 1.0])
+def test_index_of_long_rows(rows, keys, share):
+    """Rows shared by clusters of one to eight CTAs: lengths one beside a CTA's round, unaligned rows, capacity below the count."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from flash_sparse_attn.compaction import index_kept_keys
+
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(keys)
+    m = torch.rand((*rows, keys), generator=gen, device=dev) < share
+    m[..., : keys // 3] &= torch.rand((), generator=gen, device=dev) < 0.5  # some segments empty
+    key_pos, count, slots = index_kept_keys(m)
+    assert torch.equal(count, m.sum(-1, dtype=torch.int32))
+    cap = key_pos.shape[-1]
+    want = torch.where(m, torch.arange(keys, device=dev, dtype=torch.int32), 0x7FFFFFFF).sort(-1).values
+    want = torch.nn.functional.pad(want, [0, cap], value=0x7FFFFFFF)[..., :cap]
+    assert torch.equal(key_pos, want)
+    assert torch.equal(slots[:, :, 0], want != 0x7FFFFFFF)
+    if cap > 128:
+        short, total, _ = index_kept_keys(m, 128, check_capacity=False)
+        assert torch.equal(short, want[..., :128]) and torch.equal(total, count)
