@@ -61,6 +61,7 @@ struct DecodeParams {
   int k_sr, v_sr;        // row strides in elements, below 2^31: one widening multiply per address
   int64_t pos_sb, pos_sh, count_sb, count_sh, bias_sb, bias_sh;
   int h, h_k, h_pos, h_bias, d, seqlen_k, slots, nsplit;
+  int row_align;         // kPieces: bytes K and V rows are aligned to
   int heads;             // query heads per CTA
   int head_blocks;       // CTA rows per (batch, split)
   float scale_log2;
@@ -75,6 +76,19 @@ __device__ __forceinline__ uint64_t evict_first_policy() {
 }
 __device__ __forceinline__ void cp_async16(uint32_t smem, const void* gmem, uint64_t policy) {
   asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(smem), "l"(gmem), "l"(policy) : "memory");
+}
+// 16 bytes of a row whose pieces are aligned to `align` (4 or 8) bytes only
+__device__ __forceinline__ void cp_async16_in_pieces(uint32_t smem, const void* gmem, int align) {
+  const char* g = static_cast<const char*>(gmem);
+  if (align == 8) {
+#pragma unroll
+    for (int o = 0; o < 16; o += 8)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem + o), "l"(g + o) : "memory");
+  } else {
+#pragma unroll
+    for (int o = 0; o < 16; o += 4)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem + o), "l"(g + o) : "memory");
+  }
 }
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -126,16 +140,17 @@ __device__ __forceinline__ float exp2_or_zero(float x) { return x == -CUDART_INF
 
 // kM16: 9 to 16 query heads (both halves of the M rows of the products), else up to 8. Fragments of mma.m16n8k16
 // (g = lane / 4, c = lane % 4): A row g (+ 8), k = 2c, 2c+1 (+ 8); B k = 2c, 2c+1 (+ 8), n = g; C row g (+ 8), n = 2c, 2c+1.
-template <int NJ, bool kBf16, bool kM16>
-__global__ void __launch_bounds__(kThreads, NJ <= 4 ? 3 : 1) decode_rows_kernel(const DecodeParams p) {
+// kPieces: K / V rows that are aligned to 4 or 8 bytes only.
+template <int NJ, bool kBf16, bool kM16, bool kPieces>
+__global__ void __launch_bounds__(kThreads, NJ <= 4 && !kPieces ? 3 : 1) decode_rows_kernel(const DecodeParams p) {
   using L = Ring<NJ>;
   constexpr int D = NJ * 32;
   constexpr int kHalves = kM16 ? 2 : 1;
   constexpr int kHeads = 8 * kHalves;
-  // Head dims above 128: the probabilities keep their 32 bits, as sums of three 16-bit values with a product each. fp16 holds
-  // them times 2^14, away from its smallest numbers. (8 x 65536 keys, 4096 kept, 32 heads over 8, d = 256: 104 us with 16-bit
+  // Head dims above 128, and rows in pieces: the probabilities keep their 32 bits, as sums of three 16-bit values with a product
+  // each. fp16 holds them times 2^14, away from its smallest numbers. (8 x 65536 keys, 4096 kept, 32 heads over 8, d = 256: 104 us with 16-bit
   // probabilities, which are 15 % further from the exact result, 113 us so.)
-  constexpr int kTerms = D > 128 ? 3 : 1;
+  constexpr int kTerms = D > 128 || kPieces ? 3 : 1;
   constexpr float kPScale = kTerms > 1 && !kBf16 ? 16384.f : 1.f;
   extern __shared__ __align__(16) unsigned char s_dyn[];  // the warps' rings; afterwards [kWarps][kHeads][D] fp32 partials
   __shared__ uint32_t s_q[kHalves][2 * NJ][2][32];        // A fragments of Q, one word per lane
@@ -228,8 +243,14 @@ __global__ void __launch_bounds__(kThreads, NJ <= 4 ? 3 : 1) decode_rows_kernel(
       if (in) {
         const uint32_t kd = dst + r * L::kRowBytes, vd = kd + kChunk * L::kRowBytes;
         if (pos >= 0) {
-          cp_async16(kd, krow + static_cast<int64_t>(pos) * k_sr, policy);
-          cp_async16(vd, vrow + static_cast<int64_t>(pos) * v_sr, policy);
+          const uint16_t *ks = krow + static_cast<int64_t>(pos) * k_sr, *vs = vrow + static_cast<int64_t>(pos) * v_sr;
+          if (kPieces) {
+            cp_async16_in_pieces(kd, ks, p.row_align);
+            cp_async16_in_pieces(vd, vs, p.row_align);
+          } else {
+            cp_async16(kd, ks, policy);
+            cp_async16(vd, vs, policy);
+          }
         } else {
           asm volatile("st.shared.v4.b32 [%0], {%1,%1,%1,%1};" ::"r"(kd), "r"(0) : "memory");
           asm volatile("st.shared.v4.b32 [%0], {%1,%1,%1,%1};" ::"r"(vd), "r"(0) : "memory");
@@ -471,9 +492,9 @@ DecodePlan plan(const fdma_fwd_params& p, int slots, int h_pos, bool index) {
   return pl;
 }
 
-template <int NJ, bool kBf16, bool kM16>
+template <int NJ, bool kBf16, bool kM16, bool kPieces>
 int launch(const DecodeParams& dp, const DecodePlan& pl, int batch, cudaStream_t stream) {
-  auto kern = decode_rows_kernel<NJ, kBf16, kM16>;
+  auto kern = decode_rows_kernel<NJ, kBf16, kM16, kPieces>;
   constexpr int parts = kWarps * (kM16 ? 16 : 8) * NJ * 32 * static_cast<int>(sizeof(float));
   constexpr int smem = std::max(parts, kWarps * Ring<NJ>::kWarpBytes);
   if (smem > 40 * 1024) {
@@ -493,11 +514,21 @@ int launch(const DecodeParams& dp, const DecodePlan& pl, int batch, cudaStream_t
   cfg.numAttrs = 1;
   return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, dp));
 }
-template <int NJ>
+template <int NJ, bool kPieces>
 int launch_nj(const DecodeParams& dp, const DecodePlan& pl, int batch, bool bf16, cudaStream_t stream) {
-  if (NJ <= 4 && pl.heads > 8)
-    return bf16 ? launch<NJ, true, NJ <= 4>(dp, pl, batch, stream) : launch<NJ, false, NJ <= 4>(dp, pl, batch, stream);
-  return bf16 ? launch<NJ, true, false>(dp, pl, batch, stream) : launch<NJ, false, false>(dp, pl, batch, stream);
+  constexpr bool kM16 = NJ <= 4;
+  if (kM16 && pl.heads > 8)
+    return bf16 ? launch<NJ, true, kM16, kPieces>(dp, pl, batch, stream) : launch<NJ, false, kM16, kPieces>(dp, pl, batch, stream);
+  return bf16 ? launch<NJ, true, false, kPieces>(dp, pl, batch, stream) : launch<NJ, false, false, kPieces>(dp, pl, batch, stream);
+}
+
+// Bytes that every row of K and V is aligned to: 16, 8, 4 or 2.
+int row_align(const fdma_fwd_params& p) {
+  uint64_t x = reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v);
+  if (p.seqlen_k > 1) x |= static_cast<uint64_t>(p.k_row_stride | p.v_row_stride) * 2;
+  if (p.h_k > 1) x |= static_cast<uint64_t>(p.k_head_stride | p.v_head_stride) * 2;
+  if (p.b > 1) x |= static_cast<uint64_t>(p.k_batch_stride | p.v_batch_stride) * 2;
+  return x % 16 == 0 ? 16 : x % 8 == 0 ? 8 : x % 4 == 0 ? 4 : 2;
 }
 
 int run(const fdma_fwd_params& p, const DecodePlan& pl, const int32_t* pos, int64_t pos_sb, int64_t pos_sh, int h_pos,
@@ -517,16 +548,18 @@ int run(const fdma_fwd_params& p, const DecodePlan& pl, const int32_t* pos, int6
   dp.h = p.h; dp.h_k = p.h_k; dp.h_bias = p.h_bias; dp.d = p.d; dp.seqlen_k = p.seqlen_k;
   dp.slots = slots; dp.nsplit = pl.nsplit; dp.heads = pl.heads; dp.head_blocks = pl.head_blocks;
   dp.scale_log2 = p.softmax_scale * kLog2e;
+  dp.row_align = row_align(p);
+  const bool pieces = dp.row_align < 16;
   const bool bf16 = p.dtype == FDMA_BF16;
   cudaEvent_t ev0, ev1;
   take_timing_events(&ev0, &ev1);
   if (ev0) cudaEventRecord(ev0, stream);
   int st;
   switch (blocks_of(p.d)) {
-    case 2: st = launch_nj<2>(dp, pl, p.b, bf16, stream); break;
-    case 3: st = launch_nj<3>(dp, pl, p.b, bf16, stream); break;
-    case 4: st = launch_nj<4>(dp, pl, p.b, bf16, stream); break;
-    default: st = launch_nj<8>(dp, pl, p.b, bf16, stream); break;
+    case 2: st = pieces ? launch_nj<2, true>(dp, pl, p.b, bf16, stream) : launch_nj<2, false>(dp, pl, p.b, bf16, stream); break;
+    case 3: st = launch_nj<3, false>(dp, pl, p.b, bf16, stream); break;
+    case 4: st = pieces ? launch_nj<4, true>(dp, pl, p.b, bf16, stream) : launch_nj<4, false>(dp, pl, p.b, bf16, stream); break;
+    default: st = launch_nj<8, false>(dp, pl, p.b, bf16, stream); break;
   }
   if (ev1) cudaEventRecord(ev1, stream);
   if (st || pl.nsplit == 1) return st;
@@ -544,14 +577,10 @@ int mask_list_heads(const fdma_fwd_params& p) { return p.mask ? p.h_mask : 1; }
 bool decode_supported(const fdma_fwd_params& p) {
   if (p.seqlen_q != 1 || p.seqlen_k <= 0 || p.d % 8 || p.d > 256) return false;
   if (p.mask && p.mask_bits) return false;
-  // rows are read in 16-byte pieces
-  const void* ptrs[3] = {p.q, p.k, p.v};
-  for (const void* x : ptrs)
-    if (reinterpret_cast<uintptr_t>(x) & 15u) return false;
-  const int64_t strides[8] = {p.q_batch_stride, p.q_head_stride, p.k_batch_stride, p.k_row_stride,
-                              p.k_head_stride,  p.v_batch_stride, p.v_row_stride,  p.v_head_stride};
-  for (int64_t s : strides)
-    if (s % 8) return false;
+  // K and V rows are read in 16-byte pieces, at head dims 64 and 128 also in 4- and 8-byte ones; Q in 4-byte words
+  const int align = row_align(p);
+  if (align < 16 && !((p.d == 64 || p.d == 128) && align >= 4)) return false;
+  if ((reinterpret_cast<uintptr_t>(p.q) & 3u) || p.q_batch_stride % 2 || p.q_head_stride % 2) return false;
   if (p.k_row_stride < 0 || p.k_row_stride > 0x7FFFFFFF || p.v_row_stride < 0 || p.v_row_stride > 0x7FFFFFFF) return false;
   return p.b <= 65535 && p.h <= 2047;  // grid limits: head rows x up to 32 splits in y
 }

@@ -97,3 +97,41 @@ def test_probabilities_stay_in_32_bits_above_head_dim_128(dev, Sk, d, H, window,
     exact = (torch.softmax(s, -1) @ v64).transpose(1, 2)
     err, rounding = ((x.double() - exact).norm().item() for x in (out, exact.to(dtype)))
     assert err <= 1.02 * rounding, (err / rounding)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("d,pad,shift", [(64, 2, 0), (64, 4, 4), (64, 0, 2), (128, 4, 0), (128, 12, 8), (128, 0, 4)])
+@pytest.mark.parametrize("geom", [(1, 1, 4, 2), (3, 333, 8, 2), (2, 5000, 24, 2), (1, 70000, 2, 1)])
+@pytest.mark.parametrize("with_mask", [False, True])
+def test_rows_aligned_to_4_or_8_bytes(dev, geom, with_mask, d, pad, shift, dtype):
+    """K / V rows `pad` elements apart and `shift` elements off their base stay on the decode kernels, with the
+    probabilities in 32 bits, as the kernels for such rows have them: within 2 % of the rounding of the exact result."""
+    from flash_sparse_attn import flash_sparse_attn_func
+    from flash_sparse_attn.flash_sparse_attn_interface import set_kernel_path
+
+    B, Sk, H, Hk = geom
+    q, k, v, bias, _ = (t.to(dev) for t in oracle.make_inputs(B, 1, Sk, H, Hk, d, (B, Hk, 1, Sk), seed=6, dtype=dtype))
+    mask = torch.rand((B, Hk, 1, Sk), generator=torch.Generator().manual_seed(2)).to(dev) < 0.5 if with_mask else None
+    if with_mask:
+        mask[..., 0] = True
+
+    def odd(t):
+        flat = torch.full((B * Sk * Hk * (d + pad) + shift,), float("nan"), device=dev, dtype=dtype)
+        view = flat[shift:].view(B, Sk, Hk, d + pad)[..., :d]
+        return view.copy_(t)
+
+    set_kernel_path("decode")
+    try:
+        with torch.no_grad():
+            out = flash_sparse_attn_func(q, odd(k), odd(v), mask, bias)
+    finally:
+        set_kernel_path("auto")
+    torch.cuda.synchronize()
+    _kernel_status_ok()
+    k64, v64 = (t.double().repeat_interleave(H // Hk, 2).transpose(1, 2) for t in (k, v))
+    s = q.double().transpose(1, 2) @ k64.transpose(-1, -2) * d ** -0.5 + bias.double().repeat_interleave(H // Hk, 1)
+    if with_mask:
+        s = s.masked_fill(~mask.repeat_interleave(H // Hk, 1), float("-inf"))
+    exact = (torch.softmax(s, -1) @ v64).transpose(1, 2)
+    err, rounding = ((x.double() - exact).norm().item() for x in (out, exact.to(dtype)))
+    assert err <= 1.02 * rounding + 1e-6 * exact.norm().item(), (err / rounding)
