@@ -223,6 +223,18 @@ int sm_count() {
   return cached[dev];
 }
 
+int single_query_fwd_in(const fdma_fwd_params& in, cudaStream_t stream) {
+  int st = validate_fwd(in);
+  if (st) return st;
+  st = check_arch();
+  if (st) return st;
+  const fdma_fwd_params p = normalise(in);
+  if ((p.path != FDMA_PATH_AUTO && p.path != FDMA_PATH_DECODE) || !p.mask || !decode_supported(p)) return FDMA_ERR_TOO_LARGE;
+  st = decode_fwd_sliced(p, stream);
+  if (st != FDMA_ERR_WORKSPACE) return st;
+  return tc_fwd_supported(p) && tc_fwd_workspace_bytes(p) == 0 ? tc_fwd(p, stream) : simt_fwd(p, stream);
+}
+
 }  // namespace fdma
 
 using namespace fdma;

@@ -609,6 +609,49 @@ int decode_fwd(const fdma_fwd_params& p, cudaStream_t stream) {
              p.seqlen_k, stream);
 }
 
+// The same for a bool mask in less scratch than the position lists of all rows take: one batch element and as many mask heads
+// at a time as fit, one after the other. FDMA_ERR_WORKSPACE when a single row's list does not fit.
+int decode_fwd_sliced(const fdma_fwd_params& p, cudaStream_t stream) {
+  const int group = p.h / p.h_k, per_mask = p.h / p.h_mask;  // query heads per kv head, per mask head
+  auto slice = [&](int b, int m0, int m) {  // mask heads [m0, m0 + m): whole kv heads, or part of one
+    const int h0 = m0 * per_mask, hk0 = h0 / group;
+    fdma_fwd_params s = p;
+    s.b = 1;
+    s.h = m * per_mask;
+    s.h_k = std::max(1, s.h / group);
+    s.h_mask = m;
+    s.q = static_cast<const uint16_t*>(p.q) + b * p.q_batch_stride + h0 * p.q_head_stride;
+    s.k = static_cast<const uint16_t*>(p.k) + b * p.k_batch_stride + hk0 * p.k_head_stride;
+    s.v = static_cast<const uint16_t*>(p.v) + b * p.v_batch_stride + hk0 * p.v_head_stride;
+    s.out = static_cast<uint16_t*>(p.out) + b * p.o_batch_stride + h0 * p.o_head_stride;
+    s.lse = p.lse + static_cast<int64_t>(b) * p.h + h0;
+    s.mask = static_cast<const uint8_t*>(p.mask) + b * p.mask_batch_stride + m0 * p.mask_head_stride;
+    if (p.bias) {
+      const int bias_head = p.h_bias == p.h ? h0 : p.h_bias == p.h_k ? hk0 : 0;
+      s.bias = static_cast<const uint16_t*>(p.bias) + b * p.bias_batch_stride + bias_head * p.bias_head_stride;
+      s.h_bias = p.h_bias == p.h ? s.h : p.h_bias == p.h_k ? s.h_k : 1;
+    }
+    return s;
+  };
+  const int lists_per_kv = std::max(1, p.h_mask / p.h_k);  // mask heads that make up a kv head
+  int m = p.h_mask;
+  while (decode_workspace_bytes(slice(0, 0, m)) > p.workspace_bytes) {
+    if (m == 1) return FDMA_ERR_WORKSPACE;
+    if (m > lists_per_kv) {
+      m = std::max(lists_per_kv, m / 2 / lists_per_kv * lists_per_kv);
+    } else {
+      do --m;
+      while (lists_per_kv % m);
+    }
+  }
+  for (int b = 0; b < p.b; ++b)
+    for (int m0 = 0; m0 < p.h_mask; m0 += m) {
+      const int st = decode_fwd(slice(b, m0, std::min(m, p.h_mask - m0)), stream);
+      if (st) return st;
+    }
+  return 0;
+}
+
 }  // namespace fdma
 
 using namespace fdma;

@@ -85,6 +85,10 @@ int launch_bwd_finish(BwdFinishArgs a, bool bf16, bool deterministic, cudaStream
 bool decode_supported(const fdma_fwd_params& p);
 size_t decode_workspace_bytes(const fdma_fwd_params& p);
 int decode_fwd(const fdma_fwd_params& p, cudaStream_t stream);
+int decode_fwd_sliced(const fdma_fwd_params& p, cudaStream_t stream);
+// fdma_fwd for a single query with a bool mask in whatever workspace there is: position lists a few rows at a time, or where
+// not even one list fits, the kernels that need none. FDMA_ERR_TOO_LARGE for other calls.
+int single_query_fwd_in(const fdma_fwd_params& p, cudaStream_t stream);
 
 // ---- create_mask -------------------------------------------------------------------------------
 int create_mask(const fdma_mask_params& p, cudaStream_t stream);

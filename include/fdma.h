@@ -287,8 +287,10 @@ int fdma_selftest_wait_timeout(uint32_t limit_us, int* result_dev, void* stream)
  * (query it first to know):
  *   - a per-query mask: one activity byte per 128x128 tile, B * h_mask * ceil(Sq/128) * ceil(Sk/128) bytes;
  *   - a single-query call (seqlen_q == 1) on the row-gather decode kernel: with a bool mask the position lists derived
- *     from it, B * h_mask * round_up(Sk,128) * 4 bytes, and for long key ranges with few heads fp32 partials.
- * A call needing more than the limit returns FDMA_ERR_TOO_LARGE and launches nothing. The first call on each
+ *     from it, B * h_mask * round_up(Sk,128) * 4 bytes, and for long key ranges with few heads fp32 partials. With a
+ *     bool mask such a call is served beyond the limit too, its lists a few rows at a time, as long as
+ *     B * H * 8 * (d + 2) * 4 bytes are within it.
+ * Any other call needing more than the limit returns FDMA_ERR_TOO_LARGE and launches nothing. The first call on each
  * device resolves the array's address: issue it outside any stream capture. Calls share the array; calls whose
  * GPU work overlaps in time race and must be serialised by the caller.
  */

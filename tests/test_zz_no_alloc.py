@@ -113,3 +113,46 @@ def test_static_scratch_serves_single_query_calls_up_to_its_limit():
         torch.cuda.synchronize()
         assert torch.isfinite(out_new.float()).all()
         assert torch.equal(out_new, out_ref) and torch.equal(lse_new, lse_ref)
+
+
+@pytest.mark.parametrize("B,H,Hk,h_mask,h_bias,Sk,d", [
+    (1, 32, 8, 8, 8, 65536, 128),    # eight lists of 256 KB: three at a time
+    (2, 8, 2, 8, 2, 50048, 64),      # a list per query head: parts of a kv head
+    (3, 12, 4, 12, 12, 40064, 64),   # groups of three
+    (2, 4, 2, 1, 1, 200064, 128),    # one list per batch element
+    (1, 2, 1, 1, 2, 300032, 64),     # a list that does not fit at all
+])
+def test_static_scratch_serves_long_masked_rows(B, H, Hk, h_mask, h_bias, Sk, d):
+    """A single query with a bool mask whose position lists take more than the limit: made and used a few rows at a time."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from flash_sparse_attn import _lib
+    from flash_sparse_attn import flash_sparse_attn_interface as iface
+
+    lib = _lib.load()
+    dev = torch.device("cuda:0")
+    torch.cuda.set_device(dev)
+    stream = torch.cuda.current_stream(dev).cuda_stream
+    gen = torch.Generator(device=dev).manual_seed(3)
+    q, k, v, bias = (torch.randn(s, generator=gen, device=dev).to(torch.bfloat16)
+                     for s in ((B, 1, H, d), (B, Sk, Hk, d), (B, Sk, Hk, d), (B, h_bias, 1, Sk)))
+    mask = torch.rand((B, h_mask, 1, Sk), generator=gen, device=dev) < 0.05
+    mask[0, 0] = False
+    results = []
+    for static in (False, True):
+        out = torch.full_like(q, float("nan"))
+        lse = torch.full((B, H, 1), float("nan"), device=dev)
+        p = _params(_lib, iface, q, k, v, mask, bias, out, lse, False)
+        need = lib.fdma_fwd_workspace_bytes(ctypes.byref(p))
+        assert need > lib.fdma_static_scratch_limit()
+        if static:
+            assert lib.fdma_fwd_static_scratch(ctypes.byref(p), stream) == 0
+        else:
+            ws = torch.empty(need, dtype=torch.uint8, device=dev)
+            p.workspace, p.workspace_bytes = ws.data_ptr(), need
+            assert lib.fdma_fwd(ctypes.byref(p), stream) == 0
+        torch.cuda.synchronize()
+        results.append((out.float(), lse))
+    (a, la), (b, lb) = results
+    assert (a - b).norm() <= 1e-2 * a.norm()  # the keys in another order: one rounding of probabilities and results to bf16
+    assert torch.equal(torch.isposinf(la), torch.isposinf(lb)) and torch.allclose(la, lb, atol=1e-4, rtol=0)
