@@ -80,41 +80,8 @@ int validate_bwd(const fdma_bwd_params& p) {
 }
 
 // Packed sequences: one row of tokens, no mask, no bias, no gathered keys.
-bool packed_ok(const fdma_fwd_params& p) {
-  return p.b == 1 && !p.mask && !p.bias && !p.key_pos && (p.path == FDMA_PATH_AUTO || p.path == FDMA_PATH_TCGEN05);
-}
-
-// Visible ranges of packed sequences: thread r < total_q writes the keys [x, y) that query row r sees, the others the
-// query rows that see a key. Both ends ascend over the rows (a row of no sequence gets an empty range at its place), so
-// the kernels take the range of a tile from its first and last row.
-__global__ void packed_limits_kernel(const int32_t* __restrict__ cu_q, const int32_t* __restrict__ cu_k, int n, int total_q,
-                                     int total_k, int causal, int2* __restrict__ row_keys, int2* __restrict__ key_rows) {
-  const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (t >= static_cast<int64_t>(total_q) + total_k) return;
-  const bool query = t < total_q;
-  const int r = static_cast<int>(query ? t : t - total_q);
-  const int32_t* mine = query ? cu_q : cu_k;
-  int lo = 0, hi = n + 1;  // first entry above r
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (mine[mid] <= r) lo = mid + 1;
-    else hi = mid;
-  }
-  const int i = lo - 1;
-  int2 out;
-  if (i < 0 || i >= n) {
-    out.x = out.y = (query ? cu_k : cu_q)[i < 0 ? 0 : n];
-  } else {
-    const int qs = cu_q[i], qe = cu_q[i + 1], ks = cu_k[i], ke = cu_k[i + 1];
-    const int shift = (ke - ks) - (qe - qs);  // query row qs + a sees keys ks .. ks + a + shift
-    out = query ? make_int2(ks, ke) : make_int2(qs, qe);
-    if (causal && query) out.y = min(max(ks + (r - qs) + shift + 1, ks), ke);
-    if (causal && !query) out.x = min(max(qs + (r - ks) - shift, qs), qe);
-  }
-  const int limit = query ? total_k : total_q;
-  out.x = min(max(out.x, 0), limit);
-  out.y = min(max(out.y, out.x), limit);
-  (query ? row_keys : key_rows)[r] = out;
+bool packed_ok(const fdma_fwd_params& p, const PackedSeqs& s) {
+  return s.cu_q && s.cu_k && s.n > 0 && s.n <= (1 << 24) && p.b == 1 && !p.mask && !p.bias && !p.key_pos && (p.path == FDMA_PATH_AUTO || p.path == FDMA_PATH_TCGEN05);
 }
 
 // Normalised copy: absent mask/bias get head count 1 so head-ratio arithmetic never divides by zero, and
@@ -311,36 +278,29 @@ int fdma_bwd(const fdma_bwd_params* pp, void* stream_) {
   return simt_bwd(p, stream);
 }
 
-int fdma_fwd_packed(const fdma_fwd_params* pp, const int32_t* row_keys, void* stream_) {
-  if (!pp || !row_keys) return FDMA_ERR_BAD_ARG;
+int fdma_fwd_varlen(const fdma_fwd_params* pp, const int32_t* cu_q, const int32_t* cu_k, int32_t n, void* stream_) {
+  if (!pp || !cu_q || !cu_k || n <= 0) return FDMA_ERR_BAD_ARG;
   int st = validate_fwd(*pp);
   if (st) return st;
   st = check_arch();
   if (st) return st;
-  fdma_fwd_params p = normalise(*pp);
-  if (!packed_ok(p) || !tc_fwd_supported(p)) return FDMA_ERR_UNSUPPORTED;
-  return tc_fwd(p, static_cast<cudaStream_t>(stream_), row_keys);
+  const fdma_fwd_params p = normalise(*pp);
+  const PackedSeqs seqs = {cu_q, cu_k, n};
+  if (!packed_ok(p, seqs) || !tc_fwd_supported(p)) return FDMA_ERR_UNSUPPORTED;
+  return tc_fwd(p, static_cast<cudaStream_t>(stream_), seqs);
 }
 
-int fdma_bwd_packed(const fdma_bwd_params* pp, const int32_t* key_rows, void* stream_) {
-  if (!pp || !key_rows) return FDMA_ERR_BAD_ARG;
+int fdma_bwd_varlen(const fdma_bwd_params* pp, const int32_t* cu_q, const int32_t* cu_k, int32_t n, void* stream_) {
+  if (!pp || !cu_q || !cu_k || n <= 0) return FDMA_ERR_BAD_ARG;
   int st = validate_bwd(*pp);
   if (st) return st;
   st = check_arch();
   if (st) return st;
   fdma_bwd_params p = *pp;
   p.f = normalise(pp->f);
-  if (!packed_ok(p.f) || p.dbias || p.scatter_pos || p.f.d > 128 || !tc_bwd_supported(p)) return FDMA_ERR_UNSUPPORTED;
-  return tc_bwd(p, static_cast<cudaStream_t>(stream_), key_rows);
-}
-
-int fdma_packed_limits(const int32_t* cu_q, const int32_t* cu_k, int32_t n, int32_t total_q, int32_t total_k, int32_t causal,
-                       int32_t* row_keys, int32_t* key_rows, void* stream_) {
-  if (!cu_q || !cu_k || n <= 0 || total_q <= 0 || total_k <= 0 || !row_keys || !key_rows) return FDMA_ERR_BAD_ARG;
-  const int64_t rows = static_cast<int64_t>(total_q) + total_k;
-  packed_limits_kernel<<<static_cast<unsigned>((rows + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream_)>>>(
-      cu_q, cu_k, n, total_q, total_k, causal, reinterpret_cast<int2*>(row_keys), reinterpret_cast<int2*>(key_rows));
-  return static_cast<int>(cudaGetLastError());
+  const PackedSeqs seqs = {cu_q, cu_k, n};
+  if (!packed_ok(p.f, seqs) || p.dbias || p.scatter_pos || p.f.d > 128 || !tc_bwd_supported(p)) return FDMA_ERR_UNSUPPORTED;
+  return tc_bwd(p, static_cast<cudaStream_t>(stream_), seqs);
 }
 
 int fdma_create_mask(const fdma_mask_params* p, void* stream_) {

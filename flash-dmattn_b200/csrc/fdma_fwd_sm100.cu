@@ -29,6 +29,7 @@
 #include <type_traits>
 
 #include "fdma_internal.h"
+#include "fdma_packed.cuh"
 #include "fdma_ptx.cuh"
 
 namespace fdma {
@@ -70,8 +71,8 @@ struct FwdKernelParams {
   int b, seqlen_q, seqlen_k, h, h_k, h_mask, h_bias;
   int d;             // head dim, at most D: columns beyond it are zeros filled in by TMA and are not stored
   int is_causal;
-  const int2* row_keys;  // packed sequences: keys [x, y) each query row sees (both ascending), or null
-  int n_mblk;        // query blocks (of kNQ tiles) per (batch, head)
+  PackedSeqs seqs;   // packed sequences, each with query blocks and key tiles of its own
+  int n_mblk;        // query blocks (of kNQ tiles) per (batch, head); packed: places for them
   int n_items;       // work items = n_mblk * h * b
   float scale_log2;  // softmax_scale * log2(e)
 };
@@ -99,7 +100,7 @@ struct Smem {
   static constexpr int kNumBars = 2 + 2 * kStages + 2 + 2 + 2 + 2 + 2 * kBmSlots + 1 + 4 + 1 + 1;
   static constexpr int kClcOff = (kBarOff + kNumBars * 8 + 15) / 16 * 16;  // answer of the launch control
   static constexpr int kMiscOff = kClcOff + 16;
-  static constexpr int kTotal = kMiscOff + 48;
+  static constexpr int kTotal = kMiscOff + 16 + 2 * 8 * 4;
   static constexpr int kAlloc = kTotal + 1024;  // slack to align the base to 1024 B
 };
 
@@ -151,9 +152,12 @@ __global__ void tile_activity_kernel(const uint8_t* __restrict__ mask, int64_t s
 // S = Q K^T products are issued while the softmax warps still write out the current O.
 struct FwdItem {
   int mblk, h, b, hk, hm, hb;
+  int q0, sq, k0, sk;  // rows of the item's sequence: first query and their number, first key and their number
 };
 
-__device__ __forceinline__ FwdItem fwd_item(const FwdKernelParams& p, int item) {
+// `seq`: packed sequences, what warp 3 has found for the item: block and sequence (see packed_tile)
+template <bool packed>
+__device__ __forceinline__ FwdItem fwd_item(const FwdKernelParams& p, int item, const volatile int* seq) {
   FwdItem w;
   const int per_block = p.h * p.b;
   const int rem = item % per_block;
@@ -163,14 +167,23 @@ __device__ __forceinline__ FwdItem fwd_item(const FwdKernelParams& p, int item) 
   w.hk = w.h / (p.h / p.h_k);
   w.hm = w.h / (p.h / p.h_mask);
   w.hb = w.h / (p.h / p.h_bias);
+  w.q0 = w.k0 = 0;
+  w.sq = p.seqlen_q;
+  w.sk = p.seqlen_k;
+  if (packed) {
+    w.mblk = seq[0];
+    w.q0 = seq[1];
+    w.sq = seq[2];
+    w.k0 = seq[3];
+    w.sk = seq[4];
+  }
   return w;
 }
 
-// kVariant, per-query kernel: the mask holds one bit per key instead of one byte. Row-broadcast kernel: packed sequences,
-// every query row has its own first and last key (an instantiation of its own: the two limits live in the softmax
-// threads' registers, of which the ordinary kernel has none to spare). One launch instead of one per sequence, and tiles that
-// span sequences: 8192 tokens in 5 sequences, 16 heads, d = 128: forward 258 -> 185 us, backward 617 -> 486 us, the call, with
-// the fills, copies and adds of the sequences' gradients gone, 1510 -> 796 us.
+// kVariant, per-query kernel: the mask holds one bit per key instead of one byte. Row-broadcast kernel: packed sequences, whose
+// items are the blocks of each (an instantiation of its own: the ordinary kernel's softmax threads have no registers to spare
+// for an item's extents). One launch instead of one per sequence: 8192 tokens in 5 sequences, 16 heads, d = 128: forward 258 ->
+// 182 us, backward 617 -> 520 us, the call, with the fills, copies and adds of the sequences' gradients gone, 1510 -> 815 us.
 template <int D, bool kBf16, bool kBcast, bool kVariant = false>
 __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_constant__ FwdKernelParams p) {
   using L = Smem<D>;
@@ -206,32 +219,15 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + L::kMiscOff);
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem + L::kMiscOff + 4);
   volatile int* s_item = reinterpret_cast<volatile int*>(smem + L::kMiscOff + 8);  // [2]: item of the flag table
-  volatile int* s_lim = reinterpret_cast<volatile int*>(smem + L::kMiscOff + 16);  // [2][4]: packed sequences, see tile_limits
+  volatile int* s_seq = reinterpret_cast<volatile int*>(smem + L::kMiscOff + 16);  // [2][8]: packed sequences, see fwd_item
   constexpr int kFlagReaders = 3 + 4 * kNQ;  // producer, MMA issuer, addend warp, one arrival per softmax warp
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int Sq = p.seqlen_q, Sk = p.seqlen_k;
-  const int off = Sk - Sq;
-  const int nt_all = (Sk + kBN - 1) / kBN;
   const bool causal = p.is_causal != 0;
   const WaitCtl ctl{s_abort, p.status};
-  // Per item: end of the key tiles each query tile can see (causal / length limit) and the maximum of the ends, in
-  // n_begin the first tile any of them can see. Packed sequences: warp 3 has read the limits of the item's rows into
-  // `lim` (ends, then begins, of the query tiles).
-  auto tile_limits = [&](const FwdItem& w, const volatile int* lim, int (&n_end)[kNQ], const int32_t*& pos_row,
-                         int& n_begin) {
+  // Per item: number of key tiles each query tile can see at most (causal / length limit), and their maximum.
+  auto tile_limits = [&](const FwdItem& w, int (&n_end)[kNQ], const int32_t*& pos_row) {
     pos_row = nullptr;
-    n_begin = 0;
-    if (packed) {
-      int end = 0;
-#pragma unroll
-      for (int t = 0; t < kNQ; ++t) {
-        n_end[t] = lim[t];
-        end = max(end, n_end[t]);
-      }
-      n_begin = min(lim[2], end);
-      return end;
-    }
     if (kBcast && causal && p.key_pos)  // compacted keys: the causal limit is tested on the keys' positions
       pos_row = p.key_pos + w.b * p.pos_batch_stride +
                 (p.h_pos == p.h ? w.h : (p.h_pos == p.h_k ? w.hk : 0)) * p.pos_head_stride;
@@ -239,9 +235,9 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
 #pragma unroll
     for (int t = 0; t < kNQ; ++t) {
       const int m0 = (w.mblk * kNQ + t) * kBM;
-      int ne = nt_all;
-      if (causal && !pos_row) ne = min(ne, max(0, (m0 + kBM + off + kBN - 1) / kBN));
-      if (m0 >= Sq) ne = 0;
+      int ne = (w.sk + kBN - 1) / kBN;
+      if (causal && !pos_row) ne = min(ne, max(0, (m0 + kBM + w.sk - w.sq + kBN - 1) / kBN));
+      if (m0 >= w.sq) ne = 0;
       n_end[t] = ne;
       nT = max(nT, ne);
     }
@@ -302,10 +298,10 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
         if (!ok) break;
         const int item = s_item[ic & 1];
         if (item >= p.n_items) break;
-        const FwdItem w = fwd_item(p, item);
-        int n_end[kNQ], n_begin;
+        const FwdItem w = fwd_item<packed>(p, item, s_seq + (ic & 1) * 8);
+        int n_end[kNQ];
         const int32_t* pos_row;
-        const int nT = tile_limits(w, s_lim + (ic & 1) * 4, n_end, pos_row, n_begin);
+        const int nT = tile_limits(w, n_end, pos_row);
         const uint8_t* s_flags = s_flags_all + (ic & 1) * kMaxTiles;
         ok = mbar_wait(bar_q_empty, (ic & 1) ^ 1, ctl, kWaitQEmpty);
         if (!ok) break;
@@ -316,8 +312,8 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
 #pragma unroll
           for (int kb = 0; kb < D / 64; ++kb)
             tma_load_4d(s_q + t * L::kQBytes + kb * (kBM * 128), &p.tm_q, bar_q, kb * 64, w.h,
-                        (w.mblk * kNQ + t) * kBM, w.b);
-        for (int j = n_begin; j < nT && ok; ++j) {
+                        w.q0 + (w.mblk * kNQ + t) * kBM, w.b);
+        for (int j = 0; j < nT && ok; ++j) {
           if (s_flags[j] == 0) continue;
 #pragma unroll
           for (int kv = 0; kv < 2 * L::kHalves; ++kv) {  // K, then V, in halves where a slot holds half a tile
@@ -329,7 +325,7 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
             const int col = (kv % L::kHalves) * (D / L::kHalves);
 #pragma unroll
             for (int kb = 0; kb < D / L::kHalves / 64; ++kb)
-              tma_load_4d(s_kv + slot * L::kKvBytes + kb * (kBN * 128), tm, bar_kv_full + slot, col + kb * 64, w.hk, j * kBN,
+              tma_load_4d(s_kv + slot * L::kKvBytes + kb * (kBN * 128), tm, bar_kv_full + slot, col + kb * 64, w.hk, w.k0 + j * kBN,
                           w.b);
             ++it;
           }
@@ -353,17 +349,25 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
       if (!ok) break;
       const int item = s_item[ic & 1];
       if (item >= p.n_items) break;
-      const FwdItem w = fwd_item(p, item);
-      int n_end[kNQ], n_begin;
+      const FwdItem w = fwd_item<packed>(p, item, s_seq + (ic & 1) * 8);
+      int n_end[kNQ];
       const int32_t* pos_row;
-      const int nT = tile_limits(w, s_lim + (ic & 1) * 4, n_end, pos_row, n_begin);
+      const int nT = tile_limits(w, n_end, pos_row);
       const uint8_t* s_flags = s_flags_all + (ic & 1) * kMaxTiles;
       ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(0, mbar_wait(bar_q, ic & 1, ctl, kWaitQ)));
       if (!ok) break;
       tc_fence_after_sync();
       int prev_j = -1;            // previous kept tile of this item (its PV is still to be issued)
+      // packed sequences: V rows beyond the sequence, in its last tile, become zeros, as TMA fills them in at the end of a
+      // tensor (zero probabilities alone would pass a NaN on)
+      auto end_v = [&](int slot) {
+        if (!packed || w.sk - prev_j * kBN >= kBN) return;
+        zero_tile_rows(s_kv + slot * L::kKvBytes, D / L::kHalves / 64, kBN * 128, w.sk - prev_j * kBN, kBN);
+        fence_proxy_async_smem();
+        __syncwarp();
+      };
       uint32_t pv_done[2] = {0, 0};  // PV products issued for this item per query tile (0: the first one overwrites O)
-      for (int j = n_begin; j <= nT && ok; ++j) {
+      for (int j = 0; j <= nT && ok; ++j) {
         const bool last = (j == nT);
         const uint8_t fl = last ? 0 : s_flags[j];
         if (!last && fl == 0) continue;
@@ -407,6 +411,7 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
               const int it = 4 * (a - 1) + 2 + hf;
               ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(2, mbar_wait(bar_kv_full + (it & 3), (it >> 2) & 1, ctl, kWaitKvFullV)));
               if (!ok) break;
+              end_v(it & 3);
               tc_fence_after_sync();
 #pragma unroll
               for (int kk = 0; kk < kBN / 16; ++kk)
@@ -435,6 +440,7 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
           ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(2, mbar_wait(bar_kv_full + (v_it % kStages), (v_it / kStages) & 1,
                                                                      ctl, kWaitKvFullV)));
           if (!ok) break;
+          end_v(v_it % kStages);
         }
         tc_fence_after_sync();
 #pragma unroll
@@ -499,17 +505,17 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
       if (!ok) break;
       const int item = s_item[ic & 1];
       if (item >= p.n_items) break;
-      const FwdItem w = fwd_item(p, item);
-      int n_end[kNQ], n_begin;
+      const FwdItem w = fwd_item<packed>(p, item, s_seq + (ic & 1) * 8);
+      int n_end[kNQ];
       const int32_t* pos_row;
-      const int nT = tile_limits(w, s_lim + (ic & 1) * 4, n_end, pos_row, n_begin);
+      const int nT = tile_limits(w, n_end, pos_row);
       const uint8_t* s_flags = s_flags_all + (ic & 1) * kMaxTiles;
       if (kBcast) {
         const uint8_t* mrow = p.mask ? p.mask + w.b * p.mask_batch_stride + w.hm * p.mask_head_stride : nullptr;
         const uint16_t* brow = p.bias ? reinterpret_cast<const uint16_t*>(p.bias) + w.b * p.bias_batch_stride +
                                             w.hb * p.bias_head_stride
                                       : nullptr;
-        for (int j = n_begin; j < nT && ok; ++j) {
+        for (int j = 0; j < nT && ok; ++j) {
           if (s_flags[j] == 0) continue;
           const int slot = bi % kBmSlots;
           ok = __all_sync(0xffffffffu, mbar_wait(bar_bm_empty + slot, ((bi / kBmSlots) & 1) ^ 1, ctl, kWaitBmEmpty));
@@ -527,18 +533,18 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
             float bf;
             if (kBf16) bf = __uint_as_float(static_cast<uint32_t>(bh[i]) << 16);
             else bf = __half2float(__ushort_as_half(bh[i]));
-            const bool keep = ((mbits >> (8 * i)) & 0xFFu) != 0 && (k0 + i) < Sk;
+            const bool keep = ((mbits >> (8 * i)) & 0xFFu) != 0 && (k0 + i) < w.sk;
             v[i] = keep ? bf * kLog2e : -CUDART_INF_F;
           }
           *reinterpret_cast<float4*>(s_bm + slot * kBN + lane * 4) = make_float4(v[0], v[1], v[2], v[3]);
           if (pos_row) {
             int4 pv = make_int4(0x7FFFFFFF, 0x7FFFFFFF, 0x7FFFFFFF, 0x7FFFFFFF);
-            if (k0 + 3 < Sk) {
+            if (k0 + 3 < w.sk) {
               pv = *reinterpret_cast<const int4*>(pos_row + k0);
             } else {
-              if (k0 < Sk) pv.x = pos_row[k0];
-              if (k0 + 1 < Sk) pv.y = pos_row[k0 + 1];
-              if (k0 + 2 < Sk) pv.z = pos_row[k0 + 2];
+              if (k0 < w.sk) pv.x = pos_row[k0];
+              if (k0 + 1 < w.sk) pv.y = pos_row[k0 + 1];
+              if (k0 + 2 < w.sk) pv.z = pos_row[k0 + 2];
             }
             *reinterpret_cast<int4*>(s_pos + slot * kBN + lane * 4) = pv;
           }
@@ -582,26 +588,25 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
         if (lane == 0) mbar_arrive(bar_flags_full + (ic & 1));
         break;
       }
-      const FwdItem w = fwd_item(p, item);
-      volatile int* lim = s_lim + (ic & 1) * 4;
       if (packed) {
-        if (lane < kNQ) {
-          const int m0 = (w.mblk * kNQ + lane) * kBM;
-          int begin = 0, end = 0;
-          if (m0 < Sq) {
-            begin = p.row_keys[m0].x / kBN;
-            end = max(begin, (p.row_keys[min(m0 + kBM, Sq) - 1].y + kBN - 1) / kBN);
-          }
-          lim[lane] = end;
-          lim[2 + lane] = begin;
+        const PackedTile t = packed_tile(p.seqs.cu_q, p.seqs.n, p.seqlen_q, kNQ * kBM, p.n_mblk - 1 - item / (p.h * p.b));
+        const int2 keys = packed_range(p.seqs.cu_k, p.seqs.n, p.seqlen_k, t.seq);
+        if (lane == 0) {
+          volatile int* seq = s_seq + (ic & 1) * 8;
+          seq[0] = t.tile;
+          seq[1] = t.begin;
+          seq[2] = t.end - t.begin;
+          seq[3] = keys.x;
+          seq[4] = keys.y - keys.x;
         }
         __syncwarp();
       }
-      int n_end[kNQ], n_begin;
+      const FwdItem w = fwd_item<packed>(p, item, s_seq + (ic & 1) * 8);
+      int n_end[kNQ];
       const int32_t* pos_row;
-      const int nT = tile_limits(w, lim, n_end, pos_row, n_begin);
+      const int nT = tile_limits(w, n_end, pos_row);
       uint8_t* s_flags = s_flags_all + (ic & 1) * kMaxTiles;
-      for (int j = n_begin + lane; j < nT; j += 32) {
+      for (int j = lane; j < nT; j += 32) {
         uint8_t f = 0;
         if (kBcast) {
           bool any = true;
@@ -612,10 +617,10 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
             for (int i = 0; i < kBN / 16; ++i) {
               const uint4 v = *reinterpret_cast<const uint4*>(mrow + i * 16);
               uint32_t wd[4] = {v.x, v.y, v.z, v.w};
-              if (j * kBN + i * 16 + 16 > Sk) {  // ragged last tile: drop keys >= Sk
+              if (j * kBN + i * 16 + 16 > w.sk) {  // ragged last tile: drop keys beyond the last
 #pragma unroll
                 for (int e = 0; e < 16; ++e)
-                  if (j * kBN + i * 16 + e >= Sk) wd[e >> 2] &= ~(0xFFu << ((e & 3) * 8));
+                  if (j * kBN + i * 16 + e >= w.sk) wd[e >> 2] &= ~(0xFFu << ((e & 3) * 8));
               }
               acc |= wd[0] | wd[1] | wd[2] | wd[3];
             }
@@ -624,12 +629,12 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
           if (any) {
 #pragma unroll
             for (int t = 0; t < kNQ; ++t)
-              if (j < n_end[t] && (!packed || j >= lim[2 + t])) f |= (1 << t);
+              if (j < n_end[t]) f |= (1 << t);
             if (pos_row) {  // the tile's smallest position against the last row of each query tile
               const int64_t pmin = pos_row[j * kBN];
 #pragma unroll
               for (int t = 0; t < kNQ; ++t) {
-                const int qlast = min((w.mblk * kNQ + t) * kBM + kBM - 1, Sq - 1);
+                const int qlast = min((w.mblk * kNQ + t) * kBM + kBM - 1, w.sq - 1);
                 if (pmin > static_cast<int64_t>(qlast) + p.causal_shift) f &= ~(1 << t);
               }
             }
@@ -640,8 +645,8 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
             if (j < n_end[t]) {
               bool act = true;
               if (p.act) {
-                const int MT = (Sq + kBM - 1) / kBM;
-                act = p.act[((static_cast<int64_t>(w.b) * p.h_mask + w.hm) * MT + (w.mblk * kNQ + t)) * nt_all + j] != 0;
+                const int MT = (w.sq + kBM - 1) / kBM, NT = (w.sk + kBN - 1) / kBN;
+                act = p.act[((static_cast<int64_t>(w.b) * p.h_mask + w.hm) * MT + (w.mblk * kNQ + t)) * NT + j] != 0;
               }
               if (act) f |= (1 << t);
             }
@@ -680,22 +685,15 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
     if (!ok) break;
     const int item = s_item[ic & 1];
     if (item >= p.n_items) break;
-    const FwdItem w = fwd_item(p, item);
+    const FwdItem w = fwd_item<packed>(p, item, s_seq + (ic & 1) * 8);
     const int h = w.h, b = w.b;
-    int n_end[kNQ], n_begin;
+    int n_end[kNQ];
     const int32_t* pos_row;
-    const int nT = tile_limits(w, s_lim + (ic & 1) * 4, n_end, pos_row, n_begin);
+    const int nT = tile_limits(w, n_end, pos_row);
     const uint8_t* s_flags = s_flags_all + (ic & 1) * kMaxTiles;
     const int m0 = (w.mblk * kNQ + t) * kBM;
     const int qrow = m0 + row;
-    const int qclamp = min(qrow, Sq - 1);
-    int2 vis = make_int2(0, Sk);      // packed sequences: the keys this row sees,
-    int warp_lo = 0, warp_hi = Sk;    // and those that every row of the warp sees
-    if (packed) {
-      vis = p.row_keys[qclamp];
-      warp_lo = __shfl_sync(0xffffffffu, vis.x, 31);
-      warp_hi = __shfl_sync(0xffffffffu, vis.y, 0);
-    }
+    const int qclamp = min(qrow, w.sq - 1);
     const uint8_t* mrow = nullptr;
     const uint16_t* brow = nullptr;
     if (!kBcast) {
@@ -717,7 +715,7 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
     // length of both. Warpgroup 1 therefore starts only when warpgroup 0 reaches the exp2 phase of its first
     // tile, which keeps the two loops roughly half a period apart.
     if (kNQ == 2 && t == 1 && ic == 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_stagger, 0, ctl, kWaitS));
-    for (int j = n_begin; j < nT && ok; ++j) {
+    for (int j = 0; j < nT && ok; ++j) {
       const uint8_t fl = s_flags[j];
       if (fl == 0) continue;
       const int slot = bi % kBmSlots;
@@ -840,18 +838,10 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
           }
         }
         // causal / length limit, only on tiles that cross it
-        if constexpr (packed) {
-          if (kbase < warp_lo || kbase + kBN > warp_hi) {
-#pragma unroll
-            for (int i = 0; i < kBN / 2; ++i) {
-              if (kbase + 2 * i < vis.x || kbase + 2 * i >= vis.y) s2[i].x = -CUDART_INF_F;
-              if (kbase + 2 * i + 1 < vis.x || kbase + 2 * i + 1 >= vis.y) s2[i].y = -CUDART_INF_F;
-            }
-          }
-        } else {
-          int klim = Sk;  // keys < klim are visible to this row
+        {
+          int klim = w.sk;  // keys < klim are visible to this row
           const int warp_q0 = m0 + (warp & 3) * 32;  // smallest query row of this warp
-          int wlim = Sk;
+          int wlim = w.sk;
           if (pos_row) {
             const int* tp = s_pos + slot * kBN;
             if (static_cast<int64_t>(tp[kBN - 1]) > static_cast<int64_t>(warp_q0) + p.causal_shift) {
@@ -866,8 +856,8 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
               wlim = kbase;  // take the per-element path
             }
           } else if (causal) {
-            klim = min(klim, qrow + off + 1);
-            wlim = min(wlim, warp_q0 + off + 1);
+            klim = min(klim, qrow + w.sk - w.sq + 1);
+            wlim = min(wlim, warp_q0 + w.sk - w.sq + 1);
           }
           if (kbase + kBN > wlim) {
 #pragma unroll
@@ -968,17 +958,17 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
       tc_fence_after_sync();
     }
     {
-      const bool in_range = qrow < Sq;  // TMEM loads below are warp-collective: every lane runs them
+      const bool in_range = qrow < w.sq;  // TMEM loads below are warp-collective: every lane runs them
       const bool wide_o = (reinterpret_cast<uintptr_t>(p.out) & 31) == 0 &&
                           ((p.o_batch_stride | p.o_row_stride | p.o_head_stride) & 15) == 0;
       // m_ref stays -inf iff every score of the row was masked (l can then hold 2^-125 terms of exp2_poly2)
       const bool alive = sitem > 0 && l > 0.f && m_ref != -CUDART_INF_F;
       const float inv = alive ? 1.f / l : 0.f;
       unsigned char* orow = reinterpret_cast<unsigned char*>(p.out) +
-                            (b * p.o_batch_stride + static_cast<int64_t>(qclamp) * p.o_row_stride +
+                            (b * p.o_batch_stride + static_cast<int64_t>(w.q0 + qclamp) * p.o_row_stride +
                              h * p.o_head_stride) * 2;
       if (in_range)
-        p.lse[(static_cast<int64_t>(b) * p.h + h) * Sq + qrow] = alive ? (m_ref + fast_log2(l)) * kLn2 : CUDART_INF_F;
+        p.lse[(static_cast<int64_t>(b) * p.h + h) * p.seqlen_q + w.q0 + qrow] = alive ? (m_ref + fast_log2(l)) * kLn2 : CUDART_INF_F;
       if (sitem > 0) {
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
@@ -1049,7 +1039,7 @@ FwdPlan plan(const fdma_fwd_params& p) {
 bool aligned16(const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; }
 
 template <int D, bool kBf16, bool kBcast, bool kVariant = false>
-int launch(const fdma_fwd_params& p, const FwdPlan& pl, const int32_t* row_keys, cudaStream_t stream) {
+int launch(const fdma_fwd_params& p, const FwdPlan& pl, const PackedSeqs& seqs, cudaStream_t stream) {
   using L = Smem<D>;
   constexpr int kNQ = L::kNQ;
   FwdKernelParams kp;
@@ -1087,7 +1077,7 @@ int launch(const fdma_fwd_params& p, const FwdPlan& pl, const int32_t* row_keys,
   kp.b = p.b; kp.seqlen_q = p.seqlen_q; kp.seqlen_k = p.seqlen_k; kp.h = p.h; kp.h_k = p.h_k; kp.d = p.d;
   kp.h_mask = p.h_mask; kp.h_bias = p.h_bias;
   kp.is_causal = p.is_causal;
-  kp.row_keys = reinterpret_cast<const int2*>(row_keys);
+  kp.seqs = seqs;
   kp.key_pos = p.key_pos;
   kp.pos_batch_stride = p.key_pos_batch_stride; kp.pos_head_stride = p.key_pos_head_stride;
   kp.h_pos = p.h_pos; kp.causal_shift = p.causal_shift;
@@ -1107,7 +1097,7 @@ int launch(const fdma_fwd_params& p, const FwdPlan& pl, const int32_t* row_keys,
   // The attribute belongs to the (function, device) pair: set it on every call, whichever device is current.
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kAlloc);
   if (e != cudaSuccess) return static_cast<int>(e);
-  kp.n_mblk = (p.seqlen_q + kNQ * kBM - 1) / (kNQ * kBM);
+  kp.n_mblk = seqs.cu_q ? packed_slots(p.seqlen_q, seqs.n, kNQ * kBM) : (p.seqlen_q + kNQ * kBM - 1) / (kNQ * kBM);
   const int64_t n_items = static_cast<int64_t>(kp.n_mblk) * p.h * p.b;
   if (n_items > 0x7FFFFFFF) return FDMA_ERR_TOO_LARGE;
   kp.n_items = static_cast<int>(n_items);
@@ -1121,13 +1111,13 @@ int launch(const fdma_fwd_params& p, const FwdPlan& pl, const int32_t* row_keys,
 }
 
 template <int D>
-int launch_d(const fdma_fwd_params& p, const FwdPlan& pl, const int32_t* rk, cudaStream_t stream) {
+int launch_d(const fdma_fwd_params& p, const FwdPlan& pl, const PackedSeqs& seqs, cudaStream_t stream) {
   if (p.dtype == FDMA_BF16) {
-    if (pl.bcast) return rk ? launch<D, true, true, true>(p, pl, rk, stream) : launch<D, true, true>(p, pl, rk, stream);
-    return (p.mask && p.mask_bits) ? launch<D, true, false, true>(p, pl, rk, stream) : launch<D, true, false>(p, pl, rk, stream);
+    if (pl.bcast) return seqs.cu_q ? launch<D, true, true, true>(p, pl, seqs, stream) : launch<D, true, true>(p, pl, seqs, stream);
+    return (p.mask && p.mask_bits) ? launch<D, true, false, true>(p, pl, seqs, stream) : launch<D, true, false>(p, pl, seqs, stream);
   }
-  if (pl.bcast) return rk ? launch<D, false, true, true>(p, pl, rk, stream) : launch<D, false, true>(p, pl, rk, stream);
-  return (p.mask && p.mask_bits) ? launch<D, false, false, true>(p, pl, rk, stream) : launch<D, false, false>(p, pl, rk, stream);
+  if (pl.bcast) return seqs.cu_q ? launch<D, false, true, true>(p, pl, seqs, stream) : launch<D, false, true>(p, pl, seqs, stream);
+  return (p.mask && p.mask_bits) ? launch<D, false, false, true>(p, pl, seqs, stream) : launch<D, false, false>(p, pl, seqs, stream);
 }
 
 }  // namespace
@@ -1182,12 +1172,12 @@ bool tc_fwd_supported(const fdma_fwd_params& p) {
 
 size_t tc_fwd_workspace_bytes(const fdma_fwd_params& p) { return plan(p).act_bytes; }
 
-int tc_fwd(const fdma_fwd_params& p, cudaStream_t stream, const int32_t* row_keys) {
+int tc_fwd(const fdma_fwd_params& p, cudaStream_t stream, const PackedSeqs& seqs) {
   const FwdPlan pl = plan(p);
   switch (tile_head_dim(p.d)) {
-    case 64: return launch_d<64>(p, pl, row_keys, stream);
-    case 128: return launch_d<128>(p, pl, row_keys, stream);
-    default: return launch_d<256>(p, pl, row_keys, stream);
+    case 64: return launch_d<64>(p, pl, seqs, stream);
+    case 128: return launch_d<128>(p, pl, seqs, stream);
+    default: return launch_d<256>(p, pl, seqs, stream);
   }
 }
 

@@ -18,10 +18,15 @@ int simt_fwd(const fdma_fwd_params& p, cudaStream_t stream);
 int simt_bwd(const fdma_bwd_params& p, cudaStream_t stream);
 
 // ---- tcgen05 / TMA kernels ---------------------------------------------------------------------
+// Packed sequences: cumulative lengths on the device, n + 1 entries each, ascending; null: an ordinary call.
+struct PackedSeqs {
+  const int32_t *cu_q = nullptr, *cu_k = nullptr;
+  int n = 0;
+};
 bool tc_fwd_supported(const fdma_fwd_params& p);
 size_t tc_fwd_workspace_bytes(const fdma_fwd_params& p);
-// row_keys: packed sequences, int2 per query row, see fdma_packed_limits
-int tc_fwd(const fdma_fwd_params& p, cudaStream_t stream, const int32_t* row_keys = nullptr);
+// seqs: packed sequences, see fdma_fwd_varlen
+int tc_fwd(const fdma_fwd_params& p, cudaStream_t stream, const PackedSeqs& seqs = {});
 
 // Per-tile mask activity map for per-query masks: act[b][h_mask][ceil(Sq/128)][ceil(Sk/128)] bytes.
 int launch_tile_activity(const fdma_fwd_params& p, uint8_t* act, cudaStream_t stream);
@@ -33,7 +38,7 @@ int tc_bwd256(const fdma_bwd_params& p, cudaStream_t stream);
 
 bool tc_bwd_supported(const fdma_bwd_params& p);
 size_t tc_bwd_workspace_bytes(const fdma_bwd_params& p);
-int tc_bwd(const fdma_bwd_params& p, cudaStream_t stream, const int32_t* key_rows = nullptr);  // key_rows: head dims up to 128
+int tc_bwd(const fdma_bwd_params& p, cudaStream_t stream, const PackedSeqs& seqs = {});  // seqs: head dims up to 128
 
 // ---- the kernels before and after every tensor-core backward (fdma_bwd_common.cu) ---------------
 constexpr int kDetFracBits = 40;  // deterministic dQ accumulator: fixed point, |dQ / scale| < 2^23, resolution 2^-40

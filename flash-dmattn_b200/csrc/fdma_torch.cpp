@@ -45,9 +45,8 @@ struct Api {
   decltype(&fdma_fwd) fwd;
   decltype(&fdma_bwd_workspace_bytes) bwd_workspace_bytes;
   decltype(&fdma_bwd) bwd;
-  decltype(&fdma_packed_limits) packed_limits;
-  decltype(&fdma_fwd_packed) fwd_packed;
-  decltype(&fdma_bwd_packed) bwd_packed;
+  decltype(&fdma_fwd_varlen) fwd_varlen;
+  decltype(&fdma_bwd_varlen) bwd_varlen;
   decltype(&fdma_create_mask) create_mask;
   decltype(&fdma_gather_kept) gather_kept;
   decltype(&fdma_decode_kept) decode_kept;
@@ -68,9 +67,8 @@ void init(const std::string& path) {
   get(api.fwd, "fdma_fwd");
   get(api.bwd_workspace_bytes, "fdma_bwd_workspace_bytes");
   get(api.bwd, "fdma_bwd");
-  get(api.packed_limits, "fdma_packed_limits");
-  get(api.fwd_packed, "fdma_fwd_packed");
-  get(api.bwd_packed, "fdma_bwd_packed");
+  get(api.fwd_varlen, "fdma_fwd_varlen");
+  get(api.bwd_varlen, "fdma_bwd_varlen");
   get(api.create_mask, "fdma_create_mask");
   get(api.gather_kept, "fdma_gather_kept");
   get(api.decode_kept, "fdma_decode_kept");
@@ -244,7 +242,7 @@ void fill_gathered(fdma_fwd_params& p, const KvB& kv, const Tensor& key_pos, con
 // One node for the four routes. Saved: dense   q, k, v, mask, bias, out, lse
 //                                       bits    q, k, v, bits, bias, out, lse, activity
 //                                       gathered q, kvb, -, slot_mask, -, out, lse, key_pos
-//                                       packed  q, k, v, -, -, out, lse, the query rows that see each key
+//                                       packed  q, k, v, -, -, out, lse, cu (2, n + 1): the sequences' boundaries
 enum { kQ, kK, kV, kMask, kBias, kOut, kLse, kExtra, kNumSaved };
 using SavedTensors = std::array<Tensor, kNumSaved>;
 
@@ -344,7 +342,7 @@ struct AttnBackward : public torch::autograd::Node {
 
 // Gradients of packed sequences: (tokens, heads, d) tensors, one row of tokens for the kernels.
 variable_list packed_backward(const SavedTensors& t, const Call& c, const Tensor& dout, cudaStream_t stream) {
-  const Tensor &tq = t[kQ], &tk = t[kK], &tv = t[kV], &tout = t[kOut], &tlse = t[kLse], &key_rows = t[kExtra];
+  const Tensor &tq = t[kQ], &tk = t[kK], &tv = t[kV], &tout = t[kOut], &tlse = t[kLse], &cu = t[kExtra];
   variable_list res(3);
   Tensor dq = empty(tq.sizes(), tq.scalar_type(), tq), dk = empty(tk.sizes(), tk.scalar_type(), tk), dv = empty(tv.sizes(), tv.scalar_type(), tv);
   fdma_bwd_params bp = {};
@@ -368,7 +366,8 @@ variable_list packed_backward(const SavedTensors& t, const Call& c, const Tensor
     bp.f.workspace = ws.data_ptr();
     bp.f.workspace_bytes = bytes;
   }
-  check(api.bwd_packed(&bp, key_rows.data_ptr<int32_t>(), stream), "fdma_bwd_packed");
+  const int32_t* cu_q = cu.data_ptr<int32_t>();
+  check(api.bwd_varlen(&bp, cu_q, cu_q + cu.stride(0), static_cast<int32_t>(cu.size(1) - 1), stream), "fdma_bwd_varlen");
   res[0] = dq; res[1] = dk; res[2] = dv;
   return res;
 }
@@ -657,9 +656,10 @@ std::vector<Tensor> packed_attention(const Tensor& q0, const Tensor& k0, const T
   if ((type != at::kBFloat16 && type != at::kHalf) || k0.scalar_type() != type || v0.scalar_type() != type) return {};
   const int64_t Tq = q0.size(0), H = q0.size(1), d = q0.size(2), Tk = k0.size(0), Hk = k0.size(1);
   if (Tq <= 0 || Tk <= 0 || H <= 0 || Hk <= 0 || H % Hk || d <= 0 || d % 8 || d > 128 || k0.size(2) != d || v0.sizes() != k0.sizes()) return {};
-  if (Hk > 65535 || H > 65535 || Tq > (1 << 19) || Tk > (1 << 20)) return {};  // the kernels' tile tables
+  if (Hk > 65535 || H > 65535 || Tq > kMaxQueries || Tk > kMaxKeys) return {};
   for (const Tensor* t : {&cu_q, &cu_k})
     if (!t->is_cuda() || t->device() != q0.device() || t->scalar_type() != at::kInt || t->dim() != 1 || !t->is_contiguous() || t->size(0) < 2) return {};
+  if (cu_q.size(0) != cu_k.size(0)) return {};
   // what the kernels' TMA loads ask of the tensors; anything else goes sequence by sequence
   for (const Tensor* t : {&q0, &k0, &v0}) {
     if (t->stride(2) != 1 || (reinterpret_cast<uintptr_t>(t->data_ptr()) & 15)) return {};
@@ -673,7 +673,7 @@ std::vector<Tensor> packed_attention(const Tensor& q0, const Tensor& k0, const T
   c.deterministic = deterministic;
   c.packed = true;
   c.seqlen_k = Tk;
-  Tensor out, lse, key_rows;
+  Tensor out, lse, cu;
   {
     at::AutoDispatchBelowADInplaceOrView guard;
     const c10::cuda::CUDAGuard device(q0.device());
@@ -681,17 +681,16 @@ std::vector<Tensor> packed_attention(const Tensor& q0, const Tensor& k0, const T
     raise_if_timed_out(stream);
     out = empty(q0.sizes(), type, q0);
     lse = empty({1, H, Tq}, at::kFloat, q0);
-    const Tensor row_keys = empty({Tq, 2}, at::kInt, q0);
-    key_rows = empty({Tk, 2}, at::kInt, q0);
-    check(api.packed_limits(cu_q.data_ptr<int32_t>(), cu_k.data_ptr<int32_t>(), static_cast<int32_t>(cu_q.size(0) - 1),
-                            static_cast<int32_t>(Tq), static_cast<int32_t>(Tk), causal ? 1 : 0, row_keys.data_ptr<int32_t>(),
-                            key_rows.data_ptr<int32_t>(), stream), "fdma_packed_limits");
+    const int32_t *pq = cu_q.data_ptr<int32_t>(), *pk = cu_k.data_ptr<int32_t>();
+    if (grad) {  // the backward keeps boundaries of its own: the caller may fill its buffers for the next call before
+      cu = cu_q.is_same(cu_k) ? cu_q.clone().unsqueeze(0).expand({2, cu_q.size(0)}) : at::stack({cu_q, cu_k});
+    }
     fdma_fwd_params p = {};
     const Tensor q4 = q0.unsqueeze(0), k4 = k0.unsqueeze(0);
     fill_geometry(p, q4, Tk, Hk, c);
     fill_kv(p, k4, v0.unsqueeze(0));
     fill_out(p, out.unsqueeze(0), lse);
-    check(api.fwd_packed(&p, row_keys.data_ptr<int32_t>(), stream), "fdma_fwd_packed");
+    check(api.fwd_varlen(&p, pq, pk, static_cast<int32_t>(cu_q.size(0) - 1), stream), "fdma_fwd_varlen");
   }
   if (grad) {
     auto node = std::shared_ptr<AttnBackward>(new AttnBackward(), torch::autograd::deleteNode);
@@ -702,7 +701,7 @@ std::vector<Tensor> packed_attention(const Tensor& q0, const Tensor& k0, const T
     node->saved[kV] = SavedVariable(v0, false);
     node->saved[kOut] = SavedVariable(out, /*is_output=*/true);
     node->saved[kLse] = SavedVariable(lse, false);
-    node->saved[kExtra] = SavedVariable(key_rows, false);
+    node->saved[kExtra] = SavedVariable(cu, false);
     node->meta.c = std::move(c);
   }
   return {out, lse};

@@ -66,9 +66,8 @@ EXPORTED_SYMBOLS = (
     "fdma_decode_kept_workspace_bytes",
     "fdma_bwd_workspace_bytes",
     "fdma_bwd",
-    "fdma_packed_limits",
-    "fdma_fwd_packed",
-    "fdma_bwd_packed",
+    "fdma_fwd_varlen",
+    "fdma_bwd_varlen",
     "fdma_create_mask",
     "fdma_last_kernel_status",
     "fdma_poll_kernel_status",

@@ -572,9 +572,10 @@ def flash_sparse_attn_varlen_func(
     of key / value; is_causal aligns each sequence's causal mask to ITS bottom-right corner. Returns out
     (total_q, H, d), or with return_attn_probs=True (out, softmax_lse (H, total_q) fp32, empty tensor).
 
-    Sequences that cover the tokens without a gap run in one launch per direction, where every query row carries its
-    own first and last key (head dims up to 128). Anything else goes sequence by sequence: each is a contiguous slice of the packed
-    tensors, handed to the dense kernels as a zero-copy (1, L, H, d) view. No padding and no mask in either form. The
+    Sequences that cover the tokens without a gap run in one launch per direction, where every tile belongs to one of them
+    (head dims up to 128). Anything else goes sequence by sequence: each is a contiguous slice of the packed
+    tensors, handed to the dense kernels as a zero-copy (1, L, H, d) view. No padding and no mask in either form, and a
+    sequence with non-finite values leaves the others as they are. The
     boundaries are read on the host (one device synchronisation per call) for the checks below. A paged KV cache (`block_table`) is not
     built and raises NotImplementedError."""
     if block_table is not None:

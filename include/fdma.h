@@ -178,18 +178,14 @@ int fdma_bwd(const fdma_bwd_params* p, void* stream);
 
 /*
  * Packed sequences (the varlen call of flash_sparse_attn_interface.py:687-790) in one launch: the parameters describe all
- * tokens as one row (b = 1, no mask, bias or key positions) and two arrays, filled by fdma_packed_limits from the
- * cumulative lengths (n + 1 entries each, ascending), say what sees what. row_keys: int32 pairs (first, end) of the keys
- * that each query row sees; key_rows: of the query rows that see each key. is_causal of the parameters only guides the
- * split of the work. Rows outside every sequence give 0 and LSE = +inf. Workspaces as of fdma_fwd / fdma_bwd. Forward at any head
- * dim the tcgen05 kernels take, backward up to head dim 128; FDMA_ERR_UNSUPPORTED otherwise. A row of a 128-row tile
- * that several sequences share is multiplied with zero probabilities outside its own: a NaN or an infinity in one
- * sequence's rows reaches the rows of its neighbours in that tile, as it does inside one sequence.
+ * tokens as one row (b = 1, no mask, bias or key positions); cu_q and cu_k are the cumulative lengths of the n sequences on the
+ * device, n + 1 ascending entries each. Sequence i attends within queries [cu_q[i], cu_q[i + 1]) and keys [cu_k[i], cu_k[i + 1]);
+ * is_causal is aligned to its own bottom-right corner. Sequences are isolated: a NaN or an infinity in one does not reach another.
+ * Rows outside every sequence give 0 and LSE = +inf. Workspaces as of fdma_fwd / fdma_bwd. Forward at any head dim the tcgen05
+ * kernels take, backward up to head dim 128; FDMA_ERR_UNSUPPORTED otherwise.
  */
-int fdma_packed_limits(const int32_t* cu_q, const int32_t* cu_k, int32_t n, int32_t total_q, int32_t total_k, int32_t causal,
-                       int32_t* row_keys, int32_t* key_rows, void* stream);
-int fdma_fwd_packed(const fdma_fwd_params* p, const int32_t* row_keys, void* stream);
-int fdma_bwd_packed(const fdma_bwd_params* p, const int32_t* key_rows, void* stream);
+int fdma_fwd_varlen(const fdma_fwd_params* p, const int32_t* cu_q, const int32_t* cu_k, int32_t n, void* stream);
+int fdma_bwd_varlen(const fdma_bwd_params* p, const int32_t* cu_q, const int32_t* cu_k, int32_t n, void* stream);
 
 /*
  * create_mask: bool mask of the `window` largest bias entries along the key dimension of each row.
