@@ -12,7 +12,9 @@
 //     kDq      Q, dO (128 rows)  K, V                 S, dP           dQ += dS K
 // with scores[row, column] = (stationary row) . (streamed row), the probabilities or dS written back in 16 bit over the
 // scores as the A operand (from TMEM), and the B operand read MN-major from the streamed tile. dK's pass also sums dS over its queries
-// for dBias. dQ is complete in TMEM: no accumulator in memory, nothing to zero, add to or convert, and the same bits every time.
+// for dBias. dQ is complete in TMEM up to kFlush key tiles: no accumulator in memory, nothing to zero, add to or convert, and the
+// same bits every time. Beyond, the CTA adds what it has to an fp32 tile of its own in memory every kFlush steps: the tensor
+// core truncates its sums, which over 65536 keys made dQ in fp16 3 % less exact (2.95e-4 -> 3.05e-4).
 //
 // TMEM: scores[2] 2 x 64 | dP[2] 2 x 64 | accumulator 256. The products of step i+1 are issued before the gradient
 // product of step i, so the softmax of a step runs under 1536 cycles of tensor work of the next (d = 256, N = 64 products are bound by the
@@ -41,6 +43,7 @@ constexpr int kD = 256;
 constexpr int kBN = 128;  // stationary rows per CTA
 constexpr int kBM = 64;   // streamed rows per step
 constexpr int kThreads = 384;
+constexpr int kFlush = 64;  // 64-key steps whose dQ the tensor core sums up (4096 keys)
 constexpr int kMaxBits = 4096;  // 64-key tiles the activity bits of a dQ pass can hold; beyond, every tile is worked on
 constexpr float kLog2e = 1.4426950408889634f;
 
@@ -60,6 +63,7 @@ struct Bwd256Params {
   void* dk;
   void* dv;
   void* dbias;
+  float* dq_acc;       // more than kFlush key tiles: fp32 (B,H,Sq,256), each row the running sum of one dQ CTA
   float* dkv_part;     // null, or fp32 partials [2: dV, dK][nsplit][B][h_k][NT*128][256] instead of dk / dv
   float* dbias_part;   // with dkv_part: fp32 partials [nsplit][B][h_k][NT*128]
   int* status;
@@ -353,11 +357,14 @@ __device__ __forceinline__ void pass256(const Bwd256Params& p, unsigned char* sm
         if (ok && !kDp) ok = wait(bar_a_full + (i & 1), i >> 1, kW256AFull);
         if (!ok) break;
         const uint32_t a_addr = smem_u32(smem + L::kAOff + (i & 1) * L::kStep);
+        const bool fresh = kPass == kDq ? i % kFlush == 0 : i == 0;
 #pragma unroll
         for (int s = 0; s < 4; ++s)  // columns 0-31 of the step sit in [0,16) of the score block, 32-63 in [32,48)
           umma_ts(tmem_base + kColAcc, tmem_base + kColS + (i & 1) * kBM + (s < 2 ? s * 8 : 32 + (s - 2) * 8),
-                  umma_desc_sw128(a_addr + s * 2048, kBM * 128, 1024), idesc_g, (i > 0 || s > 0) ? 1u : 0u);
+                  umma_desc_sw128(a_addr + s * 2048, kBM * 128, 1024), idesc_g, (fresh && s == 0) ? 0u : 1u);
         umma_commit(bar_a_empty + (i & 1));
+        // (the next product waits for softmax warps that have read the sums by then)
+        if (kPass == kDq && i % kFlush == kFlush - 1 && i + 1 < n_steps) umma_commit(bar_final);
       }
       if (ok) umma_commit(bar_final);
     }
@@ -423,6 +430,8 @@ __device__ __forceinline__ void pass256(const Bwd256Params& p, unsigned char* sm
     }
     float colsum = 0.f;
     bool ok = true;
+    int flushed = 0;  // dQ pass: sums moved to memory so far
+    float* acc_row = kKeys ? nullptr : p.dq_acc + ((static_cast<int64_t>(b) * p.h + h) * Sq + min(row, Sq - 1)) * kD + half * 128;
     const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
     const float2 neg1 = make_float2(-1.f, -1.f);
     for (int i = 0; i < n_steps && ok; ++i, next()) {
@@ -487,6 +496,31 @@ __device__ __forceinline__ void pass256(const Bwd256Params& p, unsigned char* sm
         mbar_arrive(bar_vec_empty + (i & 1));
         mbar_arrive(bar_pds + (i & 1));
       }
+      if (kPass == kDq && i % kFlush == kFlush - 1 && i + 1 < n_steps) {
+        ok = __all_sync(0xffffffffu, mbar_wait(bar_final, flushed & 1, ctl, kW256Final));
+        if (!ok) break;
+        tc_fence_after_sync();
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t r[32];
+          tmem_ld_x32(tmem_base + lane_addr + kColAcc + half * 128 + c * 32, r);
+          tmem_wait_ld();
+          if (row_ok) {
+#pragma unroll
+            for (int v4 = 0; v4 < 8; ++v4) {
+              float4* dst = reinterpret_cast<float4*>(acc_row + c * 32 + v4 * 4);
+              float4 x = make_float4(__uint_as_float(r[v4 * 4]), __uint_as_float(r[v4 * 4 + 1]), __uint_as_float(r[v4 * 4 + 2]),
+                                     __uint_as_float(r[v4 * 4 + 3]));
+              if (flushed) {
+                const float4 y = *dst;
+                x = make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
+              }
+              *dst = x;
+            }
+          }
+        }
+        ++flushed;
+      }
     }
     // ---------------- the gradient tile; dBias sums of the dK pass ----------------
     if (kPass == kDk && p.want_dbias) {
@@ -501,7 +535,7 @@ __device__ __forceinline__ void pass256(const Bwd256Params& p, unsigned char* sm
           reinterpret_cast<uint16_t*>(p.dbias)[b * p.dbias_batch_stride + hk * p.dbias_head_stride + row] = f_to_raw16<kBf16>(tot);
       }
     }
-    if (ok && n_steps > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_final, 0, ctl, kW256Final));
+    if (ok && n_steps > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_final, flushed & 1, ctl, kW256Final));
     tc_fence_after_sync();
     if (ok) {
       const float mul = kPass == kDv ? 1.f : p.scale;
@@ -522,6 +556,16 @@ __device__ __forceinline__ void pass256(const Bwd256Params& p, unsigned char* sm
         } else {
 #pragma unroll
           for (int j = 0; j < 32; ++j) r[j] = 0u;
+        }
+        if (kPass == kDq && flushed && row_ok) {
+#pragma unroll
+          for (int v4 = 0; v4 < 8; ++v4) {
+            const float4 y = *reinterpret_cast<const float4*>(acc_row + c * 32 + v4 * 4);
+            r[v4 * 4] = __float_as_uint(__uint_as_float(r[v4 * 4]) + y.x);
+            r[v4 * 4 + 1] = __float_as_uint(__uint_as_float(r[v4 * 4 + 1]) + y.y);
+            r[v4 * 4 + 2] = __float_as_uint(__uint_as_float(r[v4 * 4 + 2]) + y.z);
+            r[v4 * 4 + 3] = __float_as_uint(__uint_as_float(r[v4 * 4 + 3]) + y.w);
+          }
         }
         if (kKeys && p.dkv_part) {
 #pragma unroll
@@ -569,7 +613,7 @@ struct Plan256 {
   int sq_r, nsplit;
   bool want_dbias;
   bool part;  // dK, dV and column sums leave the main kernel as fp32 partials
-  size_t lse2_off, dsum_off, part_off, dbpart_off, total;
+  size_t lse2_off, dsum_off, dq_off, part_off, dbpart_off, total;
 };
 
 // Query-range splits per key tile: a grid that cannot fill the GPU twice is cut along the query dimension until each of the
@@ -594,6 +638,8 @@ Plan256 plan256(const fdma_bwd_params& bp) {
   const size_t rows = static_cast<size_t>(p.b) * p.h * pl.sq_r;
   pl.lse2_off = o; o += align256(rows * 4);
   pl.dsum_off = o; o += align256(rows * 4);
+  pl.dq_off = o;
+  if (p.seqlen_k > kFlush * kBM) o += align256(static_cast<size_t>(p.b) * p.h * p.seqlen_q * kD * 4);
   pl.part_off = pl.dbpart_off = o;
   pl.part = pl.nsplit > 1 || bp.scatter_pos != nullptr;
   if (pl.part) {
@@ -655,6 +701,7 @@ int launch256(const fdma_bwd_params& bp, const Plan256& pl, cudaStream_t stream)
   kp.dk = bp.dk;
   kp.dv = bp.dv;
   kp.dbias = bp.dbias;
+  kp.dq_acc = reinterpret_cast<float*>(ws + pl.dq_off);
   kp.dkv_part = pl.part ? reinterpret_cast<float*>(ws + pl.part_off) : nullptr;
   kp.dbias_part = reinterpret_cast<float*>(ws + pl.dbpart_off);
   kp.status = kernel_status_ptr();
