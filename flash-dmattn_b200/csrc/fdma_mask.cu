@@ -910,14 +910,6 @@ __global__ void __launch_bounds__(kThreads, CHUNKS <= 4 ? 4 : 2) topk16_cluster_
       }
     }
   }
-  if (p.bits) {  // one byte per 8 keys (whole bytes: see reg_path_ok); the caller zeroed the bytes beyond the row's keys
-    uint8_t* bits_row = reinterpret_cast<uint8_t*>(p.bits + row * (((n + 127) / 128) * 4));
-#pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) {
-      const int k = k_lo + c * kChunk + tid * kPerThread;
-      if (k < k_hi) bits_row[k >> 3] = static_cast<uint8_t>(sel[c]);
-    }
-  }
   if (p.key_pos) {  // ascending positions of the selected keys
     int32_t* prow = p.key_pos + row * p.capacity;
 #pragma unroll
