@@ -69,7 +69,8 @@ class _PackedAttnFunc(torch.autograd.Function):
         keys_padded = iface.round_multiple(k.shape[1], _KEY_PAD)
         bias_keys_given = bias.shape[-1] if bias is not None else 0
         if bias is not None and bias.shape[-1] != keys_padded:
-            bias = (bias.expand(*bias.shape[:-1], keys_padded) if bias.shape[-1] == 1
+            # (the kernels read rows of keys: a bias with one key has to be written out, not expanded)
+            bias = (bias.expand(*bias.shape[:-1], keys_padded).contiguous() if bias.shape[-1] == 1
                     else torch.nn.functional.pad(bias, [0, keys_padded - bias.shape[-1]]))
         iface._check_inputs(q, k, v, None, bias)
         lib = _lib.load()

@@ -128,3 +128,30 @@ def test_create_mask_leaves_the_packed_form_on_a_per_query_mask(dev):
     # row-broadcast: position list, no packed form
     rb = create_mask(bias[:, :, :1].to(dev), None, B, Sq, Sk, 96, md)
     assert iface._cached_packed_mask(rb) is None and iface._cached_kept_keys(rb, Sk) is not None
+
+
+@pytest.mark.parametrize("bias_shape", [(1, 1, 1), (2, 2, 200)])
+@pytest.mark.parametrize("native", [True, False])
+def test_bias_with_one_key(dev, bias_shape, native):
+    """A bias that is the same for all keys, (.., .., .., 1), beside a packed mask: through the native path and through the
+    Python path, which hands the kernels rows of keys."""
+    from flash_sparse_attn import flash_sparse_attn_func
+    from flash_sparse_attn.packed import flash_sparse_attn_packed_func, pack_mask
+
+    B, Sq, Sk, H, Hk, d = 2, 200, 300, 4, 2, 128
+    q, k, v, _, dout = oracle.make_inputs(B, Sq, Sk, H, Hk, d, (B, Hk, Sq, Sk), seed=4, dtype=torch.bfloat16)
+    gen = torch.Generator().manual_seed(9)
+    bias = torch.randn(*bias_shape, 1, generator=gen).to(torch.bfloat16)
+    mask = torch.rand(B, Hk, Sq, Sk, generator=gen) < 0.3
+    ref = oracle.attention_forward_backward(q, k, v, mask, bias, dout, None, True)
+    ql, kl, vl, bl = (t.to(dev).requires_grad_(True) for t in (q, k, v, bias))
+    func = flash_sparse_attn_func if native else flash_sparse_attn_packed_func
+    out = func(ql, kl, vl, pack_mask(mask.to(dev)), bl, is_causal=True)
+    out.backward(dout.to(dev))
+    torch.cuda.synchronize()
+    _kernel_status_ok()
+    check("out", out.detach().cpu(), ref[0], torch.bfloat16)
+    check("dq", ql.grad.cpu(), ref[2], torch.bfloat16)
+    check("dk", kl.grad.cpu(), ref[3], torch.bfloat16, reduced=True)
+    check("dv", vl.grad.cpu(), ref[4], torch.bfloat16, reduced=True)
+    assert bl.grad.shape == bias.shape
