@@ -950,7 +950,7 @@ def measure_decode(args, rank: int, world: int, local_rank: int):
     q, k, v, bias = rnd(B, 1, H, d), rnd(B, Sk, Hk, d), rnd(B, Sk, Hk, d), rnd(B, Hk, 1, Sk)
     mask = create_mask(bias, None, B, 1, Sk, w, torch.finfo(torch.bfloat16).min)
     kept = int(mask.sum().item())
-    nbytes = kept * 2 * d * 2 + mask.numel() + kept * 2 + 2 * q.numel() * 2  # K+V rows, mask bytes, bias, Q, O
+    nbytes = kept * 2 * d * 2 + kept * 4 + kept * 2 + 2 * q.numel() * 2  # K+V rows, positions, bias, Q, O
     stream = torch.cuda.current_stream(dev)
     with torch.no_grad():
         for _ in range(max(args.warmup, 3)):
@@ -996,15 +996,15 @@ def measure_decode(args, rank: int, world: int, local_rank: int):
         "config": {"workload": f"decode: B={B} per GPU, Sq=1, Sk={Sk}, Hq={H}, Hkv={Hk}, d={d}, W={w}, non-causal",
                    "bytes_per_step": total_bytes, "l2": "K/V cache far larger than L2"},
         "decode_kernel_ms": kernel_ms,
-        "roofline": {"bound": "hbm", "kernel": "decode_mma_kernel",
+        "roofline": {"bound": "hbm", "kernel": "decode_rows_kernel",
                      "achieved": total_bytes / world / (kernel_ms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                      "frac": total_bytes / world / (kernel_ms * 1e-3) / 1e9 / peak, "peak_source": src,
-                     # one ncu capture of this kernel at B = 8 (profiles/decode_mma_kernel_B8_Sk65536_ncu_full.md):
-                     # 146.9 MB of DRAM traffic for 139 MB of algorithmic bytes; traffic grows with the kept rows,
+                     # one ncu capture of this kernel at B = 8 (profiles/decode_rows_kernel_B8_Sk65536_ncu.md):
+                     # 144.2 MB of DRAM traffic for 135.9 MB of algorithmic bytes; traffic grows with the kept rows,
                      # so the ratio is applied to this launch's bytes
-                     "traffic": total_bytes / world * (146.9 / 139.0),
-                     "traffic_source": "ncu capture at B=8 scaled by algorithmic bytes (x1.057)"},
-        "gpu_launches": args.steps * 2,  # decode_kernel + decode_merge_kernel
+                     "traffic": total_bytes / world * (144.2 / 135.9),
+                     "traffic_source": "ncu capture at B=8 scaled by algorithmic bytes (x1.061)"},
+        "gpu_launches": args.steps,  # decode_rows_kernel
     }
     return line
 

@@ -24,6 +24,8 @@ constexpr int kIdxPerThread = 16;  // mask bytes scanned per thread and round
 // One cluster per mask row, an even segment of the keys per CTA: running exclusive scan of the keep flags; kept key k lands in
 // slot (number of kept keys before it). Slots beyond the count are filled with INT32_MAX, mask_out marks the filled slots.
 // A CTA of a cluster first counts its segment, which gives the others their first slot; the second pass finds it in L2.
+// Bound by latency, a chain of scans per 4096 keys. With one CTA per row a single-query call with a bool mask took 356 us at
+// 1 x 1048576 keys, 4096 kept, now 84 us; 1 x 65536: 53 -> 37 us; rows enough to fill the GPU: as before.
 __global__ void __launch_bounds__(kIdxThreads) compact_index_kernel(const uint8_t* __restrict__ mask, int64_t sb,
                                                                      int64_t sh, int Hm, int Sk, int cap,
                                                                      int32_t* __restrict__ key_pos,

@@ -158,10 +158,10 @@ def _raise_if_kernel_timed_out(lib) -> None:
 
 
 def _kernel_head_dim(d: int, needs_grad: bool) -> int:
-    """Head dim the tensor-core kernels run this call at: the forward kernels exist for 64, 128 and 256, the backward
-    kernels for 128 and 256. Other head dims are zero-padded up to the next of these (zero columns change neither the
+    """Head dim this path (the calls the native path leaves) hands the operators: 64, 128 or 256, for calls with gradients
+    128 or 256. Other head dims are zero-padded up to the next of these (zero columns change neither the
     scores nor the kept columns of the results; the reference likewise runs every head dim on the next larger kernel,
-    csrc/flash_sparse_attn/src/static_switch.h:60-82)."""
+    csrc/flash_sparse_attn/src/static_switch.h:60-82). The kernels themselves take any multiple of 8."""
     if _kernel_path != _lib.PATH_AUTO:
         return d
     if needs_grad:

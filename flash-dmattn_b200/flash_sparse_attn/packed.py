@@ -5,8 +5,9 @@ read an eighth of the mask bytes on every pass and skip the kernel that derives 
 (the reference always materialises the bool tensor: flash_sparse_attn/utils/mask.py:102-110,
 csrc/flash_sparse_attn/flash_api.cpp:388-391).
 
-Served natively: head dim 128 (forward and backward), masks with one row per query, batch extent of the mask equal to
-the batch size. Anything else is expanded to the bool mask and takes the ordinary route."""
+The native path reads the bits at head dims up to 128, the functions below, for the calls that path leaves, at head dim 128:
+masks with one row per query, batch extent of the mask equal to the batch size. Anything else is expanded to the bool
+mask and takes the ordinary route."""
 import ctypes
 from dataclasses import dataclass
 from typing import Optional

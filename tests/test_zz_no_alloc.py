@@ -1,7 +1,7 @@
 """fdma_fwd_static_scratch -- the forward entry point for hosts that cannot provide scratch memory (engines with
 device memory carved up at start-up and no allocator for operators, loops where an allocation is unacceptable).
 The built-in array serves whatever fdma_fwd_workspace_bytes asks for: the tile-activity bytes of a per-query mask, or
-the split partials of a single-query (decode) call.
+the position lists (of a bool mask) and the partials of a single-query (decode) call.
 
 Called through the C ABI, twice in a row with different per-query masks (so the second call runs on top of the
 first call's left-over scratch contents), and compared with fdma_fwd given caller-allocated scratch. Same kernels,
@@ -74,9 +74,9 @@ def test_static_scratch_matches_caller_scratch_on_two_consecutive_calls():
 
 
 def test_static_scratch_serves_single_query_calls_up_to_its_limit():
-    """A single-query forward keeps its per-split partials (B, H, splits x 8 warps, d + 2) fp32 in scratch, whether or
-    not there is a mask: a call whose partials fit the 1 MiB array equals fdma_fwd bit for bit (twice in a row), one
-    whose partials do not fit is refused with FDMA_ERR_TOO_LARGE before anything is launched."""
+    """A single-query forward with a bool mask keeps the position lists of the mask's rows in scratch: a call whose lists
+    fit the 1 MiB array equals fdma_fwd bit for bit (twice in a row), one with longer lists and more query heads than
+    are served beyond the limit is refused with FDMA_ERR_TOO_LARGE before anything is launched."""
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     from flash_sparse_attn import _lib
