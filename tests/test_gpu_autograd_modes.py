@@ -168,3 +168,17 @@ def test_jit_trace_records_the_call(dev):
         traced = torch.jit.trace(f, (q, k, v, bias), check_trace=False)
         q2 = q.flip(1)
         assert torch.equal(traced(q2, k, v, bias), f(q2, k, v, bias))
+
+
+def test_create_graph_without_a_bias_gradient(dev):
+    """Inputs that are absent or not learned have no gradient; the others still carry the refusal of a second derivative."""
+    from flash_sparse_attn import flash_sparse_attn_func
+
+    leaves, dout, call = make(dev, "dense")
+    q, k, v, bias = leaves
+    for b in (None, bias.detach()):
+        out = flash_sparse_attn_func(q, k, v.detach(), None, b, is_causal=True)
+        dq, dk = torch.autograd.grad(out, (q, k), dout, create_graph=True)
+        assert dq.requires_grad and dk.requires_grad
+        with pytest.raises(RuntimeError, match="twice"):
+            (dq.float().sum() + dk.float().sum()).backward()
