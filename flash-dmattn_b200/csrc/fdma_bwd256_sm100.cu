@@ -243,7 +243,7 @@ __device__ __forceinline__ void pass256(const Bwd256Params& p, unsigned char* sm
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem_base = *s_tmem;
+  const uint32_t tmem_base = warp_uniform(*s_tmem);
   int n_steps, n_sub = 0;
   if (kKeys) {
     n_steps = (s_count[0] && M64 > m_start) ? (M64 - m_start) * G : 0;
@@ -259,6 +259,7 @@ __device__ __forceinline__ void pass256(const Bwd256Params& p, unsigned char* sm
         n_steps += __popc(s_bits[w] & (n_sub - w * 32 >= 32 ? 0xFFFFFFFFu : (1u << (n_sub - w * 32)) - 1u));
     }
   }
+  n_steps = warp_uniform(n_steps);
   // Steps: (query tile m, head g of the group), or key tile m
   int m = kKeys ? m_start : -1, g = 0;
   auto next = [&]() {
@@ -319,14 +320,16 @@ __device__ __forceinline__ void pass256(const Bwd256Params& p, unsigned char* sm
   } else if (warp == 1) {
     // ---------------- MMA issuer (whole warp, uniform control flow; the issue wrappers elect one lane) -------
     if (n_steps > 0) {
+      const uint32_t lead = umma_leader();
       constexpr uint32_t idesc_s = umma_idesc(kBN, kBM, kBf16, false, false);  // scores, dP: 128 x 64, K-major
       constexpr uint32_t idesc_g = umma_idesc(kBN, kD, kBf16, false, true);    // gradient: A from TMEM, B MN-major
       const uint32_t x_addr = smem_u32(smem + L::kXOff), x2_addr = smem_u32(smem + L::kX2Off);
       auto product = [&](uint32_t col, uint32_t x, uint32_t y) {  // [128 x 64] = x y^T
+        const uint64_t xd = umma_desc_sw128(x, 16, 1024), yd = umma_desc_sw128(y, 16, 1024);
 #pragma unroll
         for (int kk = 0; kk < kD / 16; ++kk)
-          umma_ss(tmem_base + col, umma_desc_sw128(x + (kk >> 2) * (kBN * 128) + (kk & 3) * 32, 16, 1024),
-                  umma_desc_sw128(y + (kk >> 2) * (kBM * 128) + (kk & 3) * 32, 16, 1024), idesc_s, kk > 0 ? 1u : 0u);
+          umma_ss(lead, tmem_base + col, umma_desc_at(xd, (kk >> 2) * (kBN * 128) + (kk & 3) * 32),
+                  umma_desc_at(yd, (kk >> 2) * (kBM * 128) + (kk & 3) * 32), idesc_s, kk > 0 ? 1u : 0u);
       };
       auto wait = [&](uint64_t* bar, int phase, int code) {
         const bool r = __all_sync(0xffffffffu, mbar_wait(bar, phase & 1, ctl, code));
@@ -344,8 +347,8 @@ __device__ __forceinline__ void pass256(const Bwd256Params& p, unsigned char* sm
           if (!wait(bar_b_full + (i & 1), i >> 1, kW256BFull)) return false;
           product(kColS + (i & 1) * kBM, x_addr, b_addr);
         }
-        umma_commit(bar_s_full + (i & 1));
-        umma_commit(bar_b_empty + i % kBSlots);
+        umma_commit(lead, bar_s_full + (i & 1));
+        umma_commit(lead, bar_b_empty + i % kBSlots);
         return true;
       };
       bool ok = wait(bar_x, 0, kW256X) && scores(0);
@@ -356,17 +359,17 @@ __device__ __forceinline__ void pass256(const Bwd256Params& p, unsigned char* sm
         if (ok) ok = wait(bar_pds + (i & 1), i >> 1, kW256Pds);
         if (ok && !kDp) ok = wait(bar_a_full + (i & 1), i >> 1, kW256AFull);
         if (!ok) break;
-        const uint32_t a_addr = smem_u32(smem + L::kAOff + (i & 1) * L::kStep);
+        const uint64_t ad = umma_desc_sw128(smem_u32(smem + L::kAOff + (i & 1) * L::kStep), kBM * 128, 1024);
         const bool fresh = kPass == kDq ? i % kFlush == 0 : i == 0;
 #pragma unroll
         for (int s = 0; s < 4; ++s)  // columns 0-31 of the step sit in [0,16) of the score block, 32-63 in [32,48)
-          umma_ts(tmem_base + kColAcc, tmem_base + kColS + (i & 1) * kBM + (s < 2 ? s * 8 : 32 + (s - 2) * 8),
-                  umma_desc_sw128(a_addr + s * 2048, kBM * 128, 1024), idesc_g, (fresh && s == 0) ? 0u : 1u);
-        umma_commit(bar_a_empty + (i & 1));
+          umma_ts(lead, tmem_base + kColAcc, tmem_base + kColS + (i & 1) * kBM + (s < 2 ? s * 8 : 32 + (s - 2) * 8),
+                  umma_desc_at(ad, s * 2048), idesc_g, (fresh && s == 0) ? 0u : 1u);
+        umma_commit(lead, bar_a_empty + (i & 1));
         // (the next product waits for softmax warps that have read the sums by then)
-        if (kPass == kDq && i % kFlush == kFlush - 1 && i + 1 < n_steps) umma_commit(bar_final);
+        if (kPass == kDq && i % kFlush == kFlush - 1 && i + 1 < n_steps) umma_commit(lead, bar_final);
       }
-      if (ok) umma_commit(bar_final);
+      if (ok) umma_commit(lead, bar_final);
     }
   } else if (warp == 2) {
     // ---------------- vectors of the step's 64 columns ----------------

@@ -281,8 +281,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     if (lane == 0) *s_nsteps = cnt;
   }
   __syncthreads();
-  const uint32_t tmem_base = *s_tmem;
-  const int n_steps = *s_nsteps;
+  const uint32_t tmem_base = warp_uniform(*s_tmem);
+  const int n_steps = warp_uniform(*s_nsteps);
   constexpr uint32_t kColSt = 0, kColDp = 128, kColDq = 192, kColDv = 256, kColDk = 256 + kD;
 
   if (warp < 4) {
@@ -324,6 +324,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     } else if (warp == 1) {
       // ---------------- MMA issuer (whole warp, uniform control flow; the issue wrappers elect one lane) -------
       if (n_steps > 0) {
+        const uint32_t lead = umma_leader();
         constexpr uint32_t idesc_s = umma_idesc(kBN, kBM, kBf16, false, false);  // St/dPt: 128 x 64, K-major
         constexpr uint32_t idesc_g = umma_idesc(kBN, kD, kBf16, false, true);    // dV/dK: A from TMEM, B MN-major
         // dQ^T: both MN-major, M = 128. With D = 64 the second 64-row block of A is the first one again (block stride
@@ -333,25 +334,25 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         const uint32_t k_addr = smem_u32(s_k), v_addr = smem_u32(s_v), qdo_addr = smem_u32(s_qdo),
                        ds_addr = smem_u32(s_ds);
         auto issue_st = [&](int step) {  // St[step & 1] = K Q^T
-          const uint32_t qa = qdo_addr + (step % kQStages) * L::kStageBytes;
+          const uint64_t ka = umma_desc_sw128(k_addr, 16, 1024);
+          const uint64_t qa = umma_desc_sw128(qdo_addr + (step % kQStages) * L::kStageBytes, 16, 1024);
 #pragma unroll
           for (int kk = 0; kk < kD / 16; ++kk) {
             const uint32_t ko = (kk >> 2) * (kBN * 128) + (kk & 3) * 32;
             const uint32_t qo = (kk >> 2) * (kBM * 128) + (kk & 3) * 32;
-            umma_ss(tmem_base + kColSt + (step & 1) * kBM, umma_desc_sw128(k_addr + ko, 16, 1024),
-                    umma_desc_sw128(qa + qo, 16, 1024), idesc_s, kk > 0 ? 1u : 0u);
+            umma_ss(lead, tmem_base + kColSt + (step & 1) * kBM, umma_desc_at(ka, ko), umma_desc_at(qa, qo), idesc_s, kk > 0 ? 1u : 0u);
           }
         };
         auto issue_dp = [&](int step) {  // dPt = V dO^T; the commit covers S of the same step, issued just before
-          const uint32_t ga = qdo_addr + (step % kQStages) * L::kStageBytes + L::kQBytes;
+          const uint64_t va = umma_desc_sw128(v_addr, 16, 1024);
+          const uint64_t ga = umma_desc_sw128(qdo_addr + (step % kQStages) * L::kStageBytes + L::kQBytes, 16, 1024);
 #pragma unroll
           for (int kk = 0; kk < kD / 16; ++kk) {
             const uint32_t ko = (kk >> 2) * (kBN * 128) + (kk & 3) * 32;
             const uint32_t qo = (kk >> 2) * (kBM * 128) + (kk & 3) * 32;
-            umma_ss(tmem_base + kColDp, umma_desc_sw128(v_addr + ko, 16, 1024), umma_desc_sw128(ga + qo, 16, 1024),
-                    idesc_s, kk > 0 ? 1u : 0u);
+            umma_ss(lead, tmem_base + kColDp, umma_desc_at(va, ko), umma_desc_at(ga, qo), idesc_s, kk > 0 ? 1u : 0u);
           }
-          umma_commit(bar_dp_full + (step & 1));
+          umma_commit(lead, bar_dp_full + (step & 1));
         };
         // Packed sequences: rows of other sequences that came along in a tile become zeros (queries: LSE = +inf, D = 0), as TMA
         // fills them in at the end of a tensor. Nothing they hold takes part in the sums over queries and keys below.
@@ -362,11 +363,11 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           fence_proxy_async_smem();
           __syncwarp();
         };
-        // Only the first and the last query tile can hold such rows: steps below `lead` and from `tail` on.
-        const int lead = packed && m_start * kBM < q_lo ? G : 0;
+        // Only the first and the last query tile can hold such rows: steps below `head_steps` and from `tail` on.
+        const int head_steps = packed && m_start * kBM < q_lo ? G : 0;
         const int tail = packed && M64 * kBM > q_hi ? n_steps - G : n_steps;
         auto end_qdo = [&](int step) {
-          if (!packed || (step >= lead && step < tail)) return;
+          if (!packed || (step >= head_steps && step < tail)) return;
           const int q0 = (step < G ? m_start : M64 - 1) * kBM;
           const int from = max(q_lo - q0, 0), to = min(q_hi - q0, kBM);
           unsigned char* stage = s_qdo + (step % kQStages) * L::kStageBytes;
@@ -412,6 +413,10 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           if (!ok) break;
           tc_fence_after_sync();
           const uint32_t stage_addr = qdo_addr + (i % kQStages) * L::kStageBytes;
+          const uint64_t q_desc = umma_desc_sw128(stage_addr, kBM * 128, 1024);
+          const uint64_t do_desc = umma_desc_sw128(stage_addr + L::kQBytes, kBM * 128, 1024);
+          const uint64_t kt_desc = umma_desc_sw128(k_addr, k_blk, 1024);
+          const uint64_t ds_desc = umma_desc_sw128(ds_addr + (i & 1) * L::kDsBytes, 16, 1024);
           const uint32_t acc = i > 0 ? 1u : 0u;
           // A operands from TMEM, 16-bit pairs: each softmax pass writes back into the 32 columns of the St block it
           // read -- P^T of queries 0-31 in columns [0,16), their dS^T in [16,32); queries 32-63 in [32,48) and
@@ -419,15 +424,14 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
 #pragma unroll
           for (int s = 0; s < 4; ++s) {
             const uint32_t a_col = 16 + (s < 2 ? s * 8 : 32 + (s - 2) * 8);
-            umma_ts(tmem_base + kColDk, tmem_base + kColSt + (i & 1) * kBM + a_col,
-                    umma_desc_sw128(stage_addr + s * 2048, kBM * 128, 1024), idesc_g, (acc || s > 0) ? 1u : 0u);
+            umma_ts(lead, tmem_base + kColDk, tmem_base + kColSt + (i & 1) * kBM + a_col,
+                    umma_desc_at(q_desc, s * 2048), idesc_g, (acc || s > 0) ? 1u : 0u);
           }
 #pragma unroll
           for (int s = 0; s < 4; ++s) {
             const uint32_t a_col = (s < 2 ? s * 8 : 32 + (s - 2) * 8);
-            umma_ts(tmem_base + kColDv, tmem_base + kColSt + (i & 1) * kBM + a_col,
-                    umma_desc_sw128(stage_addr + L::kQBytes + s * 2048, kBM * 128, 1024), idesc_g,
-                    (acc || s > 0) ? 1u : 0u);
+            umma_ts(lead, tmem_base + kColDv, tmem_base + kColSt + (i & 1) * kBM + a_col,
+                    umma_desc_at(do_desc, s * 2048), idesc_g, (acc || s > 0) ? 1u : 0u);
           }
           if (i > 0) {
             ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(3, mbar_wait(bar_dq_empty, (i - 1) & 1, ctl, kWaitDqEmpty)));
@@ -437,11 +441,10 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           // dQ^T = K^T dS^T : 8 k-steps of 16 keys
 #pragma unroll
           for (int s = 0; s < kBN / 16; ++s) {
-            umma_ss(tmem_base + kColDq, umma_desc_sw128(k_addr + s * 2048, k_blk, 1024),
-                    umma_desc_sw128(ds_addr + (i & 1) * L::kDsBytes + s * 2048, 16, 1024), idesc_q, s > 0 ? 1u : 0u);
+            umma_ss(lead, tmem_base + kColDq, umma_desc_at(kt_desc, s * 2048), umma_desc_at(ds_desc, s * 2048), idesc_q, s > 0 ? 1u : 0u);
           }
-          umma_commit(bar_dq_full);
-          umma_commit(bar_qdo_empty + (i % kQStages));
+          umma_commit(lead, bar_dq_full);
+          umma_commit(lead, bar_qdo_empty + (i % kQStages));
           if (i + 2 < n_steps) {
             ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(1, mbar_wait(bar_qdo_full + ((i + 2) % kQStages),
                                                                      ((i + 2) / kQStages) & 1, ctl, kWaitQdoFull)));
@@ -457,7 +460,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
             issue_dp(i + 2);
           }
         }
-        umma_commit(bar_final);
+        umma_commit(lead, bar_final);
         FDMA_PROF_END(8, lane == 0);
       }
     }

@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem_base = *s_tmem;
+  const uint32_t tmem_base = warp_uniform(*s_tmem);
 
   // ---------------- roles ----------------
   if (warp < 4) {
@@ -338,6 +338,7 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
     // whole warp, uniform control flow; the issue wrappers elect one lane
     constexpr uint32_t idesc_qk = umma_idesc(kBM, kBN, kBf16, false, false);
     constexpr uint32_t idesc_pv = umma_idesc(kBM, D / L::kHalves, kBf16, false, true);
+    const uint32_t lead = umma_leader();
     const uint32_t q_addr = smem_u32(s_q), kv_addr = smem_u32(s_kv);
     FDMA_PROF_BEGIN();
     int a = 0;                    // ring position: K of the a-th kept tile (over all items) is ring item 2a, V 2a+1
@@ -347,9 +348,14 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
     for (int ic = 0; ok; ++ic) {
       ok = __all_sync(0xffffffffu, mbar_wait(bar_flags_full + (ic & 1), (ic >> 1) & 1, ctl, kWaitFlagsFull));
       if (!ok) break;
-      const int item = s_item[ic & 1];
+      const int item = warp_uniform(s_item[ic & 1]);
       if (item >= p.n_items) break;
-      const FwdItem w = fwd_item<packed>(p, item, s_seq + (ic & 1) * 8);
+      FwdItem w = fwd_item<packed>(p, item, s_seq + (ic & 1) * 8);
+      if (packed) {
+        w.mblk = warp_uniform(w.mblk);
+        w.sq = warp_uniform(w.sq);
+        w.sk = warp_uniform(w.sk);
+      }
       int n_end[kNQ];
       const int32_t* pos_row;
       const int nT = tile_limits(w, n_end, pos_row);
@@ -358,6 +364,7 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
       if (!ok) break;
       tc_fence_after_sync();
       int prev_j = -1;            // previous kept tile of this item (its PV is still to be issued)
+      int prev_fl = 0;            // ... and its flags
       // packed sequences: V rows beyond the sequence, in its last tile, become zeros, as TMA fills them in at the end of a
       // tensor (zero probabilities alone would pass a NaN on)
       auto end_v = [&](int slot) {
@@ -369,12 +376,12 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
       uint32_t pv_done[2] = {0, 0};  // PV products issued for this item per query tile (0: the first one overwrites O)
       for (int j = 0; j <= nT && ok; ++j) {
         const bool last = (j == nT);
-        const uint8_t fl = last ? 0 : s_flags[j];
+        const int fl = last ? 0 : warp_uniform(static_cast<int>(s_flags[j]));
         if (!last && fl == 0) continue;
         if (last && prev_j < 0) break;  // the item has no kept tile at all
-        if (last) umma_commit(bar_q_empty);  // every S = Q K^T of the item has been issued: Q may be replaced as soon
+        if (last) umma_commit(lead, bar_q_empty);  // every S = Q K^T of the item has been issued: Q may be replaced as soon
                                              // as they complete, while the last P V products are still to come
-        const uint8_t pfl = prev_j >= 0 ? s_flags[prev_j] : 0;
+        const int pfl = prev_fl;
         const int k_it = 2 * a, v_it = 2 * (a - 1) + 1;
         if constexpr (kNQ == 1) {
           // S of this tile first, into the other buffer (its last reader, the P V product of the tile before the previous
@@ -387,15 +394,15 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
               ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(1, mbar_wait(bar_kv_full + (it & 3), (it >> 2) & 1, ctl, kWaitKvFullK)));
               if (!ok) break;
               tc_fence_after_sync();
-              const uint32_t ka = kv_addr + (it & 3) * L::kKvBytes, qa = q_addr + hf * 2 * (kBM * 128);
+              const uint64_t ka = umma_desc_sw128(kv_addr + (it & 3) * L::kKvBytes, 16, 1024);
+              const uint64_t qa = umma_desc_sw128(q_addr + hf * 2 * (kBM * 128), 16, 1024);
 #pragma unroll
               for (int kk = 0; kk < 8; ++kk) {
                 const uint32_t o2 = (kk >> 2) * (kBM * 128) + (kk & 3) * 32;
-                umma_ss(tmem_base + (a & 1) * kBN, umma_desc_sw128(qa + o2, 16, 1024), umma_desc_sw128(ka + o2, 16, 1024),
-                        idesc_qk, (hf > 0 || kk > 0) ? 1u : 0u);
+                umma_ss(lead, tmem_base + (a & 1) * kBN, umma_desc_at(qa, o2), umma_desc_at(ka, o2), idesc_qk, (hf > 0 || kk > 0) ? 1u : 0u);
               }
-              if (hf == 1) umma_commit(bar_s_full + (a & 1));
-              umma_commit(bar_kv_empty + (it & 3));
+              if (hf == 1) umma_commit(lead, bar_s_full + (a & 1));
+              umma_commit(lead, bar_kv_empty + (it & 3));
             }
             if (!ok) break;
           }
@@ -413,13 +420,13 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
               if (!ok) break;
               end_v(it & 3);
               tc_fence_after_sync();
+              const uint64_t va = umma_desc_sw128(kv_addr + (it & 3) * L::kKvBytes, kBN * 128, 1024);
 #pragma unroll
               for (int kk = 0; kk < kBN / 16; ++kk)
-                umma_ts(tmem_base + 2 * kBN + hf * 128, tmem_base + (pcnt[0] & 1) * kBN + kk * 8,
-                        umma_desc_sw128(kv_addr + (it & 3) * L::kKvBytes + kk * 2048, kBN * 128, 1024), idesc_pv,
+                umma_ts(lead, tmem_base + 2 * kBN + hf * 128, tmem_base + (pcnt[0] & 1) * kBN + kk * 8, umma_desc_at(va, kk * 2048), idesc_pv,
                         (pv_done[0] > 0 || kk > 0) ? 1u : 0u);
-              if (hf == 1) umma_commit(bar_pv);
-              umma_commit(bar_kv_empty + (it & 3));
+              if (hf == 1) umma_commit(lead, bar_pv);
+              umma_commit(lead, bar_kv_empty + (it & 3));
             }
             if (!ok) break;
             ++pcnt[0];
@@ -427,6 +434,7 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
           }
           if (!last) {
             prev_j = j;
+            prev_fl = fl;
             ++a;
           }
           continue;
@@ -455,41 +463,40 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
             }
             tc_fence_after_sync();
             const uint32_t o_col = tmem_base + 2 * kBN + t * 128;
-            const uint32_t v_base = kv_addr + (v_it % kStages) * L::kKvBytes;
+            const uint64_t v_base = umma_desc_sw128(kv_addr + (v_it % kStages) * L::kKvBytes, kBN * 128, 1024);
 #pragma unroll
             for (int kk = 0; kk < kBN / 16; ++kk) {
-              const uint64_t bd = umma_desc_sw128(v_base + kk * 2048, kBN * 128, 1024);
-              umma_ts(o_col, s_col + kk * 8, bd, idesc_pv, (pv_done[t] > 0 || kk > 0) ? 1u : 0u);
+              umma_ts(lead, o_col, s_col + kk * 8, umma_desc_at(v_base, kk * 2048), idesc_pv, (pv_done[t] > 0 || kk > 0) ? 1u : 0u);
             }
             ++pcnt[t];
             ++pv_done[t];
           }
           if (fl & (1 << t)) {
-            const uint32_t qa = q_addr + t * L::kQBytes;
-            const uint32_t ka = kv_addr + (k_it % kStages) * L::kKvBytes;
+            const uint64_t qa = umma_desc_sw128(q_addr + t * L::kQBytes, 16, 1024);
+            const uint64_t ka = umma_desc_sw128(kv_addr + (k_it % kStages) * L::kKvBytes, 16, 1024);
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk) {
               const uint32_t o2 = (kk >> 2) * (kBM * 128) + (kk & 3) * 32;
-              umma_ss(s_col, umma_desc_sw128(qa + o2, 16, 1024), umma_desc_sw128(ka + o2, 16, 1024), idesc_qk,
-                      kk > 0 ? 1u : 0u);
+              umma_ss(lead, s_col, umma_desc_at(qa, o2), umma_desc_at(ka, o2), idesc_qk, kk > 0 ? 1u : 0u);
             }
-            umma_commit(bar_s_full + t);
+            umma_commit(lead, bar_s_full + t);
           }
         }
         if (!ok) break;
-        if (prev_j >= 0) umma_commit(bar_kv_empty + (v_it % kStages));
-        if (!last) umma_commit(bar_kv_empty + (k_it % kStages));
+        if (prev_j >= 0) umma_commit(lead, bar_kv_empty + (v_it % kStages));
+        if (!last) umma_commit(lead, bar_kv_empty + (k_it % kStages));
         if (!last) {
           prev_j = j;
+          prev_fl = fl;
           ++a;
         }
       }
       if (!ok) break;
-      if (prev_j < 0) umma_commit(bar_q_empty);  // (an item without kept tiles never read its Q)
+      if (prev_j < 0) umma_commit(lead, bar_q_empty);  // (an item without kept tiles never read its Q)
 #pragma unroll
       for (int t = 0; t < kNQ; ++t)
         if (pv_done[t] > 0) {
-          umma_commit(bar_o_done + t);
+          umma_commit(lead, bar_o_done + t);
           ++ocnt[t];
         }
       __syncwarp();

@@ -29,6 +29,11 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
   return t;
 }
 
+// A value that is the same in every lane of a converged warp, in a form the compiler knows to be: what is read from shared
+// memory counts as different per lane, and so does everything computed from it or in a loop it bounds.
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(
@@ -263,6 +268,12 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr, uint32_t
   return d;
 }
 
+// The same descriptor, `bytes` further on in shared memory (a multiple of 16; everything lies below 256 KB, so the address field
+// cannot overflow): one 32-bit add where building it anew takes five instructions of the issuing warp.
+__device__ __forceinline__ uint64_t umma_desc_at(uint64_t desc, uint32_t bytes) {
+  return (desc & 0xFFFFFFFF00000000ull) | (static_cast<uint32_t>(desc) + (bytes >> 4));
+}
+
 // Instruction descriptor for kind::f16 with fp32 accumulation.
 //   bits [4,6) D format (1 = f32), [7,10) A format, [10,13) B format (0 = f16, 1 = bf16),
 //   bit 15 A is MN-major, bit 16 B is MN-major, [17,23) N>>3, [24,29) M>>4.
@@ -272,43 +283,50 @@ __host__ __device__ constexpr uint32_t umma_idesc(int m, int n, bool is_bf16, bo
          (static_cast<uint32_t>(m >> 4) << 24);
 }
 
-// The three issue wrappers below are called by ALL lanes of a converged warp with warp-uniform arguments; one
-// elected lane issues. Keeping the surrounding control flow uniform lets the compiler hold descriptors in
-// uniform registers instead of moving them there one by one for every instruction.
+// The three issue wrappers below are called by ALL lanes of a converged warp with warp-uniform arguments; the instruction is
+// predicated on `lead`, which is 1 in one lane (umma_leader, found once per kernel). Uniform control flow and values known to be
+// uniform (warp_uniform) let the compiler hold descriptors in uniform registers instead of moving them there one by one for every
+// instruction. What one product costs the issuing warp matters: its instructions queue behind those of the softmax warps of the
+// same scheduler, and its code is displaced by theirs. Issue of eight products, alone / beside dense code of 16 KB: 190 / 980
+// cycles with an election and a branch around each, 129 / 697 with one predicate.
+__device__ __forceinline__ uint32_t umma_leader() { return elect_one() ? 1u : 0u; }
 // D[tmem] (+)= A[smem] * B[smem]
-__device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+__device__ __forceinline__ void umma_ss(uint32_t lead, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                         uint32_t accumulate) {
-  if (elect_one())
   asm volatile(
       "{\n\t"
-      ".reg .pred p;\n\t"
+      ".reg .pred p, q;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
       "}\n"
       :
-      : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(lead)
       : "memory");
 }
 // D[tmem] (+)= A[tmem] * B[smem]; A holds 16-bit values packed two per 32-bit column (lane = M row).
-__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+__device__ __forceinline__ void umma_ts(uint32_t lead, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
                                         uint32_t accumulate) {
-  if (elect_one())
   asm volatile(
       "{\n\t"
-      ".reg .pred p;\n\t"
+      ".reg .pred p, q;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
       "}\n"
       :
-      : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(lead)
       : "memory");
 }
-// The mbarrier receives one arrival once every tcgen05.mma issued so far by the electing warp has completed
-// (elect.sync picks the same lane every time for a full, converged warp).
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  if (elect_one())
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
+// The mbarrier receives one arrival once every tcgen05.mma issued so far by the leading lane has completed.
+__device__ __forceinline__ void umma_commit(uint32_t lead, uint64_t* bar) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+      "}\n" ::"r"(smem_u32(bar)), "r"(lead)
+      : "memory");
 }
 
 // ---------------------------------------------------------------------------------------------
