@@ -604,8 +604,7 @@ __device__ __forceinline__ void pass256(const Bwd256Params& p, unsigned char* sm
 template <bool kBf16>
 __global__ void __launch_bounds__(kThreads, 1) bwd256_kernel(const __grid_constant__ Bwd256Params p) {
   extern __shared__ unsigned char smem_dyn[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) &
-                                                         ~static_cast<uintptr_t>(1023));
+  unsigned char* smem = align_smem_1024(smem_dyn);
   const int item = blockIdx.x;
   if (item < p.n_kv_ctas) pass256<kBf16, kDk>(p, smem, item);
   else if (item < 2 * p.n_kv_ctas) pass256<kBf16, kDv>(p, smem, item - p.n_kv_ctas);

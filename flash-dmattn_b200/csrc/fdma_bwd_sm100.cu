@@ -143,8 +143,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   // work on every step, 32 queries each.
   constexpr bool kTeams = kBcast;
   extern __shared__ unsigned char smem_dyn[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) &
-                                                         ~static_cast<uintptr_t>(1023));
+  unsigned char* smem = align_smem_1024(smem_dyn);
   unsigned char* s_k = smem + L::kKOff;
   unsigned char* s_v = smem + L::kVOff;
   unsigned char* s_qdo = smem + L::kQdoOff;

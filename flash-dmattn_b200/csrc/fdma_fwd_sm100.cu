@@ -190,8 +190,7 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
   constexpr int kNQ = L::kNQ, kStages = L::kStages;
   constexpr bool kBits = !kBcast && kVariant, packed = kBcast && kVariant;
   extern __shared__ unsigned char smem_dyn[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) &
-                                                         ~static_cast<uintptr_t>(1023));
+  unsigned char* smem = align_smem_1024(smem_dyn);
   unsigned char* s_q = smem + L::kQOff;
   unsigned char* s_kv = smem + L::kKvOff;
   float* s_bm = reinterpret_cast<float*>(smem + L::kBmOff);

@@ -23,6 +23,10 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// The next multiple of 1024 in shared memory, as an offset from the array it is in: a pointer that went through an integer would
+// be a generic one, and every access through it a generic load or store.
+__device__ __forceinline__ unsigned char* align_smem_1024(unsigned char* p) { return p + ((0u - smem_u32(p)) & 1023u); }
+
 __device__ __forceinline__ uint64_t globaltimer_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
