@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(kThreads) bwd_prep_kernel(const BwdPrepArgs a)
       y[u] = *reinterpret_cast<const uint4*>(g + static_cast<int64_t>(q) * a.do_sr);
     }
   }
-  if (D <= 128) {  // accumulator rows of this warp: (B,H,Sq,D) elements of acc_bytes each
+  if (D <= 128 && a.dq_acc) {  // accumulator rows of this warp: (B,H,Sq,D) elements of acc_bytes each
     char* base = static_cast<char*>(a.dq_acc) + (static_cast<int64_t>(bh) * a.sq + q0) * D * a.acc_bytes;
     const int n16 = min(8, a.sq - q0) * D * a.acc_bytes / 16;
     for (int i = lane; i < n16; i += 32) reinterpret_cast<uint4*>(base)[i] = make_uint4(0, 0, 0, 0);

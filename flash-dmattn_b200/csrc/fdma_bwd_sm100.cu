@@ -1256,12 +1256,14 @@ bool tc_bwd_supported(const fdma_bwd_params& bp) {
 }
 
 size_t tc_bwd_workspace_bytes(const fdma_bwd_params& p) {
-  return tile_head_dim(p.f.d) == 256 ? tc_bwd256_workspace_bytes(p) : plan(p).total;
+  if (tile_head_dim(p.f.d) == 256) return tc_bwd256_workspace_bytes(p);
+  return bwd_rows_taken(p) ? bwd_rows_workspace_bytes(p) : plan(p).total;
 }
 
 int tc_bwd(const fdma_bwd_params& p, cudaStream_t stream, const PackedSeqs& seqs) {
   const bool bf16 = p.f.dtype == FDMA_BF16;
   if (tile_head_dim(p.f.d) == 256) return tc_bwd256(p, stream);
+  if (bwd_rows_taken(p)) return bwd_rows(p, stream, seqs);
   const BwdPlan pl = plan(p);
   if (pl.D == 64) return bf16 ? launch<64, true>(p, pl, seqs, stream) : launch<64, false>(p, pl, seqs, stream);
   return bf16 ? launch<128, true>(p, pl, seqs, stream) : launch<128, false>(p, pl, seqs, stream);

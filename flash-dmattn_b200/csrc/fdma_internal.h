@@ -36,6 +36,11 @@ bool tc_bwd256_supported(const fdma_bwd_params& p);
 size_t tc_bwd256_workspace_bytes(const fdma_bwd_params& p);
 int tc_bwd256(const fdma_bwd_params& p, cudaStream_t stream);
 
+// head dims up to 128, row-broadcast mask / bias, packed sequences (fdma_bwd_rows_sm100.cu); also reached through tc_bwd
+bool bwd_rows_taken(const fdma_bwd_params& p);
+size_t bwd_rows_workspace_bytes(const fdma_bwd_params& p);
+int bwd_rows(const fdma_bwd_params& p, cudaStream_t stream, const PackedSeqs& seqs);
+
 bool tc_bwd_supported(const fdma_bwd_params& p);
 size_t tc_bwd_workspace_bytes(const fdma_bwd_params& p);
 int tc_bwd(const fdma_bwd_params& p, cudaStream_t stream, const PackedSeqs& seqs = {});  // seqs: head dims up to 128
@@ -51,7 +56,7 @@ struct BwdPrepArgs {
   const void *out, *dout;
   const float* lse;
   float *lse2, *dsum;  // (B,H,sq_r)
-  void* dq_acc;        // D <= 128: zeroed, (B,H,Sq,D) elements of acc_bytes
+  void* dq_acc;        // null, or (D <= 128) zeroed: (B,H,Sq,D) elements of acc_bytes
   int b, h, sq, sq_r, d, acc_bytes;
   int64_t o_sb, o_sr, o_sh, do_sb, do_sr, do_sh;
 };
