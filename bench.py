@@ -336,9 +336,9 @@ class AttentionStep:
         self.ws = torch.empty(max(ws_f, ws_b, 1), dtype=torch.uint8, device=dev)
         self.fp.workspace, self.fp.workspace_bytes = self.ws.data_ptr(), ws_f
         bp.f.workspace, bp.f.workspace_bytes = self.ws.data_ptr(), ws_b
-        # launches per step, from the code paths above: gathers 3 | fwd_kernel 1 | bwd_prep, bwd_kernel,
-        # convert_dq 3 (+ 3 partial reductions when the backward grid is split) | scatters 3 (their zero fills are memsets)
-        self.launches = (3 + 1 + 6 + 3) if compact else 4
+        # launches per step, from the code paths above: gathers 3 | fwd_kernel 1 | bwd_prep, bwd_rows_kernel, bwd_finish 3 |
+        # scatters 3 (their zero fills are memsets); full key range: no query-range splits, so nothing for bwd_finish to do
+        self.launches = (3 + 1 + 3 + 3) if compact else 3
 
     def run_pre(self):
         for fn, prm in self.pre:
@@ -727,13 +727,12 @@ def run_ours(args, rank: int, world: int, local_rank: int):
         "tflops_element_level": elem_fl / (ms_per_step * 1e-3) / 1e12,
         "tflops_causal_dense_equivalent": dense / (ms_per_step * 1e-3) / 1e12,
         "utilisation_of_nominal_2250": value / world / NOMINAL_TFLOPS,
-        "roofline": {"bound": "tensor", "kernel": "bwd_kernel", "achieved": bwd_tflops, "peak": peaks["peak"],
+        # (achieved: the five products of the gradients; the kernel forms seven, in two passes)
+        "roofline": {"bound": "tensor", "kernel": "bwd_rows_kernel", "achieved": bwd_tflops, "peak": peaks["peak"],
                      "unit": "TFLOP/s", "frac": bwd_tflops / peaks["peak"], "peak_source": peaks["source"],
                      "frac_sustained": bwd_tflops / peaks["sustained"], "peak_sustained": peaks["sustained"],
                      "frac_of_nominal_2250": bwd_tflops / NOMINAL_TFLOPS,
-                     # dram__bytes_read + dram__bytes_write of one bwd_kernel launch of exactly this workload, one ncu
-                     # capture (profiles/fwd_bwd_kernel_S32768_compaction_dram_traffic.md); other geometries: null
-                     "traffic": (2364e6 if (compact and (S, WINDOW, D, B) == (32768, 2048, 128, 1)) else None),
+                     "traffic": None,
                      "fwd_kernel_achieved": fwd_tflops, "fwd_kernel_frac": fwd_tflops / peaks["peak"]},
         "e2e": {"value": tot / (e2e_ms * 1e-3) / 1e12 if e2e_ms == e2e_ms else None, "unit": "TFLOP/s",
                 "ms_per_step": e2e_ms if e2e_ms == e2e_ms else None,
