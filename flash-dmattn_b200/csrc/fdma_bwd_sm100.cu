@@ -1,4 +1,5 @@
-// Backward dynamic-mask attention for sm_100a (head dims up to 128): dQ, dK, dV and dBias from dO, O, LSE.
+// Backward dynamic-mask attention for sm_100a (head dims up to 128) with a mask or bias per query: dQ, dK, dV and dBias from dO, O,
+// LSE. Row-broadcast ones and packed sequences: fdma_bwd_rows_sm100.cu.
 //
 // Math of the reference's compute_dq_dk_dv_1colblock (csrc/flash_sparse_attn/src/flash_bwd_kernel.h:79-1142):
 //   P = exp(S - LSE), dP = dO V^T, dS = P o (dP - D), D = rowsum(dO o O),
@@ -13,7 +14,8 @@
 //   dV += P^T dO,  dK += dS^T Q   (B = dO / Q tiles read MN-major from the same shared-memory copy)
 //   dQ^T = K^T dS^T    (A = K MN-major, B = dS^T staged in shared memory), added to an fp32 dQ buffer by a
 //                      dedicated warpgroup: transpose through shared memory, one bulk reduce-add per 32 queries
-// Query-broadcast bias gives dBias = column sums of dS: one fp32 register per softmax thread for the whole CTA.
+// One pass, with dQ^T added up in memory: a second pass over the scores, as in the row-broadcast kernel, would fetch the bias and mask
+// of every (query, key) again, once per query head instead of once per group.
 //
 // Warps: 0 TMA producer | 1 MMA issuer | 4-7, 8-11 softmax (query columns 0-31 / 32-63) | 12-15 dQ writer.
 // TMEM: St[2] 2x64 | dPt 64 | dQ^T 64 | dV D | dK D = 512 columns (D = 128) or 384 (D = 64).
@@ -27,7 +29,6 @@
 #include <algorithm>
 
 #include "fdma_internal.h"
-#include "fdma_packed.cuh"
 #include "fdma_ptx.cuh"
 
 namespace fdma {
@@ -77,8 +78,6 @@ struct BwdKernelParams {
   const int32_t* key_pos;  // ascending positions of compacted keys, or null
   int64_t pos_batch_stride, pos_head_stride;
   int h_pos, causal_shift;
-  PackedSeqs seqs;     // packed sequences, each with key tiles of its own; 64-row query tiles are cut at fixed rows
-  int n_tiles;         // packed: places for key tiles
   float scale_log2, scale;
 };
 
@@ -132,16 +131,10 @@ __device__ __forceinline__ uint16_t float_to_raw16(float x) {
   return static_cast<uint16_t>(pack_16x2<kBf16>(x, 0.f) & 0xFFFFu);
 }
 
-// packed (row-broadcast kernel): an instantiation of its own, whose bounds of a sequence would cost the others registers.
-template <int D, bool kBf16, bool kBcast, bool kDet, bool packed = false>
+template <int D, bool kBf16, bool kDet>
 __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant__ BwdKernelParams p) {
   using L = SmemB<D>;
   constexpr int kD = D;
-  // Row-broadcast kernel: the two softmax warpgroups are two teams that take alternate steps (all 64 queries of
-  // a step, in two passes of 32), so the fixed latencies of one team's step -- barrier round trips, TMEM loads and
-  // stores, the hand-over to the MMA warp -- overlap the other team's arithmetic. Per-query kernel: both warpgroups
-  // work on every step, 32 queries each.
-  constexpr bool kTeams = kBcast;
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* smem = align_smem_1024(smem_dyn);
   unsigned char* s_k = smem + L::kKOff;
@@ -157,7 +150,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   uint64_t* bar_qdo_empty = bar_qdo_full + kQStages;
   uint64_t* bar_dp_full = bar_qdo_empty + kQStages;
   uint64_t* bar_pds = bar_dp_full + 2;              // bar_dp_full: [2], by step parity
-  uint64_t* bar_dq_full = bar_pds + 2;              // bar_pds: [2], one per softmax team (broadcast kernel)
+  uint64_t* bar_dq_full = bar_pds + 2;              // bar_pds: [2], by step parity
   uint64_t* bar_dq_empty = bar_dq_full + 1;
   uint64_t* bar_dp_free = bar_dq_empty + 1;
   uint64_t* bar_final = bar_dp_free + 1;
@@ -175,39 +168,26 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   // blockIdx.x = (query-range split, key tile). With more than one split a CTA covers the 64-row query tiles
   // [m_lo, M64) of its key tile and leaves fp32 partial dK / dV / column sums for a reduction kernel. The last
   // query ranges, which causal masking never empties, are scheduled first.
-  const int tiles = packed ? p.n_tiles : NT;
-  const int n = blockIdx.x % tiles;  // key tile
-  const int split = p.nsplit - 1 - blockIdx.x / tiles;
+  const int n = blockIdx.x % NT;  // key tile
+  const int split = p.nsplit - 1 - blockIdx.x / NT;
   const int M64_all = (Sq + kBM - 1) / kBM;
   const int m_chunk = (M64_all + p.nsplit - 1) / p.nsplit;
   const int m_lo = split * m_chunk;
-  int M64 = min(M64_all, m_lo + m_chunk);  // end of this CTA's query range
+  const int M64 = min(M64_all, m_lo + m_chunk);  // end of this CTA's query range
   const bool causal = p.is_causal != 0;
   const int act_g = (p.h_mask == p.h && G > 1) ? G : 1;  // activity differs per query head only for per-head masks
   // Compacted keys carry their original positions (ascending); the causal test then runs on positions.
   const int32_t* pos_row = nullptr;
   if (causal && p.key_pos)
     pos_row = p.key_pos + b * p.pos_batch_stride + (p.h_pos == p.h_k ? hk : 0) * p.pos_head_stride;
-  int coff = pos_row ? p.causal_shift : off;
-  // Packed sequences: the tile covers the keys [key0, key_end) of one of them, whose queries are [q_lo, q_hi).
-  int key0 = n * kBN, key_end = Sk, q_lo = 0, q_hi = Sq;
+  const int coff = pos_row ? p.causal_shift : off;
+  const int key0 = n * kBN;
   int m_start = 0;
   if (pos_row) {
     const int64_t first = (static_cast<int64_t>(pos_row[n * kBN]) - coff) / kBM;
     m_start = static_cast<int>(max(static_cast<int64_t>(0), min(first, static_cast<int64_t>(M64))));
   } else if (causal) {
     m_start = max(0, (n * kBN - off) / kBM);  // first query tile with a row that sees key n*128
-  }
-  if (packed) {
-    const PackedTile t = packed_tile(p.seqs.cu_k, p.seqs.n, Sk, kBN, n);
-    const int2 q = packed_range(p.seqs.cu_q, p.seqs.n, Sq, t.seq);
-    key0 = t.begin + t.tile * kBN;
-    key_end = t.end;
-    q_lo = q.x;
-    q_hi = key0 < key_end ? q.y : q.x;  // (an empty place has no queries)
-    coff = key_end - q_hi;              // the last query sees the last key
-    m_start = (causal ? max(q_lo, key0 - coff) : q_lo) / kBM;
-    M64 = q_lo < q_hi ? min(M64, (q_hi + kBM - 1) / kBM) : 0;
   }
   m_start = max(m_start, m_lo);
   const WaitCtl ctl{s_abort, p.status};
@@ -222,11 +202,11 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     }
     mbar_init(bar_dp_full + 0, 1);
     mbar_init(bar_dp_full + 1, 1);
-    mbar_init(bar_pds + 0, kTeams ? 4 : 8);  // one arrival per softmax warp that works on the step
-    mbar_init(bar_pds + 1, kTeams ? 4 : 8);
+    mbar_init(bar_pds + 0, 8);  // one arrival per softmax warp
+    mbar_init(bar_pds + 1, 8);
     mbar_init(bar_dq_full, 1);
     mbar_init(bar_dq_empty, 4);   // one arrival per dQ-writer warp
-    mbar_init(bar_dp_free, kTeams ? 4 : 8);
+    mbar_init(bar_dp_free, 8);
     mbar_init(bar_final, 1);
     fence_mbar_init();
   }
@@ -247,7 +227,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     const int hm = hq / (p.h / p.h_mask);
     uint8_t a = 1;
     if (p.mask) {
-      if (kBcast || p.mask_row_stride == 0) {
+      if (p.mask_row_stride == 0) {
         const uint8_t* mrow = p.mask + b * p.mask_batch_stride + hm * p.mask_head_stride + n * kBN;
         uint32_t accw = 0;
 #pragma unroll
@@ -353,43 +333,10 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           }
           umma_commit(lead, bar_dp_full + (step & 1));
         };
-        // Packed sequences: rows of other sequences that came along in a tile become zeros (queries: LSE = +inf, D = 0), as TMA
-        // fills them in at the end of a tensor. Nothing they hold takes part in the sums over queries and keys below.
-        auto end_kv = [&]() {
-          if (!packed || key_end - key0 >= kBN) return;
-          zero_tile_rows(s_k, kD / 64, kBN * 128, key_end - key0, kBN);
-          zero_tile_rows(s_v, kD / 64, kBN * 128, key_end - key0, kBN);
-          fence_proxy_async_smem();
-          __syncwarp();
-        };
-        // Only the first and the last query tile can hold such rows: steps below `head_steps` and from `tail` on.
-        const int head_steps = packed && m_start * kBM < q_lo ? G : 0;
-        const int tail = packed && M64 * kBM > q_hi ? n_steps - G : n_steps;
-        auto end_qdo = [&](int step) {
-          if (!packed || (step >= head_steps && step < tail)) return;
-          const int q0 = (step < G ? m_start : M64 - 1) * kBM;
-          const int from = max(q_lo - q0, 0), to = min(q_hi - q0, kBM);
-          unsigned char* stage = s_qdo + (step % kQStages) * L::kStageBytes;
-          for (int t = 0; t < 2; ++t) {
-            zero_tile_rows(stage + t * L::kQBytes, kD / 64, kBM * 128, 0, from);
-            zero_tile_rows(stage + t * L::kQBytes, kD / 64, kBM * 128, to, kBM);
-          }
-          float* ld = s_ld + (step % kQStages) * (2 * kBM);
-          for (int r = lane; r < kBM; r += 32)
-            if (r < from || r >= to) {
-              ld[r] = CUDART_INF_F;
-              ld[kBM + r] = 0.f;
-            }
-          fence_proxy_async_smem();
-          __threadfence_block();
-          __syncwarp();
-        };
         FDMA_PROF_BEGIN();
         bool ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(0, mbar_wait(bar_kv, 0, ctl, kWaitKv)));
         if (ok) ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(1, mbar_wait(bar_qdo_full + 0, 0, ctl, kWaitQdoFull)));
         if (ok) {
-          end_kv();
-          end_qdo(0);
           tc_fence_after_sync();
           issue_st(0);
           issue_dp(0);
@@ -397,7 +344,6 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         if (ok && n_steps > 1) {
           ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(1, mbar_wait(bar_qdo_full + 1, 0, ctl, kWaitQdoFull)));
           if (ok) {
-            end_qdo(1);
             tc_fence_after_sync();
             issue_st(1);
           }
@@ -448,7 +394,6 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
             ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(1, mbar_wait(bar_qdo_full + ((i + 2) % kQStages),
                                                                      ((i + 2) / kQStages) & 1, ctl, kWaitQdoFull)));
             if (!ok) break;
-            end_qdo(i + 2);
             tc_fence_after_sync();
             issue_st(i + 2);
             // dP of step i+2 goes out two steps ahead as well, as soon as the softmax threads have read dP of step
@@ -475,19 +420,11 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     const int key = key0 + krow;
     unsigned char* s_tr = smem + L::kTrOff + (warp - 4) * 1024;
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const bool key_ok = key < key_end;
+    const bool key_ok = key < Sk;
     // value compared with q + coff in the causal test: the key's position
     // (clamped so that ckey - coff cannot overflow; padding slots hold INT_MAX and are masked out anyway)
     const int ckey = pos_row ? (key_ok ? min(pos_row[key], 0x3FFFFFFF) : 0x3FFFFFFF) : key;
     const int ckey_wmax = pos_row ? __shfl_sync(0xffffffffu, ckey, 31) : key0 + (warp & 3) * 32 + 31;
-    // Row-broadcast kernel: query rows [qlo, qhi) see this key, those of [qlo_max, qhi_min) all keys of the warp.
-    int qlo = causal ? ckey - coff : -0x7FFFFFFF, qhi = 0x7FFFFFFF;
-    int qlo_max = causal ? ckey_wmax - coff : -0x7FFFFFFF, qhi_min = 0x7FFFFFFF;
-    if (packed) {
-      qlo = max(qlo, q_lo);
-      qlo_max = max(qlo_max, q_lo);
-      qhi = qhi_min = q_hi;
-    }
     const int mode = p.dbias_mode;
     float colsum = 0.f;       // column-sum mode
     float dacc[32];           // direct mode with dbias_h == h_k: sum over the head group
@@ -527,22 +464,11 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
             dst_key[static_cast<int64_t>(q_first + j) * p.dbias_row_stride] = vals ? float_to_raw16<kBf16>(vals[j]) : 0;
       }
     };
-    // Row-broadcast bias / mask that do not depend on the query head: one value per thread for the whole CTA.
+    // bias and mask that do not depend on the query head: fetched once per query tile
     const bool group_inv = G == 1 || ((!p.bias || p.h_bias != p.h) && (!p.mask || p.h_mask != p.h));
-    const bool hoist = kBcast && group_inv;
     // mask / bias head of query head h, without integer division (extents are 1, h_k or h)
     auto hm_of = [&](int h) { return p.h_mask == p.h ? h : (p.h_mask == p.h_k ? hk : 0); };
     auto hb_of = [&](int h) { return p.h_bias == p.h ? h : (p.h_bias == p.h_k ? hk : 0); };
-    float bv_h = -CUDART_INF_F;  // bias*log2e of this key, or -inf when the key is masked out
-    if (hoist) {
-      const int hm0 = hm_of(hk * G), hb0 = hb_of(hk * G);
-      bool kp = key_ok;
-      if (p.mask && kp) kp = p.mask[b * p.mask_batch_stride + hm0 * p.mask_head_stride + key] != 0;
-      if (kp)
-        bv_h = p.bias ? raw16_to_float<kBf16>(reinterpret_cast<const uint16_t*>(
-                            p.bias)[b * p.bias_batch_stride + hb0 * p.bias_head_stride + key]) * kLog2e
-                      : 0.f;
-    }
     int i = 0;
     bool ok = true;
     FDMA_PROF_BEGIN();
@@ -562,27 +488,9 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
             store_dbias(dbias16 + b * p.dbias_batch_stride + h * p.dbias_head_stride + key, q0, nullptr);
           continue;
         }
-        if (kTeams && (i & 1) != half) {  // the other team's step
-          ++i;
-          continue;
-        }
         group_touched = true;
-        // ---- bias (log2 units) for this thread's key; masked elements get -inf, which turns into
-        //      P = exp2(-inf) = 0 without any per-element select. Row-broadcast bias: one scalar per thread; the
-        //      per-element array is only filled for per-query bias/mask and on tiles that cross the causal limit ----
-        float bv = bv_h;
-        if (kBcast) {
-          if (!hoist) {
-            const int hm = hm_of(h), hb = hb_of(h);
-            bool kp = key_ok;
-            if (p.mask && kp) kp = p.mask[b * p.mask_batch_stride + hm * p.mask_head_stride + key] != 0;
-            bv = -CUDART_INF_F;
-            if (kp)
-              bv = p.bias ? raw16_to_float<kBf16>(reinterpret_cast<const uint16_t*>(
-                                p.bias)[b * p.bias_batch_stride + hb * p.bias_head_stride + key]) * kLog2e
-                          : 0.f;
-          }
-        } else {
+        // ---- bias (log2 units) for this thread's key and 32 queries; masked elements get -inf, which turns into
+        //      P = exp2(-inf) = 0 without any per-element select ----
           if (!(group_inv && bias2_loaded)) {
           bias2_loaded = true;
           {
@@ -681,55 +589,36 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
             }
           }
           }
-        }
 
         // ---- P^T and dS^T in one pass: both accumulators are loaded together ----
-        // Barriers that alternate between the teams come in pairs indexed by step parity, so that a team only ever
-        // waits on consecutive phases of a barrier. dP of step i is committed after S of step i was issued, so
+        // dP of step i is committed after S of step i was issued, so
         // dp_full covers both accumulators. The dS^T buffer (i & 1) was last read by the dQ product of step i-2,
         // issued before dP of step i: the tcgen05.commit behind dP covers every earlier MMA of the issuing thread, so
         // dp_full(i) also says that buffer is free. The LSE / D values of the stage were bulk-copied under the
-        // stage barrier, which the MMA warp observed before it issued S and dP of this step; the per-query kernel
-        // waits on that barrier itself as well.
-        if (!kTeams) {
-          ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(0, mbar_wait(bar_qdo_full + (i % kQStages),
-                                                                     (i / kQStages) & 1, ctl, kWaitQdoFull)));
-          if (!ok) break;
-        }
+        // stage barrier.
+        ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(0, mbar_wait(bar_qdo_full + (i % kQStages),
+                                                                   (i / kQStages) & 1, ctl, kWaitQdoFull)));
+        if (!ok) break;
         ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(2, mbar_wait(bar_dp_full + (i & 1), (i >> 1) & 1, ctl, kWaitDpFull)));
         if (!ok) break;
         tc_fence_after_sync();
         float step_sum = 0.f;
-#pragma unroll 1
-        for (int sub = 0; sub < (kTeams ? 2 : 1); ++sub) {
-          const int qh = kTeams ? sub : half;  // which 32 of the step's 64 queries
-          const int q0s = m * kBM + qh * 32;
+        {
           // LSE*log2e and D of the step's 64 queries arrive in shared memory with the Q/dO stage
-          const float* lrow = s_ld + (i % kQStages) * (2 * kBM) + qh * 32;
+          const float* lrow = s_ld + (i % kQStages) * (2 * kBM) + half * 32;
           const float* drow = lrow + kBM;
-          const bool diag = qlo_max > q0s || qhi_min < q0s + 32;  // warp-uniform
-          const bool per_elem = !kBcast || diag;
-          if (kBcast && diag) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-              bias2[j] = make_float2(q0s + 2 * j < qlo || q0s + 2 * j >= qhi ? -CUDART_INF_F : bv,
-                                     q0s + 2 * j + 1 < qlo || q0s + 2 * j + 1 >= qhi ? -CUDART_INF_F : bv);
-          }
           uint32_t dsk[16];
           uint32_t rs[32], rp[32];
-          tmem_ld_x32(tmem_base + lane_addr + kColSt + (i & 1) * kBM + qh * 32, rs);
-          tmem_ld_x32(tmem_base + lane_addr + kColDp + qh * 32, rp);
+          tmem_ld_x32(tmem_base + lane_addr + kColSt + (i & 1) * kBM + half * 32, rs);
+          tmem_ld_x32(tmem_base + lane_addr + kColDp + half * 32, rp);
           tmem_wait_ld();
-          if (!kTeams || sub == 1) {
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_dp_free);  // the dPt block may be overwritten from here on
-          }
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_dp_free);  // the dPt block may be overwritten from here on
           // packed fp32x2 arithmetic: two queries per instruction
           float2 pp[16], dd[16];
           float2 part[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
           const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
-          const float2 bv2 = make_float2(bv, bv);
           const float2 neg1 = make_float2(-1.f, -1.f);
 #pragma unroll
           for (int j4 = 0; j4 < 8; ++j4) {
@@ -740,7 +629,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
               const int j = j4 * 2 + e;  // pair index
               const float2 lv = e == 0 ? make_float2(l4.x, l4.y) : make_float2(l4.z, l4.w);
               const float2 dv = e == 0 ? make_float2(d4.x, d4.y) : make_float2(d4.z, d4.w);
-              const float2 addend = __ffma2_rn(lv, neg1, per_elem ? bias2[j] : bv2);       // bias - LSE
+              const float2 addend = __ffma2_rn(lv, neg1, bias2[j]);       // bias - LSE
               const float2 x = __ffma2_rn(make_float2(__uint_as_float(rs[2 * j]), __uint_as_float(rs[2 * j + 1])), sc2,
                                           addend);
               const float2 pj = make_float2(fast_exp2(x.x), fast_exp2(x.y));
@@ -765,14 +654,14 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
             dsk[j] = pack_16x2<kBf16>(pv[2 * j], pv[2 * j + 1]);
           }
           // back into the 32 columns just read: P^T pairs in the first 16, dS^T pairs in the last 16
-          tmem_st_x16(tmem_base + lane_addr + kColSt + (i & 1) * kBM + qh * 32, pk);
-          tmem_st_x16(tmem_base + lane_addr + kColSt + (i & 1) * kBM + qh * 32 + 16, dsk);
-          if (mode == kDbDirect) {  // only reached by the per-query kernel (one pass: q0s == q0)
+          tmem_st_x16(tmem_base + lane_addr + kColSt + (i & 1) * kBM + half * 32, pk);
+          tmem_st_x16(tmem_base + lane_addr + kColSt + (i & 1) * kBM + half * 32 + 16, dsk);
+          if (mode == kDbDirect) {
             if (direct_group) {
 #pragma unroll
               for (int j = 0; j < 32; ++j) dacc[j] += pv[j];
             } else {
-              store_dbias(dbias16 + b * p.dbias_batch_stride + h * p.dbias_head_stride + key, q0s, pv);
+              store_dbias(dbias16 + b * p.dbias_batch_stride + h * p.dbias_head_stride + key, q0, pv);
             }
           } else if (mode == kDbAtomic && key_ok && p.dbias_rows != 1) {
             const int b2 = p.dbias_b == 1 ? 0 : b;
@@ -780,14 +669,14 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
             float* base = p.dbias_acc + (static_cast<int64_t>(b2) * p.dbias_h + h2) * p.dbias_rows * p.dbias_keys + key;
 #pragma unroll
             for (int j = 0; j < 32; ++j)
-              if (q0s + j < Sq && pv[j] != 0.f) atomicAdd(base + static_cast<int64_t>(q0s + j) * p.dbias_keys, pv[j]);
+              if (q0 + j < Sq && pv[j] != 0.f) atomicAdd(base + static_cast<int64_t>(q0 + j) * p.dbias_keys, pv[j]);
           }
           // ---- dS^T tile to shared memory for the dQ MMA: row = key, 64 queries x 2 B = 128 B, 128-byte swizzle ----
           {
             unsigned char* rowp = s_ds + (i & 1) * L::kDsBytes + krow * 128;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-              const int chunk = (qh * 4 + c) ^ (krow & 7);
+              const int chunk = (half * 4 + c) ^ (krow & 7);
               *reinterpret_cast<uint4*>(rowp + chunk * 16) = make_uint4(dsk[c * 4], dsk[c * 4 + 1], dsk[c * 4 + 2], dsk[c * 4 + 3]);
             }
           }
@@ -851,7 +740,6 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         }
         if (p.dkv_part) {
           // fp32 partial: part[dv|dk][split][b][hk][key][d]
-          if (packed && !key_ok) continue;  // (after the warp-wide load)
           float* part = p.dkv_part + ((((static_cast<int64_t>(half) * p.nsplit + split) * p.b + b) * p.h_k + hk) *
                                           (NT * kBN) + key) * kD + c * 32;
 #pragma unroll
@@ -927,14 +815,14 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
             fence_proxy_async_smem();
             named_bar_sync(3, 128);
             if (tid == 384) {
-              const int r0 = packed ? max(0, q_lo - (m * kBM + c * 32)) : 0, rows = min(2 * kPer, q_hi - (m * kBM + c * 32)) - r0;
+              const int rows = min(2 * kPer, Sq - (m * kBM + c * 32));
               if (rows > 0) {
                 if constexpr (kDet)
                   bulk_reduce_add_u64(reinterpret_cast<long long*>(p.dq_acc) +
-                                          ((static_cast<int64_t>(b) * p.h + h) * Sq + m * kBM + c * 32 + r0) * kD,
-                                      reinterpret_cast<long long*>(s_dq) + r0 * kD, rows * kD * 8);
+                                          ((static_cast<int64_t>(b) * p.h + h) * Sq + m * kBM + c * 32) * kD,
+                                      s_dq, rows * kD * 8);
                 else
-                  bulk_reduce_add_f32(gdst + r0 * kD, s_dq + r0 * kD, rows * kD * 4);
+                  bulk_reduce_add_f32(gdst, s_dq, rows * kD * 4);
               }
               asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             }
@@ -967,8 +855,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
             fence_proxy_async_smem();
             named_bar_sync(3, 128);
             if (tid == 384) {
-              const int r0 = packed ? max(0, q_lo - (m * kBM + c * 16)) : 0, rows = min(16, q_hi - (m * kBM + c * 16)) - r0;
-              if (rows > 0) bulk_reduce_add_u64(gdst64 + (c * 16 + r0) * kD, s_dq64 + r0 * kD, rows * kD * 8);
+              const int rows = min(16, Sq - (m * kBM + c * 16));
+              if (rows > 0) bulk_reduce_add_u64(gdst64 + c * 16 * kD, s_dq64, rows * kD * 8);
               asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             }
           }
@@ -984,8 +872,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           fence_proxy_async_smem();
           named_bar_sync(3, 128);
           if (tid == 384) {
-            const int r0 = packed ? max(0, q_lo - (m * kBM + c * 32)) : 0, rows = min(32, q_hi - (m * kBM + c * 32)) - r0;
-            if (rows > 0) bulk_reduce_add_f32(gdst + (c * 32 + r0) * kD, s_dq + r0 * kD, rows * kD * 4);
+            const int rows = min(32, Sq - (m * kBM + c * 32));
+            if (rows > 0) bulk_reduce_add_f32(gdst + c * 32 * kD, s_dq, rows * kD * 4);
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
         }
@@ -1007,7 +895,6 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
 
 struct BwdPlan {
   int D;
-  bool bcast;
   bool part;  // dK, dV (and column sums) leave the main kernel as fp32 partials
   bool needs_act;
   int dbias_mode;
@@ -1040,10 +927,7 @@ BwdPlan plan(const fdma_bwd_params& bp) {
   const fdma_fwd_params& p = bp.f;
   BwdPlan pl;
   pl.D = tile_head_dim(p.d);
-  const bool mask_b = !p.mask || p.mask_row_stride == 0 || p.seqlen_q == 1;
-  const bool bias_b = !p.bias || p.bias_row_stride == 0 || p.seqlen_q == 1;
-  pl.bcast = mask_b && bias_b;
-  pl.needs_act = p.mask != nullptr && !mask_b;
+  pl.needs_act = p.mask != nullptr && p.mask_row_stride != 0 && p.seqlen_q != 1;
   pl.sq_r = static_cast<int>(round_up(p.seqlen_q, kBM));
   const int G = p.h / p.h_k;
   if (!bp.dbias) {
@@ -1056,8 +940,6 @@ BwdPlan plan(const fdma_bwd_params& bp) {
   } else {
     pl.dbias_mode = kDbAtomic;
   }
-  // per-(query, key) dBias is written by the per-query kernel, whose softmax threads keep one query range per step
-  if (pl.dbias_mode == kDbDirect) pl.bcast = false;
   size_t o = 0;
   const size_t rows = static_cast<size_t>(p.b) * p.h * pl.sq_r;
   pl.lse2_off = o; o += align256(rows * 4);
@@ -1085,7 +967,7 @@ BwdPlan plan(const fdma_bwd_params& bp) {
 bool aligned16(const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; }
 
 template <int D, bool kBf16>
-int launch(const fdma_bwd_params& bp, const BwdPlan& pl, const PackedSeqs& seqs, cudaStream_t stream) {
+int launch(const fdma_bwd_params& bp, const BwdPlan& pl, cudaStream_t stream) {
   using L = SmemB<D>;
   const fdma_fwd_params& p = bp.f;
   if (!p.workspace || p.workspace_bytes < pl.total) return FDMA_ERR_WORKSPACE;
@@ -1171,21 +1053,17 @@ int launch(const fdma_bwd_params& bp, const BwdPlan& pl, const PackedSeqs& seqs,
   kp.dbias_keys = bp.scatter_pos ? p.seqlen_k : bp.dbias_keys;
   kp.dbias_mode = pl.dbias_mode;
   kp.is_causal = p.is_causal;
-  kp.seqs = seqs;
-  kp.n_tiles = seqs.cu_q ? packed_slots(p.seqlen_k, seqs.n, kBN) : (p.seqlen_k + kBN - 1) / kBN;
   kp.key_pos = p.key_pos;
   kp.pos_batch_stride = p.key_pos_batch_stride; kp.pos_head_stride = p.key_pos_head_stride;
   kp.h_pos = p.h_pos; kp.causal_shift = p.causal_shift;
   kp.scale_log2 = p.softmax_scale * kLog2e;
   kp.scale = p.softmax_scale;
 
-  auto kern = bp.deterministic ? (pl.bcast ? bwd_kernel<D, kBf16, true, true> : bwd_kernel<D, kBf16, false, true>)
-                               : (pl.bcast ? bwd_kernel<D, kBf16, true, false> : bwd_kernel<D, kBf16, false, false>);
-  if (seqs.cu_q) kern = bp.deterministic ? bwd_kernel<D, kBf16, true, true, true> : bwd_kernel<D, kBf16, true, false, true>;
+  auto kern = bp.deterministic ? bwd_kernel<D, kBf16, true> : bwd_kernel<D, kBf16, false>;
   const int smem_bytes = L::kAlloc;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
   if (e != cudaSuccess) return static_cast<int>(e);
-  dim3 grid(static_cast<unsigned>(kp.n_tiles) * pl.nsplit, p.h_k, p.b);
+  dim3 grid(static_cast<unsigned>((p.seqlen_k + kBN - 1) / kBN) * pl.nsplit, p.h_k, p.b);
   cudaEvent_t ev0, ev1;
   take_timing_events(&ev0, &ev1);
   if (ev0) cudaEventRecord(ev0, stream);
@@ -1265,8 +1143,8 @@ int tc_bwd(const fdma_bwd_params& p, cudaStream_t stream, const PackedSeqs& seqs
   if (tile_head_dim(p.f.d) == 256) return tc_bwd256(p, stream);
   if (bwd_rows_taken(p)) return bwd_rows(p, stream, seqs);
   const BwdPlan pl = plan(p);
-  if (pl.D == 64) return bf16 ? launch<64, true>(p, pl, seqs, stream) : launch<64, false>(p, pl, seqs, stream);
-  return bf16 ? launch<128, true>(p, pl, seqs, stream) : launch<128, false>(p, pl, seqs, stream);
+  if (pl.D == 64) return bf16 ? launch<64, true>(p, pl, stream) : launch<64, false>(p, pl, stream);
+  return bf16 ? launch<128, true>(p, pl, stream) : launch<128, false>(p, pl, stream);
 }
 
 }  // namespace fdma
