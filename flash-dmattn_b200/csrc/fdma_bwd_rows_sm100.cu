@@ -45,7 +45,7 @@ constexpr int kBM = 64;       // streamed rows per step
 constexpr int kThreads = 384;
 constexpr int kStages = 4;    // ring of streamed tiles
 constexpr int kVecSlots = 4;  // ring of key addends and positions (row pass)
-constexpr int kFlush = 64;    // 64-key steps whose dQ the tensor core sums up (4096 keys)
+constexpr int kFlush = 32;    // 64-key steps whose dQ the tensor core sums up (2048 keys)
 constexpr int kMaxBits = 4096;   // 64-key tiles the activity bits of a row-pass item can hold; beyond, every tile is worked on
 constexpr int kMaxHeads = 4096;  // query heads of a group whose activity differs from head to head
 constexpr float kLog2e = 1.4426950408889634f;
@@ -1069,16 +1069,16 @@ struct RowsPlan {
   size_t lse2_off, dsum_off, dq_off, dbias_off, part_off, dbpart_off, total;
 };
 
-// Query-range splits per key tile: two CTAs per SM at least, as long as a split keeps 32 steps, and on to eight where causal masking
-// makes the CTAs unequal, as long as it keeps 80 (a split writes and reads fp32 partials of its key tile).
+// Query-range splits per key tile: two CTAs per SM, as long as a split keeps 32 steps. The row pass, whose many short CTAs run last, evens
+// out what unequal key CTAs leave, and every further split writes and reads fp32 partials of its key tile. (Up to eight CTAs per SM with
+// 80 steps each for causal calls, as a kernel without a row pass wants them, against this, with the sum of the partials: 8192 packed tokens
+// 427 -> 364 us, 8192 queries over 2048 kept keys 557 -> 501, plain 4096 462 -> 448, 32768 queries over 2048 1828 -> 1785; up to four:
+// 384, 527, 463, 1781.)
 int pick_nsplit(const fdma_fwd_params& p) {
   const int64_t ctas = static_cast<int64_t>((p.seqlen_k + kBN - 1) / kBN) * p.h_k * p.b;
-  const bool causal = p.is_causal != 0 && p.seqlen_q > 1;
-  if (ctas >= (causal ? 8 : 2) * sm_count()) return 1;
   const int64_t steps = static_cast<int64_t>((p.seqlen_q + kBM - 1) / kBM) * (p.h / p.h_k);
-  const int64_t fill = std::min((2 * sm_count() + ctas - 1) / ctas, steps / 32);
-  const int64_t even = std::min((8 * sm_count() + ctas - 1) / ctas, steps / 80);
-  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(std::max(fill, even), 64)));
+  const int64_t want = std::min((2 * sm_count() + ctas - 1) / ctas, steps / 32);
+  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(want, 64)));
 }
 
 // Query heads a row-pass CTA works on, one after the other: as many as leave six CTAs per SM, so that set-up and the first loads

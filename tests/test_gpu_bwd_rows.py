@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 # (batch, queries, keys, heads, kv heads, head dim, mask heads, bias heads, bias batch, causal)
 CASES = [
-    (1, 300, 4200, 4, 2, 64, 0, 0, 1, False),     # 66 steps a row: sums leave tensor memory once
+    (1, 300, 4200, 4, 2, 64, 0, 0, 1, False),     # 66 steps a row: sums leave tensor memory on the way
     (1, 130, 8256, 3, 1, 128, 1, 1, 1, False),    # 129 steps less the masked tiles
     (2, 4300, 4300, 2, 2, 72, 0, 2, 2, True),
     (1, 129, 127, 4, 1, 128, 0, 1, 1, True),      # two rows see no key
