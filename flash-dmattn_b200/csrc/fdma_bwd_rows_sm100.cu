@@ -15,8 +15,8 @@
 // 32 KB of fp32 dQ on its way to a buffer in global memory, which also had to be zeroed, added to and converted. Here dQ is complete in
 // tensor memory, up to kFlush steps, and the same bits every time: nothing changes for `deterministic`. Beyond, a row-pass CTA adds its
 // sums to an fp32 tile of its own every kFlush steps (the tensor core truncates its sums).
-// Whole backward, single pass -> this: plain causal 4096 x 32 heads 538 -> 481 us; 8192 packed tokens 528 -> 443; 32768 queries, 2048
-// kept keys 2118 -> 1965.
+// Whole backward, single pass -> this: plain causal 4096 x 32 heads 538 -> 484 us; 8192 packed tokens 528 -> 397; 32768 queries, 2048
+// kept keys 2118 -> 1893; deterministic, 8192 queries, 2048 kept keys 1016 (before the change to issuing) -> 530.
 //
 // Tensor memory, columns: scores[2] 2 x 64 | dP 64 (key pass at D = 128) or 2 x 64 | accumulators | stationary operands.
 // Only V in the key pass at D = 128 finds no room there (scores 128, dP 64, K 64, dV 128, dK 128) and stays in shared memory.

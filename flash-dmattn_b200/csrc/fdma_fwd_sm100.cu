@@ -82,7 +82,7 @@ struct FwdKernelParams {
 // owns ONE query tile. Its K/V ring has four slots too, of half a tile (128 columns) each: the products take the halves one after
 // the other, so that a slot is on its way again while the other half is being read. The scores have two buffers (TMEM S[2]|O = 2 x 128 +
 // 256 columns): S of the next key tile is formed while the softmax warps work on this one, before this tile's P V.
-// 65536 queries, 16 heads, 2048 kept keys: 1498 -> 1365 us (with two slots of a whole tile and one buffer, load, products and softmax took turns).
+// 65536 queries, 16 heads, 2048 kept keys: 1498 -> 1365 us, 1290 with cheaper issue (with two slots of a whole tile and one buffer, load, products and softmax took turns).
 template <int D>
 struct Smem {
   static constexpr int kNQ = D == 256 ? 1 : 2;          // query tiles per CTA
