@@ -12,9 +12,9 @@
 // written back over the scores in 16 bit; the tensor core reads little but the 64 streamed rows from shared memory (a 128 x 64 x 16
 // product takes 33 cycles with A in tensor memory and 54 with A in shared memory). The single pass this replaces formed five products
 // instead of seven, but moved 48 + 48 KB per step through shared memory for the scores, 48 KB for dQ^T = K^T dS^T, 16 KB of dS and twice
-// 32 KB of fp32 dQ on its way to a buffer in global memory, which also had to be zeroed, added to and converted. Here dQ is complete in
-// tensor memory, up to kFlush steps, and the same bits every time: nothing changes for `deterministic`. Beyond, a row-pass CTA adds its
-// sums to an fp32 tile of its own every kFlush steps (the tensor core truncates its sums).
+// 32 KB of fp32 dQ on its way to a buffer in global memory, which also had to be zeroed, added to and converted. Here dQ stays in the
+// CTA: the tensor core sums up 128 keys at a time (it truncates its sums: over 2048 keys dQ lost 1.1e-5 of its size), and the softmax
+// threads add those sums up in registers, rounding to nearest. It is the same bits every time: nothing changes for `deterministic`.
 // Whole backward, single pass -> this: plain causal 4096 x 32 heads 538 -> 484 us; 8192 packed tokens 528 -> 397; 32768 queries, 2048
 // kept keys 2118 -> 1893; deterministic, 8192 queries, 2048 kept keys 1016 (before the change to issuing) -> 530.
 //
@@ -45,7 +45,10 @@ constexpr int kBM = 64;       // streamed rows per step
 constexpr int kThreads = 384;
 constexpr int kStages = 4;    // ring of streamed tiles
 constexpr int kVecSlots = 4;  // ring of key addends and positions (row pass)
-constexpr int kFlush = 32;    // 64-key steps whose dQ the tensor core sums up (2048 keys)
+// 64-key steps whose dQ the tensor core sums up (128 keys, as a key tile's dQ was added to a buffer in memory before). Taking the sums out
+// at the start of a step, with no wait of their own, against at the end of it: plain causal 8192 x 16 heads 850 against 883 us, 32768
+// queries over 2048 gathered keys 1988 against 2020 (1936 with sums over all 2048 keys).
+constexpr int kFlush = 2;
 constexpr int kMaxBits = 4096;   // 64-key tiles the activity bits of a row-pass item can hold; beyond, every tile is worked on
 constexpr int kMaxHeads = 4096;  // query heads of a group whose activity differs from head to head
 constexpr float kLog2e = 1.4426950408889634f;
@@ -67,7 +70,6 @@ struct BwdRowsParams {
   void* dk;
   void* dv;
   void* dbias;         // column-sum mode: the output tensor
-  float* dq_acc;       // more than kFlush key tiles: fp32 (B,H,Sq,D), each row the running sum of one row-pass CTA
   float* dbias_acc;    // atomic mode: fp32 buffer (dbias_b, dbias_h, dbias_keys), zeroed
   float* dkv_part;     // null, or fp32 partials [2: dV, dK][nsplit][B][h_k][NT*128][D] instead of dk / dv
   float* dbias_part;   // with dkv_part, column-sum mode: fp32 partials [nsplit][B][h_k][NT*128]
@@ -840,83 +842,55 @@ __device__ __forceinline__ void row_pass(const BwdRowsParams& p, unsigned char* 
     const int row_g = q0 + min(row, sq - 1);  // row in the tensors
     constexpr int kHalfCols = D / 2;          // columns of dQ each team takes out
     int g0 = 0, xc = 0, sums = 0;  // steps, items with steps, sums received so far
-    int todo = -1, todo_steps = 0, flushed = 0;  // head whose dQ is to be stored
+    int todo = -1, todo_steps = 0;  // head whose dQ is to be stored
     bool ok = true;
-    auto acc_row = [&](int h) { return p.dq_acc + ((static_cast<int64_t>(b) * p.h + h) * p.seqlen_q + row_g) * D + half * kHalfCols; };
-    // 32 of this thread's dQ sums out of tensor memory; the accumulator is free after the last ones
-    auto take = [&](int c, uint32_t (&r)[32]) {
-      tmem_ld_x32(tmem_base + lane_addr + C::kAcc + half * kHalfCols + c * 32, r);
-      tmem_wait_ld();
-      if (c == kHalfCols / 32 - 1) {
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar.acc_free);
-      }
+    float2 acc[kHalfCols / 2];  // dQ of this thread's row and team
+#pragma unroll
+    for (int j = 0; j < kHalfCols / 2; ++j) acc[j] = make_float2(0.f, 0.f);
+    auto load_sums = [&](uint32_t (&r)[kHalfCols / 32][32]) {
+#pragma unroll
+      for (int c = 0; c < kHalfCols / 32; ++c) tmem_ld_x32(tmem_base + lane_addr + C::kAcc + half * kHalfCols + c * 32, r[c]);
     };
-    auto sums_ready = [&]() {
-      ok = __all_sync(0xffffffffu, mbar_wait(bar.final_, sums & 1, ctl, kWaitFinal));
+    auto add_sums = [&](const uint32_t (&r)[kHalfCols / 32][32]) {
       ++sums;
-      tc_fence_after_sync();
-      return ok;
+#pragma unroll
+      for (int c = 0; c < kHalfCols / 32; ++c)
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          acc[c * 16 + j] = __fadd2_rn(acc[c * 16 + j], make_float2(__uint_as_float(r[c][2 * j]), __uint_as_float(r[c][2 * j + 1])));
     };
-    auto flush = [&](int h) {
-      if (!sums_ready()) return;
-#pragma unroll
-      for (int c = 0; c < kHalfCols / 32; ++c) {
-        uint32_t r[32];
-        take(c, r);
-        if (!row_ok) continue;
-#pragma unroll
-        for (int v4 = 0; v4 < 8; ++v4) {
-          float4* dst = reinterpret_cast<float4*>(acc_row(h) + c * 32 + v4 * 4);
-          float4 x = make_float4(__uint_as_float(r[v4 * 4]), __uint_as_float(r[v4 * 4 + 1]), __uint_as_float(r[v4 * 4 + 2]),
-                                 __uint_as_float(r[v4 * 4 + 3]));
-          if (flushed) {
-            const float4 y = *dst;
-            x = make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
-          }
-          *dst = x;
-        }
-      }
-      ++flushed;
+    auto sums_taken = [&]() {  // after tmem_wait_ld: the accumulator may be overwritten from here on
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar.acc_free);
+    };
+    auto collect = [&]() {  // the oldest sums not yet taken
+      ok = __all_sync(0xffffffffu, mbar_wait(bar.final_, sums & 1, ctl, kWaitFinal));
+      if (!ok) return;
+      tc_fence_after_sync();
+      uint32_t r[kHalfCols / 32][32];
+      load_sums(r);
+      tmem_wait_ld();
+      sums_taken();
+      add_sums(r);
     };
     auto store = [&](int h, int n_steps) {  // dQ of a finished item
-      if (n_steps > 0 && !sums_ready()) return;
+      if (n_steps > 0) collect();
+      if (!ok) return;
       uint16_t* dst = reinterpret_cast<uint16_t*>(p.dq) + b * p.dq_batch_stride + h * p.dq_head_stride +
-                      static_cast<int64_t>(row_g) * p.dq_row_stride;
+                      static_cast<int64_t>(row_g) * p.dq_row_stride + half * kHalfCols;
 #pragma unroll
-      for (int c = 0; c < kHalfCols / 32; ++c) {
-        const int col = half * kHalfCols + c * 32;
-        uint32_t r[32];
-        if (n_steps > 0) {
-          take(c, r);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) r[j] = 0u;
-        }
-        if (!row_ok) continue;
-        if (flushed) {
-#pragma unroll
-          for (int v4 = 0; v4 < 8; ++v4) {
-            const float4 y = *reinterpret_cast<const float4*>(acc_row(h) + c * 32 + v4 * 4);
-            r[v4 * 4] = __float_as_uint(__uint_as_float(r[v4 * 4]) + y.x);
-            r[v4 * 4 + 1] = __float_as_uint(__uint_as_float(r[v4 * 4 + 1]) + y.y);
-            r[v4 * 4 + 2] = __float_as_uint(__uint_as_float(r[v4 * 4 + 2]) + y.z);
-            r[v4 * 4 + 3] = __float_as_uint(__uint_as_float(r[v4 * 4 + 3]) + y.w);
-          }
-        }
-#pragma unroll
-        for (int v4 = 0; v4 < 4; ++v4) {
-          if (col + v4 * 8 >= p.d) break;
-          uint4 o;
-          o.x = pack_16x2<kBf16>(__uint_as_float(r[v4 * 8 + 0]) * p.scale, __uint_as_float(r[v4 * 8 + 1]) * p.scale);
-          o.y = pack_16x2<kBf16>(__uint_as_float(r[v4 * 8 + 2]) * p.scale, __uint_as_float(r[v4 * 8 + 3]) * p.scale);
-          o.z = pack_16x2<kBf16>(__uint_as_float(r[v4 * 8 + 4]) * p.scale, __uint_as_float(r[v4 * 8 + 5]) * p.scale);
-          o.w = pack_16x2<kBf16>(__uint_as_float(r[v4 * 8 + 6]) * p.scale, __uint_as_float(r[v4 * 8 + 7]) * p.scale);
-          *reinterpret_cast<uint4*>(dst + col + v4 * 8) = o;
-        }
+      for (int v = 0; v < kHalfCols / 8; ++v) {
+        if (!row_ok || half * kHalfCols + v * 8 >= p.d) break;
+        uint4 o;
+        o.x = pack_16x2<kBf16>(acc[v * 4].x * p.scale, acc[v * 4].y * p.scale);
+        o.y = pack_16x2<kBf16>(acc[v * 4 + 1].x * p.scale, acc[v * 4 + 1].y * p.scale);
+        o.z = pack_16x2<kBf16>(acc[v * 4 + 2].x * p.scale, acc[v * 4 + 2].y * p.scale);
+        o.w = pack_16x2<kBf16>(acc[v * 4 + 3].x * p.scale, acc[v * 4 + 3].y * p.scale);
+        *reinterpret_cast<uint4*>(dst + v * 8) = o;
       }
-      flushed = 0;
+#pragma unroll
+      for (int j = 0; j < kHalfCols / 2; ++j) acc[j] = make_float2(0.f, 0.f);
     };
     for (int ic = 0; ok; ++ic) {
       const int h = h0 + ic, buf = ic & 1;
@@ -958,8 +932,6 @@ __device__ __forceinline__ void row_pass(const BwdRowsParams& p, unsigned char* 
       const float2 nlse2 = make_float2(-lse, -lse), dsum2 = make_float2(dsum, dsum);
       for (int i = 0; i < n_steps && ok; ++i) {
         const int g = g0 + i, slot = g % kVecSlots;
-        while (ok && flushed < i / kFlush) flush(h);
-        if (!ok) break;
         ok = __all_sync(0xffffffffu, mbar_wait(bar.vec_full + slot, (g / kVecSlots) & 1, ctl, kWaitVecFull));
         if (!ok) break;
         ok = __all_sync(0xffffffffu, mbar_wait(bar.s_full + (g & 1), (g >> 1) & 1, ctl, kWaitS));
@@ -967,6 +939,15 @@ __device__ __forceinline__ void row_pass(const BwdRowsParams& p, unsigned char* 
         tc_fence_after_sync();
         uint32_t rs[32], rp[32], dsk[16];
         const uint32_t s_col = tmem_base + lane_addr + C::kS + (g & 1) * kBM + half * 32;
+        // Sums that ended two steps ago: their product was issued before the scores just waited for, so it is complete; the next
+        // one, which starts new sums, waits for this.
+        if (i > kFlush && i % kFlush == 1 % kFlush) {
+          uint32_t r[kHalfCols / 32][32];
+          load_sums(r);
+          tmem_wait_ld();
+          sums_taken();
+          add_sums(r);
+        }
         tmem_ld_x32(s_col, rs);
         tmem_ld_x32(tmem_base + lane_addr + C::kDp + (g & 1) * kBM + half * 32, rp);
         tmem_wait_ld();
@@ -999,7 +980,7 @@ __device__ __forceinline__ void row_pass(const BwdRowsParams& p, unsigned char* 
           mbar_arrive(bar.vec_empty + slot);
         }
       }
-      while (ok && n_steps > 0 && flushed < (n_steps - 1) / kFlush) flush(h);
+      if (ok && n_steps > 1 && (n_steps - 1) % kFlush == 0) collect();  // (those of the step before the last)
       g0 += n_steps;
     }
   }
@@ -1066,7 +1047,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_rows_kernel(const __grid_cons
 struct RowsPlan {
   int D, sq_r, nsplit, dbias_mode;
   bool part;  // dK, dV (and column sums) leave the kernel as fp32 partials
-  size_t lse2_off, dsum_off, dq_off, dbias_off, part_off, dbpart_off, total;
+  size_t lse2_off, dsum_off, dbias_off, part_off, dbpart_off, total;
 };
 
 // Query-range splits per key tile: two CTAs per SM, as long as a split keeps 32 steps. The row pass, whose many short CTAs run last, evens
@@ -1102,8 +1083,6 @@ RowsPlan plan(const fdma_bwd_params& bp) {
   const size_t rows = static_cast<size_t>(p.b) * p.h * pl.sq_r;
   pl.lse2_off = o; o += align256(rows * 4);
   pl.dsum_off = o; o += align256(rows * 4);
-  pl.dq_off = o;
-  if (p.seqlen_k > kFlush * kBM) o += align256(static_cast<size_t>(p.b) * p.seqlen_q * p.h * pl.D * 4);
   pl.dbias_off = o;
   if (pl.dbias_mode == kDbAtomic) o += align256(static_cast<size_t>(bp.dbias_b) * bp.dbias_h * atomic_keys(bp) * 4);
   pl.nsplit = pick_nsplit(p);
@@ -1174,7 +1153,6 @@ int launch(const fdma_bwd_params& bp, const RowsPlan& pl, const PackedSeqs& seqs
   kp.dk = bp.dk;
   kp.dv = bp.dv;
   kp.dbias = bp.dbias;
-  kp.dq_acc = reinterpret_cast<float*>(ws + pl.dq_off);
   kp.dkv_part = pl.part ? reinterpret_cast<float*>(ws + pl.part_off) : nullptr;
   kp.dbias_part = reinterpret_cast<float*>(ws + pl.dbpart_off);
   kp.status = kernel_status_ptr();
