@@ -49,6 +49,9 @@ constexpr int kVecSlots = 4;  // ring of key addends and positions (row pass)
 // at the start of a step, with no wait of their own, against at the end of it: plain causal 8192 x 16 heads 850 against 883 us, 32768
 // queries over 2048 gathered keys 1988 against 2020 (1936 with sums over all 2048 keys).
 constexpr int kFlush = 2;
+// 64-query steps whose dK and dV the tensor core sums up: 192 additions, no more than one CTA of the single pass made (that took up to a
+// whole group's queries, or 80 steps and more of them). Moving them out costs some 1700 cycles (0.9 us), the time of 128 KB on their way to L2.
+constexpr int kKeyFlush = 48;
 constexpr int kMaxBits = 4096;   // 64-key tiles the activity bits of a row-pass item can hold; beyond, every tile is worked on
 constexpr int kMaxHeads = 4096;  // query heads of a group whose activity differs from head to head
 constexpr float kLog2e = 1.4426950408889634f;
@@ -71,6 +74,7 @@ struct BwdRowsParams {
   void* dv;
   void* dbias;         // column-sum mode: the output tensor
   float* dbias_acc;    // atomic mode: fp32 buffer (dbias_b, dbias_h, dbias_keys), zeroed
+  float* dkv_sums;     // more than kKeyFlush steps: fp32 [2: dV, dK][nsplit][B][h_k][NT*128 * D], a CTA's rows as [D / 4][rows][4]
   float* dkv_part;     // null, or fp32 partials [2: dV, dK][nsplit][B][h_k][NT*128][D] instead of dk / dv
   float* dbias_part;   // with dkv_part, column-sum mode: fp32 partials [nsplit][B][h_k][NT*128]
   int* status;
@@ -373,12 +377,20 @@ __device__ __forceinline__ void key_pass(const BwdRowsParams& p, unsigned char* 
           if constexpr (kX2Tmem) product_ts<D, kBf16>(lead, dst, tmem_base + C::kX2, g);
           else product_ss<D, kBf16>(lead, dst, smem_u32(smem + L::kX2Off), g);
         };
+        int summed = 0, acc = 0;  // steps in the sums so far, sums before these
         auto gradients = [&](int step) {
+          const bool fresh = summed == 0;
           if (!wait(bar.pds + (step & 1), step >> 1, kWaitPds)) return false;
+          if (fresh && acc > 0 && !wait(bar.acc_free, acc - 1, kWaitAccFree)) return false;  // the sums before have been read
           const uint32_t st = st_addr + (step % kStages) * 2 * L::kStep, pc = tmem_base + C::kS + (step & 1) * kBM;
-          gradient<D, kBf16>(lead, tmem_base + C::kAcc, pc, st + L::kStep, step == 0);
-          gradient<D, kBf16>(lead, tmem_base + kAcc2, pc + 16, st, step == 0);
+          gradient<D, kBf16>(lead, tmem_base + C::kAcc, pc, st + L::kStep, fresh);
+          gradient<D, kBf16>(lead, tmem_base + kAcc2, pc + 16, st, fresh);
           umma_commit(lead, bar.st_empty + (step % kStages));
+          if (++summed == kKeyFlush || step == n_steps - 1) {
+            umma_commit(lead, bar.final_);
+            summed = 0;
+            ++acc;
+          }
           return true;
         };
         bool ok = wait(bar.x_full, 0, kWaitX) && wait(bar.ready, 0, kWaitReady) && stage_ready(0);
@@ -410,8 +422,7 @@ __device__ __forceinline__ void key_pass(const BwdRowsParams& p, unsigned char* 
             umma_commit(lead, bar.s_full + ((i + 1) & 1));
           }
         }
-        if (ok) ok = gradients(n_steps - 1);
-        if (ok) umma_commit(lead, bar.final_);
+        if (ok) gradients(n_steps - 1);
       }
     }
   } else {
@@ -454,62 +465,104 @@ __device__ __forceinline__ void key_pass(const BwdRowsParams& p, unsigned char* 
       if (!p.bias) return 0.f;
       return raw16_to_f<kBf16>(reinterpret_cast<const uint16_t*>(p.bias)[b * p.bias_batch_stride + hb * p.bias_head_stride + key]) * kLog2e;
     };
+    // dV (team 0) and dK (team 1) out of tensor memory: 128 columns of this thread's key, in pieces that a warp stores in one go
+    const uint32_t acc_addr = tmem_base + lane_addr + (half == 0 ? C::kAcc : kAcc2);
+    const int rows = min(kBN, key_end - key0);
+    float4* const sums = reinterpret_cast<float4*>(p.dkv_sums) +
+                         ((((static_cast<int64_t>(half) * p.nsplit + split) * p.b + b) * p.h_k + hk) * (NT * kBN) + key0) * (D / 4) + krow;
+    int moved = 0;  // how often
+    auto move_sums = [&]() {
+#pragma unroll 1  // (little code: it lies in the loop over the steps)
+      for (int c = 0; c < D / 32; ++c) {
+        uint32_t r[32];
+        tmem_ld_x32(acc_addr + c * 32, r);
+        tmem_wait_ld();
+        if (c == D / 32 - 1) {  // the next sums may take their place
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar.acc_free);
+        }
+        if (key_ok) {
+#pragma unroll
+          for (int v4 = 0; v4 < 8; ++v4) {
+            float4* dst = sums + (c * 8 + v4) * rows;
+            const float4 x = make_float4(__uint_as_float(r[v4 * 4]), __uint_as_float(r[v4 * 4 + 1]), __uint_as_float(r[v4 * 4 + 2]),
+                                         __uint_as_float(r[v4 * 4 + 3]));
+            if (moved) red_add_f32x4(dst, x);
+            else *dst = x;
+          }
+        }
+        __syncwarp();
+      }
+      ++moved;
+    };
     const bool hoist = G == 1 || ((!p.bias || p.h_bias != p.h) && (!p.mask || p.h_mask != p.h));
     float bv = addend(hk * G);
     float colsum = 0.f;  // dBias: sum of dS over the CTA's queries and heads
     int m = m_start, a = 0;  // the step's query tile and place in the list of heads
-    for (int i = 0; i < n_steps && ok; ++i) {
-      const int h = hk * G + (list ? s_heads[a] : a);
-      if (!hoist) bv = addend(h);
-      ok = __all_sync(0xffffffffu, mbar_wait(bar.s_full + (i & 1), (i >> 1) & 1, ctl, kWaitS));
-      if (!ok) break;
+    auto sums_ready = [&]() {
+      ok = __all_sync(0xffffffffu, mbar_wait(bar.final_, moved & 1, ctl, kWaitFinal));
       tc_fence_after_sync();
-      uint32_t rs[32], rp[32], pk[16], dsk[16];
-      const uint32_t s_col = tmem_base + lane_addr + C::kS + (i & 1) * kBM + half * 32;
-      tmem_ld_x32(s_col, rs);
-      tmem_ld_x32(tmem_base + lane_addr + C::kDp + (kDpBufs == 2 ? (i & 1) * kBM : 0) + half * 32, rp);
-      tmem_wait_ld();
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar.dp_free + (i & 1));  // the dP block may be overwritten from here on
-      // LSE and D of the step's queries: bulk-copied under the stage barrier, which the MMA warp observed before it issued the
-      // products this team has just waited for
-      const float4* l4 = reinterpret_cast<const float4*>(s_ld + (i % kStages) * (2 * kBM) + half * 32);
-      const float4* d4 = l4 + kBM / 4;
-      const int q0 = m * kBM + half * 32;
-      auto pair = [](const float4* v, int j) {
-        const float4 x = v[j >> 1];
-        return (j & 1) ? make_float2(x.z, x.w) : make_float2(x.x, x.y);
-      };
-      const float2 neg1 = make_float2(-1.f, -1.f);
-      float sum;
-      if (qlo_max > q0 || qhi_min < q0 + 32) {  // warp-uniform: some (query, key) of the warp is out of sight
-        sum = softmax_step<kBf16, true>(rs, rp, p.scale_log2, [&](int j) {
-          const int q = q0 + 2 * j;
-          return __ffma2_rn(pair(l4, j), neg1, make_float2(q < qlo || q >= qhi ? -CUDART_INF_F : bv, q + 1 < qlo || q + 1 >= qhi ? -CUDART_INF_F : bv));
-        }, [&](int j) { return pair(d4, j); }, pk, dsk);
-      } else {
-        const float2 bv2 = make_float2(bv, bv);
-        sum = softmax_step<kBf16, true>(rs, rp, p.scale_log2, [&](int j) { return __ffma2_rn(pair(l4, j), neg1, bv2); },
-                                        [&](int j) { return pair(d4, j); }, pk, dsk);
+      return ok;
+    };
+    int i = 0;
+    while (true) {
+      const int end = min(n_steps, (moved + 1) * kKeyFlush + 1);
+      for (; i < end && ok; ++i) {
+        const int h = hk * G + (list ? s_heads[a] : a);
+        if (!hoist) bv = addend(h);
+        ok = __all_sync(0xffffffffu, mbar_wait(bar.s_full + (i & 1), (i >> 1) & 1, ctl, kWaitS));
+        if (!ok) break;
+        tc_fence_after_sync();
+        uint32_t rs[32], rp[32], pk[16], dsk[16];
+        const uint32_t s_col = tmem_base + lane_addr + C::kS + (i & 1) * kBM + half * 32;
+        tmem_ld_x32(s_col, rs);
+        tmem_ld_x32(tmem_base + lane_addr + C::kDp + (kDpBufs == 2 ? (i & 1) * kBM : 0) + half * 32, rp);
+        tmem_wait_ld();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar.dp_free + (i & 1));  // the dP block may be overwritten from here on
+        // LSE and D of the step's queries: bulk-copied under the stage barrier, which the MMA warp observed before it issued the
+        // products this team has just waited for
+        const float4* l4 = reinterpret_cast<const float4*>(s_ld + (i % kStages) * (2 * kBM) + half * 32);
+        const float4* d4 = l4 + kBM / 4;
+        const int q0 = m * kBM + half * 32;
+        auto pair = [](const float4* v, int j) {
+          const float4 x = v[j >> 1];
+          return (j & 1) ? make_float2(x.z, x.w) : make_float2(x.x, x.y);
+        };
+        const float2 neg1 = make_float2(-1.f, -1.f);
+        float sum;
+        if (qlo_max > q0 || qhi_min < q0 + 32) {  // warp-uniform: some (query, key) of the warp is out of sight
+          sum = softmax_step<kBf16, true>(rs, rp, p.scale_log2, [&](int j) {
+            const int q = q0 + 2 * j;
+            return __ffma2_rn(pair(l4, j), neg1, make_float2(q < qlo || q >= qhi ? -CUDART_INF_F : bv, q + 1 < qlo || q + 1 >= qhi ? -CUDART_INF_F : bv));
+          }, [&](int j) { return pair(d4, j); }, pk, dsk);
+        } else {
+          const float2 bv2 = make_float2(bv, bv);
+          sum = softmax_step<kBf16, true>(rs, rp, p.scale_log2, [&](int j) { return __ffma2_rn(pair(l4, j), neg1, bv2); },
+                                          [&](int j) { return pair(d4, j); }, pk, dsk);
+        }
+        // back into the 32 columns just read: P^T pairs in the first 16, dS^T pairs in the last 16
+        tmem_st_x16(s_col, pk);
+        tmem_st_x16(s_col + 16, dsk);
+        tmem_wait_st();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar.pds + (i & 1));
+        if (p.dbias_mode == kDbAtomic && key_ok) {
+          const int b2 = p.dbias_b == 1 ? 0 : b, h2 = h / (p.h / p.dbias_h);
+          atomicAdd(p.dbias_acc + (static_cast<int64_t>(b2) * p.dbias_h + h2) * p.dbias_keys + key, sum);
+        } else {
+          colsum += sum;
+        }
+        if (++a == GA) {
+          a = 0;
+          ++m;
+        }
       }
-      // back into the 32 columns just read: P^T pairs in the first 16, dS^T pairs in the last 16
-      tmem_st_x16(s_col, pk);
-      tmem_st_x16(s_col + 16, dsk);
-      tmem_wait_st();
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar.pds + (i & 1));
-      if (p.dbias_mode == kDbAtomic && key_ok) {
-        const int b2 = p.dbias_b == 1 ? 0 : b, h2 = h / (p.h / p.dbias_h);
-        atomicAdd(p.dbias_acc + (static_cast<int64_t>(b2) * p.dbias_h + h2) * p.dbias_keys + key, sum);
-      } else {
-        colsum += sum;
-      }
-      if (++a == GA) {
-        a = 0;
-        ++m;
-      }
+      if (!ok || n_steps <= (moved + 1) * kKeyFlush || !sums_ready()) break;
+      move_sums();  // one step behind: the first product of the next sums follows that step
     }
     // ---------------- epilogue: dV (team 0) and dK (team 1), column-sum dBias ----------------
     if (p.dbias_mode == kDbColsum) {
@@ -524,10 +577,8 @@ __device__ __forceinline__ void key_pass(const BwdRowsParams& p, unsigned char* 
           reinterpret_cast<uint16_t*>(p.dbias)[b * p.dbias_batch_stride + hk * p.dbias_head_stride + key] = f_to_raw16<kBf16>(key_ok ? tot : 0.f);
       }
     }
-    if (ok && n_steps > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar.final_, 0, ctl, kWaitFinal));
-    tc_fence_after_sync();
+    if (ok && n_steps > 0) sums_ready();
     if (ok) {
-      const uint32_t col = half == 0 ? C::kAcc : kAcc2;
       const float mul = half == 0 ? 1.f : p.scale;
       uint16_t* dst = half == 0 ? reinterpret_cast<uint16_t*>(p.dv) + b * p.dv_batch_stride + hk * p.dv_head_stride +
                                       static_cast<int64_t>(min(key, Sk - 1)) * p.dv_row_stride
@@ -537,8 +588,18 @@ __device__ __forceinline__ void key_pass(const BwdRowsParams& p, unsigned char* 
       for (int c = 0; c < D / 32; ++c) {
         uint32_t r[32];
         if (n_steps > 0) {
-          tmem_ld_x32(tmem_base + lane_addr + col + c * 32, r);
+          tmem_ld_x32(acc_addr + c * 32, r);
           tmem_wait_ld();
+          if (moved && key_ok) {
+#pragma unroll
+            for (int v4 = 0; v4 < 8; ++v4) {
+              const float4 x = __ldcg(sums + (c * 8 + v4) * rows);  // (from L2, where they were added up)
+              r[v4 * 4] = __float_as_uint(__uint_as_float(r[v4 * 4]) + x.x);
+              r[v4 * 4 + 1] = __float_as_uint(__uint_as_float(r[v4 * 4 + 1]) + x.y);
+              r[v4 * 4 + 2] = __float_as_uint(__uint_as_float(r[v4 * 4 + 2]) + x.z);
+              r[v4 * 4 + 3] = __float_as_uint(__uint_as_float(r[v4 * 4 + 3]) + x.w);
+            }
+          }
         } else {
 #pragma unroll
           for (int j = 0; j < 32; ++j) r[j] = 0u;
@@ -1047,7 +1108,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_rows_kernel(const __grid_cons
 struct RowsPlan {
   int D, sq_r, nsplit, dbias_mode;
   bool part;  // dK, dV (and column sums) leave the kernel as fp32 partials
-  size_t lse2_off, dsum_off, dbias_off, part_off, dbpart_off, total;
+  size_t lse2_off, dsum_off, dbias_off, sums_off, part_off, dbpart_off, total;
 };
 
 // Query-range splits per key tile: two CTAs per SM, as long as a split keeps 32 steps. The row pass, whose many short CTAs run last, evens
@@ -1086,6 +1147,10 @@ RowsPlan plan(const fdma_bwd_params& bp) {
   pl.dbias_off = o;
   if (pl.dbias_mode == kDbAtomic) o += align256(static_cast<size_t>(bp.dbias_b) * bp.dbias_h * atomic_keys(bp) * 4);
   pl.nsplit = pick_nsplit(p);
+  pl.sums_off = o;
+  const int64_t m_tiles = (p.seqlen_q + kBM - 1) / kBM;
+  if ((m_tiles + pl.nsplit - 1) / pl.nsplit * (p.h / p.h_k) > kKeyFlush)
+    o += align256(static_cast<size_t>(2) * pl.nsplit * p.b * p.h_k * round_up(p.seqlen_k, kBN) * pl.D * 4);
   pl.part = pl.nsplit > 1 || bp.scatter_pos != nullptr;
   pl.part_off = pl.dbpart_off = o;
   if (pl.part) {
@@ -1153,6 +1218,7 @@ int launch(const fdma_bwd_params& bp, const RowsPlan& pl, const PackedSeqs& seqs
   kp.dk = bp.dk;
   kp.dv = bp.dv;
   kp.dbias = bp.dbias;
+  kp.dkv_sums = reinterpret_cast<float*>(ws + pl.sums_off);
   kp.dkv_part = pl.part ? reinterpret_cast<float*>(ws + pl.part_off) : nullptr;
   kp.dbias_part = reinterpret_cast<float*>(ws + pl.dbpart_off);
   kp.status = kernel_status_ptr();

@@ -199,6 +199,13 @@ __device__ __forceinline__ void bulk_reduce_add_f32(float* gmem_dst, const void*
                : "l"(reinterpret_cast<uint64_t>(gmem_dst)), "r"(smem_u32(smem_src)), "r"(bytes)
                : "memory");
 }
+// *dst += x, rounded to nearest, in L2: nothing waits for it.
+__device__ __forceinline__ void red_add_f32x4(float4* dst, float4 x) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
+               :
+               : "l"(reinterpret_cast<uint64_t>(dst)), "f"(x.x), "f"(x.y), "f"(x.z), "f"(x.w)
+               : "memory");
+}
 __device__ __forceinline__ void bulk_reduce_add_u64(long long* gmem_dst, const void* smem_src, uint32_t bytes) {
   asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.u64 [%0], [%1], %2;"
                :
