@@ -218,8 +218,15 @@ __global__ void __launch_bounds__(kThreads) bwd_finish_kernel(const BwdFinishArg
         for (int j = 0; j < 8; ++j) x[j] = __int_as_float(0x7FC00000);
       }
     } else {
-      const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(a.dq_acc) + i * 8);
-      const float4 u = p[0], v = p[1];
+      const float* p = static_cast<const float*>(a.dq_acc) + i * 8;
+      float4 u = *reinterpret_cast<const float4*>(p), v = *reinterpret_cast<const float4*>(p + 4);
+#pragma unroll 4
+      for (int s = 1; s < a.dq_nsplit; ++s) {
+        const float4 y = *reinterpret_cast<const float4*>(p + s * a.dq_split_stride);
+        const float4 z = *reinterpret_cast<const float4*>(p + s * a.dq_split_stride + 4);
+        u.x += y.x; u.y += y.y; u.z += y.z; u.w += y.w;
+        v.x += z.x; v.y += z.y; v.z += z.z; v.w += z.w;
+      }
       x[0] = u.x * a.scale; x[1] = u.y * a.scale; x[2] = u.z * a.scale; x[3] = u.w * a.scale;
       x[4] = v.x * a.scale; x[5] = v.y * a.scale; x[6] = v.z * a.scale; x[7] = v.w * a.scale;
     }

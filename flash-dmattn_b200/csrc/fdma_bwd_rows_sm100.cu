@@ -74,6 +74,7 @@ struct BwdRowsParams {
   void* dv;
   void* dbias;         // column-sum mode: the output tensor
   float* dbias_acc;    // atomic mode: fp32 buffer (dbias_b, dbias_h, dbias_keys), zeroed
+  float* dq_part;      // more than one key range: fp32 partials [ranges][B][H][Sq][D] instead of dq
   float* dkv_sums;     // more than kKeyFlush steps: fp32 [2: dV, dK][nsplit][B][h_k][NT*128 * D], a CTA's rows as [D / 4][rows][4]
   float* dkv_part;     // null, or fp32 partials [2: dV, dK][nsplit][B][h_k][NT*128][D] instead of dk / dv
   float* dbias_part;   // with dkv_part, column-sum mode: fp32 partials [nsplit][B][h_k][NT*128]
@@ -95,6 +96,7 @@ struct BwdRowsParams {
   int nsplit;        // query-range splits per key tile
   int n_key_ctas;    // CTAs of the key pass
   int heads_per_cta; // query heads a row-pass CTA works on, one after the other
+  int ranges;        // key ranges a row-pass tile is cut into, a CTA each
   float scale_log2, scale;
 };
 
@@ -642,14 +644,16 @@ __device__ __forceinline__ void row_pass(const BwdRowsParams& p, unsigned char* 
   using C = Cols<D, false>;
   float* s_vec = reinterpret_cast<float*>(smem + L::kVecOff);
   uint32_t* s_bits_all = reinterpret_cast<uint32_t*>(smem + L::kBitsOff);
-  volatile int* s_item = reinterpret_cast<volatile int*>(smem + L::kMiscOff + 16);  // [2][2]: 64-key tiles in sight, steps
+  volatile int* s_item = reinterpret_cast<volatile int*>(smem + L::kMiscOff + 16);  // [2][4]: first 64-key tile, end of them, steps
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = p.h / p.h_k;
   const bool causal = p.is_causal != 0;
   const int hgroups = (p.h + p.heads_per_cta - 1) / p.heads_per_cta;
   const int idx = blockIdx.x - p.n_key_ctas;
   // the last query tiles, which see most keys, run first; heads that share K and V meet in L2
-  int n = p.q_tiles - 1 - idx / (hgroups * p.b);
+  const int per_tile = hgroups * p.b * p.ranges;
+  int n = p.q_tiles - 1 - idx / per_tile;
+  const int range = idx % per_tile / (hgroups * p.b);
   const int b = idx % (hgroups * p.b) / hgroups;
   const int h0 = idx % hgroups * p.heads_per_cta, h1 = min(p.h, h0 + p.heads_per_cta);
   int q0 = 0, sq = p.seqlen_q, k0 = 0, sk = p.seqlen_k;  // rows of the tile's sequence: first query and their number, keys
@@ -673,10 +677,10 @@ __device__ __forceinline__ void row_pass(const BwdRowsParams& p, unsigned char* 
     return p.mask ? p.mask + b * p.mask_batch_stride + (p.h_mask == p.h ? h : (p.h_mask == p.h_k ? h / G : 0)) * p.mask_head_stride : nullptr;
   };
   const bool use_bits = p.mask && (p.seqlen_k + kBM - 1) / kBM <= kMaxBits;
-  // Steps of an item: the 64-key tiles below n_sub that hold a kept key
-  auto next = [&](int m, int n_sub, const uint32_t* bits) {
+  // Steps of an item: the 64-key tiles [first, end) that hold a kept key
+  auto next = [&](int m, int first, int end, const uint32_t* bits) {
     do ++m;
-    while (use_bits && m < n_sub && !((bits[m >> 5] >> (m & 31)) & 1u));
+    while (use_bits && m < end && !((bits[(m - first) >> 5] >> ((m - first) & 31)) & 1u));
     return m;
   };
 
@@ -691,7 +695,7 @@ __device__ __forceinline__ void row_pass(const BwdRowsParams& p, unsigned char* 
           const int h = h0 + ic, buf = ic & 1;
           ok = mbar_wait(bar.item_full + buf, (ic >> 1) & 1, ctl, kWaitItemFull);
           if (!ok) break;
-          const int n_sub = s_item[buf * 2], n_steps = s_item[buf * 2 + 1];
+          const int first = s_item[buf * 4], end = s_item[buf * 4 + 1], n_steps = s_item[buf * 4 + 2];
           const uint32_t* bits = s_bits_all + buf * (kMaxBits / 32);
           if (n_steps > 0) {
             ok = mbar_wait(bar.x_empty, (xc & 1) ^ 1, ctl, kWaitXEmpty);
@@ -707,7 +711,7 @@ __device__ __forceinline__ void row_pass(const BwdRowsParams& p, unsigned char* 
                 tma_load_4d(smem + L::kX2Off + dst, &p.tm_do, bar.x_full, kb * 64, h, row, b);
               }
           }
-          for (int i = 0, m = next(-1, n_sub, bits); i < n_steps; ++i, m = next(m, n_sub, bits), ++it) {
+          for (int i = 0, m = next(first - 1, first, end, bits); i < n_steps; ++i, m = next(m, first, end, bits), ++it) {
             const int stage = it % kStages;
             ok = mbar_wait(bar.st_empty + stage, ((it / kStages) & 1) ^ 1, ctl, kWaitStEmpty);
             if (!ok) break;
@@ -743,15 +747,15 @@ __device__ __forceinline__ void row_pass(const BwdRowsParams& p, unsigned char* 
         const int buf = ic & 1;
         ok = wait(bar.item_full + buf, ic >> 1, kWaitItemFull);
         if (!ok) break;
-        const int n_sub = warp_uniform(s_item[buf * 2]), n_steps = warp_uniform(s_item[buf * 2 + 1]);
+        const int end = warp_uniform(s_item[buf * 4 + 1]), n_steps = warp_uniform(s_item[buf * 4 + 2]);
         // Packed sequences: K and V rows beyond the sequence, in its last tile, become zeros, as TMA fills them in at the end of a
         // tensor (zero probabilities alone would pass a NaN on).
         auto stage_ready = [&](int i) {
           const int stage = (g0 + i) % kStages;
           if (!wait(bar.st_full + stage, (g0 + i) / kStages, kWaitStFull)) return false;
-          if (packed && i == n_steps - 1 && sk - (n_sub - 1) * kBM < kBM) {
+          if (packed && i == n_steps - 1 && sk - (end - 1) * kBM < kBM) {
             unsigned char* st = smem + L::kStOff + stage * 2 * L::kStep;
-            for (int t = 0; t < 2; ++t) zero_tile_rows(st + t * L::kStep, D / 64, kBM * 128, sk - (n_sub - 1) * kBM, kBM);
+            for (int t = 0; t < 2; ++t) zero_tile_rows(st + t * L::kStep, D / 64, kBM * 128, sk - (end - 1) * kBM, kBM);
             fence_proxy_async_smem();
             __syncwarp();
           }
@@ -802,13 +806,13 @@ __device__ __forceinline__ void row_pass(const BwdRowsParams& p, unsigned char* 
         const int h = h0 + ic, buf = ic & 1;
         ok = __all_sync(0xffffffffu, mbar_wait(bar.item_full + buf, (ic >> 1) & 1, ctl, kWaitItemFull));
         if (!ok) break;
-        const int n_sub = s_item[buf * 2], n_steps = s_item[buf * 2 + 1];
+        const int first = s_item[buf * 4], end = s_item[buf * 4 + 1], n_steps = s_item[buf * 4 + 2];
         const uint32_t* bits = s_bits_all + buf * (kMaxBits / 32);
         const uint8_t* mrow = mask_of(h);
         const uint16_t* brow = p.bias ? reinterpret_cast<const uint16_t*>(p.bias) + b * p.bias_batch_stride +
                                             (p.h_bias == p.h ? h : (p.h_bias == p.h_k ? h / G : 0)) * p.bias_head_stride : nullptr;
         const int32_t* pos_row = pos_of(h);
-        for (int i = 0, m = next(-1, n_sub, bits); i < n_steps; ++i, m = next(m, n_sub, bits), ++vi) {
+        for (int i = 0, m = next(first - 1, first, end, bits); i < n_steps; ++i, m = next(m, first, end, bits), ++vi) {
           const int k = m * kBM + lane * 2;
           const uint32_t mb = mrow ? *reinterpret_cast<const uint16_t*>(mrow + k) : 0x0101u;
           const uint32_t bb = brow ? *reinterpret_cast<const uint32_t*>(brow + k) : 0u;
@@ -853,16 +857,17 @@ __device__ __forceinline__ void row_pass(const BwdRowsParams& p, unsigned char* 
         } else if (causal) {
           vis = static_cast<int>(max(static_cast<int64_t>(0), min(static_cast<int64_t>(sk), static_cast<int64_t>(q_last) + coff + 1)));
         }
-        const int n_sub = (vis + kBM - 1) / kBM;
-        int n_steps = n_sub;
+        const int n_sub = (vis + kBM - 1) / kBM, chunk = (n_sub + p.ranges - 1) / p.ranges;
+        const int first = min(range * chunk, n_sub), end = min(first + chunk, n_sub);
+        int n_steps = end - first;
         if (use_bits) {
           const uint8_t* mrow = mask_of(h);
           uint32_t* bits = s_bits_all + buf * (kMaxBits / 32);
           n_steps = 0;
-          for (int w = 0; w * 32 < n_sub; ++w) {  // a lane per tile
-            const int m = w * 32 + lane;
+          for (int w = 0; first + w * 32 < end; ++w) {  // a lane per tile
+            const int m = first + w * 32 + lane;
             uint32_t any = 0;
-            if (m < n_sub) {
+            if (m < end) {
 #pragma unroll
               for (int c = 0; c < 4; ++c) {
                 const uint4 v = *reinterpret_cast<const uint4*>(mrow + m * kBM + c * 16);
@@ -881,8 +886,9 @@ __device__ __forceinline__ void row_pass(const BwdRowsParams& p, unsigned char* 
           }
         }
         if (lane == 0) {
-          s_item[buf * 2] = n_sub;
-          s_item[buf * 2 + 1] = n_steps;
+          s_item[buf * 4] = first;
+          s_item[buf * 4 + 1] = end;
+          s_item[buf * 4 + 2] = n_steps;
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(bar.item_full + buf);
@@ -938,11 +944,18 @@ __device__ __forceinline__ void row_pass(const BwdRowsParams& p, unsigned char* 
     auto store = [&](int h, int n_steps) {  // dQ of a finished item
       if (n_steps > 0) collect();
       if (!ok) return;
+      if (p.ranges > 1) {  // a partial sum
+        float4* part = reinterpret_cast<float4*>(
+            p.dq_part + (((static_cast<int64_t>(range) * p.b + b) * p.h + h) * p.seqlen_q + row_g) * D + half * kHalfCols);
+#pragma unroll
+        for (int v = 0; v < kHalfCols / 4; ++v)
+          if (row_ok) part[v] = make_float4(acc[v * 2].x, acc[v * 2].y, acc[v * 2 + 1].x, acc[v * 2 + 1].y);
+      }
       uint16_t* dst = reinterpret_cast<uint16_t*>(p.dq) + b * p.dq_batch_stride + h * p.dq_head_stride +
                       static_cast<int64_t>(row_g) * p.dq_row_stride + half * kHalfCols;
 #pragma unroll
       for (int v = 0; v < kHalfCols / 8; ++v) {
-        if (!row_ok || half * kHalfCols + v * 8 >= p.d) break;
+        if (p.ranges > 1 || !row_ok || half * kHalfCols + v * 8 >= p.d) break;
         uint4 o;
         o.x = pack_16x2<kBf16>(acc[v * 4].x * p.scale, acc[v * 4].y * p.scale);
         o.y = pack_16x2<kBf16>(acc[v * 4 + 1].x * p.scale, acc[v * 4 + 1].y * p.scale);
@@ -965,7 +978,7 @@ __device__ __forceinline__ void row_pass(const BwdRowsParams& p, unsigned char* 
         }
         ok = __all_sync(0xffffffffu, mbar_wait(bar.item_full + buf, (ic >> 1) & 1, ctl, kWaitItemFull));
         if (!ok) break;
-        n_steps = s_item[buf * 2 + 1];
+        n_steps = s_item[buf * 4 + 2];
         __syncwarp();
         if (lane == 0) mbar_arrive(bar.item_empty + buf);
         if (n_steps > 0) {
@@ -1105,10 +1118,17 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_rows_kernel(const __grid_cons
   }
 }
 
+// (row tile, head, batch element) of a call: the CTAs of the row pass at one range and head each
+int64_t row_tiles(const fdma_fwd_params& p) { return static_cast<int64_t>((p.seqlen_q + kBN - 1) / kBN) * p.h * p.b; }
+
+// The workspace is asked for without the sequences: calls that may be about packed ones.
+bool maybe_packed(const fdma_bwd_params& bp) { return bp.f.b == 1 && !bp.f.mask && !bp.f.bias && !bp.dbias && !bp.f.key_pos; }
+
 struct RowsPlan {
   int D, sq_r, nsplit, dbias_mode;
+  int ranges, packed_ranges;  // key ranges of an ordinary call; at most so many of one with packed sequences
   bool part;  // dK, dV (and column sums) leave the kernel as fp32 partials
-  size_t lse2_off, dsum_off, dbias_off, sums_off, part_off, dbpart_off, total;
+  size_t lse2_off, dsum_off, dq_off, dbias_off, sums_off, part_off, dbpart_off, total;
 };
 
 // Query-range splits per key tile: two CTAs per SM, as long as a split keeps 32 steps. The row pass, whose many short CTAs run last, evens
@@ -1121,6 +1141,22 @@ int pick_nsplit(const fdma_fwd_params& p) {
   const int64_t steps = static_cast<int64_t>((p.seqlen_q + kBM - 1) / kBM) * (p.h / p.h_k);
   const int64_t want = std::min((2 * sm_count() + ctas - 1) / ctas, steps / 32);
   return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(want, 64)));
+}
+
+// Key ranges per row-pass tile, where there are few rows and at least four times as many keys: else a few CTAs walk all keys one tile after
+// the other. Their fp32 partials are added up in one order by bwd_finish_kernel. `ctas`: row-pass CTAs without ranges.
+// Packed sequences: up to two CTAs per SM with 16 steps each. 2 x 64 queries over 2 x 16384 keys, 8 heads over 2 243 -> 104 us (82 in a
+// single pass over the keys), 32 over 8 378 -> 333 (265). A long sequence among many short ones still walks its keys in one chain.
+int packed_ranges(const fdma_fwd_params& p, int64_t ctas, int64_t steps) {
+  if (p.seqlen_k < 4ll * p.seqlen_q || steps < 32) return 1;
+  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(2 * sm_count() / ctas, steps / 16)));
+}
+// Other calls, of those this file takes (see bwd_rows_taken): half a CTA per SM, so that both passes fit in one wave, with eight steps
+// each: 128 queries over 4096 keys, 8 heads over 2 61 -> 28 us (29 in a single pass), over 2048 34 -> 27 (29), over 1024 (not cut) 25.
+int pick_ranges(const fdma_fwd_params& p) {
+  const int64_t ctas = row_tiles(p), steps = (p.seqlen_k + kBM - 1) / kBM;
+  if (p.seqlen_k < 4ll * p.seqlen_q || steps < 32 || ctas > sm_count() / 8) return 1;
+  return static_cast<int>(std::min<int64_t>(sm_count() / 2 / ctas, steps / 8));
 }
 
 // Query heads a row-pass CTA works on, one after the other: as many as leave six CTAs per SM, so that set-up and the first loads
@@ -1144,6 +1180,11 @@ RowsPlan plan(const fdma_bwd_params& bp) {
   const size_t rows = static_cast<size_t>(p.b) * p.h * pl.sq_r;
   pl.lse2_off = o; o += align256(rows * 4);
   pl.dsum_off = o; o += align256(rows * 4);
+  pl.ranges = pick_ranges(p);
+  pl.packed_ranges = maybe_packed(bp) ? packed_ranges(p, row_tiles(p), (p.seqlen_k + kBM - 1) / kBM) : 1;
+  pl.dq_off = o;
+  const int dq_parts = std::max(pl.ranges, pl.packed_ranges);
+  if (dq_parts > 1) o += align256(static_cast<size_t>(dq_parts) * p.b * p.h * p.seqlen_q * pl.D * 4);
   pl.dbias_off = o;
   if (pl.dbias_mode == kDbAtomic) o += align256(static_cast<size_t>(bp.dbias_b) * bp.dbias_h * atomic_keys(bp) * 4);
   pl.nsplit = pick_nsplit(p);
@@ -1218,6 +1259,7 @@ int launch(const fdma_bwd_params& bp, const RowsPlan& pl, const PackedSeqs& seqs
   kp.dk = bp.dk;
   kp.dv = bp.dv;
   kp.dbias = bp.dbias;
+  kp.dq_part = reinterpret_cast<float*>(ws + pl.dq_off);
   kp.dkv_sums = reinterpret_cast<float*>(ws + pl.sums_off);
   kp.dkv_part = pl.part ? reinterpret_cast<float*>(ws + pl.part_off) : nullptr;
   kp.dbias_part = reinterpret_cast<float*>(ws + pl.dbpart_off);
@@ -1242,7 +1284,10 @@ int launch(const fdma_bwd_params& bp, const RowsPlan& pl, const PackedSeqs& seqs
   kp.n_tiles = seqs.cu_q ? packed_slots(p.seqlen_k, seqs.n, kBN) : (p.seqlen_k + kBN - 1) / kBN;
   kp.q_tiles = seqs.cu_q ? packed_slots(p.seqlen_q, seqs.n, kBN) : (p.seqlen_q + kBN - 1) / kBN;
   kp.nsplit = pl.nsplit;
-  kp.heads_per_cta = pick_heads_per_cta(static_cast<int64_t>(kp.q_tiles) * p.b, p.h);
+  kp.ranges = pl.ranges;
+  if (seqs.cu_q)  // by the tiles there can be, and the average sequence
+    kp.ranges = std::min(pl.packed_ranges, packed_ranges(p, static_cast<int64_t>(p.seqlen_q / kBN + seqs.n) * p.h, (p.seqlen_k / seqs.n + kBM - 1) / kBM));
+  kp.heads_per_cta = pick_heads_per_cta(static_cast<int64_t>(kp.q_tiles) * p.b * kp.ranges, p.h);
   kp.scale_log2 = p.softmax_scale * kLog2e;
   kp.scale = p.softmax_scale;
 
@@ -1250,7 +1295,7 @@ int launch(const fdma_bwd_params& bp, const RowsPlan& pl, const PackedSeqs& seqs
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kAlloc);
   if (e != cudaSuccess) return static_cast<int>(e);
   const int64_t key_ctas = static_cast<int64_t>(kp.n_tiles) * pl.nsplit * p.h_k * p.b;
-  const int64_t ctas = key_ctas + static_cast<int64_t>(kp.q_tiles) * p.b * ((p.h + kp.heads_per_cta - 1) / kp.heads_per_cta);
+  const int64_t ctas = key_ctas + static_cast<int64_t>(kp.q_tiles) * p.b * kp.ranges * ((p.h + kp.heads_per_cta - 1) / kp.heads_per_cta);
   if (ctas > 0x7FFFFFFF) return FDMA_ERR_TOO_LARGE;
   kp.n_key_ctas = static_cast<int>(key_ctas);
   cudaEvent_t ev0, ev1;
@@ -1265,6 +1310,12 @@ int launch(const fdma_bwd_params& bp, const RowsPlan& pl, const PackedSeqs& seqs
   f.b = p.b; f.h = p.h; f.sq = p.seqlen_q; f.sq_r = pl.sq_r; f.d = p.d; f.D = D;
   f.h_k = p.h_k; f.keys_r = static_cast<int>(round_up(p.seqlen_k, kBN));
   f.rows_out = bp.scatter_pos ? bp.scatter_rows : p.seqlen_k;
+  f.scale = p.softmax_scale;
+  if (kp.ranges > 1) {
+    f.dq_acc = kp.dq_part; f.dq_nsplit = kp.ranges;
+    f.dq_split_stride = static_cast<int64_t>(p.b) * p.h * p.seqlen_q * D;
+    f.dq = bp.dq; f.dq_sb = bp.dq_batch_stride; f.dq_sr = bp.dq_row_stride; f.dq_sh = bp.dq_head_stride;
+  }
   f.pos = bp.scatter_pos; f.pos_sb = bp.scatter_batch_stride; f.pos_sh = bp.scatter_head_stride;
   f.h_pos = bp.scatter_h; f.cap = p.seqlen_k;
   if (pl.part) {
@@ -1288,15 +1339,30 @@ int launch(const fdma_bwd_params& bp, const RowsPlan& pl, const PackedSeqs& seqs
 }  // namespace
 
 // Calls of tc_bwd (head dims up to 128) that this file takes: mask and bias broadcast over the queries, or absent, and a dBias,
-// if asked for, that is summed over them.
+// if asked for, that is summed over them; but not those of few queries over many keys, beyond what fits in one wave of CTAs. There the row
+// pass is a few long chains of key tiles, while the single pass of fdma_bwd_sm100.cu spreads dQ over all key tiles. Backward in us, here
+// without ranges / single pass, head dim 128 (queries x keys, heads): 128 x 65536, 8 over 2 962 / 150, 32 over 8 1286 / 540; 1024 x 16384,
+// 32 over 8 856 / 682; 512 x 4096, 16 over 4 98 / 65; 1024 x 4096 gathered, 8 over 2 138 / 94; 256 x 2048, 32 over 8 56 / 42; but 512 x 2048,
+// 8 over 2 39 / 63, 1024 x 512, 16 over 4 64 / 77.
+// Per tile the single pass is the slower one at head dim 64 (4096 x 8192, 16 over 4 686 / 830), with less than three query heads to share
+// what a query tile needs (8192 x 1024 gathered, MHA 491 / 684), with addends per query head and with fixed-point sums (2048 x 8192
+// 502 / 729). Such calls go there only while row tiles x heads leave half the SMs idle, three quarters in fixed point (256 x 8192, 32 heads,
+// 64 row tiles: d = 64 152 / 120, MHA 280 / 224, per head 230 / 176, fixed point 183 / 180).
 bool bwd_rows_taken(const fdma_bwd_params& bp) {
   const fdma_fwd_params& p = bp.f;
   const bool mask_b = !p.mask || p.mask_row_stride == 0 || p.seqlen_q == 1;
   const bool bias_b = !p.bias || p.bias_row_stride == 0 || p.seqlen_q == 1;
-  return mask_b && bias_b && (!bp.dbias || bp.dbias_rows == 1);
+  if (!mask_b || !bias_b || (bp.dbias && bp.dbias_rows != 1)) return false;
+  if (p.seqlen_k < 2048 || p.seqlen_k < (p.seqlen_k < 4096 ? 8ll : 4ll) * p.seqlen_q) return true;
+  const int half_sms = sm_count() / 2;
+  const int64_t key_tiles = static_cast<int64_t>((p.seqlen_k + kBN - 1) / kBN) * p.h_k * p.b;
+  if (key_tiles <= half_sms && row_tiles(p) <= half_sms / 4) return true;
+  const bool per_head = (p.mask && p.h_mask == p.h) || (p.bias && p.h_bias == p.h);
+  if (tile_head_dim(p.d) == 128 && p.h >= 3 * p.h_k && !per_head && !bp.deterministic) return false;
+  return row_tiles(p) > (bp.deterministic ? half_sms / 2 : half_sms);
 }
 
-size_t bwd_rows_workspace_bytes(const fdma_bwd_params& bp) { return plan(bp).total; }
+size_t bwd_rows_workspace_bytes(const fdma_bwd_params& bp) { return bwd_rows_taken(bp) || maybe_packed(bp) ? plan(bp).total : 0; }
 
 int bwd_rows(const fdma_bwd_params& bp, cudaStream_t stream, const PackedSeqs& seqs) {
   const RowsPlan pl = plan(bp);

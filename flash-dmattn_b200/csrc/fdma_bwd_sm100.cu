@@ -1,5 +1,5 @@
 // Backward dynamic-mask attention for sm_100a (head dims up to 128) with a mask or bias per query: dQ, dK, dV and dBias from dO, O,
-// LSE. Row-broadcast ones and packed sequences: fdma_bwd_rows_sm100.cu.
+// LSE; also of few queries over many keys with row-broadcast ones. Other row-broadcast ones and packed sequences: fdma_bwd_rows_sm100.cu.
 //
 // Math of the reference's compute_dq_dk_dv_1colblock (csrc/flash_sparse_attn/src/flash_bwd_kernel.h:79-1142):
 //   P = exp(S - LSE), dP = dO V^T, dS = P o (dP - D), D = rowsum(dO o O),
@@ -464,6 +464,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
             dst_key[static_cast<int64_t>(q_first + j) * p.dbias_row_stride] = vals ? float_to_raw16<kBf16>(vals[j]) : 0;
       }
     };
+    // all queries have the same addends (calls of few queries): one value per key and head
+    const bool same_rows = (!p.bias || p.bias_row_stride == 0) && (!p.mask || (p.mask_row_stride == 0 && !p.mask_bits));
     // bias and mask that do not depend on the query head: fetched once per query tile
     const bool group_inv = G == 1 || ((!p.bias || p.h_bias != p.h) && (!p.mask || p.h_mask != p.h));
     // mask / bias head of query head h, without integer division (extents are 1, h_k or h)
@@ -493,7 +495,15 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         //      P = exp2(-inf) = 0 without any per-element select ----
           if (!(group_inv && bias2_loaded)) {
           bias2_loaded = true;
-          {
+          if (same_rows) {
+            float bv = -CUDART_INF_F;
+            if (key_ok && (!p.mask || p.mask[b * p.mask_batch_stride + hm_of(h) * p.mask_head_stride + key] != 0))
+              bv = p.bias ? raw16_to_float<kBf16>(reinterpret_cast<const uint16_t*>(
+                                p.bias)[b * p.bias_batch_stride + hb_of(h) * p.bias_head_stride + key]) * kLog2e
+                          : 0.f;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) bias2[j] = make_float2(bv, bv);
+          } else {
             const int hm = hm_of(h), hb = hb_of(h);
             const uint16_t* bcol = p.bias ? reinterpret_cast<const uint16_t*>(p.bias) + b * p.bias_batch_stride +
                                                 hb * p.bias_head_stride + key
@@ -1135,13 +1145,14 @@ bool tc_bwd_supported(const fdma_bwd_params& bp) {
 
 size_t tc_bwd_workspace_bytes(const fdma_bwd_params& p) {
   if (tile_head_dim(p.f.d) == 256) return tc_bwd256_workspace_bytes(p);
-  return bwd_rows_taken(p) ? bwd_rows_workspace_bytes(p) : plan(p).total;
+  // (both: it may be about packed sequences, which only the other kernel takes)
+  return std::max(bwd_rows_workspace_bytes(p), bwd_rows_taken(p) ? 0 : plan(p).total);
 }
 
 int tc_bwd(const fdma_bwd_params& p, cudaStream_t stream, const PackedSeqs& seqs) {
   const bool bf16 = p.f.dtype == FDMA_BF16;
   if (tile_head_dim(p.f.d) == 256) return tc_bwd256(p, stream);
-  if (bwd_rows_taken(p)) return bwd_rows(p, stream, seqs);
+  if (seqs.cu_q || bwd_rows_taken(p)) return bwd_rows(p, stream, seqs);
   const BwdPlan pl = plan(p);
   if (pl.D == 64) return bf16 ? launch<64, true>(p, pl, stream) : launch<64, false>(p, pl, stream);
   return bf16 ? launch<128, true>(p, pl, stream) : launch<128, false>(p, pl, stream);

@@ -38,7 +38,7 @@ int tc_bwd256(const fdma_bwd_params& p, cudaStream_t stream);
 
 // head dims up to 128, row-broadcast mask / bias, packed sequences (fdma_bwd_rows_sm100.cu); also reached through tc_bwd
 bool bwd_rows_taken(const fdma_bwd_params& p);
-size_t bwd_rows_workspace_bytes(const fdma_bwd_params& p);
+size_t bwd_rows_workspace_bytes(const fdma_bwd_params& p);  // 0: not taken, nor with packed sequences
 int bwd_rows(const fdma_bwd_params& p, cudaStream_t stream, const PackedSeqs& seqs);
 
 bool tc_bwd_supported(const fdma_bwd_params& p);
@@ -63,8 +63,10 @@ struct BwdPrepArgs {
 int launch_bwd_prep(const BwdPrepArgs& a, int D, bool bf16, cudaStream_t stream);
 
 struct BwdFinishArgs {
-  // dQ, or dq_acc = null (already written by the main kernel)
+  // dQ, or dq_acc = null (already written by the main kernel); fp32: the sum of dq_nsplit partials (0: of one)
   const void* dq_acc;
+  int dq_nsplit;
+  int64_t dq_split_stride;
   void* dq;
   const float* dsum;  // deterministic mode: rows with a non-finite D become NaN
   int64_t dq_sb, dq_sr, dq_sh;

@@ -153,8 +153,9 @@ typedef struct fdma_bwd_params {
   int32_t dbias_b, dbias_h, dbias_rows; /* extents of dbias dims 0..2 (1 where bias is broadcast) */
   int32_t dbias_keys;                   /* extent of the key dimension of dbias (>= Sk)          */
   int32_t deterministic;                /* flash_api.cpp:809. Non-zero: the tensor-core backward kernel of per-query
-                                           masks and biases sums dQ in 64-bit fixed point (order-independent, bit-identical
-                                           between runs, slower); those of row-broadcast masks have a fixed order without it.
+                                           masks and biases, which also takes few queries over many keys, sums dQ in 64-bit
+                                           fixed point (order-independent, bit-identical between runs, slower); those of
+                                           row-broadcast masks have a fixed order without it.
                                            The CUDA-core backward computes each dQ row in one warp (fixed order) but
                                            sums dK, dV and dBias with fp32 atomics. On the tensor-core kernels dK, dV and
                                            dBias (except dBias shared across batch / kv heads) have a fixed summation

@@ -1,0 +1,176 @@
+"""Gradients of row-broadcast masks and biases (head dims up to 128) against 64 bits, over the routes the backward takes: the two-pass
+kernel, the single pass for few queries over many keys, gathered keys with positions, packed sequences.
+
+Bound: 1.01 times the error of the same formulas in 64 bits with the roundings the data type asks for and no others: O (as the forward
+pass returned it, through D = rowsum(dO o O)), P and dS before they enter a product, and the result. Rounding is the same in both but
+where 32-bit sums fall on the other side of a boundary, which moves the error by far less than the hundredth."""
+import pytest
+import torch
+
+from flash_sparse_attn import flash_sparse_attn_func, flash_sparse_attn_varlen_func
+from flash_sparse_attn import flash_sparse_attn_interface as iface
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _gradients(q, k, v, dout, out, mask, bias, causal, dtype):
+    """dq, dk, dv, dbias of (Sq, H, d) queries over (Sk, Hk, d) keys in 64 bits; `dtype`: with the roundings to it, D from `out`.
+    mask, bias: (heads, Sk) or None; dbias: per query head."""
+    rnd = (lambda t: t.to(dtype).double()) if dtype else (lambda t: t)
+    H, Hk, d, Sq, Sk = q.shape[1], k.shape[1], q.shape[2], q.shape[0], k.shape[0]
+    dq, dk, dv = (torch.zeros(t.shape, dtype=torch.float64, device=q.device) for t in (q, k, v))
+    dbias = torch.zeros(H, Sk, dtype=torch.float64, device=q.device)
+    seen = torch.ones(Sq, Sk, dtype=torch.bool, device=q.device).tril(Sk - Sq) if causal else None
+    for h in range(H):
+        Q, K, V, G = q[:, h].double(), k[:, h * Hk // H].double(), v[:, h * Hk // H].double(), dout[:, h].double()
+        s = Q @ K.T * d ** -0.5
+        if bias is not None:
+            s += bias[h * bias.shape[0] // H].double()
+        if causal:
+            s = s.masked_fill(~seen, float("-inf"))
+        if mask is not None:
+            s = s.masked_fill(~mask[h * mask.shape[0] // H], float("-inf"))
+        p = torch.softmax(s, -1).nan_to_num(0.0)  # (rows that see no key)
+        dp = G @ V.T
+        D = (G * (out[:, h].double() if dtype else p @ V)).sum(-1, keepdim=True)
+        ds = p * (dp - D)
+        dq[:, h] = rnd(ds) @ K * d ** -0.5
+        dk[:, h * Hk // H] += rnd(ds).T @ Q * d ** -0.5
+        dv[:, h * Hk // H] += rnd(p).T @ G
+        dbias[h] = ds.sum(0)
+    return dq, dk, dv, dbias
+
+
+def _check(got, exact, rounded, dtype, what):
+    err, model = (got.double() - exact).norm().item(), (rounded.to(dtype).double() - exact).norm().item()
+    assert err <= 1.01 * model, (what, err / model, model / exact.norm().item())
+
+
+def _run(B, Sq, Sk, H, Hk, d, hm, hb, bb, causal, route, deterministic, dtype, keep=0.4, edit_mask=None):
+    g = torch.Generator(device="cuda").manual_seed(Sq + Sk)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda", dtype=dtype)  # noqa: E731
+    q, k, v, dout = r(B, Sq, H, d), r(B, Sk, Hk, d), r(B, Sk, Hk, d), r(B, Sq, H, d)
+    mask = bias = None
+    if hm:
+        mask = torch.rand((B, hm, 1, Sk), generator=g, device="cuda") < keep
+        mask[..., Sk // 3: Sk // 3 + 150] = False  # whole 64-key tiles
+        if edit_mask:
+            edit_mask(mask)
+    if hb:
+        bias = r(bb, hb, 1, Sk).requires_grad_()
+    for t in (q, k, v):
+        t.requires_grad_()
+    learned = [q, k, v] + ([bias] if hb else [])
+    iface.set_compaction(route)
+    try:
+        out = flash_sparse_attn_func(q, k, v, attn_mask=mask, attn_bias=bias, is_causal=causal, deterministic=deterministic)
+        runs = [torch.autograd.grad(out, learned, dout, retain_graph=True) for _ in range(2)]
+    finally:
+        iface.set_compaction("auto")
+    with torch.no_grad():
+        sides = []
+        for rounding in (None, dtype):
+            per = [_gradients(q[b], k[b], v[b], dout[b], out[b], None if mask is None else mask[b, :, 0],
+                              None if bias is None else bias[b % bb, :, 0], causal, rounding) for b in range(B)]
+            sides.append([torch.stack(x) for x in zip(*per)])
+        if hb:
+            for side in sides:
+                side[3] = side[3].view(B, hb, H // hb, 1, Sk).sum(2)
+                if bb == 1:
+                    side[3] = side[3].sum(0, keepdim=True)
+        for name, got, exact, rounded in zip(("dq", "dk", "dv", "dbias"), runs[0], *sides):
+            _check(got, exact, rounded, dtype, name)
+    fixed = 3 + (hb == Hk and bb == B)  # (dBias summed over heads or the batch by atomics: in no fixed order)
+    if deterministic:
+        assert all(torch.equal(a, b) for a, b in zip(runs[0][:fixed], runs[1][:fixed]))
+
+
+def _packed(lq, lk, H, Hk, d, causal, dtype):
+    g = torch.Generator(device="cuda").manual_seed(sum(lk))
+    r = lambda *s: torch.randn(s, generator=g, device="cuda", dtype=dtype)  # noqa: E731
+    q, k, v, dout = r(sum(lq), H, d), r(sum(lk), Hk, d), r(sum(lk), Hk, d), r(sum(lq), H, d)
+    cq, ck = (torch.tensor([0] + x, device="cuda").cumsum(0).to(torch.int32) for x in (lq, lk))
+    leaves = [t.requires_grad_() for t in (q, k, v)]
+    out = flash_sparse_attn_varlen_func(*leaves, cq, ck, max(lq), max(lk), is_causal=causal)
+    grads = torch.autograd.grad(out, leaves, dout)
+    with torch.no_grad():
+        sides = []
+        for rounding in (None, dtype):
+            per = []
+            for i in range(len(lq)):
+                rows, keys = slice(cq[i], cq[i + 1]), slice(ck[i], ck[i + 1])
+                per.append(_gradients(q[rows], k[keys], v[keys], dout[rows], out[rows], None, None, causal, rounding)[:3])
+            sides.append([torch.cat(x) for x in zip(*per)])
+        for name, got, exact, rounded in zip(("dq", "dk", "dv"), grads, *sides):
+            _check(got, exact, rounded, dtype, name)
+
+
+# (batch, queries, keys, heads, kv heads, head dim, mask heads, bias heads, bias batch, causal, route, deterministic)
+FEW_QUERIES = [
+    (1, 128, 8192, 8, 2, 128, 0, 0, 1, False, "off", False),
+    (2, 65, 3000, 6, 2, 96, 2, 2, 2, True, "off", False),
+    (1, 200, 5000, 4, 4, 128, 4, 4, 1, False, "off", False),
+    (2, 100, 4200, 4, 1, 72, 0, 1, 1, False, "off", False),     # dBias summed over the batch
+    (1, 300, 6000, 12, 4, 128, 4, 4, 1, True, "off", False),
+    (1, 129, 2050, 8, 2, 128, 8, 8, 1, True, "off", False),     # mask and bias per query head
+    (1, 128, 16384, 8, 2, 128, 2, 2, 1, True, "auto", False),   # gathered keys and their positions
+    (1, 70, 9000, 4, 2, 64, 2, 2, 1, True, "auto", True),
+    (1, 128, 4096, 4, 2, 64, 0, 0, 1, True, "off", True),
+    (1, 128, 8192, 8, 2, 64, 2, 2, 1, False, "off", True),
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("case", FEW_QUERIES, ids=lambda c: "x".join(map(str, c)))
+def test_few_queries(case, dtype):
+    _run(*case, dtype)
+
+
+@pytest.mark.parametrize("B,Sk,H,Hk,d", [(1, 4101, 4, 1, 64), (2, 9001, 8, 2, 128)])
+def test_single_query(B, Sk, H, Hk, d):
+    """Against the oracle, with its tolerances (the few numbers of one row say little about the error of rounding)."""
+    q, k, v, bias, dout = oracle.make_inputs(B, 1, Sk, H, Hk, d, (B, Hk, 1, Sk), seed=Sk, dtype=torch.bfloat16, device="cpu")
+    mask = torch.rand(B, Hk, 1, Sk, generator=torch.Generator().manual_seed(1)) < 0.4
+    want = oracle.attention_forward_backward(q, k, v, mask, bias, dout, None, False)
+    iface.set_compaction("off")
+    try:
+        leaves = [t.cuda().requires_grad_() for t in (q, k, v, bias)]
+        out = flash_sparse_attn_func(*leaves[:3], attn_mask=mask.cuda(), attn_bias=leaves[3])
+        grads = torch.autograd.grad(out, leaves, dout.cuda())
+    finally:
+        iface.set_compaction("auto")
+    for name, got, ref in zip(("dq", "dk", "dv", "dbias"), grads, want[2:]):
+        ok, msg = oracle.within_tolerance(oracle.error_report(name, got.cpu(), ref), name != "dq")
+        assert ok, msg
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("lq,lk,H,Hk,d", [([64, 70], [4100, 3000], 4, 2, 128), ([60, 3, 100], [70, 5000, 3000], 4, 4, 64)])
+def test_packed_few_queries(lq, lk, H, Hk, d, causal, dtype):
+    """Packed sequences of few queries over many keys: a row tile's keys are cut into ranges, of which a short sequence has none in some."""
+    _packed(lq, lk, H, Hk, d, causal, dtype)
+
+
+def test_few_queries_time():
+    """128 queries over 65536 keys take no more than three times as long as the same number of scores in 2048 rows: their dQ is not
+    left to the eight chains of 1024 key tiles that eight heads have."""
+    times = []
+    for Sq, Sk in ((128, 65536), (2048, 4096)):
+        q, k, v, dout = (torch.randn(1, n, h, 128, device="cuda", dtype=torch.bfloat16) for n, h in ((Sq, 8), (Sk, 2), (Sk, 2), (Sq, 8)))
+        leaves = [t.requires_grad_() for t in (q, k, v)]
+        out = flash_sparse_attn_func(*leaves)
+        torch.autograd.grad(out, leaves, dout, retain_graph=True)
+        best = float("inf")
+        for _ in range(3):
+            start, stop = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            torch.cuda._sleep(10_000_000)  # the launches queue up behind it
+            start.record()
+            for _ in range(5):
+                torch.autograd.grad(out, leaves, dout, retain_graph=True)
+            stop.record()
+            stop.synchronize()
+            best = min(best, start.elapsed_time(stop))
+        times.append(best)
+    assert times[0] <= 3 * times[1], times
