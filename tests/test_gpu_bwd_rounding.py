@@ -175,6 +175,38 @@ def _normal(Sq, Sk, H, Hk, d):
     return [t.requires_grad_() for t in (q, k, v)], dout
 
 
+def _some_heads_empty(mask):
+    mask[:, 1] = False  # between heads that have kept keys
+    mask[0, 4:7] = False
+
+
+# Two-pass kernel, several query heads per CTA of the row pass (from 12 row tiles x heads per SM on): Q and dO of the next head come in
+# while the last one's dQ is stored, activity bits alternate between two tables, sums start again; odd and even numbers of key tiles
+MANY_HEADS = [
+    (8, 1024, 320, 32, 8, 128, 0, 0, 1, False, "off", False),
+    (8, 1000, 1100, 32, 4, 64, 32, 32, 8, True, "off", True),   # mask and bias per head, some heads without a kept key
+    (4, 2048, 128, 32, 32, 128, 1, 0, 1, False, "off", False),
+]
+# ... and more keys than the 2048 that dQ was once summed over: positions, ragged ends, fixed order
+MANY_KEYS = [
+    (1, 2100, 8256, 2, 1, 64, 1, 1, 1, True, "off", True),
+    (1, 5000, 6000, 4, 2, 128, 2, 2, 1, True, "auto", False),
+    (1, 1400, 5000, 8, 4, 128, 4, 4, 1, False, "auto", True),
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("case", MANY_HEADS + MANY_KEYS, ids=lambda c: "x".join(map(str, c)))
+def test_two_passes(case, dtype):
+    _run(*case, dtype, keep=0.6, edit_mask=_some_heads_empty if case[6] > 8 else None)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("causal", [False, True])
+def test_packed_long(causal, dtype):
+    _packed([2500, 300, 2177], [2500, 333, 4200], 4, 2, 128, causal, dtype)
+
+
 def test_few_queries_time():
     """128 queries over 65536 keys take no more than three times as long as the same number of scores in 2048 rows: their dQ is not
     left to the eight chains of 1024 key tiles that eight heads have."""
