@@ -158,8 +158,9 @@ typedef struct fdma_bwd_params {
                                            row-broadcast masks have a fixed order without it.
                                            The CUDA-core backward computes each dQ row in one warp (fixed order) but
                                            sums dK, dV and dBias with fp32 atomics. On the tensor-core kernels dK, dV and
-                                           dBias (except dBias shared across batch / kv heads) have a fixed summation
-                                           order in both modes */
+                                           dBias have a fixed summation order in both modes, except a dBias that is shared
+                                           across batch or kv heads, or held per query head where several share a kv head:
+                                           CTAs add to it with fp32 atomics, in no fixed order, also when this is set */
   int32_t reserved;
   float* softmax_d; /* optional out, may be NULL: D = rowsum(dOut o Out) as fp32 (B, H, round_up(Sq,128)) contiguous,
                        zeros in the padding columns -- the `softmax_d` tensor mha_bwd returns (flash_api.cpp:952,

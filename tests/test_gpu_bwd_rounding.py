@@ -154,8 +154,11 @@ def test_packed_few_queries(lq, lk, H, Hk, d, causal, dtype):
 
 
 def _time(leaves, dout, **kwargs):
+    return _backward_time(flash_sparse_attn_func(*leaves, **kwargs), leaves, dout)
+
+
+def _backward_time(out, leaves, dout):
     """Device time of five backward passes, the best of three."""
-    out = flash_sparse_attn_func(*leaves, **kwargs)
     torch.autograd.grad(out, leaves, dout, retain_graph=True)
     best = float("inf")
     for _ in range(3):
@@ -195,8 +198,19 @@ MANY_KEYS = [
 ]
 
 
+# dBias per query head of a group (in shared memory up to 16 heads, beyond in memory), summed over the batch, over the heads
+DBIAS = [
+    (2, 300, 400, 16, 1, 128, 0, 16, 1, True, "off", False),
+    (1, 300, 400, 17, 1, 64, 17, 17, 1, False, "off", False),
+    (2, 500, 900, 4, 2, 64, 2, 4, 2, True, "auto", False),
+    (3, 300, 400, 6, 2, 128, 0, 2, 1, False, "off", False),
+    (3, 300, 400, 6, 2, 96, 2, 1, 3, True, "off", False),
+    (2, 300, 400, 4, 4, 128, 1, 1, 1, False, "off", False),
+]
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
-@pytest.mark.parametrize("case", MANY_HEADS + MANY_KEYS, ids=lambda c: "x".join(map(str, c)))
+@pytest.mark.parametrize("case", MANY_HEADS + MANY_KEYS + DBIAS, ids=lambda c: "x".join(map(str, c)))
 def test_two_passes(case, dtype):
     _run(*case, dtype, keep=0.6, edit_mask=_some_heads_empty if case[6] > 8 else None)
 
@@ -228,3 +242,16 @@ def test_long_masks():
     finally:
         iface.set_compaction("auto")
     assert times[0] <= 0.4 * times[1], times
+
+
+def test_dbias_per_head_time():
+    """A bias per query head adds its sums to memory once per CTA, not in every step: no more than 1.12 of the time with one per kv head."""
+    times = []
+    for heads in (16, 4):
+        g = torch.Generator(device="cuda").manual_seed(heads)
+        r = lambda *s: torch.randn(s, generator=g, device="cuda", dtype=torch.bfloat16)  # noqa: E731
+        leaves = [t.requires_grad_() for t in (r(4, 2048, 16, 128), r(4, 2048, 4, 128), r(4, 2048, 4, 128), r(4, heads, 1, 2048))]
+        dout = r(4, 2048, 16, 128)
+        out = flash_sparse_attn_func(*leaves[:3], attn_bias=leaves[3])
+        times.append(_backward_time(out, leaves, dout))
+    assert times[0] <= 1.12 * times[1], times
