@@ -1144,16 +1144,17 @@ struct RowsPlan {
   size_t lse2_off, dsum_off, dq_off, dbias_off, sums_off, part_off, dbpart_off, total;
 };
 
-// Query-range splits per key tile: two CTAs per SM, as long as a split keeps 32 steps. The row pass, whose many short CTAs run last, evens
-// out what unequal key CTAs leave, and every further split writes and reads fp32 partials of its key tile. (Up to eight CTAs per SM with
-// 80 steps each for causal calls, as a kernel without a row pass wants them, against this, with the sum of the partials: 8192 packed tokens
-// 427 -> 364 us, 8192 queries over 2048 kept keys 557 -> 501, plain 4096 462 -> 448, 32768 queries over 2048 1828 -> 1785; up to four:
-// 384, 527, 463, 1781.)
+// Query-range splits per key tile: one CTA per SM, as long as a split keeps 32 steps, and on to two per SM while it keeps 160. The row pass,
+// whose many short CTAs run last, evens out what unequal key CTAs leave; every split writes and reads fp32 partials of its key tile. (What
+// the tensor core sums up has its own bound, kKeyFlush.) Backward in us, at least one / two CTAs per SM: 8192 x 16 heads over 4, causal
+// 847 / 880, plain 4096 x 32 over 8 465 / 507, 8192 packed tokens 365 / 409, 4 x 2048, 512 gathered keys, d = 64 251 / 267; but 32768 over 2048
+// gathered keys (splits of 1024 / 683 steps) 2100 / 2063, 8192 over 2048 (256 / 171 steps) 613 / 598.
 int pick_nsplit(const fdma_fwd_params& p) {
   const int64_t ctas = static_cast<int64_t>((p.seqlen_k + kBN - 1) / kBN) * p.h_k * p.b;
   const int64_t steps = static_cast<int64_t>((p.seqlen_q + kBM - 1) / kBM) * (p.h / p.h_k);
-  const int64_t want = std::min((2 * sm_count() + ctas - 1) / ctas, steps / 32);
-  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(want, 64)));
+  if (ctas >= sm_count()) return 1;
+  const int64_t one = std::min((sm_count() + ctas - 1) / ctas, steps / 32), two = std::min((2 * sm_count() + ctas - 1) / ctas, steps / 160);
+  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(std::max(one, two), 64)));
 }
 
 // Key ranges per row-pass tile, where there are few rows and at least four times as many keys: else a few CTAs walk all keys one tile after
