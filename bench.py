@@ -336,9 +336,13 @@ class AttentionStep:
         self.ws = torch.empty(max(ws_f, ws_b, 1), dtype=torch.uint8, device=dev)
         self.fp.workspace, self.fp.workspace_bytes = self.ws.data_ptr(), ws_f
         bp.f.workspace, bp.f.workspace_bytes = self.ws.data_ptr(), ws_b
-        # launches per step, from the code paths above: gathers 3 | fwd_kernel 1 | bwd_prep, bwd_rows_kernel, bwd_finish 3 |
-        # scatters 3 (their zero fills are memsets); full key range: no query-range splits, so nothing for bwd_finish to do
-        self.launches = (3 + 1 + 3 + 3) if compact else 3
+        # launches per step, from the code paths above: gathers 3 | fwd_kernel 1 | bwd_prep, bwd_rows_kernel (per query: bwd_kernel),
+        # bwd_finish 3 (row-broadcast: the last one only if query ranges are split, for fewer key tiles than SMs and at least
+        # 32 steps each) | scatters 3 (their zero fills are memsets)
+        split = (-(-kk.shape[1] // 128) * Hk * B < torch.cuda.get_device_properties(dev).multi_processor_count
+                 and -(-Sq // 64) * (H // Hk) >= 64)
+        finish = split or bias.shape[2] > 1
+        self.launches = len(self.pre) + 1 + (3 if finish else 2) + len(self.post)
 
     def run_pre(self):
         for fn, prm in self.pre:
@@ -732,7 +736,9 @@ def run_ours(args, rank: int, world: int, local_rank: int):
                      "unit": "TFLOP/s", "frac": bwd_tflops / peaks["peak"], "peak_source": peaks["source"],
                      "frac_sustained": bwd_tflops / peaks["sustained"], "peak_sustained": peaks["sustained"],
                      "frac_of_nominal_2250": bwd_tflops / NOMINAL_TFLOPS,
-                     "traffic": None,
+                     # dram__bytes_read + dram__bytes_write of one bwd_rows_kernel launch of exactly this workload, one ncu
+                     # capture (profiles/bench_S32768_compaction_launch_list.md); other geometries: null
+                     "traffic": (3060e6 if (compact and (S, WINDOW, D, B) == (32768, 2048, 128, 1)) else None),
                      "fwd_kernel_achieved": fwd_tflops, "fwd_kernel_frac": fwd_tflops / peaks["peak"]},
         "e2e": {"value": tot / (e2e_ms * 1e-3) / 1e12 if e2e_ms == e2e_ms else None, "unit": "TFLOP/s",
                 "ms_per_step": e2e_ms if e2e_ms == e2e_ms else None,

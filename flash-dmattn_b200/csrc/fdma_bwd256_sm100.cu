@@ -318,7 +318,7 @@ __device__ __forceinline__ void pass256(const Bwd256Params& p, unsigned char* sm
       }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer (whole warp, uniform control flow; the issue wrappers elect one lane) -------
+    // ---------------- MMA issuer (whole warp, uniform control flow; the issue wrappers are predicated on one lane) -------
     if (n_steps > 0) {
       const uint32_t lead = umma_leader();
       constexpr uint32_t idesc_s = umma_idesc(kBN, kBM, kBf16, false, false);  // scores, dP: 128 x 64, K-major

@@ -15,8 +15,8 @@
 // 32 KB of fp32 dQ on its way to a buffer in global memory, which also had to be zeroed, added to and converted. Here dQ stays in the
 // CTA: the tensor core sums up 128 keys at a time (it truncates its sums: over 2048 keys dQ lost 1.1e-5 of its size), and the softmax
 // threads add those sums up in registers, rounding to nearest. It is the same bits every time: nothing changes for `deterministic`.
-// Whole backward, single pass -> this: plain causal 4096 x 32 heads 538 -> 484 us; 8192 packed tokens 528 -> 397; 32768 queries, 2048
-// kept keys 2118 -> 1893; deterministic, 8192 queries, 2048 kept keys 1016 (before the change to issuing) -> 530.
+// Whole backward in us, single pass (with the slower issue it had) -> this: plain causal 4096 x 32 heads 580 -> 464, 8192 packed tokens
+// 583 -> 364, 32768 queries over 2048 kept keys 2246 -> 2059, deterministic, 8192 queries over 2048 kept keys 1020 -> 609.
 //
 // Tensor memory, columns: scores[2] 2 x 64 | dP 64 (key pass at D = 128) or 2 x 64 | accumulators | stationary operands.
 // Only V in the key pass at D = 128 finds no room there (scores 128, dP 64, K 64, dV 128, dK 128) and stays in shared memory.
@@ -1174,7 +1174,9 @@ int pick_ranges(const fdma_fwd_params& p) {
 }
 
 // Query heads a row-pass CTA works on, one after the other: as many as leave six CTAs per SM, so that set-up and the first loads
-// of a CTA are paid once for several items and the last ones still even out.
+// of a CTA are paid once for several items and the last ones still even out. 32768 queries, 32 heads, backward in us with one head / 12 / 6 / 3
+// CTAs per SM: 2048 gathered keys 2265 / 2077 / 2057 / 2058, 128 keys 808 / 654 / 651 / 656; three per SM also 4 x 2048 at head dim 64 265 -> 251,
+// but 16384 x 8 heads at head dim 64 2523 -> 2690.
 int pick_heads_per_cta(int64_t tiles, int h) {
   return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(std::min(h, 16), tiles * h / (6 * sm_count()))));
 }

@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         FDMA_PROF_END(0, true);
       }
     } else if (warp == 1) {
-      // ---------------- MMA issuer (whole warp, uniform control flow; the issue wrappers elect one lane) -------
+      // ---------------- MMA issuer (whole warp, uniform control flow; the issue wrappers are predicated on one lane) -------
       if (n_steps > 0) {
         const uint32_t lead = umma_leader();
         constexpr uint32_t idesc_s = umma_idesc(kBN, kBM, kBf16, false, false);  // St/dPt: 128 x 64, K-major
@@ -916,10 +916,9 @@ struct BwdPlan {
 // Query-range splits per key tile. A grid of (key tiles x kv heads x batch) CTAs that cannot fill the GPU twice
 // (eight times when causal masking makes the CTAs unequal) is cut along the query dimension: into two CTAs per SM at least, as long as
 // every split keeps 32 steps, and on to about eight per SM, which evens out the causal imbalance between key tiles and the last wave of equal
-// ones, as long as it keeps 80. (Not causal, eight against two CTAs per SM: 8192 x 16 heads over 4 1.64 against 1.74 ms, 16384 x 8 over 1 3.1
-// against 3.4, 32768 x 4 over 1 at d = 64 5.5 against 6.15; 4 x 2048 x 16 over 4 and 4096 x 32 over 8 the same; 3001 x 12 over 4 278 against 261 us.)
-// (Each split writes and reads fp32 partials of its key tile, the time of some 6 steps. Plain causal attention at 4096, 8 kv heads: 3 splits
-// of 85 steps instead of 5 of 51, 815 -> 791 us for the whole step; deterministic at 8192, 2048 kept: 1301 -> 1270 us; 32768 queries over 2048 kept keys keep 10 splits of 205: 5 are 3 % slower.)
+// ones, as long as it keeps 80 (each split writes and reads fp32 partials of its key tile, the time of some 6 steps). With / without the
+// part beyond two: a bias per query, causal, 8 heads over 2, 8192 queries 640 / 659 us, 4096 229 / 228; 4096 queries over 16384 keys, 8 heads
+// over 2, causal 660 / 664, 8 over 1, not causal 775 / 741.
 int pick_nsplit(const fdma_fwd_params& p) {
   const int64_t ctas = static_cast<int64_t>((p.seqlen_k + kBN - 1) / kBN) * p.h_k * p.b;
   const bool causal = p.is_causal != 0 && p.seqlen_q > 1;

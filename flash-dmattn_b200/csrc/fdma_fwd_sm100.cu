@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(Smem<D>::kThreads, 1) fwd_kernel(const __grid_
       FDMA_PROF_END(0, true);
     }
   } else if (warp == 1) {
-    // whole warp, uniform control flow; the issue wrappers elect one lane
+    // whole warp, uniform control flow; the issue wrappers are predicated on one lane
     constexpr uint32_t idesc_qk = umma_idesc(kBM, kBN, kBf16, false, false);
     constexpr uint32_t idesc_pv = umma_idesc(kBM, D / L::kHalves, kBf16, false, true);
     const uint32_t lead = umma_leader();
