@@ -1134,12 +1134,9 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_rows_kernel(const __grid_cons
 // (row tile, head, batch element) of a call: the CTAs of the row pass at one range and head each
 int64_t row_tiles(const fdma_fwd_params& p) { return static_cast<int64_t>((p.seqlen_q + kBN - 1) / kBN) * p.h * p.b; }
 
-// The workspace is asked for without the sequences: calls that may be about packed ones.
-bool maybe_packed(const fdma_bwd_params& bp) { return bp.f.b == 1 && !bp.f.mask && !bp.f.bias && !bp.dbias && !bp.f.key_pos; }
-
 struct RowsPlan {
   int D, sq_r, nsplit, dbias_mode;
-  int ranges, packed_ranges;  // key ranges of an ordinary call; at most so many of one with packed sequences
+  int ranges;  // key ranges per row-pass tile
   bool part;  // dK, dV (and column sums) leave the kernel as fp32 partials
   size_t lse2_off, dsum_off, dq_off, dbias_off, sums_off, part_off, dbpart_off, total;
 };
@@ -1158,15 +1155,9 @@ int pick_nsplit(const fdma_fwd_params& p) {
 }
 
 // Key ranges per row-pass tile, where there are few rows and at least four times as many keys: else a few CTAs walk all keys one tile after
-// the other. Their fp32 partials are added up in one order by bwd_finish_kernel. `ctas`: row-pass CTAs without ranges.
-// Packed sequences: up to two CTAs per SM with 16 steps each. 2 x 64 queries over 2 x 16384 keys, 8 heads over 2 243 -> 104 us (82 in a
-// single pass over the keys), 32 over 8 378 -> 333 (265). A long sequence among many short ones still walks its keys in one chain.
-int packed_ranges(const fdma_fwd_params& p, int64_t ctas, int64_t steps) {
-  if (p.seqlen_k < 4ll * p.seqlen_q || steps < 32) return 1;
-  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(2 * sm_count() / ctas, steps / 16)));
-}
-// Other calls, of those this file takes (see bwd_rows_taken): half a CTA per SM, so that both passes fit in one wave, with eight steps
+// the other. Of the calls this file takes (see bwd_rows_taken) half a CTA per SM, so that both passes fit in one wave, with eight steps
 // each: 128 queries over 4096 keys, 8 heads over 2 61 -> 28 us (29 in a single pass), over 2048 34 -> 27 (29), over 1024 (not cut) 25.
+// The fp32 partials are added up in one order by bwd_finish_kernel.
 int pick_ranges(const fdma_fwd_params& p) {
   const int64_t ctas = row_tiles(p), steps = (p.seqlen_k + kBM - 1) / kBM;
   if (p.seqlen_k < 4ll * p.seqlen_q || steps < 32 || ctas > sm_count() / 8) return 1;
@@ -1197,10 +1188,8 @@ RowsPlan plan(const fdma_bwd_params& bp) {
   pl.lse2_off = o; o += align256(rows * 4);
   pl.dsum_off = o; o += align256(rows * 4);
   pl.ranges = pick_ranges(p);
-  pl.packed_ranges = maybe_packed(bp) ? packed_ranges(p, row_tiles(p), (p.seqlen_k + kBM - 1) / kBM) : 1;
   pl.dq_off = o;
-  const int dq_parts = std::max(pl.ranges, pl.packed_ranges);
-  if (dq_parts > 1) o += align256(static_cast<size_t>(dq_parts) * p.b * p.h * p.seqlen_q * pl.D * 4);
+  if (pl.ranges > 1) o += align256(static_cast<size_t>(pl.ranges) * p.b * p.h * p.seqlen_q * pl.D * 4);
   pl.dbias_off = o;
   if (pl.dbias_mode == kDbAtomic) o += align256(static_cast<size_t>(bp.dbias_b) * bp.dbias_h * atomic_keys(bp) * 4);
   pl.nsplit = pick_nsplit(p);
@@ -1300,9 +1289,7 @@ int launch(const fdma_bwd_params& bp, const RowsPlan& pl, const PackedSeqs& seqs
   kp.n_tiles = seqs.cu_q ? packed_slots(p.seqlen_k, seqs.n, kBN) : (p.seqlen_k + kBN - 1) / kBN;
   kp.q_tiles = seqs.cu_q ? packed_slots(p.seqlen_q, seqs.n, kBN) : (p.seqlen_q + kBN - 1) / kBN;
   kp.nsplit = pl.nsplit;
-  kp.ranges = pl.ranges;
-  if (seqs.cu_q)  // by the tiles there can be, and the average sequence
-    kp.ranges = std::min(pl.packed_ranges, packed_ranges(p, static_cast<int64_t>(p.seqlen_q / kBN + seqs.n) * p.h, (p.seqlen_k / seqs.n + kBM - 1) / kBM));
+  kp.ranges = seqs.cu_q ? 1 : pl.ranges;
   kp.heads_per_cta = pick_heads_per_cta(static_cast<int64_t>(kp.q_tiles) * p.b * kp.ranges, p.h);
   kp.scale_log2 = p.softmax_scale * kLog2e;
   kp.scale = p.softmax_scale;
@@ -1381,7 +1368,12 @@ bool bwd_rows_taken(const fdma_bwd_params& bp) {
   return row_tiles(p) > (bp.deterministic ? half_sms / 2 : half_sms);
 }
 
-size_t bwd_rows_workspace_bytes(const fdma_bwd_params& bp) { return bwd_rows_taken(bp) || maybe_packed(bp) ? plan(bp).total : 0; }
+// Packed sequences, whose lengths only the device knows: by all their queries and keys. Here / single pass, us, 8 heads over 2: 2 x 64 queries
+// over 2 x 16384 keys 244 / 70, one query over 65536 keys beside 127 over 64 919 / 169, 2 x 128 over 2 x 1024 25 / 31; 16 over 4: 2 x 1024 over 2 x
+// 16384 875 / 706, 4 x 512 over 4 x 2048 170 / 163, 4 x 256 over 4 x 1024 71 / 72; MHA at head dim 64, 2 x 256 over 2 x 4096 182 / 195.
+bool bwd_rows_taken_packed(const fdma_bwd_params& bp) { return bp.f.seqlen_k < 4096 || bp.f.seqlen_k < 4ll * bp.f.seqlen_q; }
+
+size_t bwd_rows_workspace_bytes(const fdma_bwd_params& bp) { return plan(bp).total; }
 
 int bwd_rows(const fdma_bwd_params& bp, cudaStream_t stream, const PackedSeqs& seqs) {
   const RowsPlan pl = plan(bp);

@@ -1,5 +1,5 @@
 // Backward dynamic-mask attention for sm_100a (head dims up to 128) with a mask or bias per query: dQ, dK, dV and dBias from dO, O,
-// LSE; also of few queries over many keys with row-broadcast ones. Other row-broadcast ones and packed sequences: fdma_bwd_rows_sm100.cu.
+// LSE; also of few queries over many keys with row-broadcast ones, packed sequences among them. Others of both: fdma_bwd_rows_sm100.cu.
 //
 // Math of the reference's compute_dq_dk_dv_1colblock (csrc/flash_sparse_attn/src/flash_bwd_kernel.h:79-1142):
 //   P = exp(S - LSE), dP = dO V^T, dS = P o (dP - D), D = rowsum(dO o O),
@@ -29,6 +29,7 @@
 #include <algorithm>
 
 #include "fdma_internal.h"
+#include "fdma_packed.cuh"
 #include "fdma_ptx.cuh"
 
 namespace fdma {
@@ -78,6 +79,8 @@ struct BwdKernelParams {
   const int32_t* key_pos;  // ascending positions of compacted keys, or null
   int64_t pos_batch_stride, pos_head_stride;
   int h_pos, causal_shift;
+  PackedSeqs seqs;     // packed sequences, each with key tiles of its own; 64-row query tiles are cut at fixed rows
+  int n_tiles;         // packed: places for key tiles
   float scale_log2, scale;
 };
 
@@ -131,7 +134,8 @@ __device__ __forceinline__ uint16_t float_to_raw16(float x) {
   return static_cast<uint16_t>(pack_16x2<kBf16>(x, 0.f) & 0xFFFFu);
 }
 
-template <int D, bool kBf16, bool kDet>
+// packed: an instantiation of its own, whose bounds of a sequence would cost the others registers.
+template <int D, bool kBf16, bool kDet, bool packed = false>
 __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant__ BwdKernelParams p) {
   using L = SmemB<D>;
   constexpr int kD = D;
@@ -168,26 +172,39 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   // blockIdx.x = (query-range split, key tile). With more than one split a CTA covers the 64-row query tiles
   // [m_lo, M64) of its key tile and leaves fp32 partial dK / dV / column sums for a reduction kernel. The last
   // query ranges, which causal masking never empties, are scheduled first.
-  const int n = blockIdx.x % NT;  // key tile
-  const int split = p.nsplit - 1 - blockIdx.x / NT;
+  const int tiles = packed ? p.n_tiles : NT;
+  const int n = blockIdx.x % tiles;  // key tile
+  const int split = p.nsplit - 1 - blockIdx.x / tiles;
   const int M64_all = (Sq + kBM - 1) / kBM;
   const int m_chunk = (M64_all + p.nsplit - 1) / p.nsplit;
   const int m_lo = split * m_chunk;
-  const int M64 = min(M64_all, m_lo + m_chunk);  // end of this CTA's query range
+  int M64 = min(M64_all, m_lo + m_chunk);  // end of this CTA's query range
   const bool causal = p.is_causal != 0;
   const int act_g = (p.h_mask == p.h && G > 1) ? G : 1;  // activity differs per query head only for per-head masks
   // Compacted keys carry their original positions (ascending); the causal test then runs on positions.
   const int32_t* pos_row = nullptr;
   if (causal && p.key_pos)
     pos_row = p.key_pos + b * p.pos_batch_stride + (p.h_pos == p.h_k ? hk : 0) * p.pos_head_stride;
-  const int coff = pos_row ? p.causal_shift : off;
-  const int key0 = n * kBN;
+  int coff = pos_row ? p.causal_shift : off;
+  // Packed sequences: the tile covers the keys [key0, key_end) of one of them, whose queries are [q_lo, q_hi).
+  int key0 = n * kBN, key_end = Sk, q_lo = 0, q_hi = Sq;
   int m_start = 0;
   if (pos_row) {
     const int64_t first = (static_cast<int64_t>(pos_row[n * kBN]) - coff) / kBM;
     m_start = static_cast<int>(max(static_cast<int64_t>(0), min(first, static_cast<int64_t>(M64))));
   } else if (causal) {
     m_start = max(0, (n * kBN - off) / kBM);  // first query tile with a row that sees key n*128
+  }
+  if (packed) {
+    const PackedTile t = packed_tile(p.seqs.cu_k, p.seqs.n, Sk, kBN, n);
+    const int2 q = packed_range(p.seqs.cu_q, p.seqs.n, Sq, t.seq);
+    key0 = t.begin + t.tile * kBN;
+    key_end = t.end;
+    q_lo = q.x;
+    q_hi = key0 < key_end ? q.y : q.x;  // (an empty place has no queries)
+    coff = key_end - q_hi;              // the last query sees the last key
+    m_start = (causal ? max(q_lo, key0 - coff) : q_lo) / kBM;
+    M64 = q_lo < q_hi ? min(M64, (q_hi + kBM - 1) / kBM) : 0;
   }
   m_start = max(m_start, m_lo);
   const WaitCtl ctl{s_abort, p.status};
@@ -333,10 +350,43 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           }
           umma_commit(lead, bar_dp_full + (step & 1));
         };
+        // Packed sequences: rows of other sequences that came along in a tile become zeros (queries: LSE = +inf, D = 0), as TMA
+        // fills them in at the end of a tensor. Nothing they hold takes part in the sums over queries and keys below.
+        auto end_kv = [&]() {
+          if (!packed || key_end - key0 >= kBN) return;
+          zero_tile_rows(s_k, kD / 64, kBN * 128, key_end - key0, kBN);
+          zero_tile_rows(s_v, kD / 64, kBN * 128, key_end - key0, kBN);
+          fence_proxy_async_smem();
+          __syncwarp();
+        };
+        // Only the first and the last query tile can hold such rows: steps below `head_steps` and from `tail` on.
+        const int head_steps = packed && m_start * kBM < q_lo ? G : 0;
+        const int tail = packed && M64 * kBM > q_hi ? n_steps - G : n_steps;
+        auto end_qdo = [&](int step) {
+          if (!packed || (step >= head_steps && step < tail)) return;
+          const int q0 = (step < G ? m_start : M64 - 1) * kBM;
+          const int from = max(q_lo - q0, 0), to = min(q_hi - q0, kBM);
+          unsigned char* stage = s_qdo + (step % kQStages) * L::kStageBytes;
+          for (int t = 0; t < 2; ++t) {
+            zero_tile_rows(stage + t * L::kQBytes, kD / 64, kBM * 128, 0, from);
+            zero_tile_rows(stage + t * L::kQBytes, kD / 64, kBM * 128, to, kBM);
+          }
+          float* ld = s_ld + (step % kQStages) * (2 * kBM);
+          for (int r = lane; r < kBM; r += 32)
+            if (r < from || r >= to) {
+              ld[r] = CUDART_INF_F;
+              ld[kBM + r] = 0.f;
+            }
+          fence_proxy_async_smem();
+          __threadfence_block();
+          __syncwarp();
+        };
         FDMA_PROF_BEGIN();
         bool ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(0, mbar_wait(bar_kv, 0, ctl, kWaitKv)));
         if (ok) ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(1, mbar_wait(bar_qdo_full + 0, 0, ctl, kWaitQdoFull)));
         if (ok) {
+          end_kv();
+          end_qdo(0);
           tc_fence_after_sync();
           issue_st(0);
           issue_dp(0);
@@ -344,6 +394,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         if (ok && n_steps > 1) {
           ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(1, mbar_wait(bar_qdo_full + 1, 0, ctl, kWaitQdoFull)));
           if (ok) {
+            end_qdo(1);
             tc_fence_after_sync();
             issue_st(1);
           }
@@ -394,6 +445,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
             ok = __all_sync(0xffffffffu, FDMA_PROF_WAIT(1, mbar_wait(bar_qdo_full + ((i + 2) % kQStages),
                                                                      ((i + 2) / kQStages) & 1, ctl, kWaitQdoFull)));
             if (!ok) break;
+            end_qdo(i + 2);
             tc_fence_after_sync();
             issue_st(i + 2);
             // dP of step i+2 goes out two steps ahead as well, as soon as the softmax threads have read dP of step
@@ -420,7 +472,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     const int key = key0 + krow;
     unsigned char* s_tr = smem + L::kTrOff + (warp - 4) * 1024;
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const bool key_ok = key < Sk;
+    const bool key_ok = key < key_end;
     // value compared with q + coff in the causal test: the key's position
     // (clamped so that ckey - coff cannot overflow; padding slots hold INT_MAX and are masked out anyway)
     const int ckey = pos_row ? (key_ok ? min(pos_row[key], 0x3FFFFFFF) : 0x3FFFFFFF) : key;
@@ -750,6 +802,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         }
         if (p.dkv_part) {
           // fp32 partial: part[dv|dk][split][b][hk][key][d]
+          if (packed && !key_ok) continue;  // (after the warp-wide load)
           float* part = p.dkv_part + ((((static_cast<int64_t>(half) * p.nsplit + split) * p.b + b) * p.h_k + hk) *
                                           (NT * kBN) + key) * kD + c * 32;
 #pragma unroll
@@ -825,14 +878,14 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
             fence_proxy_async_smem();
             named_bar_sync(3, 128);
             if (tid == 384) {
-              const int rows = min(2 * kPer, Sq - (m * kBM + c * 32));
+              const int r0 = packed ? max(0, q_lo - (m * kBM + c * 32)) : 0, rows = min(2 * kPer, q_hi - (m * kBM + c * 32)) - r0;
               if (rows > 0) {
                 if constexpr (kDet)
                   bulk_reduce_add_u64(reinterpret_cast<long long*>(p.dq_acc) +
-                                          ((static_cast<int64_t>(b) * p.h + h) * Sq + m * kBM + c * 32) * kD,
-                                      s_dq, rows * kD * 8);
+                                          ((static_cast<int64_t>(b) * p.h + h) * Sq + m * kBM + c * 32 + r0) * kD,
+                                      reinterpret_cast<long long*>(s_dq) + r0 * kD, rows * kD * 8);
                 else
-                  bulk_reduce_add_f32(gdst, s_dq, rows * kD * 4);
+                  bulk_reduce_add_f32(gdst + r0 * kD, s_dq + r0 * kD, rows * kD * 4);
               }
               asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             }
@@ -865,8 +918,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
             fence_proxy_async_smem();
             named_bar_sync(3, 128);
             if (tid == 384) {
-              const int rows = min(16, Sq - (m * kBM + c * 16));
-              if (rows > 0) bulk_reduce_add_u64(gdst64 + c * 16 * kD, s_dq64, rows * kD * 8);
+              const int r0 = packed ? max(0, q_lo - (m * kBM + c * 16)) : 0, rows = min(16, q_hi - (m * kBM + c * 16)) - r0;
+              if (rows > 0) bulk_reduce_add_u64(gdst64 + (c * 16 + r0) * kD, s_dq64 + r0 * kD, rows * kD * 8);
               asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             }
           }
@@ -882,8 +935,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           fence_proxy_async_smem();
           named_bar_sync(3, 128);
           if (tid == 384) {
-            const int rows = min(32, Sq - (m * kBM + c * 32));
-            if (rows > 0) bulk_reduce_add_f32(gdst + c * 32 * kD, s_dq, rows * kD * 4);
+            const int r0 = packed ? max(0, q_lo - (m * kBM + c * 32)) : 0, rows = min(32, q_hi - (m * kBM + c * 32)) - r0;
+            if (rows > 0) bulk_reduce_add_f32(gdst + (c * 32 + r0) * kD, s_dq + r0 * kD, rows * kD * 4);
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
         }
@@ -976,7 +1029,7 @@ BwdPlan plan(const fdma_bwd_params& bp) {
 bool aligned16(const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; }
 
 template <int D, bool kBf16>
-int launch(const fdma_bwd_params& bp, const BwdPlan& pl, cudaStream_t stream) {
+int launch(const fdma_bwd_params& bp, const BwdPlan& pl, const PackedSeqs& seqs, cudaStream_t stream) {
   using L = SmemB<D>;
   const fdma_fwd_params& p = bp.f;
   if (!p.workspace || p.workspace_bytes < pl.total) return FDMA_ERR_WORKSPACE;
@@ -1062,6 +1115,8 @@ int launch(const fdma_bwd_params& bp, const BwdPlan& pl, cudaStream_t stream) {
   kp.dbias_keys = bp.scatter_pos ? p.seqlen_k : bp.dbias_keys;
   kp.dbias_mode = pl.dbias_mode;
   kp.is_causal = p.is_causal;
+  kp.seqs = seqs;
+  kp.n_tiles = seqs.cu_q ? packed_slots(p.seqlen_k, seqs.n, kBN) : (p.seqlen_k + kBN - 1) / kBN;
   kp.key_pos = p.key_pos;
   kp.pos_batch_stride = p.key_pos_batch_stride; kp.pos_head_stride = p.key_pos_head_stride;
   kp.h_pos = p.h_pos; kp.causal_shift = p.causal_shift;
@@ -1069,10 +1124,11 @@ int launch(const fdma_bwd_params& bp, const BwdPlan& pl, cudaStream_t stream) {
   kp.scale = p.softmax_scale;
 
   auto kern = bp.deterministic ? bwd_kernel<D, kBf16, true> : bwd_kernel<D, kBf16, false>;
+  if (seqs.cu_q) kern = bp.deterministic ? bwd_kernel<D, kBf16, true, true> : bwd_kernel<D, kBf16, false, true>;
   const int smem_bytes = L::kAlloc;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
   if (e != cudaSuccess) return static_cast<int>(e);
-  dim3 grid(static_cast<unsigned>((p.seqlen_k + kBN - 1) / kBN) * pl.nsplit, p.h_k, p.b);
+  dim3 grid(static_cast<unsigned>(kp.n_tiles) * pl.nsplit, p.h_k, p.b);
   cudaEvent_t ev0, ev1;
   take_timing_events(&ev0, &ev1);
   if (ev0) cudaEventRecord(ev0, stream);
@@ -1142,19 +1198,23 @@ bool tc_bwd_supported(const fdma_bwd_params& bp) {
   return true;
 }
 
+// The workspace is asked for without the sequences: calls that may be about packed ones.
+static bool maybe_packed(const fdma_bwd_params& bp) { return bp.f.b == 1 && !bp.f.mask && !bp.f.bias && !bp.dbias && !bp.f.key_pos; }
+
 size_t tc_bwd_workspace_bytes(const fdma_bwd_params& p) {
   if (tile_head_dim(p.f.d) == 256) return tc_bwd256_workspace_bytes(p);
-  // (both: it may be about packed sequences, which only the other kernel takes)
-  return std::max(bwd_rows_workspace_bytes(p), bwd_rows_taken(p) ? 0 : plan(p).total);
+  // Either kernel where it may be about packed sequences, whose route is another one
+  const bool rows = bwd_rows_taken(p), packed_rows = maybe_packed(p) ? bwd_rows_taken_packed(p) : rows;
+  return std::max(rows || packed_rows ? bwd_rows_workspace_bytes(p) : 0, rows && packed_rows ? 0 : plan(p).total);
 }
 
 int tc_bwd(const fdma_bwd_params& p, cudaStream_t stream, const PackedSeqs& seqs) {
   const bool bf16 = p.f.dtype == FDMA_BF16;
   if (tile_head_dim(p.f.d) == 256) return tc_bwd256(p, stream);
-  if (seqs.cu_q || bwd_rows_taken(p)) return bwd_rows(p, stream, seqs);
+  if (seqs.cu_q ? bwd_rows_taken_packed(p) : bwd_rows_taken(p)) return bwd_rows(p, stream, seqs);
   const BwdPlan pl = plan(p);
-  if (pl.D == 64) return bf16 ? launch<64, true>(p, pl, stream) : launch<64, false>(p, pl, stream);
-  return bf16 ? launch<128, true>(p, pl, stream) : launch<128, false>(p, pl, stream);
+  if (pl.D == 64) return bf16 ? launch<64, true>(p, pl, seqs, stream) : launch<64, false>(p, pl, seqs, stream);
+  return bf16 ? launch<128, true>(p, pl, seqs, stream) : launch<128, false>(p, pl, seqs, stream);
 }
 
 }  // namespace fdma

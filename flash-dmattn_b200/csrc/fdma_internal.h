@@ -38,7 +38,8 @@ int tc_bwd256(const fdma_bwd_params& p, cudaStream_t stream);
 
 // head dims up to 128, row-broadcast mask / bias, packed sequences (fdma_bwd_rows_sm100.cu); also reached through tc_bwd
 bool bwd_rows_taken(const fdma_bwd_params& p);
-size_t bwd_rows_workspace_bytes(const fdma_bwd_params& p);  // 0: not taken, nor with packed sequences
+bool bwd_rows_taken_packed(const fdma_bwd_params& p);  // the same call, about packed sequences
+size_t bwd_rows_workspace_bytes(const fdma_bwd_params& p);
 int bwd_rows(const fdma_bwd_params& p, cudaStream_t stream, const PackedSeqs& seqs);
 
 bool tc_bwd_supported(const fdma_bwd_params& p);

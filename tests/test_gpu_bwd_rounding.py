@@ -147,10 +147,42 @@ def test_single_query(B, Sk, H, Hk, d):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
 @pytest.mark.parametrize("causal", [False, True])
-@pytest.mark.parametrize("lq,lk,H,Hk,d", [([64, 70], [4100, 3000], 4, 2, 128), ([60, 3, 100], [70, 5000, 3000], 4, 4, 64)])
+@pytest.mark.parametrize("lq,lk,H,Hk,d", [([64, 70], [4100, 3000], 4, 2, 128), ([60, 3, 100], [70, 5000, 3000], 4, 4, 64),
+                                          ([129, 1, 200, 31], [129, 900, 4000, 128], 8, 2, 96)])
 def test_packed_few_queries(lq, lk, H, Hk, d, causal, dtype):
-    """Packed sequences of few queries over many keys: a row tile's keys are cut into ranges, of which a short sequence has none in some."""
+    """Packed sequences of few queries over many keys: key tiles and query tiles that hold rows of several sequences."""
     _packed(lq, lk, H, Hk, d, causal, dtype)
+
+
+def test_packed_few_queries_isolated():
+    """Fixed-point sums twice the same; a NaN in one sequence stays there; rows outside every sequence are zero."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda", dtype=torch.bfloat16)  # noqa: E731
+    q, k, v, dout = r(200, 4, 128), r(6000, 2, 128), r(6000, 2, 128), r(200, 4, 128)
+    cq, ck = (torch.tensor(x, device="cuda", dtype=torch.int32) for x in ([0, 70, 190], [0, 2500, 5900]))
+    grads = []
+    for nan in (False, False, True):
+        if nan:
+            q[10, 1], k[20, 0], v[2499, 1] = float("nan"), float("nan"), float("inf")
+        leaves = [t.clone().requires_grad_() for t in (q, k, v)]
+        out = flash_sparse_attn_varlen_func(*leaves, cq, ck, 120, 3400, is_causal=True, deterministic=True)
+        grads.append(torch.autograd.grad(out, leaves, dout))
+    for a, b, c, rows, end in zip(*grads, (70, 2500, 2500), (190, 5900, 5900)):
+        assert torch.equal(a, b)
+        assert torch.equal(a[rows:end], c[rows:end]) and not c[:rows].isfinite().all()
+        assert not a[end:].any() and not c[end:].any()
+
+
+def test_packed_few_queries_time():
+    """2 x 64 queries over 2 x 16384 keys take no more than three times as long as the same number of scores in 2 x 1024 rows."""
+    def run(lq, lk):
+        q, k, v, dout = (torch.randn(2 * n, h, 128, device="cuda", dtype=torch.bfloat16) for n, h in ((lq, 8), (lk, 2), (lk, 2), (lq, 8)))
+        leaves = [t.requires_grad_() for t in (q, k, v)]
+        cq, ck = (torch.tensor([0, n, 2 * n], device="cuda", dtype=torch.int32) for n in (lq, lk))
+        return _backward_time(flash_sparse_attn_varlen_func(*leaves, cq, ck, lq, lk), leaves, dout)
+
+    few, many = run(64, 16384), run(1024, 1024)
+    assert few <= 3 * many, (few, many)
 
 
 def _time(leaves, dout, **kwargs):
