@@ -5,8 +5,9 @@ one column, with few bits there and pairs of keys of opposite sign, so that D = 
 exact. K takes the sign of V's column: the terms of each dQ element are positive. Q and dO are positive, so are those of dV, and those of
 a row of dK have one sign.
 
-Bound: a sum of n additions in tensor memory, each of which loses less than one unit in the last of 24 bits (2^-23 of it) and on average
-half of that, is too small by at most n 2^-24 on average; the 32-bit sums of what leaves tensor memory round to nearest. A result is the
+Bound: what n additions in tensor memory lose if each loses half a unit in the last of 24 bits, n 2^-24 (an addition takes in 16 products,
+aligned to the largest of them, and measured it loses up to 1.5 times that; the kernel makes fewer of them than the bounds of dK and dV
+allow for); the 32-bit sums of what leaves tensor memory round to nearest. A result is the
 rounded exact one unless such a loss moves it over a boundary of rounding, one fp16 step (at most 2^-10 of it) further on, which
 happens with a probability of loss / step: that mean has a standard deviation of at most sqrt(loss 2^-10 / N) over N elements, and four
 of them are allowed."""
